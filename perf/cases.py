@@ -20,15 +20,10 @@ memory of its own; weights are random 4-bit codes.
 """
 import importlib
 import math
-import os
 import random
-import sys
 
 import torch
 
-ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-if ROOT not in sys.path:
-    sys.path.insert(0, ROOT)
 api = importlib.import_module("llada2-orin-cuda_b200.api")
 wl = importlib.import_module("llada2-orin-cuda_b200.workload")
 
