@@ -1,8 +1,8 @@
-// Dense W4.A8 projection with residual add on tcgen05 tensor cores (kind::i8: u8 x s8 -> s32 in tensor memory).
+// Dense W4.A8 projection with residual add.
 //
-// It consumes the int8 activations the merge kernel writes (values in fragment order inside every 128-group, one fp32
-// scale and one int32 sum per token and group) and the reference's 4-bit weight strips as the engine holds them on the
-// device, and computes what the reference's attention-output projection computes (engine/engine.cu:434,
+// It consumes the int8 activations the attention epilogue writes (values in fragment order inside every 128-group, one
+// fp32 scale and one int32 sum per token and group) and the reference's 4-bit weight strips as the engine holds them on
+// the device, and computes what the reference's attention-output projection computes (engine/engine.cu:434,
 // moe8::gemm<.., MODE 2>, engine/moe_i8.cu:295-400), for any number of tokens:
 //     Y[n][r] += sum over 128-groups g, in order, of  (s_w[r][g] * s_x[n][g]) * float(P[r][n][g] - z[r][g] * Sxq[n][g])
 // with P the exact integer dot product of the group. Every float operation is the reference's (one fp32 product of
@@ -15,11 +15,15 @@
 // 16 h + 4 t + e (e = byte index), the code of row g in the low nibble and of row g + 8 in the high nibble
 // (engine/moe_i8.cu:127-160). A meta holds fp16 scale pairs (rows g | g + 8) at 4 g and zero-point pairs at 32 + 2 g.
 //
-// One CTA computes 128 weight rows x 64 tokens. Per 128-group: 128 threads unpack the eight strips' codes into a u8
-// operand tile and copy the tokens' int8 rows (both K-major, 128-byte swizzle; the weights are stored at the
-// activations' fragment positions, so the activations are copied as they are), a fifth warp issues four K = 32 MMAs
-// into one of two 64-column accumulators, and the 128 threads (thread = weight row = tensor-memory lane) fold the
-// previous group's integers into 64 fp32 accumulators while the next group's MMAs run.
+// Both kernels use mma.sync m16n8k32 (u8 x s8 -> s32), whose fragments these layouts are: a lane's eight code words ARE its
+// A fragments (one nibble mask per register) and a token's B fragments are 32 contiguous bytes per lane, so operands go
+// from memory to the tensor core without being unpacked into shared memory, and the integers come out in registers,
+// where the fold into fp32 needs them. What the path costs is that fold, 16 float steps per output which cannot be
+// reordered, not the products: the tcgen05 form (unpack to shared memory, proxy fence, MMA, commit, tensor-memory load)
+// took 1.2 us for every group at any number of tokens, a chain longer than the group's arithmetic.
+//   dense_strip_kernel  a decode step's few tokens: a CTA takes ONE strip and one warp per 128-group works on it; the
+//                       integers of all groups exist at once, only the multiply-adds run in group order.
+//   dense_tile_kernel   many tokens: 128 rows x 64 tokens per CTA, a warp per strip.
 #pragma once
 #include <cuda_fp16.h>
 #include "common.cuh"
@@ -27,22 +31,8 @@
 
 namespace llattn {
 
-constexpr int DN_ROWS = 128, DN_TOK = 64, DN_GROUP = 128;
+constexpr int DN_ROWS = 128, DN_GROUP = 128;
 constexpr int DN_TILE_BYTES = 1024, DN_META_BYTES = 48;
-constexpr int DN_STAGES = 3;                                      // slots for data coming from global memory
-constexpr int DN_A_BYTES = DN_ROWS * 128, DN_B_BYTES = DN_TOK * 128, DN_RAW_BYTES = 8 * DN_TILE_BYTES;
-constexpr int DN_SM_A = 0;                                        // two unpacked weight tiles
-constexpr int DN_SM_B = DN_SM_A + 2 * DN_A_BYTES;                 // DN_STAGES activation tiles, written by cp.async
-constexpr int DN_SM_RAW = DN_SM_B + DN_STAGES * DN_B_BYTES;       // eight code tiles as they lie in memory (every thread copies and
-                                                                  // unpacks its own 64 bytes, so one slot is enough)
-// Token scales and sums are read by the folding threads themselves; a thread may be one group ahead of the slowest one
-// when it refills a slot, so these have twice as many slots as there are stages.
-constexpr int DN_SM_SX = DN_SM_RAW + DN_RAW_BYTES;                // [8][64] float token scales
-constexpr int DN_SM_SQ = DN_SM_SX + 8 * DN_TOK * 4;               // [8][64] int token sums
-constexpr int DN_SM_BAR = DN_SM_SQ + 8 * DN_TOK * 4;
-constexpr int DN_SMEM_BYTES = DN_SM_BAR + 64;
-constexpr int DN_THREADS = 160;
-enum { DB_FULL = 0, DB_DONE = 2, DB_COUNT = 4 };
 
 struct DenseParams {
     const uint8_t* W;      // strips
@@ -51,14 +41,127 @@ struct DenseParams {
     const int32_t* sum;    // [ntokens][K / 128]
     float* Y;              // [ntokens][rows], accumulated into
     int ntokens, rows, K;
-    int* err;
 };
 
-__device__ __forceinline__ void mma_i8_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n"
-                 :: "r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+__device__ __forceinline__ void mma_m16n8k32_u8s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// 16-byte and 4-byte asynchronous copies global -> shared (per-thread completion groups); `live` false writes zeros.
+// int -> float through the float whose bits are 1.5 * 2^23 + v: exact for |v| < 2^22 (here |v| <= 255 * 127 * 128). An
+// integer add and a float subtract at full rate; the conversion instruction has an eighth of it.
+__device__ __forceinline__ float small_int_to_float(int v) { return __int_as_float(v + 0x4B400000) - 12582912.0f; }
+
+// ------------------------------------------------------------------------------------------------------------- few tokens
+// Bound by latency: 2.2 MB of weights are 0.34 us of HBM time and 32 tokens x 2048 x 2048 are nothing, so what counts is
+// the length of the dependent chain and how many SMs pull on the weights: one CTA per (strip, 32 tokens), 128 CTAs at
+// 2048 rows, warp w on group w (w + 16, ... when K > 2048). Each warp leaves the two factors of its group's multiply-add
+// in shared memory; then thread = output element runs the sixteen in order.
+// Measured, 2048 x 2048, launches in a graph over 20 different weights: 32 tokens 3.8 us (a 128-row tile per CTA, group after group: 18.7),
+// 1 token 2.4 us.
+constexpr int DS_WARPS = 16, DS_THREADS = 32 * DS_WARPS, DS_TOK = 32;
+constexpr int DS_LD = 18;                          // (value, scale) pairs per token row of 16: keeps the fragment writes conflict-free
+constexpr int DS_SMEM_BYTES = DS_WARPS * DS_TOK * DS_LD * 8;
+
+__global__ void __launch_bounds__(DS_THREADS, 1) dense_strip_kernel(const DenseParams p) {
+    extern __shared__ __align__(16) uint8_t ds_smem[];
+    float2* pairs = reinterpret_cast<float2*>(ds_smem);               // [warp][token][DS_LD]: (float of the integer, s_w * s_x)
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int strip = blockIdx.x, n0 = blockIdx.y * DS_TOK, live = min(DS_TOK, p.ntokens - n0);
+    const int ktot = p.K / DN_GROUP;
+    const uint8_t* codes = p.W + size_t(strip) * ktot * (DN_TILE_BYTES + DN_META_BYTES);
+    const uint8_t* metas = codes + size_t(ktot) * DN_TILE_BYTES;
+    // this thread's output element: row tid % 16 of the strip, token tid / 16; its old value is on its way from the start
+    const int row = tid & 15, tok = tid >> 4;
+    float* yp = p.Y + size_t(n0 + tok) * p.rows + strip * 16 + row;
+    float y = 0.f, c = 0.f;
+#pragma unroll 1
+    for (int k0 = 0; k0 < ktot; k0 += DS_WARPS) {
+        const int gi = k0 + warp;
+        if (gi < ktot) {
+            const uint4 lo = __ldg(reinterpret_cast<const uint4*>(codes + size_t(gi) * DN_TILE_BYTES + 16 * lane));
+            const uint4 hi = __ldg(reinterpret_cast<const uint4*>(codes + size_t(gi) * DN_TILE_BYTES + 512 + 16 * lane));
+            const uint32_t sw2 = __ldg(reinterpret_cast<const uint32_t*>(metas + size_t(gi) * DN_META_BYTES + 4 * g));
+            const uint32_t z2 = __ldg(reinterpret_cast<const uint16_t*>(metas + size_t(gi) * DN_META_BYTES + 32 + 2 * g));
+            uint4 b[4][2];
+            float sx[4][2];
+            int sq[4][2];
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const int n = 8 * nt + g;
+                b[nt][0] = b[nt][1] = make_uint4(0u, 0u, 0u, 0u);
+                if (n < live) {
+                    const uint4* src = reinterpret_cast<const uint4*>(p.q + size_t(n0 + n) * p.K + size_t(gi) * DN_GROUP + 32 * t);
+                    b[nt][0] = __ldg(src);
+                    b[nt][1] = __ldg(src + 1);
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const size_t at = size_t(n0 + min(8 * nt + 2 * t + e, live - 1)) * ktot + gi;
+                    sx[nt][e] = __ldg(p.s + at);
+                    sq[nt][e] = __ldg(p.sum + at);
+                }
+            }
+            if (k0 == 0 && tok < live) y = __ldcg(yp);
+            const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+            const uint32_t mk = 0x0F0F0F0Fu;
+            const float swa = __half2float(__ushort_as_half(uint16_t(sw2 & 0xffffu))), swb = __half2float(__ushort_as_half(uint16_t(sw2 >> 16)));
+            const int za = int(z2 & 0xffu), zb = int(z2 >> 8);
+            float2* out = pairs + warp * DS_TOK * DS_LD;
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                if (8 * nt >= live) break;
+                int acc[4] = {0, 0, 0, 0};
+                const uint32_t bw[8] = {b[nt][0].x, b[nt][0].y, b[nt][0].z, b[nt][0].w, b[nt][1].x, b[nt][1].y, b[nt][1].z, b[nt][1].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    mma_m16n8k32_u8s8(acc, w[2 * j] & mk, (w[2 * j] >> 4) & mk, w[2 * j + 1] & mk, (w[2 * j + 1] >> 4) & mk, bw[2 * j], bw[2 * j + 1]);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    float2* o = out + (8 * nt + 2 * t + e) * DS_LD + g;
+                    o[0] = make_float2(small_int_to_float(acc[e] - za * sq[nt][e]), __fmul_rn(swa, sx[nt][e]));
+                    o[8] = make_float2(small_int_to_float(acc[2 + e] - zb * sq[nt][e]), __fmul_rn(swb, sx[nt][e]));
+                }
+            }
+        } else if (k0 == 0 && tok < live) {
+            y = __ldcg(yp);
+        }
+        __syncthreads();
+        if (tok < live) {
+            const int ng = min(DS_WARPS, ktot - k0);
+            const float2* in = pairs + tok * DS_LD + row;
+#pragma unroll 16
+            for (int k = 0; k < ng; ++k) {
+                const float2 vs = in[k * DS_TOK * DS_LD];
+                c = __fmaf_rn(vs.y, vs.x, c);
+            }
+        }
+        if (k0 + DS_WARPS < ktot) __syncthreads();
+    }
+    if (tok < live) __stcg(yp, y + c);
+}
+
+// ------------------------------------------------------------------------------------------------------------ many tokens
+// CTA = 128 rows x 64 tokens, 8 warps; warp = strip. Everything a group needs comes in through cp.async, DT_STAGES - 1
+// groups ahead: the strips' codes and metas (each warp its own), the 64 tokens' codes, scales and sums (shared; 16-byte
+// chunk c of token n at chunk position c ^ (n % 8): conflict-free fragment loads). Then 32 MMAs, four output tiles in
+// turn so that a chain of four K-steps hides behind the others, and the fold of 32 outputs per thread, two per
+// instruction where fp32 comes in pairs.
+// What bounds it: about 200 issue slots and 32 MMAs (8.8 cycles each on a scheduler) per warp and group of 1,024 outputs -
+// 2048 tokens x 2048 x 2048: 17 us of tensor pipe over 148 SMs - then reading and writing Y (33.6 MB, 5.1 us; brought
+// into L2 while the groups run).
+// Measured, 2048 x 2048, launches in a graph: 2048 tokens 54 us (tcgen05, 128 x 64 tiles: 61), 128 tokens 16.8 us.
+constexpr int DT_TOK = 64, DT_THREADS = 256, DT_STAGES = 4;
+constexpr int DT_CODES = 0, DT_Q = 8 * DN_TILE_BYTES, DT_SX = DT_Q + DT_TOK * 128, DT_SQ = DT_SX + DT_TOK * 4, DT_META = DT_SQ + DT_TOK * 4;
+constexpr int DT_STAGE_BYTES = DT_META + 8 * DN_META_BYTES;        // 17,280
+constexpr int DT_SMEM_BYTES = DT_STAGES * DT_STAGE_BYTES;
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(uint32_t a, uint32_t b) { f32x2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(a), "r"(b)); return d; }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f32x2 fma2v(f32x2 a, f32x2 b, f32x2 c) { f32x2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+
+// 16- and 4-byte asynchronous copies global -> shared (per-thread completion groups); `live` false writes zeros.
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool live) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
 }
@@ -68,197 +171,108 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, bool li
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int kPending> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
 
-// kind::i8 instruction descriptor: s32 accumulator, A u8 (format 0), B s8 (format 1), both K-major.
-__host__ __device__ constexpr uint32_t idesc_i8_u8s8(int M, int N) {
-    return (2u << 4) | (0u << 7) | (1u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
-}
-
-__global__ void __launch_bounds__(DN_THREADS) dense_i8_kernel(const DenseParams p) {
-    extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint32_t tmem_slot;
-    __shared__ int abort_flag_s;
-    volatile int* abort_flag = &abort_flag_s;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int row0 = blockIdx.x * DN_ROWS, n0 = blockIdx.y * DN_TOK;
+__global__ void __launch_bounds__(DT_THREADS, 2) dense_tile_kernel(const DenseParams p) {
+    extern __shared__ __align__(128) uint8_t dt_smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int row0 = blockIdx.x * DN_ROWS, n0 = blockIdx.y * DT_TOK, live = min(DT_TOK, p.ntokens - n0);
     const int ktot = p.K / DN_GROUP;
-    const uint32_t bar0 = ptx::smem_u32(smem + DN_SM_BAR);
-    auto BAR = [&](int i) -> uint32_t { return bar0 + 8u * uint32_t(i); };
-    if (ptx::smem_u32(smem) & 1023u) {
-        if (tid == 0 && p.err) atomicOr(p.err, ERR_SMEM_ALIGN);
-        return;
-    }
-    if (tid == 0) {
-        for (int i = 0; i < 2; ++i) { ptx::mbar_init(BAR(DB_FULL + i), 128); ptx::mbar_init(BAR(DB_DONE + i), 1); }
-        ptx::fence_mbar_init();
-        abort_flag_s = 0;
-    }
-    if (warp == 4) { ptx::tmem_alloc(ptx::smem_u32(&tmem_slot), 128); ptx::tmem_relinquish(); }
-    ptx::tc_fence_before();
-    __syncthreads();
-    ptx::tc_fence_after();
-    const uint32_t tmem = tmem_slot;
-    const size_t strip_bytes = size_t(ktot) * (DN_TILE_BYTES + DN_META_BYTES), meta_off = size_t(ktot) * DN_TILE_BYTES;
-    int errbits = 0;
-
-    if (warp < 4) {
-        // ---- this thread's weight row: strip, row inside the strip, where its scale and zero point sit in a meta
-        const int r = tid, strip = (row0 + r) >> 4, rr = r & 15, g8 = rr & 7, hi = rr >> 3;
-        const uint8_t* my_meta = p.W + size_t(strip) * strip_bytes + meta_off + 4 * g8 + 2 * hi;
-        const uint8_t* my_zero = p.W + size_t(strip) * strip_bytes + meta_off + 32 + 2 * g8 + hi;
-        // what this thread brings in and stages per group: two (strip, reference lane) tasks of weight codes - it unpacks
-        // exactly the bytes it copied itself - and half a token's 128-byte row, copied straight into the operand tile
-        const int sl0 = tid >> 5, l = tid & 31, g = l >> 2, t = l & 3;       // task 0: strip sl0, task 1: strip sl0 + 4
-        const uint8_t* code0 = p.W + size_t((row0 >> 4) + sl0) * strip_bytes + 16 * l;
-        const uint8_t* code1 = code0 + 4 * strip_bytes;
-        const int tn = tid >> 1, hf = tid & 1;
-        const bool tlive = n0 + tn < p.ntokens;
-        const int8_t* arow = p.q + size_t(tlive ? n0 + tn : 0) * p.K + 64 * hf;
-        const bool slive = tid < DN_TOK && n0 + tid < p.ntokens;
-        const size_t srow = size_t(slive ? n0 + tid : 0) * ktot;
-        const uint32_t sm0 = ptx::smem_u32(smem);
-        const uint32_t raw_mine = sm0 + DN_SM_RAW + 64 * tid;             // 4 x 16 bytes per stage
-        const uint32_t b_mine = sm0 + DN_SM_B + tn * 128;
-        auto fetch = [&](int i) {          // asynchronous copies of group i (always one commit, so groups count uniformly)
-            if (i < ktot) {
-                const int sg = i % DN_STAGES;
-                const size_t co = size_t(i) * DN_TILE_BYTES;
-                cp_async16(raw_mine, code0 + co, true);
-                cp_async16(raw_mine + 16, code0 + co + 512, true);
-                cp_async16(raw_mine + 32, code1 + co, true);
-                cp_async16(raw_mine + 48, code1 + co + 512, true);
-                const int8_t* src = arow + size_t(i) * DN_GROUP;
+    const uint8_t* codes = p.W + size_t((row0 >> 4) + warp) * ktot * (DN_TILE_BYTES + DN_META_BYTES);
+    const uint8_t* metas = codes + size_t(ktot) * DN_TILE_BYTES;
+    const uint32_t sm0 = ptx::smem_u32(dt_smem);
+    // this thread's part of a stage: its lane's code words, one of the strip's three meta chunks, two chunks of tokens tid / 8 and tid / 8 + 32, and one scale or sum
+    const int cn = tid >> 3, cc = tid & 7;
+    const int8_t* src0 = p.q + size_t(n0 + min(cn, live - 1)) * p.K + 16 * cc;
+    const int8_t* src1 = p.q + size_t(n0 + min(cn + 32, live - 1)) * p.K + 16 * cc;
+    const uint32_t dst0 = sm0 + DT_Q + cn * 128 + ((cc ^ (cn & 7)) << 4);
+    const bool live0 = cn < live, live1 = cn + 32 < live;
+    const int sn = tid & 63;
+    const size_t sat = size_t(n0 + min(sn, live - 1)) * ktot;
+    const void* ssrc = tid < 64 ? static_cast<const void*>(p.s + sat) : static_cast<const void*>(p.sum + sat);
+    const uint32_t sdst = sm0 + DT_SX + 4 * (tid & 127);
+    auto fetch = [&](int i) {                  // one commit per call, so groups count uniformly
+        if (i < ktot) {
+            const uint32_t st = uint32_t(i % DT_STAGES) * DT_STAGE_BYTES;
+            const uint32_t mine = sm0 + DT_CODES + warp * DN_TILE_BYTES + 16 * lane + st;
+            cp_async16(mine, codes + size_t(i) * DN_TILE_BYTES + 16 * lane, true);
+            cp_async16(mine + 512, codes + size_t(i) * DN_TILE_BYTES + 512 + 16 * lane, true);
+            if (lane < 3) cp_async16(sm0 + DT_META + warp * DN_META_BYTES + 16 * lane + st, metas + size_t(i) * DN_META_BYTES + 16 * lane, true);
+            cp_async16(dst0 + st, src0 + size_t(i) * DN_GROUP, live0);
+            cp_async16(dst0 + st + 32 * 128, src1 + size_t(i) * DN_GROUP, live1);
+            if (tid < 128) cp_async4(sdst + st, static_cast<const uint8_t*>(ssrc) + 4 * size_t(i), sn < live);
+        }
+        cp_async_commit();
+    };
+    for (int i = 0; i < DT_STAGES - 1; ++i) fetch(i);
+    // the tile's 64 x 512 bytes of Y into L2: wanted when the last group is folded
+    if ((tid >> 2) < live) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.Y + size_t(n0 + (tid >> 2)) * p.rows + row0 + 32 * (tid & 3)));
+    f32x2 c[8][2];                             // per n-tile: rows g and g + 8, tokens 8 nt + 2 t and + 1
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    cp_async16(b_mine + sg * DN_B_BYTES + (((4 * hf + k) ^ (tn & 7)) << 4), src + 16 * k, tlive);
-                if (tid < DN_TOK) {
-                    cp_async4(sm0 + DN_SM_SX + ((i & 7) * DN_TOK + tid) * 4, p.s + srow + i, slive);
-                    cp_async4(sm0 + DN_SM_SQ + ((i & 7) * DN_TOK + tid) * 4, p.sum + srow + i, slive);
-                }
-            }
-            cp_async_commit();
-        };
-        float c[DN_TOK];
-#pragma unroll
-        for (int n = 0; n < DN_TOK; ++n) c[n] = 0.f;
-        const bool second_half = p.ntokens - n0 > 32;
-        bool alive = true;
-        uint16_t sw_next = 0;
-        int z_next = 0;
-        fetch(0);
+    for (int nt = 0; nt < 8; ++nt) c[nt][0] = c[nt][1] = 0ull;
+    const f32x2 magic = 0xCB400000CB400000ull; // -1.5 * 2^23 twice
 #pragma unroll 1
-        for (int i = 0; i <= ktot && alive; ++i) {
-            // scale and zero point of the group folded in this iteration (loaded one iteration ago, behind the proxy fence:
-            // a fence with loads in flight waits for them)
-            const uint16_t sw_bits = sw_next;
-            const int z = z_next;
-            if (i < ktot) {
-                const int st = i & 1;
-                // group i has landed (this thread's copies; nothing else is in flight: a proxy fence with copies in flight
-                // would wait for them). The A tile's previous MMAs (group i - 2) were seen complete when this thread folded
-                // that group.
-                cp_async_wait<0>();
-                uint8_t* As = smem + DN_SM_A + st * DN_A_BYTES;
-                const uint4* raw = reinterpret_cast<const uint4*>(smem + DN_SM_RAW + 64 * tid);
-                // weights: each task yields 8 words for row g of its strip and 8 for row g + 8, stored at the codes'
-                // fragment positions
+    for (int i = 0; i < ktot; ++i) {
+        cp_async_wait<DT_STAGES - 2>();
+        __syncthreads();                       // group i is in for everybody; group i - 1 is done with, its stage can be refilled
+        fetch(i + DT_STAGES - 1);
+        const uint8_t* st = dt_smem + (i % DT_STAGES) * DT_STAGE_BYTES;
+        const uint8_t* meta = st + DT_META + warp * DN_META_BYTES;
+        const uint32_t sw2 = *reinterpret_cast<const uint32_t*>(meta + 4 * g), z2 = *reinterpret_cast<const uint16_t*>(meta + 32 + 2 * g);
+        uint32_t a[4][4];                      // A fragments of the four K-steps
+        {
+            const uint4 lo = *reinterpret_cast<const uint4*>(st + DT_CODES + warp * DN_TILE_BYTES + 16 * lane);
+            const uint4 hi = *reinterpret_cast<const uint4*>(st + DT_CODES + warp * DN_TILE_BYTES + 512 + 16 * lane);
+            const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}, mk = 0x0F0F0F0Fu;
 #pragma unroll
-                for (int task = 0; task < 2; ++task) {
-                    const uint4 lo = raw[2 * task], h4 = raw[2 * task + 1];
-                    const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, h4.x, h4.y, h4.z, h4.w};
-                    const int ra = (sl0 + 4 * task) * 16 + g, rb = ra + 8;            // rows inside the CTA tile
-                    // word k holds the codes at fragment positions 32 t + 8 (k / 2) + 4 (k % 2): words 0-3 are the 16-byte chunk
-                    // 2 t of the row, words 4-7 chunk 2 t + 1. Two 16-byte stores per row; a quarter warp covers eight
-                    // different chunk positions, so they are conflict-free.
-                    const uint32_t m = 0x0F0F0F0Fu;
-                    *reinterpret_cast<uint4*>(As + ra * 128 + (((2 * t) ^ (ra & 7)) << 4)) = make_uint4(w[0] & m, w[1] & m, w[2] & m, w[3] & m);
-                    *reinterpret_cast<uint4*>(As + ra * 128 + (((2 * t + 1) ^ (ra & 7)) << 4)) = make_uint4(w[4] & m, w[5] & m, w[6] & m, w[7] & m);
-                    *reinterpret_cast<uint4*>(As + rb * 128 + (((2 * t) ^ (rb & 7)) << 4)) =
-                        make_uint4((w[0] >> 4) & m, (w[1] >> 4) & m, (w[2] >> 4) & m, (w[3] >> 4) & m);
-                    *reinterpret_cast<uint4*>(As + rb * 128 + (((2 * t + 1) ^ (rb & 7)) << 4)) =
-                        make_uint4((w[4] >> 4) & m, (w[5] >> 4) & m, (w[6] >> 4) & m, (w[7] >> 4) & m);
-                }
-                ptx::fence_proxy_async_smem();         // the A tile, and the activation tile the copies wrote, for the tensor core
-                ptx::mbar_arrive(BAR(DB_FULL + st));
-                // group i + 1 comes in while group i - 1 is folded; its slots were last read by the MMAs of group i - 2
-                fetch(i + 1);
-                sw_next = __ldg(reinterpret_cast<const uint16_t*>(my_meta + size_t(i) * DN_META_BYTES));
-                z_next = int(__ldg(my_zero + size_t(i) * DN_META_BYTES));
-            }
-            if (i >= 1) {
-                // ---- fold group i - 1: its integers are complete in accumulator (i - 1) % 2. The token scales were
-                // written by other threads' copies: their arrivals on db_full order them before this read.
-                const int gi = i - 1, st = gi & 1;
-                if (!ptx::mbar_wait(BAR(DB_FULL + st), (gi >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_DEQUANT; break; }
-                if (!ptx::mbar_wait(BAR(DB_DONE + st), (gi >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_DEQUANT; break; }
-                ptx::tc_fence_after();
-                const float sw = __half2float(__ushort_as_half(sw_bits));
-                const float* sx = reinterpret_cast<const float*>(smem + DN_SM_SX) + (gi & 7) * DN_TOK;
-                const int* sq = reinterpret_cast<const int*>(smem + DN_SM_SQ) + (gi & 7) * DN_TOK;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (h == 1 && !second_half) break;       // a tile with at most 32 live tokens (the reference's decode shape)
-                    uint32_t d[32];
-                    ptx::tmem_ld32(tmem + (uint32_t(warp * 32) << 16) + st * DN_TOK + 32 * h, d);
-                    ptx::tmem_wait_ld();
-#pragma unroll
-                    for (int n4 = 0; n4 < 32; n4 += 4) {
-                        const float4 sx4 = *reinterpret_cast<const float4*>(sx + 32 * h + n4);      // broadcast 16-byte loads
-                        const int4 sq4 = *reinterpret_cast<const int4*>(sq + 32 * h + n4);
-                        const float sxv[4] = {sx4.x, sx4.y, sx4.z, sx4.w};
-                        const int sqv[4] = {sq4.x, sq4.y, sq4.z, sq4.w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            // int -> float through the float whose bits are 1.5 * 2^23 + v: exact for |v| < 2^22 (here
-                            // |v| <= 255 * 127 * 128), integer adds and one float subtract at full rate
-                            const int n = n4 + e;
-                            const int v = int(d[n]) - z * sqv[e];
-                            const float vf = __int_as_float(v + 0x4B400000) - 12582912.0f;
-                            c[32 * h + n] = __fmaf_rn(__fmul_rn(sw, sxv[e]), vf, c[32 * h + n]);
-                        }
-                    }
-                }
-                ptx::tc_fence_before();
-            }
+            for (int j = 0; j < 4; ++j) { a[j][0] = w[2 * j] & mk; a[j][1] = (w[2 * j] >> 4) & mk; a[j][2] = w[2 * j + 1] & mk; a[j][3] = (w[2 * j + 1] >> 4) & mk; }
         }
-        cp_async_wait<0>();
-        if (alive) {
-            // Y += c, sixteen tokens at a time: all loads of a batch are issued before the first add, so the round trips
-            // to memory overlap instead of queueing behind one another (one coalesced 128-byte line per warp and token)
-            float* ybase = p.Y + size_t(n0) * p.rows + row0 + r;
+        const float swa = __half2float(__ushort_as_half(uint16_t(sw2 & 0xffffu))), swb = __half2float(__ushort_as_half(uint16_t(sw2 >> 16)));
+        const int za = int(z2 & 0xffu), zb = int(z2 >> 8);
+        const f32x2 swa2 = pack2(__float_as_uint(swa), __float_as_uint(swa)), swb2 = pack2(__float_as_uint(swb), __float_as_uint(swb));
 #pragma unroll
-            for (int nb = 0; nb < DN_TOK; nb += 16) {
-                float y[16];
+        for (int nq = 0; nq < 8; nq += 4) {
+            int acc[4][4] = {};
 #pragma unroll
-                for (int j = 0; j < 16; ++j) y[j] = n0 + nb + j < p.ntokens ? __ldcg(ybase + size_t(nb + j) * p.rows) : 0.f;
+            for (int h = 0; h < 2; ++h) {
+                uint4 b[4];
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (n0 + nb + j < p.ntokens) __stcg(ybase + size_t(nb + j) * p.rows, y[j] + c[nb + j]);
+                for (int k = 0; k < 4; ++k) b[k] = *reinterpret_cast<const uint4*>(st + DT_Q + (8 * (nq + k) + g) * 128 + (((2 * t + h) ^ g) << 4));
+#pragma unroll
+                for (int k = 0; k < 4; ++k) mma_m16n8k32_u8s8(acc[k], a[2 * h][0], a[2 * h][1], a[2 * h][2], a[2 * h][3], b[k].x, b[k].y);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) mma_m16n8k32_u8s8(acc[k], a[2 * h + 1][0], a[2 * h + 1][1], a[2 * h + 1][2], a[2 * h + 1][3], b[k].z, b[k].w);
             }
-        }
-    } else {
-        // ---- MMA issue: group i = four K-steps of 32 into accumulator i % 2, overwriting it
-        const uint32_t id = idesc_i8_u8s8(DN_ROWS, DN_TOK);
-        bool alive = true;
-#pragma unroll 1
-        for (int i = 0; i < ktot && alive; ++i) {
-            const int st = i & 1;
-            if (!ptx::mbar_wait(BAR(DB_FULL + st), (i >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_MMA; break; }
-            ptx::tc_fence_after();
-            if (ptx::elect_one()) {
-                const uint32_t a_s = ptx::smem_u32(smem + DN_SM_A + st * DN_A_BYTES);
-                const uint32_t b_s = ptx::smem_u32(smem + DN_SM_B + (i % DN_STAGES) * DN_B_BYTES);
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    mma_i8_ss(tmem + st * DN_TOK, ptx::smem_desc_sw128(a_s + 32 * k, 16, 1024), ptx::smem_desc_sw128(b_s + 32 * k, 16, 1024), id, k > 0);
-                ptx::mma_commit(BAR(DB_DONE + st));
+            for (int k = 0; k < 4; ++k) {
+                const int nt = nq + k;
+                const f32x2 sx = *reinterpret_cast<const f32x2*>(st + DT_SX + 8 * t + 32 * nt);
+                const int2 sq = *reinterpret_cast<const int2*>(st + DT_SQ + 8 * t + 32 * nt);
+                const f32x2 va = add2(pack2(uint32_t(acc[k][0] + (0x4B400000 - za * sq.x)), uint32_t(acc[k][1] + (0x4B400000 - za * sq.y))), magic);
+                const f32x2 vb = add2(pack2(uint32_t(acc[k][2] + (0x4B400000 - zb * sq.x)), uint32_t(acc[k][3] + (0x4B400000 - zb * sq.y))), magic);
+                c[nt][0] = fma2v(mul2(swa2, sx), va, c[nt][0]);
+                c[nt][1] = fma2v(mul2(swb2, sx), vb, c[nt][1]);
             }
-            __syncwarp();
         }
     }
-    if (errbits && p.err) atomicOr(p.err, errbits);
-    ptx::tc_fence_before();
-    __syncthreads();
-    if (warp == 4) ptx::tmem_dealloc(tmem, 128);
+    cp_async_wait<0>();
+    // Y += c: a warp's access covers the 8 rows of four tokens, whole 32-byte sectors
+    float* ybase = p.Y + size_t(n0 + 2 * t) * p.rows + row0 + 16 * warp + g;
+#pragma unroll
+    for (int nh = 0; nh < 8; nh += 4) {
+        float y[4][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                y[k][e] = 8 * (nh + k) + 2 * t + (e & 1) < live ? __ldcg(ybase + size_t(8 * (nh + k) + (e & 1)) * p.rows + 8 * (e >> 1)) : 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (8 * (nh + k) + 2 * t + (e & 1) < live) {
+                    const f32x2 v = c[nh + k][e >> 1];
+                    __stcg(ybase + size_t(8 * (nh + k) + (e & 1)) * p.rows + 8 * (e >> 1), y[k][e] + __uint_as_float(uint32_t(e & 1 ? v >> 32 : v)));
+                }
+    }
 }
 
 }  // namespace llattn

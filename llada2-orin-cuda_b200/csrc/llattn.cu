@@ -191,23 +191,36 @@ int llattn_qkv_prepare_commit(const float* qkv, const int32_t* pos, const float*
 // ------------------------------------------------------------------------------------------------------ consumer
 // The attention-output projection on the int8 activations the merge kernel writes.
 
+namespace {
+// At most this many tokens go to the strip kernel: it reads the weights once per 32 tokens, with every SM, and a call is
+// 3.8 us at 32 tokens and 6.6 at 64; the tile kernel's 16 row tiles at 65 tokens leave most SMs idle (15.5 us).
+constexpr int DENSE_STRIP_MAX_TOKENS = 64;
+}  // namespace
+
 int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int32_t* sum, float* Y, int ntokens, int rows, int K,
                       int* err_word, void* stream) {
     if (!W || !q || !s || !sum || !Y) return fail(LLATTN_EINVAL, "dense_w4a8: null pointer");
     if (ntokens < 0 || ntokens > 1 << 22) return fail(LLATTN_EINVAL, "dense_w4a8: ntokens = %d", ntokens);
     if (rows <= 0 || rows % llattn::DN_ROWS || K <= 0 || K % llattn::DN_GROUP || K > 1 << 20 || rows > 1 << 20)
         return fail(LLATTN_EINVAL, "dense_w4a8: rows = %d, K = %d (both multiples of 128)", rows, K);
+    if (!aligned16(W) || !aligned16(q)) return fail(LLATTN_EINVAL, "dense_w4a8: W and q must be 16-byte aligned");
     if (ntokens == 0) return LLATTN_OK;
+    const llattn::DenseParams p{static_cast<const uint8_t*>(W), q, s, sum, Y, ntokens, rows, K};
     static std::once_flag once[64];
     int dev = 0;
     CU(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64)
         std::call_once(once[dev], [] {
-            cudaFuncSetAttribute(llattn::dense_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DN_SMEM_BYTES);
+            cudaFuncSetAttribute(llattn::dense_strip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DS_SMEM_BYTES);
+            cudaFuncSetAttribute(llattn::dense_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DT_SMEM_BYTES);
         });
-    llattn::DenseParams p{static_cast<const uint8_t*>(W), q, s, sum, Y, ntokens, rows, K, err_word};
-    const dim3 grid(rows / llattn::DN_ROWS, (ntokens + llattn::DN_TOK - 1) / llattn::DN_TOK);
-    llattn::dense_i8_kernel<<<grid, llattn::DN_THREADS, llattn::DN_SMEM_BYTES, as_stream(stream)>>>(p);
+    if (ntokens <= DENSE_STRIP_MAX_TOKENS) {
+        const dim3 grid(rows / 16, (ntokens + llattn::DS_TOK - 1) / llattn::DS_TOK);
+        llattn::dense_strip_kernel<<<grid, llattn::DS_THREADS, llattn::DS_SMEM_BYTES, as_stream(stream)>>>(p);
+    } else {
+        const dim3 grid(rows / llattn::DN_ROWS, (ntokens + llattn::DT_TOK - 1) / llattn::DT_TOK);
+        llattn::dense_tile_kernel<<<grid, llattn::DT_THREADS, llattn::DT_SMEM_BYTES, as_stream(stream)>>>(p);
+    }
     CU(cudaGetLastError());
     return LLATTN_OK;
 }

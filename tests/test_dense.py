@@ -73,6 +73,38 @@ def test_dense_bit_exact_vs_oracle(api, orc, pkg, ntokens, rows, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("ntokens,rows,K,odd", [
+    (7, 128, 128, False), (8, 256, 2176, False), (31, 128, 2048, True), (33, 128, 4224, False), (63, 384, 256, False),   # a strip's tokens, one group, more groups than warps
+    (65, 128, 128, False), (97, 128, 4224, True), (127, 256, 384, True), (129, 128, 2176, False), (257, 2048, 256, False),
+    (1000, 384, 512, True), (2500, 1024, 128, False)])
+def test_dense_tile_edges(api, orc, pkg, ntokens, rows, K, odd):
+    """Token counts around the tile sizes of both kernels, one to more groups than pipeline stages or warps. `odd`: zero
+    points over the whole byte and sums that are not the sums of the codes, which the formula allows."""
+    wl = pkg.workload
+    strips, _, _, zero = wl.dense_weights(rows, K, 41)
+    q, s, qsum = wl.int8_activations(ntokens, K, 42)
+    rng = np.random.default_rng(43)
+    if odd:
+        ktot = K // 128
+        meta = strips.reshape(rows // 16, -1)[:, ktot * 1024:].reshape(rows // 16, ktot, 48)
+        meta[..., 32:] = rng.integers(0, 256, meta[..., 32:].shape)
+        qsum = qsum.copy()
+        qsum[rng.random(qsum.shape) < 0.1] += 77
+        q = q.copy()
+        q[0, :5] = -128
+    Y0 = rng.normal(size=(ntokens, rows)).astype(np.float32)
+    want = Y0.copy()
+    orc.dense_w4a8(strips, q, s, qsum, want)
+    pad = torch.full((ntokens + 2, rows), 7.0, device="cuda")          # rows before and after Y must not change
+    pad[1:-1] = _dev(Y0)
+    api.dense_w4a8(_dev(strips), _dev(q), _dev(s), _dev(qsum), pad[1:-1])
+    torch.cuda.synchronize()
+    got = pad.cpu().numpy()
+    assert (got[0] == 7).all() and (got[-1] == 7).all()
+    assert np.array_equal(got[1:-1].view(np.uint32), want.view(np.uint32)), float(np.abs(got[1:-1] - want).max())
+
+
+@pytest.mark.gpu
 def test_dense_bit_exact_vs_reference_kernel(api, pkg):
     import refkernel
     if not refkernel.gemm_available():
