@@ -104,9 +104,9 @@ attn_combine(const float* Opart, const float* Mpart, const float* Lpart, int nch
     llattn::fold_row_warp(Opart, Mpart, Lpart, md, r, int(threadIdx.x & 31), o);
 }
 
-__global__ void __launch_bounds__(llattn::COMMIT_THREADS)
+__global__ void __launch_bounds__(llattn::COMMIT_SHIM_THREADS)
 kv_commit(const half* Kf, const half* Vf, uint8_t* cache, int max_blocks, int blk) {
-    llattn::kv_commit_body(Kf, Vf, cache, nullptr, max_blocks, blk);
+    llattn::kv_commit_body<llattn::COMMIT_SHIM_THREADS>(Kf, Vf, cache, nullptr, max_blocks, blk);
 }
 
 }  // namespace attn

@@ -161,7 +161,9 @@ int launch_prepare(const float* qkv, const int32_t* pos, const float* gq, const 
                    void* q, void* k, void* v, int T, void* records, const int32_t* pages, int max_blocks, int blk, void* stream) {
     llattn::PrepArgs a{qkv, pos, gq, gk, inv_freq, eps, static_cast<half*>(q), static_cast<half*>(k), static_cast<half*>(v), T,
                        static_cast<uint8_t*>(records), pages, max_blocks, blk};
-    llattn::qkv_prepare_kernel<<<dim3((T + llattn::BLK - 1) / llattn::BLK, 8), llattn::PREP_THREADS, 0, as_stream(stream)>>>(a);
+    const int blocks = (T + llattn::BLK - 1) / llattn::BLK;
+    if (records) llattn::qkv_prepare_kernel<true><<<dim3(blocks, 20), llattn::PREP_THREADS, 0, as_stream(stream)>>>(a);
+    else llattn::qkv_prepare_kernel<false><<<dim3(blocks, 24), llattn::PREP_THREADS, 0, as_stream(stream)>>>(a);
     CU(cudaGetLastError());
     return LLATTN_OK;
 }

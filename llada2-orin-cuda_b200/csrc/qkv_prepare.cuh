@@ -9,8 +9,14 @@
 // (kv_commit.cuh), so a prefill block goes from fp32 qkv to its 4736-byte record in one pass: 12,288 B read and
 // 6,144 + 592 B written per token, against 14,336 read and the same written by the two-kernel sequence.
 //
-// Grid (blocks of 32 tokens, 8): y < 4 is a group of four q heads, y >= 4 the k and v head of kv head y - 4.
-// 256 threads; a warp takes whole (token, head) rows, lane l holding dims l, l+32, l+64, l+96: the rotate-half partners
+// A warp takes the four heads of one group for one token: sixteen loads in flight, one sine and cosine for all of them.
+// Groups 0-3 are q heads, 4 the k heads, 5 the v heads; grid (blocks of 32 tokens, 24): group y / 4, tokens 8 (y % 4) ..,
+// 8 warps a CTA. With the commit, K and V of a (block, kv head) stay with one CTA: grid (blocks, 20), y < 16 as above,
+// y >= 16 kv head y - 16, a warp per four tokens.
+// Bound by latency in a decode step: the former split, 8 CTAs per block whose warps walked 16 rows one after the
+// other, took 7.8 us for one block in a graph; now 1.8 (with the commit 9.5 -> 5.1). HBM-bound from a few thousand tokens
+// on: 8192 tokens 38.9 -> 24.7 us = 6.1 TB/s.
+// Lane l holds dims l, l+32, l+64, l+96 of a row: the rotate-half partners
 // then share a lane and every global access of a warp is one contiguous segment. The float operations and their order
 // are the reference kernel's (sum of squares folded lane-wise then by a xor butterfly, rsqrtf, x*r*g, sincosf, one
 // fused multiply-add per rotated output), which is what makes the outputs bit-identical to it.
@@ -58,67 +64,75 @@ __device__ __forceinline__ void norm_rope_lane(float (&x)[4], const float* __res
     x[0] = lo; x[1] = hi;
 }
 
+__device__ __forceinline__ void rope_angle(const PrepArgs& a, int t, float freq, float& cs, float& sn) {
+    sincosf(float(a.pos[t]) * freq, &sn, &cs);
+    cs = __bfloat162float(__float2bfloat16(cs));
+    sn = __bfloat162float(__float2bfloat16(sn));
+}
+
+template <bool COMMIT>
 __global__ void __launch_bounds__(PREP_THREADS) qkv_prepare_kernel(const PrepArgs a) {
-    __shared__ CommitSmem sm;
-    const int jb = blockIdx.x, grp = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int jb = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = jb * BLK;
     const float freq = a.inv_freq[lane];
-    if (grp < 4) {
-        // ---- four q heads x 32 tokens = 128 rows, 16 per warp
-        for (int i = warp; i < 4 * BLK; i += PREP_THREADS / 32) {
-            const int t = t0 + (i >> 2), hd = 4 * grp + (i & 3);
-            if (t >= a.T) break;
-            const float* src = a.qkv + size_t(t) * 3072 + hd * D;
-            float x[4];
+    if (!COMMIT || blockIdx.y < 16) {
+        // ---- four heads of one token
+        const int grp = blockIdx.y >> 2, t = t0 + 8 * (blockIdx.y & 3) + warp;
+        if (t >= a.T) return;
+        const float* src = a.qkv + size_t(t) * 3072 + 4 * grp * D + lane;
+        float x[4][4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) x[c] = src[lane + 32 * c];
-            float sn, cs;
-            sincosf(float(a.pos[t]) * freq, &sn, &cs);
-            cs = __bfloat162float(__float2bfloat16(cs));
-            sn = __bfloat162float(__float2bfloat16(sn));
-            norm_rope_lane(x, a.gq, lane, a.eps, cs, sn);
-            half* dst = a.q + (size_t(t) * NQH + hd) * D;
+        for (int h = 0; h < 4; ++h)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) dst[lane + 32 * c] = __float2half(x[c]);
+            for (int c = 0; c < 4; ++c) x[h][c] = src[h * D + 32 * c];
+        if (grp < 5) {
+            const float* gain = grp < 4 ? a.gq : a.gk;
+            float cs, sn;
+            rope_angle(a, t, freq, cs, sn);
+#pragma unroll
+            for (int h = 0; h < 4; ++h) norm_rope_lane(x[h], gain, lane, a.eps, cs, sn);
         }
+        half* dst = (grp < 4 ? a.q + (size_t(t) * NQH + 4 * grp) * D : (grp == 4 ? a.k : a.v) + size_t(t) * NKV * D) + lane;
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) dst[h * D + 32 * c] = __float2half(x[h][c]);
         return;
     }
-    // ---- kv head h: the block's K (normalised, rotated) and V (converted) as fp16 tiles in shared memory
-    const int h = grp - 4;
-    for (int tok = warp; tok < BLK; tok += PREP_THREADS / 32) {
-        const int t = t0 + tok;
-        float xk[4], xv[4];
-        if (t < a.T) {
-            const float* ks = a.qkv + size_t(t) * 3072 + (NQH + h) * D;
-            const float* vs = a.qkv + size_t(t) * 3072 + (NQH + NKV + h) * D;
+    if constexpr (COMMIT) {
+        // ---- kv head h: the block's K (normalised, rotated) and V (converted) as fp16 tiles in shared memory. Whole blocks.
+        __shared__ CommitSmem sm;
+        const int h = blockIdx.y - 16;
+        constexpr int TOKS = BLK / (PREP_THREADS / 32);
+        float xk[TOKS][4], xv[TOKS][4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) { xk[c] = ks[lane + 32 * c]; xv[c] = vs[lane + 32 * c]; }
-            float sn, cs;
-            sincosf(float(a.pos[t]) * freq, &sn, &cs);
-            cs = __bfloat162float(__float2bfloat16(cs));
-            sn = __bfloat162float(__float2bfloat16(sn));
-            norm_rope_lane(xk, a.gk, lane, a.eps, cs, sn);
-        } else {
+        for (int k = 0; k < TOKS; ++k) {
+            const float* ks = a.qkv + size_t(t0 + TOKS * warp + k) * 3072 + (NQH + h) * D + lane;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) { xk[c] = 0.f; xv[c] = 0.f; }
+            for (int c = 0; c < 4; ++c) { xk[k][c] = ks[32 * c]; xv[k][c] = ks[NKV * D + 32 * c]; }
         }
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            sm.Ks[tok][lane + 32 * c] = __float2half(xk[c]);
-            sm.Vs[tok][lane + 32 * c] = __float2half(xv[c]);
+        for (int k = 0; k < TOKS; ++k) {
+            const int tok = TOKS * warp + k;
+            float cs, sn;
+            rope_angle(a, t0 + tok, freq, cs, sn);
+            norm_rope_lane(xk[k], a.gk, lane, a.eps, cs, sn);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                sm.Ks[tok][lane + 32 * c] = __float2half(xk[k][c]);
+                sm.Vs[tok][lane + 32 * c] = __float2half(xv[k][c]);
+            }
         }
-    }
-    __syncthreads();
-    // ---- fp16 K and V of the block to global memory, 16 bytes per thread and store
-    for (int i = threadIdx.x; i < BLK * 16; i += PREP_THREADS) {
-        const int tok = i >> 4, ch = i & 15, t = t0 + tok;
-        if (t >= a.T) continue;
-        *reinterpret_cast<uint4*>(a.k + (size_t(t) * NKV + h) * D + ch * 8) = *reinterpret_cast<const uint4*>(&sm.Ks[tok][ch * 8]);
-        *reinterpret_cast<uint4*>(a.v + (size_t(t) * NKV + h) * D + ch * 8) = *reinterpret_cast<const uint4*>(&sm.Vs[tok][ch * 8]);
-    }
-    if (a.records) {
+        __syncthreads();
+        // ---- fp16 K and V of the block to global memory, 16 bytes per thread and store
+        for (int i = threadIdx.x; i < BLK * 16; i += PREP_THREADS) {
+            const int tok = i >> 4, ch = i & 15;
+            const size_t at = (size_t(t0 + tok) * NKV + h) * D + ch * 8;
+            *reinterpret_cast<uint4*>(a.k + at) = *reinterpret_cast<const uint4*>(&sm.Ks[tok][ch * 8]);
+            *reinterpret_cast<uint4*>(a.v + at) = *reinterpret_cast<const uint4*>(&sm.Vs[tok][ch * 8]);
+        }
         const size_t ridx = a.pages ? size_t(a.pages[jb * NKV + h]) : size_t(h) * a.max_blocks + a.blk + jb;
-        commit_tiles(sm, a.records + ridx * REC_BYTES, threadIdx.x, PREP_THREADS);
+        commit_tiles<PREP_THREADS>(sm, a.records + ridx * REC_BYTES, threadIdx.x);
     }
 }
 
