@@ -84,8 +84,11 @@ constexpr int SM_V = SM_K + 2 * TILE_BYTES;        // two V tiles
 constexpr int SM_RAW = SM_V + 2 * VTILE_BYTES;
 constexpr int SM_BAR = SM_RAW + NRAW * RAW_STRIDE;
 constexpr int SM_MISC = SM_BAR + 512;
-constexpr int SM_FIRST = SM_MISC + 16;             // the CTA's first run descriptor (64 bytes), fetched during set-up
-constexpr int ATTN_SMEM_BYTES = SM_FIRST + 64;
+constexpr int SM_FIRST = SM_MISC + 16;             // the CTA's first run descriptor, fetched during set-up
+// A softmax warp's way between its row-per-thread tensor memory and row-major global memory: 32 rows x 128 bytes, the 16-byte
+// chunk c of row r at chunk position c ^ (r % 8). Without it a warp's 16-byte accesses touch 32 lines each.
+constexpr int SM_STAGE = (SM_FIRST + int(sizeof(RunDesc)) + 127) / 128 * 128, STAGE_BYTES = 32 * 128;
+constexpr int ATTN_SMEM_BYTES = SM_STAGE + 4 * STAGE_BYTES;
 // warps 0-3 softmax (warp w: TMEM lanes 32 w .. 32 w + 31, one query row per thread), 4-11 dequant (four groups of two
 // warps, group g takes unit g of every tile: a thread's scale / minimum words then serve eight passes over the record),
 // then the service warps. Every scheduler carries one softmax warp, two dequantising warps and one service warp.
@@ -128,6 +131,7 @@ static_assert((GROUP_WARPS == 2 || GROUP_WARPS == 4) && DEQUANT_WARPS % GROUP_WA
 struct KParams {
     const RunDesc* items;          // list mode: runs in plan order, each with its sequence; nullptr = reference-grid mode
     const int32_t* cta_first;      // [gridDim.x + 1]
+    const RunDesc* first_runs;     // [gridDim.x]: items[cta_first[cta]], so that a CTA need not load the one to find the other
     const half* Q;
     const half* Kf;
     const half* Vf;
@@ -136,8 +140,8 @@ struct KParams {
     float* Lpart;
     float sl2;                     // softmax scale * log2(e)
     int* err;
-    // list mode with folding in the kernel (merge != nullptr)
-    const MergeDesc* merge;        // per output tile (WorkItem::tile indexes it)
+    // list mode with folding in the kernel
+    bool fused;
     int* tile_counters;            // [tiles][4]: [0] softmax warps whose rows of a run are out (4 per run), [1] warps that
                                    // have folded their share (16 per run); both back at 0 when the launch ends
     MergeOut out;
@@ -148,16 +152,17 @@ struct KParams {
     int ref_nchunks;
 };
 
-__device__ __forceinline__ bool fetch_item(const KParams& p, int idx, WorkItem& w, SeqDesc& s, const RunDesc* first, int first_idx) {
+__device__ __forceinline__ bool fetch_item(const KParams& p, int idx, WorkItem& w, SeqDesc& s, const RunDesc* first, int first_idx, MergeDesc* md = nullptr) {
     if (p.items) {
         const uint4* src = reinterpret_cast<const uint4*>(idx == first_idx ? first : p.items + idx);   // the first one is in shared memory
         RunDesc r;
         uint4* dst = reinterpret_cast<uint4*>(&r);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) dst[k] = src[k];
+        for (int k = 0; k < int(sizeof(RunDesc) / 16); ++k) dst[k] = src[k];
         w = r.w;
         s = r.s;
         s.cache += p.cache_offset;
+        if (md) *md = MergeDesc{s.q_first + w.qblk, w.kvh, r.slot_begin, r.nslots};
         return true;
     }
     const int kvh = idx & 3, chunk = (idx >> 2) % p.ref_nchunks, jb = (idx >> 2) / p.ref_nchunks;
@@ -527,8 +532,8 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
     }
     // the first run's descriptor comes in while the barriers and tensor memory are being set up
     const RunDesc* first_run = reinterpret_cast<const RunDesc*>(smem + SM_FIRST);
-    if (p.items && i0 < i1 && warp == 1 && lane < 16)
-        reinterpret_cast<uint32_t*>(smem + SM_FIRST)[lane] = __ldg(reinterpret_cast<const uint32_t*>(p.items + i0) + lane);
+    if (p.items && warp == 1 && lane < int(sizeof(RunDesc) / 4))
+        reinterpret_cast<uint32_t*>(smem + SM_FIRST)[lane] = __ldg(reinterpret_cast<const uint32_t*>(p.first_runs + cta) + lane);
     if (warp == WARP_MMA) { ptx::tmem_alloc(ptx::smem_u32(tmem_slot), TMEM_COLS); ptx::tmem_relinquish(); }
     ptx::tc_fence_before();
     __syncthreads();
@@ -550,11 +555,13 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
         const int row = warp * 32 + lane;
         const uint32_t tlane = tmem + (uint32_t(warp * 32) << 16);
         const unsigned long long sl2x2 = dup2(p.sl2);
+        uint8_t* const stage = smem + SM_STAGE + warp * STAGE_BYTES;
+        auto stage_in = [&](int r, int c) -> uint8_t* { return stage + r * 128 + ((c ^ (r & 7)) << 4); };
         uint32_t t = 0;
         bool alive = true;
 #pragma unroll 1
         for (int ii = i0; ii < i1 && alive; ++ii) {
-            WorkItem w; SeqDesc s;
+            WorkItem w; SeqDesc s; MergeDesc md{0, 0, 0, 1};
             if (!fetch_item(p, ii, w, s, first_run, i0_any)) continue;
             const int U = w.rec_count + w.fresh, ntiles = (U + TILE_UNITS - 1) / TILE_UNITS;
             // Reference exponent of the row, log2 units: the exact maximum of the run's first tile (a row dominated by a
@@ -562,18 +569,26 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
             // more than RESCALE_SLACK (engine/attn.cu:237-255 moves its reference lazily in the same way).
             float mref = -INFINITY;
             bool s_ready = false;              // the tile's S has been seen complete already (tested during the previous tile)
-            {   // this thread's query row into tensor memory as fp16 pairs. Every S MMA of the previous item has completed:
-                // this warp has seen the S of its last tile.
-                const half* src = p.Q + ((size_t(s.q_first + w.qblk) * BLK + (row >> 2)) * NQH + 4 * w.kvh + (row & 3)) * D;
-#pragma unroll 1
-                for (int c = 0; c < 4; ++c) {
-                    uint32_t r[16];
+            {   // the warp's 32 query rows into tensor memory as fp16 pairs, row = lane. Every S MMA of the previous item has
+                // completed: this warp has seen the S of its last tile. The rows come in as whole lines (8 lanes per 128-byte half
+                // row), all of them on their way at once, and change hands through the staging rows.
+                const half* src = p.Q + ((size_t(s.q_first + w.qblk) * BLK + 8 * warp) * NQH + 4 * w.kvh) * D + (lane >> 3) * D + (lane & 7) * 8;
+                uint4 v[16];
 #pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        const uint4 v = permute8(__ldg(reinterpret_cast<const uint4*>(src + 32 * c + 8 * g)));
-                        r[4 * g] = v.x; r[4 * g + 1] = v.y; r[4 * g + 2] = v.z; r[4 * g + 3] = v.w;
+                for (int g = 0; g < 16; ++g) v[g] = __ldg(reinterpret_cast<const uint4*>(src + size_t(g & 7) * NQH * D + 64 * (g >> 3)));      // token g % 8, half g / 8
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) *reinterpret_cast<uint4*>(stage_in(4 * g + (lane >> 3), lane & 7)) = permute8(v[8 * hf + g]);
+                    __syncwarp();
+                    uint32_t r[32];
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const uint4 x = *reinterpret_cast<const uint4*>(stage_in(lane, c));
+                        r[4 * c] = x.x; r[4 * c + 1] = x.y; r[4 * c + 2] = x.z; r[4 * c + 3] = x.w;
                     }
-                    ptx::tmem_st16(tlane + TM_Q + 16 * c, r);
+                    ptx::tmem_st32(tlane + TM_Q + 32 * hf, r);
+                    __syncwarp();
                 }
                 ptx::tmem_wait_st();
                 ptx::tc_fence_before();
@@ -623,6 +638,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
             // the tile's arrival counter; the tile's runs fold it together once the CTAs have no runs left (end of this
             // function).
             const uint32_t tl = t - 1;
+            fetch_item(p, ii, w, s, first_run, i0_any, &md);     // again: cheaper than a dozen registers through the loop above
             if (!ptx::mbar_wait(BAR(B_PV_DONE + (tl & 1)), (tl >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; break; }
             ptx::tc_fence_after();
             float lsum;
@@ -632,13 +648,10 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                 ptx::tmem_wait_ld_tied(r);
                 lsum = __uint_as_float(r[0]);
             }
-            const bool fused = p.merge != nullptr;
-            MergeDesc md{0, 0, 0, 1};
-            if (fused) md = p.merge[w.tile];
-            bool finish = fused && md.nslots == 1;
+            const bool fused = p.fused, finish = fused && md.nslots == 1;
             float M = mref, den = lsum;
             if (!finish) {
-                float* orow = p.Opart + (size_t(w.slot) * QR + row) * D;
+                float* out = p.Opart + (size_t(w.slot) * QR + 32 * warp + (lane >> 3)) * D + 4 * (lane & 7);
 #pragma unroll 1
                 for (int c = 0; c < 4; ++c) {
                     uint32_t r[32];
@@ -646,13 +659,14 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                     ptx::tmem_wait_ld_tied(r);
 #pragma unroll
                     for (int g = 0; g < 4; ++g) {      // positions (0..7) hold dims (0,4,1,5,2,6,3,7)
-                        const float4 lo = make_float4(__uint_as_float(r[8 * g]), __uint_as_float(r[8 * g + 2]),
-                                                      __uint_as_float(r[8 * g + 4]), __uint_as_float(r[8 * g + 6]));
-                        const float4 hi = make_float4(__uint_as_float(r[8 * g + 1]), __uint_as_float(r[8 * g + 3]),
-                                                      __uint_as_float(r[8 * g + 5]), __uint_as_float(r[8 * g + 7]));
-                        *reinterpret_cast<float4*>(orow + 32 * c + 8 * g) = lo;
-                        *reinterpret_cast<float4*>(orow + 32 * c + 8 * g + 4) = hi;
+                        *reinterpret_cast<uint4*>(stage_in(lane, 2 * g)) = make_uint4(r[8 * g], r[8 * g + 2], r[8 * g + 4], r[8 * g + 6]);
+                        *reinterpret_cast<uint4*>(stage_in(lane, 2 * g + 1)) = make_uint4(r[8 * g + 1], r[8 * g + 3], r[8 * g + 5], r[8 * g + 7]);
                     }
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)        // four rows x 128 bytes
+                        *reinterpret_cast<uint4*>(out + 4 * i * D + 32 * c) = *reinterpret_cast<const uint4*>(stage_in(4 * i + (lane >> 3), lane & 7));
+                    __syncwarp();
                 }
                 // the accumulator has been read: the next run's PV may start while the stores below drain
                 ptx::tc_fence_before();
@@ -693,7 +707,35 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                             v[8 * g + k] = __uint_as_float(r[8 * g + 2 * k]) * inv;
                             v[8 * g + 4 + k] = __uint_as_float(r[8 * g + 2 * k + 1]) * inv;
                         }
-                    row_store(p.out, ro, c, v);
+                    if (p.out.O32) {
+#pragma unroll
+                        for (int g = 0; g < 8; ++g)
+                            *reinterpret_cast<float4*>(stage_in(lane, g)) = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+                        __syncwarp();
+                        float* out = p.out.O32 + ((size_t(md.q_index) * BLK + 8 * warp) * NQH + 4 * md.kvh + (lane >> 3)) * D + 32 * c + 4 * (lane & 7);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)    // the four heads of token 8 warp + i
+                            *reinterpret_cast<uint4*>(out + size_t(i) * NQH * D) = *reinterpret_cast<const uint4*>(stage_in(4 * i + (lane >> 3), lane & 7));
+                        __syncwarp();
+                    }
+                    if (p.out.O16) {
+#pragma unroll
+                        for (int g = 0; g < 4; ++g) {
+                            const half2 h0 = __floats2half2_rn(v[8 * g], v[8 * g + 1]), h1 = __floats2half2_rn(v[8 * g + 2], v[8 * g + 3]);
+                            const half2 h2 = __floats2half2_rn(v[8 * g + 4], v[8 * g + 5]), h3 = __floats2half2_rn(v[8 * g + 6], v[8 * g + 7]);
+                            *reinterpret_cast<uint4*>(stage_in(lane, g)) = make_uint4(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1),
+                                                                                      *reinterpret_cast<const uint32_t*>(&h2), *reinterpret_cast<const uint32_t*>(&h3));
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {  // eight rows x 64 bytes
+                            const int rr = 8 * i + (lane >> 2);
+                            half* out = p.out.O16 + ((size_t(md.q_index) * BLK + 8 * warp + (rr >> 2)) * NQH + 4 * md.kvh + (rr & 3)) * D + 32 * c + 8 * (lane & 3);
+                            *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(stage_in(rr, lane & 3));
+                        }
+                        __syncwarp();
+                    }
+                    if (p.out.q8) row_store_q8(p.out, ro, c, v);
                 }
                 row_finish(p.out, ro, M, den);
                 ptx::tc_fence_before();
@@ -707,13 +749,6 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
         const DqThread dq = dq_thread(dt);
         uint32_t t = 0, r = 0;
         bool alive = true;
-        // third block of both V tiles: column 128 of V is all ones (O column 128 accumulates sum(P)), 129..143 zero.
-        // Published by the first v_full arrival.
-        for (int idx = da; idx < 2 * 128 * 8; idx += 32 * DEQUANT_WARPS) {
-            const int buf = idx >> 10, key = (idx >> 3) & 127, pos = idx & 7;
-            *reinterpret_cast<uint4*>(smem + SM_V + buf * VTILE_BYTES + 2 * KBLOCK + key * 128 + pos * 16) =
-                make_uint4(pos == (key & 7) ? 0x00003C00u : 0u, 0u, 0u, 0u);
-        }
 #pragma unroll 1
         for (int ii = i0; ii < i1 && alive; ++ii) {
             WorkItem w; SeqDesc s;
@@ -946,6 +981,15 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
         // ================================================================== O += P V issue
         uint32_t t = 0, itc = 0;
         bool alive = true;
+        // third block of both V tiles: column 128 of V is all ones (O column 128 accumulates sum(P)), 129..143 zero. Written by
+        // the warp whose MMAs read it, which has nothing else to do while the first tile is on its way.
+        for (int idx = lane; idx < 2 * 128 * 8; idx += 32) {
+            const int buf = idx >> 10, key = (idx >> 3) & 127, pos = idx & 7;
+            *reinterpret_cast<uint4*>(smem + SM_V + buf * VTILE_BYTES + 2 * KBLOCK + key * 128 + pos * 16) =
+                make_uint4(pos == (key & 7) ? 0x00003C00u : 0u, 0u, 0u, 0u);
+        }
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
         const uint32_t v_s = ptx::smem_u32(smem + SM_V);
         const uint32_t idO = ptx::idesc_f16(128, PV_N, false, true);
         // one base descriptor per V buffer (MN-major, 128-byte swizzle: 8-key groups 1024 B apart, 64-dim blocks KBLOCK apart)
@@ -1007,13 +1051,12 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
     // counted in, then all sixteen warps finish this run's share of the rows, a warp per row. The last warp to leave a
     // tile puts both of its counters back to zero for the next launch. Every thread of the CTA walks this loop the same
     // way (same runs, same outcome), so the CTA barrier inside it is reached by all.
-    if (p.merge != nullptr) {
+    if (p.fused) {
         int nsplit = 0;
 #pragma unroll 1
         for (int ii = i0_any; ii < i1_any; ++ii) {
-            WorkItem w; SeqDesc sq;
-            if (!fetch_item(p, ii, w, sq, first_run, i0_any)) continue;
-            const MergeDesc md = p.merge[w.tile];
+            WorkItem w; SeqDesc sq; MergeDesc md{0, 0, 0, 1};
+            if (!fetch_item(p, ii, w, sq, first_run, i0_any, &md)) continue;
             if (md.nslots <= 1) continue;
             int* counters = p.tile_counters + 4 * w.tile;
             // one warp polls the counter for the whole CTA (hundreds of finished CTAs polling with every warp would load
@@ -1032,7 +1075,9 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
             }
             constexpr int NW = ATTN_THREADS / 32;
             const int r0 = (w.slot - md.slot_begin) + md.nslots * warp, step = md.nslots * NW;
-            if (md.nslots == 2) {
+            if (md.nslots > FOLD_PART) {
+                fold_rows_shared(p.Opart, p.Mpart, p.Lpart, md, w.slot - md.slot_begin, warp, lane, smem + SM_K, p.out);      // the tiles are done with
+            } else if (md.nslots == 2) {
 #pragma unroll 1
                 for (int r = r0; r < QR; r += 4 * step) {
                     const int rows[4] = {r, r + step < QR ? r + step : -1, r + 2 * step < QR ? r + 2 * step : -1, r + 3 * step < QR ? r + 3 * step : -1};

@@ -37,13 +37,15 @@ struct WorkItem {
     int32_t tile;             // output tile (query block x kv head) the run belongs to: index of its MergeDesc
 };
 
-// What the kernel reads per run: the run and its sequence side by side, 64 bytes, so that a CTA reaches everything about
-// its first run with two dependent loads (its item range, then this) instead of three.
+// What the kernel reads per run: the run, its sequence and the slots of its tile side by side, 80 bytes, so that nothing a
+// CTA does on the way of a run waits for a second, dependent load.
 struct alignas(16) RunDesc {
     WorkItem w;
     SeqDesc s;
+    int32_t slot_begin, nslots;   // the tile's partial slots (its MergeDesc)
+    int32_t pad[2];
 };
-static_assert(sizeof(RunDesc) == 64, "RunDesc layout");
+static_assert(sizeof(RunDesc) == 80, "RunDesc layout");
 
 // One output tile (query block x kv head) and the partial slots that make it up.
 struct MergeDesc {

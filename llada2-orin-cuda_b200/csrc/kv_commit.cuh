@@ -12,21 +12,26 @@
 
 namespace llattn {
 
-constexpr int COMMIT_THREADS = 512, COMMIT_SHIM_THREADS = 128;       // 128: the launch shape of the reference (attn_shim.cuh)
+constexpr int COMMIT_SHIM_THREADS = 128;        // the launch shape of the reference (attn_shim.cuh)
 
 __device__ __forceinline__ void commit_meta(float mn, float mx, half& sh, half& mh) {
     sh = __float2half_rn(fmaxf(__fdiv_rn(__fsub_rn(mx, mn), 15.f), 6.2e-5f));
     mh = __float2half_rn(mn);
 }
-// clamp(rint((v - m0) / s), 0, 15) with the division rounded as IEEE says, r = 1 / s correctly rounded. The product with r
-// is within 16 x 2^-22 of that quotient wherever the clamp lets the difference show, so only a product that lies this
-// close to a tie (or is not finite) needs the division itself: about one value in a thousand. The divisions were half of
-// the kernel's instructions.
-__device__ __forceinline__ uint32_t commit_code(float v, float m0, float s, float r) {
+// clamp(rint((v - m0) / s), 0, 15) as a float, with the division rounded as IEEE says, r = 1 / s correctly rounded. The
+// product with r is within 16 x 2^-22 of that quotient wherever the clamp lets the difference show, so only a product that
+// lies this close to a tie (or is not finite) needs the division itself: about one value in a thousand. Rounding to an
+// integer is the addition of 1.5 x 2^23 (larger products end at the clamp either way): the divisions and the conversion
+// instructions, an eighth of the rate of an addition, were most of the kernel's time.
+__device__ __forceinline__ float commit_code(float v, float m0, float s, float r) {
     const float x = __fsub_rn(v, m0), a = __fmul_rn(x, r);
-    int n = __float2int_rn(a);
-    if (!(fabsf(a - float(n)) < 0.4995f)) n = __float2int_rn(__fdiv_rn(x, s));
-    return uint32_t(max(0, min(15, n)));
+    float n = __fsub_rn(__fadd_rn(a, 12582912.f), 12582912.f);
+    if (!(fabsf(a - n) < 0.4995f)) n = rintf(__fdiv_rn(x, s));
+    return fminf(fmaxf(n, 0.f), 15.f);
+}
+// Four codes, the first in the low nibble.
+__device__ __forceinline__ uint32_t pack_codes(float c0, float c1, float c2, float c3) {
+    return __float_as_uint(fmaf(c3, 4096.f, fmaf(c2, 256.f, fmaf(c1, 16.f, c0))) + 12582912.f) & 0xffffu;
 }
 
 constexpr int TILE_LD = D + 8;           // halves per tile row: rows 272 B apart, 16-byte aligned, no bank conflicts by column
@@ -46,7 +51,7 @@ struct CommitSmem {
 // through their shuffles together. fminf and fmaxf order -0 below +0 and pass NaN by whatever the order of the operands,
 // so the extrema do not depend on the split.
 // In a graph, 128 threads with a channel per thread and a division per value -> this: 1 block 9.5 -> 3.0 us, 64 blocks
-// 10.2 -> 4.3, 2048 blocks 102 -> 73 (its bytes: 26).
+// 10.2 -> 4.3, 2048 blocks 102 -> 68 (its bytes: 26).
 template <int NT>
 __device__ __forceinline__ void commit_tiles(CommitSmem& sm, uint8_t* __restrict__ dst, int tid) {
     constexpr int PARTS = NT / D, KT = BLK / PARTS, VT = BLK / (NT / 32);
@@ -89,8 +94,8 @@ __device__ __forceinline__ void commit_tiles(CommitSmem& sm, uint8_t* __restrict
             half sh, mh;
             commit_meta(mn[k], mx[k], sh, mh);
             const float s = __half2float(sh), m0 = __half2float(mh), r = __frcp_rn(s);
-            const uint32_t packed = commit_code(v[k][0], m0, s, r) | (commit_code(v[k][1], m0, s, r) << 4) |
-                                    (commit_code(v[k][2], m0, s, r) << 8) | (commit_code(v[k][3], m0, s, r) << 12);
+            const uint32_t packed = pack_codes(commit_code(v[k][0], m0, s, r), commit_code(v[k][1], m0, s, r),
+                                               commit_code(v[k][2], m0, s, r), commit_code(v[k][3], m0, s, r));
             *reinterpret_cast<uint16_t*>(sm.rec + VOFF + tok * 64 + lane * 2) = uint16_t(packed);
             if (lane == 0) {
                 reinterpret_cast<half*>(sm.rec + VOFF_META)[tok] = sh;
@@ -110,9 +115,10 @@ __device__ __forceinline__ void commit_tiles(CommitSmem& sm, uint8_t* __restrict
         // four of the eight tokens' bytes
 #pragma unroll
         for (int k0 = 0; k0 < KT; k0 += 8) {
-            uint32_t w = 0;
+            float code[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) w |= commit_code(__half2float(kv[k0 + k]), m0, s, r) << (4 * k);
+            for (int k = 0; k < 8; ++k) code[k] = commit_code(__half2float(kv[k0 + k]), m0, s, r);
+            const uint32_t w = pack_codes(code[0], code[1], code[2], code[3]) | pack_codes(code[4], code[5], code[6], code[7]) << 16;
             const uint32_t other = __shfl_xor_sync(0xffffffffu, w, 1);
             const uint32_t lo = (lane & 1) ? other >> 16 : w, hi = (lane & 1) ? w >> 16 : other;     // even channel, odd channel
             const int tok = part * KT + k0 + 4 * (lane & 1);
@@ -159,10 +165,11 @@ __device__ __forceinline__ void kv_commit_body(const half* __restrict__ Kf, cons
     commit_tiles<NT>(sm, records + ridx * REC_BYTES, tid);
 }
 
-__global__ void __launch_bounds__(COMMIT_THREADS)
+template <int NT>
+__global__ void __launch_bounds__(NT)
 kv_commit_kernel(const half* __restrict__ Kf, const half* __restrict__ Vf, uint8_t* __restrict__ records,
                  const int32_t* __restrict__ pages, int max_blocks, int blk) {
-    kv_commit_body<COMMIT_THREADS>(Kf, Vf, records, pages, max_blocks, blk);
+    kv_commit_body<NT>(Kf, Vf, records, pages, max_blocks, blk);
 }
 
 }  // namespace llattn

@@ -63,17 +63,16 @@ struct llattn_ctx {
 struct llattn_plan {
     llattn_ctx* ctx = nullptr;
     llattn_plan_stats stats{};
-    void* dev_blob = nullptr;         // seq descriptors, work items, per-CTA ranges, tile descriptors (fixed section offsets)
+    void* dev_blob = nullptr;         // run descriptors, per-CTA ranges, each CTA's first run (fixed section offsets)
     void* host_blob = nullptr;        // pinned mirror: llattn_plan_update fills it and copies it up asynchronously
-    size_t blob_bytes = 0, off_seqs = 0, off_items = 0, off_cta = 0, off_merge = 0;
+    size_t blob_bytes = 0, off_items = 0, off_cta = 0, off_first = 0;
     size_t cap_seqs = 0, cap_items = 0, cap_tiles = 0;
     int launch_ctas = 0;              // grid of every launch of this plan (CTAs beyond the used ones find no items)
     cudaEvent_t ev_upload = nullptr;
     bool upload_pending = false;
-    const llattn::SeqDesc* d_seqs = nullptr;
     const llattn::RunDesc* d_items = nullptr;
     const int32_t* d_cta_first = nullptr;
-    const llattn::MergeDesc* d_merge = nullptr;
+    const llattn::RunDesc* d_first = nullptr;
 };
 
 namespace {
@@ -130,6 +129,21 @@ int llattn_tile_units(void) { return llattn::TILE_UNITS; }
 
 // ------------------------------------------------------------------------------------------------------ commit
 
+namespace {
+// Few blocks: 512 threads a record, for the shortest chain. From the number of blocks on whose records no longer fit on the
+// chip at four of those CTAs an SM: 256 threads, eight records an SM in flight (2048 blocks 75 -> 68 us; 64
+// blocks 4.3 us with 512).
+int launch_commit(const void* Kf, const void* Vf, void* records, const int32_t* pages, int max_blocks, int blk, int nb, void* stream) {
+    const dim3 grid(llattn::NKV, nb);
+    const half *k = static_cast<const half*>(Kf), *v = static_cast<const half*>(Vf);
+    uint8_t* r = static_cast<uint8_t*>(records);
+    if (nb <= 128) llattn::kv_commit_kernel<512><<<grid, 512, 0, as_stream(stream)>>>(k, v, r, pages, max_blocks, blk);
+    else llattn::kv_commit_kernel<256><<<grid, 256, 0, as_stream(stream)>>>(k, v, r, pages, max_blocks, blk);
+    CU(cudaGetLastError());
+    return LLATTN_OK;
+}
+}  // namespace
+
 int llattn_kv_commit(const void* Kf, const void* Vf, void* cache, int max_blocks, int blk, int nb, void* stream) {
     if (!Kf || !Vf || !cache) return fail(LLATTN_EINVAL, "kv_commit: null pointer");
     if (nb < 0 || blk < 0 || max_blocks <= 0 || blk + nb > max_blocks)
@@ -137,10 +151,7 @@ int llattn_kv_commit(const void* Kf, const void* Vf, void* cache, int max_blocks
     if (!aligned16(Kf) || !aligned16(Vf) || !aligned16(cache)) return fail(LLATTN_EINVAL, "kv_commit: pointers must be 16-byte aligned");
     if (nb == 0) return LLATTN_OK;
     if (nb > 65535) return fail(LLATTN_EINVAL, "kv_commit: at most 65535 blocks per call");
-    llattn::kv_commit_kernel<<<dim3(llattn::NKV, nb), llattn::COMMIT_THREADS, 0, as_stream(stream)>>>(
-        static_cast<const half*>(Kf), static_cast<const half*>(Vf), static_cast<uint8_t*>(cache), nullptr, max_blocks, blk);
-    CU(cudaGetLastError());
-    return LLATTN_OK;
+    return launch_commit(Kf, Vf, cache, nullptr, max_blocks, blk, nb, stream);
 }
 
 int llattn_kv_commit_paged(const void* Kf, const void* Vf, void* pool, const int32_t* pages, int nb, void* stream) {
@@ -148,10 +159,7 @@ int llattn_kv_commit_paged(const void* Kf, const void* Vf, void* pool, const int
     if (nb < 0 || nb > 65535) return fail(LLATTN_EINVAL, "kv_commit_paged: nb must be in [0, 65535]");
     if (!aligned16(Kf) || !aligned16(Vf) || !aligned16(pool)) return fail(LLATTN_EINVAL, "kv_commit_paged: pointers must be 16-byte aligned");
     if (nb == 0) return LLATTN_OK;
-    llattn::kv_commit_kernel<<<dim3(llattn::NKV, nb), llattn::COMMIT_THREADS, 0, as_stream(stream)>>>(
-        static_cast<const half*>(Kf), static_cast<const half*>(Vf), static_cast<uint8_t*>(pool), pages, 0, 0);
-    CU(cudaGetLastError());
-    return LLATTN_OK;
+    return launch_commit(Kf, Vf, pool, pages, 0, 0, nb, stream);
 }
 
 // ------------------------------------------------------------------------------------------------------ producer

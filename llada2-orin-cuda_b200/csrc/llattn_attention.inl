@@ -308,11 +308,15 @@ int stage_plan(llattn_plan* pl, const HostPlan& hp) {
         return fail(LLATTN_ENOMEM, "plan: %zu sequences, %zu runs, %zu tiles; the plan was created for %zu, %zu, %zu",
                     hp.seqs.size(), hp.items.size(), hp.merge.size(), pl->cap_seqs, pl->cap_items, pl->cap_tiles);
     uint8_t* h = static_cast<uint8_t*>(pl->host_blob);
-    memcpy(h + pl->off_seqs, hp.seqs.data(), hp.seqs.size() * sizeof(llattn::SeqDesc));
     llattn::RunDesc* runs = reinterpret_cast<llattn::RunDesc*>(h + pl->off_items);
-    for (size_t i = 0; i < hp.items.size(); ++i) runs[i] = llattn::RunDesc{hp.items[i], hp.seqs[hp.items[i].seq]};
+    for (size_t i = 0; i < hp.items.size(); ++i) {
+        const llattn::MergeDesc& md = hp.merge[hp.items[i].tile];
+        runs[i] = llattn::RunDesc{hp.items[i], hp.seqs[hp.items[i].seq], md.slot_begin, md.nslots, {0, 0}};
+    }
     memcpy(h + pl->off_cta, hp.cta_first.data(), hp.cta_first.size() * sizeof(int32_t));
-    memcpy(h + pl->off_merge, hp.merge.data(), hp.merge.size() * sizeof(llattn::MergeDesc));
+    llattn::RunDesc* first = reinterpret_cast<llattn::RunDesc*>(h + pl->off_first);      // of a CTA without runs: any bytes, not used
+    for (int c = 0; c < pl->launch_ctas; ++c)
+        if (hp.cta_first[c] < hp.cta_first[c + 1]) first[c] = runs[hp.cta_first[c]];
     return LLATTN_OK;
 }
 
@@ -342,11 +346,10 @@ int llattn_plan_create(llattn_ctx* c, const llattn_seq* seqs, int nseq, int ncta
     pl->cap_seqs = hp.seqs.size();
     pl->cap_tiles = hp.merge.size();
     pl->cap_items = hp.merge.size() + size_t(nctas);
-    pl->off_seqs = 0;
-    pl->off_items = pl->off_seqs + up256(pl->cap_seqs * sizeof(SeqDesc));
+    pl->off_items = 0;
     pl->off_cta = pl->off_items + up256(pl->cap_items * sizeof(RunDesc));
-    pl->off_merge = pl->off_cta + up256((size_t(nctas) + 1) * sizeof(int32_t));
-    pl->blob_bytes = pl->off_merge + up256(pl->cap_tiles * sizeof(MergeDesc));
+    pl->off_first = pl->off_cta + up256((size_t(nctas) + 1) * sizeof(int32_t));
+    pl->blob_bytes = pl->off_first + up256(size_t(nctas) * sizeof(RunDesc));
     auto bail = [&](int code, const char* what) {
         if (pl->dev_blob) cudaFree(pl->dev_blob);
         if (pl->host_blob) cudaFreeHost(pl->host_blob);
@@ -362,10 +365,9 @@ int llattn_plan_create(llattn_ctx* c, const llattn_seq* seqs, int nseq, int ncta
     if (int rc = stage_plan(pl, hp)) { bail(rc, "internal"); return rc; }
     if (cudaMemcpy(pl->dev_blob, pl->host_blob, pl->blob_bytes, cudaMemcpyHostToDevice) != cudaSuccess) return bail(LLATTN_ECUDA, "upload failed");
     const uint8_t* d = static_cast<const uint8_t*>(pl->dev_blob);
-    pl->d_seqs = reinterpret_cast<const SeqDesc*>(d + pl->off_seqs);
     pl->d_items = reinterpret_cast<const RunDesc*>(d + pl->off_items);
     pl->d_cta_first = reinterpret_cast<const int32_t*>(d + pl->off_cta);
-    pl->d_merge = reinterpret_cast<const MergeDesc*>(d + pl->off_merge);
+    pl->d_first = reinterpret_cast<const RunDesc*>(d + pl->off_first);
     fill_stats(pl, hp, nseq);
     // the scratch is sized for the most runs any update can bring, so that an update never allocates
     pl->stats.workspace_bytes = COUNTER_BYTES + pl->cap_items * (SLOT_O_BYTES + 2 * SLOT_ML_BYTES);
@@ -450,12 +452,12 @@ int llattn_attention(llattn_ctx* c, const llattn_plan* pl, const llattn_io* io, 
     float* Mpart = Opart + ns * QR * D;
     float* Lpart = Mpart + ns * QR;
     KParams p{};
-    p.items = pl->d_items; p.cta_first = pl->d_cta_first;
+    p.items = pl->d_items; p.cta_first = pl->d_cta_first; p.first_runs = pl->d_first;
     p.Q = static_cast<const half*>(io->Q); p.Kf = static_cast<const half*>(io->Kf); p.Vf = static_cast<const half*>(io->Vf);
     p.Opart = Opart; p.Mpart = Mpart; p.Lpart = Lpart;
     p.sl2 = (io->scale > 0.f ? io->scale : 0.08838834764831845f) * 1.4426950408889634f;
     p.err = c->err_word;
-    p.merge = pl->d_merge;
+    p.fused = true;
     p.tile_counters = static_cast<int*>(c->workspace);
     p.out = MergeOut{static_cast<half*>(io->O16), io->O32, io->LSE, io->q8, io->s8, io->sum8};
     p.cache_offset = io->cache_offset;

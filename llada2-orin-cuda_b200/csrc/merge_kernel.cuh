@@ -6,8 +6,8 @@
 // stored in the fragment order of engine/attn.cu:308-312, plus the integer row sum).
 //
 // Two forms. In the attention kernel's epilogue one THREAD owns one query row (that is how the kernel holds its
-// accumulator: one tensor-memory lane per row) and writes a row 32 dims at a time straight from tensor memory
-// (row_store, row_finish): a tile that a single run covers needs no folding. Everywhere partial slots have to be folded -
+// accumulator: one tensor-memory lane per row) and writes a row 32 dims at a time from tensor memory
+// (the kernel itself, row_store_q8, row_finish): a tile that a single run covers needs no folding. Everywhere partial slots have to be folded -
 // the attention kernel's split tiles, the reference-shaped operator pair, the allocation-free entry point, the source
 // shim - a WARP owns a row (fold_row_warp and friends, below). The slots of a tile are always added in slot order, so
 // the result does not depend on which run finishes last.
@@ -42,44 +42,19 @@ struct RowOut {
     int qsum;          // int8 form: running sum of the codes
 };
 
-// 32 normalised values of a row (dims [32 c, 32 c + 32), dim order) to every requested output.
-__device__ __forceinline__ void row_store(const MergeOut& o, RowOut& ro, int c, const float (&v)[32]) {
-    const size_t base = (ro.row * NQH + ro.head) * D + 32 * c;
-    if (o.O32) {
+// 32 normalised values of a row (dims [32 c, 32 c + 32), dim order) to the int8 output.
+__device__ __forceinline__ void row_store_q8(const MergeOut& o, RowOut& ro, int c, const float (&v)[32]) {
 #pragma unroll
-        for (int g = 0; g < 8; ++g)
-            *reinterpret_cast<float4*>(o.O32 + base + 4 * g) = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
-    }
-    if (o.O16) {
+    for (int g = 0; g < 8; ++g) {      // a run of 4 dims stays contiguous in fragment order
+        char4 qv;
+        int8_t* qq = reinterpret_cast<int8_t*>(&qv);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            const half2 a = __floats2half2_rn(v[8 * g], v[8 * g + 1]), b = __floats2half2_rn(v[8 * g + 2], v[8 * g + 3]);
-            const half2 cc = __floats2half2_rn(v[8 * g + 4], v[8 * g + 5]), d = __floats2half2_rn(v[8 * g + 6], v[8 * g + 7]);
-            uint4 pk;
-            pk.x = *reinterpret_cast<const uint32_t*>(&a); pk.y = *reinterpret_cast<const uint32_t*>(&b);
-            pk.z = *reinterpret_cast<const uint32_t*>(&cc); pk.w = *reinterpret_cast<const uint32_t*>(&d);
-            *reinterpret_cast<uint4*>(o.O16 + base + 8 * g) = pk;
+        for (int k = 0; k < 4; ++k) {
+            qq[k] = int8_t(max(-127, min(127, __float2int_rn(__fdiv_rn(v[4 * g + k], ro.qscale)))));
+            ro.qsum += qq[k];
         }
+        *reinterpret_cast<char4*>(o.q8 + ro.row * 2048 + frag_pos(ro.head * D + 32 * c + 4 * g)) = qv;
     }
-    if (o.q8) {
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {      // a run of 4 dims stays contiguous in fragment order
-            char4 qv;
-            int8_t* qq = reinterpret_cast<int8_t*>(&qv);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                qq[k] = int8_t(max(-127, min(127, __float2int_rn(__fdiv_rn(v[4 * g + k], ro.qscale)))));
-                ro.qsum += qq[k];
-            }
-            *reinterpret_cast<char4*>(o.q8 + ro.row * 2048 + frag_pos(ro.head * D + 32 * c + 4 * g)) = qv;
-        }
-    }
-}
-__device__ __forceinline__ float absmax32(const float (&v)[32]) {
-    float m = 0.f;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) m = fmaxf(m, fabsf(v[j]));
-    return m;
 }
 // Per-row scalars once all values are out: the log-sum-exp and the int8 form's scale and code sum.
 __device__ __forceinline__ void row_finish(const MergeOut& o, const RowOut& ro, float M, float den) {
@@ -149,11 +124,46 @@ __device__ __forceinline__ void emit_row_warp(float M, float den, const float4& 
     }
 }
 
+// Up to FOLD_PART slots of one row, by one warp: reference exponent, row sum and weighted dims of those slots. Every load
+// - the slots' scalars and their rows - is on its way before the first is used: one round trip to the L2.
+constexpr int FOLD_PART = 16;
+__device__ __forceinline__ void fold_part(const float* Opart, const float* Mpart, const float* Lpart, size_t slot0, int cnt, int r, int lane,
+                                          float& M, float& den, float4& acc) {
+    const size_t i0 = slot0 * QR + r;
+    const float m = lane < cnt ? __ldcg(Mpart + i0 + size_t(lane) * QR) : -INFINITY;
+    const float l = lane < cnt ? __ldcg(Lpart + i0 + size_t(lane) * QR) : 0.f;
+    float4 v[FOLD_PART];
+#pragma unroll
+    for (int k = 0; k < FOLD_PART; ++k)                // past the end: the last slot again, not used below
+        v[k] = __ldcg(reinterpret_cast<const float4*>(Opart + (i0 + size_t(min(k, cnt - 1)) * QR) * D) + lane);
+    M = m;
+#pragma unroll
+    for (int d = 16; d; d >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, d));
+    const float w = exp2f(m - M);
+    den = 0.f;
+    acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < FOLD_PART; ++k) {
+        const float f = __shfl_sync(0xffffffffu, w, k), lk = __shfl_sync(0xffffffffu, l, k);
+        if (k < cnt) {
+            den += f * lk;
+            acc.x += f * v[k].x; acc.y += f * v[k].y; acc.z += f * v[k].z; acc.w += f * v[k].w;
+        }
+    }
+}
+
 // One row of a split tile, by one warp: fold the slots, normalise, write every requested output.
 constexpr int FOLD_MAX_SLOTS = 160;           // slots of one tile: at most one per CTA of the launch (148 SMs)
 __device__ __forceinline__ void fold_row_warp(const float* Opart, const float* Mpart, const float* Lpart, const MergeDesc& md,
                                               int r, int lane, const MergeOut& o) {
     const int n = md.nslots;
+    if (n <= FOLD_PART) {
+        float M, den;
+        float4 acc;
+        fold_part(Opart, Mpart, Lpart, md.slot_begin, n, r, lane, M, den, acc);
+        emit_row_warp(M, den, acc, md, r, lane, o);
+        return;
+    }
     const size_t i0 = size_t(md.slot_begin) * QR + r;              // the row in the tile's first slot; + QR per slot
     // reference exponents and row sums of all slots at once: lane l holds slots l, l + 32, ...
     float mm[FOLD_MAX_SLOTS / 32], ll[FOLD_MAX_SLOTS / 32];
@@ -192,6 +202,41 @@ __device__ __forceinline__ void fold_row_warp(const float* Opart, const float* M
         }
     }
     emit_row_warp(M, den, acc, md, r, lane, o);
+}
+
+// This CTA's rows k, k + n, ... (n > FOLD_PART slots, so at most 7 rows) of a tile cut into n runs, by 16 warps: W warps share
+// a row, each folds n / W of its slots (at most FOLD_PART), the row's first warp adds their results up in slot order. With a
+// warp per row, most of the warps had none and the others went through their slots in several round trips:
+// 22 runs a tile, 7,000 cycles from the last count-in to the outputs. `scratch`: 16 x 544 bytes of shared memory; every
+// thread of the CTA calls.
+__device__ __noinline__ void fold_rows_shared(const float* Opart, const float* Mpart, const float* Lpart, const MergeDesc& md, int k, int warp,
+                                                 int lane, uint8_t* scratch, const MergeOut& o) {
+    const int n = md.nslots, W = n <= 32 ? 2 : n <= 64 ? 4 : n <= 128 ? 8 : 16;
+    const int part = warp & (W - 1), per = (n + W - 1) / W, s0 = part * per, cnt = min(per, n - s0);
+    const int r = k + n * (warp / W);
+    float M = -INFINITY, den = 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < QR && cnt > 0) fold_part(Opart, Mpart, Lpart, size_t(md.slot_begin) + s0, cnt, r, lane, M, den, acc);
+    float4* rows = reinterpret_cast<float4*>(scratch);
+    float2* ml = reinterpret_cast<float2*>(scratch + 16 * 512);
+    __syncthreads();                                   // the scratch of a previous tile has been read
+    rows[warp * 32 + lane] = acc;
+    if (lane == 0) ml[warp] = make_float2(M, den);
+    __syncthreads();
+    if (part == 0 && r < QR) {
+        float top = M;
+        for (int q = 1; q < W; ++q) top = fmaxf(top, ml[warp + q].x);
+        float f = exp2f(M - top), d = f * den;
+        float4 a = make_float4(f * acc.x, f * acc.y, f * acc.z, f * acc.w);
+        for (int q = 1; q < W; ++q) {
+            const float2 e = ml[warp + q];
+            const float4 b = rows[(warp + q) * 32 + lane];
+            f = exp2f(e.x - top);
+            d += f * e.y;
+            a.x += f * b.x; a.y += f * b.y; a.z += f * b.z; a.w += f * b.w;
+        }
+        emit_row_warp(top, d, a, md, r, lane, o);
+    }
 }
 
 // A few rows at once for tiles cut into NS <= 4 runs (what a large batch produces: a tile straddling two CTAs): the
