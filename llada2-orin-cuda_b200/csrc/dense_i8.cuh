@@ -141,15 +141,16 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dense_strip_kernel(const DenseP
 }
 
 // ------------------------------------------------------------------------------------------------------------ many tokens
-// CTA = 128 rows x 64 tokens, 8 warps; warp = strip. Everything a group needs comes in through cp.async, DT_STAGES - 1
-// groups ahead: the strips' codes and metas (each warp its own), the 64 tokens' codes, scales and sums (shared; 16-byte
+// CTA = 128 rows x 64 tokens, 8 warps of 32 rows x 32 tokens. Everything a group needs comes in through cp.async, DT_STAGES - 1
+// groups ahead: the strips' codes and metas, the 64 tokens' codes, scales and sums (16-byte
 // chunk c of token n at chunk position c ^ (n % 8): conflict-free fragment loads). Then 32 MMAs, four output tiles in
 // turn so that a chain of four K-steps hides behind the others, and the fold of 32 outputs per thread, two per
 // instruction where fp32 comes in pairs.
 // What bounds it: about 200 issue slots and 32 MMAs (8.8 cycles each on a scheduler) per warp and group of 1,024 outputs -
 // 2048 tokens x 2048 x 2048: 17 us of tensor pipe over 148 SMs - then reading and writing Y (33.6 MB, 5.1 us; brought
 // into L2 while the groups run).
-// Measured, 2048 x 2048, launches in a graph: 2048 tokens 54 us (tcgen05, 128 x 64 tiles: 61), 128 tokens 16.8 us.
+// Measured, 2048 x 2048, launches in a graph: 2048 tokens 49.4 us (a warp per strip and 64 tokens, whose
+// fragment loads took half of the shared-memory bandwidth: 54; the tcgen05 form it replaces: 61), 128 tokens 16.6 us.
 constexpr int DT_TOK = 64, DT_THREADS = 256, DT_STAGES = 4;
 constexpr int DT_CODES = 0, DT_Q = 8 * DN_TILE_BYTES, DT_SX = DT_Q + DT_TOK * 128, DT_SQ = DT_SX + DT_TOK * 4, DT_META = DT_SQ + DT_TOK * 4;
 constexpr int DT_STAGE_BYTES = DT_META + 8 * DN_META_BYTES;        // 17,280
@@ -205,9 +206,11 @@ __global__ void __launch_bounds__(DT_THREADS, 2) dense_tile_kernel(const DensePa
     for (int i = 0; i < DT_STAGES - 1; ++i) fetch(i);
     // the tile's 64 x 512 bytes of Y into L2: wanted when the last group is folded
     if ((tid >> 2) < live) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.Y + size_t(n0 + (tid >> 2)) * p.rows + row0 + 32 * (tid & 3)));
-    f32x2 c[8][2];                             // per n-tile: rows g and g + 8, tokens 8 nt + 2 t and + 1
+    // this warp: strips 2 (warp / 2) and + 1, tokens 32 (warp % 2) .. + 31
+    const int sp = 2 * (warp >> 1), tb = 32 * (warp & 1);
+    f32x2 c[2][4][2];                          // per strip and n-tile: rows g and g + 8, tokens tb + 8 nt + 2 t and + 1
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) c[nt][0] = c[nt][1] = 0ull;
+    for (int k = 0; k < 16; ++k) (&c[0][0][0])[k] = 0ull;
     const f32x2 magic = 0xCB400000CB400000ull; // -1.5 * 2^23 twice
 #pragma unroll 1
     for (int i = 0; i < ktot; ++i) {
@@ -215,62 +218,65 @@ __global__ void __launch_bounds__(DT_THREADS, 2) dense_tile_kernel(const DensePa
         __syncthreads();                       // group i is in for everybody; group i - 1 is done with, its stage can be refilled
         fetch(i + DT_STAGES - 1);
         const uint8_t* st = dt_smem + (i % DT_STAGES) * DT_STAGE_BYTES;
-        const uint8_t* meta = st + DT_META + warp * DN_META_BYTES;
-        const uint32_t sw2 = *reinterpret_cast<const uint32_t*>(meta + 4 * g), z2 = *reinterpret_cast<const uint16_t*>(meta + 32 + 2 * g);
-        uint32_t a[4][4];                      // A fragments of the four K-steps
-        {
-            const uint4 lo = *reinterpret_cast<const uint4*>(st + DT_CODES + warp * DN_TILE_BYTES + 16 * lane);
-            const uint4 hi = *reinterpret_cast<const uint4*>(st + DT_CODES + warp * DN_TILE_BYTES + 512 + 16 * lane);
-            const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}, mk = 0x0F0F0F0Fu;
+        uint32_t w[2][8];                      // the lane's code words of both strips
+        float swa[2], swb[2];
+        int za[2], zb[2];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) { a[j][0] = w[2 * j] & mk; a[j][1] = (w[2 * j] >> 4) & mk; a[j][2] = w[2 * j + 1] & mk; a[j][3] = (w[2 * j + 1] >> 4) & mk; }
+        for (int u = 0; u < 2; ++u) {
+            const uint8_t* meta = st + DT_META + (sp + u) * DN_META_BYTES;
+            const uint32_t sw2 = *reinterpret_cast<const uint32_t*>(meta + 4 * g), z2 = *reinterpret_cast<const uint16_t*>(meta + 32 + 2 * g);
+            swa[u] = __half2float(__ushort_as_half(uint16_t(sw2 & 0xffffu))); swb[u] = __half2float(__ushort_as_half(uint16_t(sw2 >> 16)));
+            za[u] = int(z2 & 0xffu); zb[u] = int(z2 >> 8);
+            *reinterpret_cast<uint4*>(&w[u][0]) = *reinterpret_cast<const uint4*>(st + DT_CODES + (sp + u) * DN_TILE_BYTES + 16 * lane);
+            *reinterpret_cast<uint4*>(&w[u][4]) = *reinterpret_cast<const uint4*>(st + DT_CODES + (sp + u) * DN_TILE_BYTES + 512 + 16 * lane);
         }
-        const float swa = __half2float(__ushort_as_half(uint16_t(sw2 & 0xffffu))), swb = __half2float(__ushort_as_half(uint16_t(sw2 >> 16)));
-        const int za = int(z2 & 0xffu), zb = int(z2 >> 8);
-        const f32x2 swa2 = pack2(__float_as_uint(swa), __float_as_uint(swa)), swb2 = pack2(__float_as_uint(swb), __float_as_uint(swb));
+        const uint32_t mk = 0x0F0F0F0Fu;
+        int acc[2][4][4] = {};
 #pragma unroll
-        for (int nq = 0; nq < 8; nq += 4) {
-            int acc[4][4] = {};
+        for (int h = 0; h < 2; ++h) {
+            uint4 b[4];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint4 b[4];
+            for (int k = 0; k < 4; ++k) b[k] = *reinterpret_cast<const uint4*>(st + DT_Q + (tb + 8 * k + g) * 128 + (((2 * t + h) ^ g) << 4));
 #pragma unroll
-                for (int k = 0; k < 4; ++k) b[k] = *reinterpret_cast<const uint4*>(st + DT_Q + (8 * (nq + k) + g) * 128 + (((2 * t + h) ^ g) << 4));
+            for (int j = 0; j < 2; ++j)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mma_m16n8k32_u8s8(acc[k], a[2 * h][0], a[2 * h][1], a[2 * h][2], a[2 * h][3], b[k].x, b[k].y);
+                for (int u = 0; u < 2; ++u) {
+                    const uint32_t x = w[u][4 * h + 2 * j], y = w[u][4 * h + 2 * j + 1], a0 = x & mk, a1 = (x >> 4) & mk, a2 = y & mk, a3 = (y >> 4) & mk;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mma_m16n8k32_u8s8(acc[k], a[2 * h + 1][0], a[2 * h + 1][1], a[2 * h + 1][2], a[2 * h + 1][3], b[k].z, b[k].w);
-            }
+                    for (int k = 0; k < 4; ++k) mma_m16n8k32_u8s8(acc[u][k], a0, a1, a2, a3, j ? b[k].z : b[k].x, j ? b[k].w : b[k].y);
+                }
+        }
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int nt = nq + k;
-                const f32x2 sx = *reinterpret_cast<const f32x2*>(st + DT_SX + 8 * t + 32 * nt);
-                const int2 sq = *reinterpret_cast<const int2*>(st + DT_SQ + 8 * t + 32 * nt);
-                const f32x2 va = add2(pack2(uint32_t(acc[k][0] + (0x4B400000 - za * sq.x)), uint32_t(acc[k][1] + (0x4B400000 - za * sq.y))), magic);
-                const f32x2 vb = add2(pack2(uint32_t(acc[k][2] + (0x4B400000 - zb * sq.x)), uint32_t(acc[k][3] + (0x4B400000 - zb * sq.y))), magic);
-                c[nt][0] = fma2v(mul2(swa2, sx), va, c[nt][0]);
-                c[nt][1] = fma2v(mul2(swb2, sx), vb, c[nt][1]);
+        for (int k = 0; k < 4; ++k) {
+            const f32x2 sx = *reinterpret_cast<const f32x2*>(st + DT_SX + 4 * tb + 8 * t + 32 * k);
+            const int2 sq = *reinterpret_cast<const int2*>(st + DT_SQ + 4 * tb + 8 * t + 32 * k);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const f32x2 va = add2(pack2(uint32_t(acc[u][k][0] + (0x4B400000 - za[u] * sq.x)), uint32_t(acc[u][k][1] + (0x4B400000 - za[u] * sq.y))), magic);
+                const f32x2 vb = add2(pack2(uint32_t(acc[u][k][2] + (0x4B400000 - zb[u] * sq.x)), uint32_t(acc[u][k][3] + (0x4B400000 - zb[u] * sq.y))), magic);
+                c[u][k][0] = fma2v(mul2(pack2(__float_as_uint(swa[u]), __float_as_uint(swa[u])), sx), va, c[u][k][0]);
+                c[u][k][1] = fma2v(mul2(pack2(__float_as_uint(swb[u]), __float_as_uint(swb[u])), sx), vb, c[u][k][1]);
             }
         }
     }
     cp_async_wait<0>();
     // Y += c: a warp's access covers the 8 rows of four tokens, whole 32-byte sectors
-    float* ybase = p.Y + size_t(n0 + 2 * t) * p.rows + row0 + 16 * warp + g;
+    float* ybase = p.Y + size_t(n0 + tb + 2 * t) * p.rows + row0 + 16 * sp + g;
 #pragma unroll
-    for (int nh = 0; nh < 8; nh += 4) {
+    for (int u = 0; u < 2; ++u) {
         float y[4][4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-                y[k][e] = 8 * (nh + k) + 2 * t + (e & 1) < live ? __ldcg(ybase + size_t(8 * (nh + k) + (e & 1)) * p.rows + 8 * (e >> 1)) : 0.f;
+                y[k][e] = tb + 8 * k + 2 * t + (e & 1) < live ? __ldcg(ybase + size_t(8 * k + (e & 1)) * p.rows + 16 * u + 8 * (e >> 1)) : 0.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-                if (8 * (nh + k) + 2 * t + (e & 1) < live) {
-                    const f32x2 v = c[nh + k][e >> 1];
-                    __stcg(ybase + size_t(8 * (nh + k) + (e & 1)) * p.rows + 8 * (e >> 1), y[k][e] + __uint_as_float(uint32_t(e & 1 ? v >> 32 : v)));
+                if (tb + 8 * k + 2 * t + (e & 1) < live) {
+                    const f32x2 v = c[u][k][e >> 1];
+                    __stcg(ybase + size_t(8 * k + (e & 1)) * p.rows + 16 * u + 8 * (e >> 1), y[k][e] + __uint_as_float(uint32_t(e & 1 ? v >> 32 : v)));
                 }
     }
 }

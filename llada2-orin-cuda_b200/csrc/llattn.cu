@@ -203,7 +203,7 @@ int llattn_qkv_prepare_commit(const float* qkv, const int32_t* pos, const float*
 
 namespace {
 // At most this many tokens go to the strip kernel: it reads the weights once per 32 tokens, with every SM, and a call is
-// 3.8 us at 32 tokens and 6.6 at 64; the tile kernel's 16 row tiles at 65 tokens leave most SMs idle (15.5 us).
+// 3.8 us at 32 tokens and 6.6 at 64; the tile kernel's 16 row tiles at 65 tokens leave most SMs idle (16.3 us).
 constexpr int DENSE_STRIP_MAX_TOKENS = 64;
 }  // namespace
 
