@@ -128,10 +128,25 @@ def _ptr(t) -> Optional[int]:
     return t.data_ptr()
 
 
+_raw_stream = None
+
+
+def _current_stream() -> int:
+    """The current stream's handle. torch.cuda.current_stream() builds a Stream object for it, 3 us of a 9 us call on the
+    host; the handle alone is 0.2 us. (Where this torch has no such function, and before CUDA is up: the long way.)"""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        handle, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+        if handle is None or device is None or not torch.cuda.is_initialized():
+            return torch.cuda.current_stream().cuda_stream
+        _raw_stream = lambda: handle(device())
+    return _raw_stream()
+
+
 def _stream(stream) -> Optional[int]:
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        return _current_stream()
     return getattr(stream, "cuda_stream", stream)
 
 
