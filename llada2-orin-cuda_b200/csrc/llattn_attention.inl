@@ -20,7 +20,7 @@ int grow_workspace(llattn_ctx* c, size_t need) {
 // Splits the flattened unit sequence (every (sequence, query block, kv head) tile contributes nblocks + j records and
 // one fresh block, in that order) into `nctas` contiguous shares of near-equal size. A share boundary inside a tile
 // falls on a multiple of 4 units from the tile's start so that 128-key MMA tiles stay full, and a run is never
-// shorter than `min_units` unless the tile itself is. Every run gets its own partial slot; the slots of one tile are
+// shorter than `shortest` unless the tile itself is. Every run gets its own partial slot; the slots of one tile are
 // consecutive. When there are no more output tiles than CTAs the tiles are cut one by one instead (see build_plan).
 struct HostPlan {
     std::vector<llattn::SeqDesc> seqs;
@@ -35,8 +35,6 @@ struct HostPlan {
 // (query load, first records, the pipeline filling up, the epilogue), and for a run of a split tile the partial result's
 // round trip through the L2 and its share of the folding.
 constexpr int64_t RUN_STARTUP_UNITS = 20, RUN_SPLIT_UNITS = 4;
-// A piece of a tile shorter than this is not worth a run of its own: the cut moves to the tile's end (or start) instead.
-constexpr int SHORTEST_PIECE = 12;
 
 void finish_plan(HostPlan& hp, int nctas) {
     if (hp.cta_first.back() != int32_t(hp.items.size())) hp.cta_first.push_back(int32_t(hp.items.size()));
@@ -56,7 +54,8 @@ void finish_plan(HostPlan& hp, int nctas) {
 }
 
 // Contiguous shares of the flattened unit sequence (see above).
-void cut_contiguous(const llattn_seq* seqs, int nseq, int nctas, int64_t total, int64_t MIN_UNITS, HostPlan& hp) {
+// A piece of a tile shorter than `shortest` gets no run of its own: the cut moves to the tile's end (or start) instead.
+void cut_contiguous(const llattn_seq* seqs, int nseq, int nctas, int64_t total, int64_t MIN_UNITS, int shortest, HostPlan& hp) {
     using namespace llattn;
     // The share of the CTA being filled is re-derived from what is left (units and CTAs), so rounding a cut down to a
     // tile boundary never pushes work into an extra CTA: the plan uses at most `nctas` CTAs.
@@ -86,8 +85,8 @@ void cut_contiguous(const llattn_seq* seqs, int nseq, int nctas, int64_t total, 
                     int take = int(std::min<int64_t>(room, U - done));
                     if (take < U - done) {
                         take = take / TILE_UNITS * TILE_UNITS;                      // keep the cut on a tile boundary
-                        if (U - done - take < SHORTEST_PIECE) take = U - done;      // no short tail for the next CTA
-                        else if (take < SHORTEST_PIECE && int(hp.items.size()) > hp.cta_first.back()) take = 0;   // no short head here
+                        if (U - done - take < shortest) take = U - done;      // no short tail for the next CTA
+                        else if (take < shortest && int(hp.items.size()) > hp.cta_first.back()) take = 0;   // no short head here
                     }
                     if (take == 0) { next_cta(); continue; }
                     const int rec_cnt = std::min(take, nrec - done);
@@ -169,12 +168,25 @@ int build_plan(const llattn_seq* seqs, int nseq, int nctas, HostPlan& hp) {
             hp.used_ctas = alt.used_ctas; hp.max_cta_units = alt.max_cta_units; hp.max_cta_cost = alt.max_cta_cost;
         }
     };
-    cut_contiguous(seqs, nseq, nctas, total, 16, hp);
-    if (total < 16 * int64_t(nctas)) {       // little work: shorter shares on more CTAs may beat several runs per CTA
+    // Contiguous shares, with pieces allowed down to 12, 24, 48 or 96 units: the longer they must be, the fewer runs and
+    // tiles shared between CTAs, and the less equal the shares; the model decides. (64 sequences of 1 K tokens, two and a bit
+    // tiles of 33 units per CTA: 47.6 us with pieces of 12, 35.2 without any; 16 ragged sequences 86 -> 76 us with 24.)
+    cut_contiguous(seqs, nseq, nctas, total, 16, 12, hp);
+    for (int shortest : {24, 48, 96}) {
         HostPlan alt;
-        cut_contiguous(seqs, nseq, nctas, total, TILE_UNITS, alt);
+        cut_contiguous(seqs, nseq, nctas, total, 16, shortest, alt);
         take_if_cheaper(alt);
     }
+    // Little work: shorter shares on more CTAs may beat several runs per CTA. Down to a single 128-key tile where the tiles
+    // outnumber the CTAs (64 x 128 tokens 22.0 -> 17.9 us) or the units do not (one sequence at 1 K tokens 14.6 -> 12.1);
+    // between the two, the runs of about 0.75 sqrt(units) below are within 2 us of it with half the slots to fold.
+    if (total < 16 * int64_t(nctas))
+        for (int shortest : {12, TILE_UNITS}) {
+            if (shortest < 12 && total > nctas && ntile_out <= nctas) break;
+            HostPlan alt;
+            cut_contiguous(seqs, nseq, nctas, total, TILE_UNITS, shortest, alt);
+            take_if_cheaper(alt);
+        }
     if (ntile_out <= nctas) {
         HostPlan alt;
         cut_per_tile(seqs, nseq, nctas, total, alt);

@@ -190,3 +190,16 @@ def test_decoder_commit_policy(api):
     assert api.commit_needs_forward(blk, other) and api.commit_needs_forward(blk, blk[:31])
     with pytest.raises(ValueError):
         api.commit_block(blk, other, None, None, None, 4, 0)        # a forward pass is needed and none was given
+
+
+def test_planner_prefers_whole_tiles_to_short_pieces(api):
+    """Pieces of a tile cost a start-up and a fold each: a batch of short sequences keeps its tiles whole although the shares
+    then differ by a tile; a single short context is cut to one run per 128-key tile."""
+    st, items, cta_first = api.plan_preview([32] * 64, 148)                   # 256 tiles of 33 units
+    assert st.nitems == 256 and st.max_cta_units <= 66
+    st, items, cta_first = api.plan_preview([4] * 64, 148)
+    assert st.nitems == 256 and st.max_cta_units <= 10
+    for nblocks in (4, 20, 32, 36):                                          # fewer units than CTAs
+        st, items, cta_first = api.plan_preview([nblocks], 148)
+        units = items[:, 4] + items[:, 5]
+        assert st.nitems == st.nctas and st.nitems <= 148 and units.max() <= 8
