@@ -23,7 +23,7 @@
 // took 1.2 us for every group at any number of tokens, a chain longer than the group's arithmetic.
 //   dense_strip_kernel  a decode step's few tokens: a CTA takes ONE strip and one warp per 128-group works on it; the
 //                       integers of all groups exist at once, only the multiply-adds run in group order.
-//   dense_tile_kernel   many tokens: 128 rows x 64 tokens per CTA, a warp per strip.
+//   dense_tile_kernel   many tokens: 128 rows x 16, 32 or 64 tokens per CTA.
 #pragma once
 #include <cuda_fp16.h>
 #include "common.cuh"
@@ -141,20 +141,22 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dense_strip_kernel(const DenseP
 }
 
 // ------------------------------------------------------------------------------------------------------------ many tokens
-// CTA = 128 rows x 64 tokens, 8 warps of 32 rows x 32 tokens. Everything a group needs comes in through cp.async, DT_STAGES - 1
-// groups ahead: the strips' codes and metas, the 64 tokens' codes, scales and sums (16-byte
-// chunk c of token n at chunk position c ^ (n % 8): conflict-free fragment loads). Then 32 MMAs, four output tiles in
-// turn so that a chain of four K-steps hides behind the others, and the fold of 32 outputs per thread, two per
+// CTA = 128 rows x TOK (16, 32 or 64) tokens, 8 warps of 32 rows x TOK / 2 tokens. Everything a group needs comes in through cp.async, DT_STAGES - 1
+// groups ahead: the strips' codes and metas, the tokens' codes, scales and sums (16-byte
+// chunk c of token n at chunk position c ^ (n % 8): conflict-free fragment loads). Then two strips' MMAs, all output tiles in
+// turn so that a chain of four K-steps hides behind the others, and the fold of TOK / 2 outputs per thread, two per
 // instruction where fp32 comes in pairs.
 // What bounds it: about 200 issue slots and 32 MMAs (8.8 cycles each on a scheduler) per warp and group of 1,024 outputs -
 // 2048 tokens x 2048 x 2048: 17 us of tensor pipe over 148 SMs - then reading and writing Y (33.6 MB, 5.1 us; brought
 // into L2 while the groups run).
 // Measured, 2048 x 2048, launches in a graph: 2048 tokens 49.4 us (a warp per strip and 64 tokens, whose
-// fragment loads took half of the shared-memory bandwidth: 54; the tcgen05 form it replaces: 61), 128 tokens 16.6 us.
-constexpr int DT_TOK = 64, DT_THREADS = 256, DT_STAGES = 4;
-constexpr int DT_CODES = 0, DT_Q = 8 * DN_TILE_BYTES, DT_SX = DT_Q + DT_TOK * 128, DT_SQ = DT_SX + DT_TOK * 4, DT_META = DT_SQ + DT_TOK * 4;
-constexpr int DT_STAGE_BYTES = DT_META + 8 * DN_META_BYTES;        // 17,280
-constexpr int DT_SMEM_BYTES = DT_STAGES * DT_STAGE_BYTES;
+// fragment loads took half of the shared-memory bandwidth: 54; the tcgen05 form it replaces: 61), 128 tokens 8.6 us (16-token
+// tiles; 16.6 with 64).
+constexpr int DT_THREADS = 256, DT_STAGES = 4;
+template <int TOK> struct DenseTile {                              // shared-memory layout of a stage: codes, q, scales, sums, metas
+    static constexpr int Q = 8 * DN_TILE_BYTES, SX = Q + TOK * 128, SQ = SX + TOK * 4, META = SQ + TOK * 4, STAGE = META + 8 * DN_META_BYTES;
+    static constexpr int SMEM = DT_STAGES * STAGE, NT = TOK / 16;  // NT: 8-token output tiles per warp and strip
+};
 
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pack2(uint32_t a, uint32_t b) { f32x2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(a), "r"(b)); return d; }
@@ -172,84 +174,86 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, bool li
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int kPending> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
 
-__global__ void __launch_bounds__(DT_THREADS, 2) dense_tile_kernel(const DenseParams p) {
+template <int TOK>
+__global__ void __launch_bounds__(DT_THREADS, TOK == 64 ? 2 : 3) dense_tile_kernel(const DenseParams p) {
+    using T = DenseTile<TOK>;
     extern __shared__ __align__(128) uint8_t dt_smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int row0 = blockIdx.x * DN_ROWS, n0 = blockIdx.y * DT_TOK, live = min(DT_TOK, p.ntokens - n0);
+    const int row0 = blockIdx.x * DN_ROWS, n0 = blockIdx.y * TOK, live = min(TOK, p.ntokens - n0);
     const int ktot = p.K / DN_GROUP;
     const uint8_t* codes = p.W + size_t((row0 >> 4) + warp) * ktot * (DN_TILE_BYTES + DN_META_BYTES);
     const uint8_t* metas = codes + size_t(ktot) * DN_TILE_BYTES;
     const uint32_t sm0 = ptx::smem_u32(dt_smem);
-    // this thread's part of a stage: its lane's code words, one of the strip's three meta chunks, two chunks of tokens tid / 8 and tid / 8 + 32, and one scale or sum
+    // this thread's part of a stage: its lane's code words, one of the strip's three meta chunks, chunk tid % 8 of tokens
+    // tid / 8 and tid / 8 + 32, and one scale or sum
     const int cn = tid >> 3, cc = tid & 7;
-    const int8_t* src0 = p.q + size_t(n0 + min(cn, live - 1)) * p.K + 16 * cc;
-    const int8_t* src1 = p.q + size_t(n0 + min(cn + 32, live - 1)) * p.K + 16 * cc;
-    const uint32_t dst0 = sm0 + DT_Q + cn * 128 + ((cc ^ (cn & 7)) << 4);
-    const bool live0 = cn < live, live1 = cn + 32 < live;
-    const int sn = tid & 63;
+    const int8_t* src = p.q + size_t(n0 + min(cn, live - 1)) * p.K + 16 * cc;
+    const int8_t* src32 = p.q + size_t(n0 + min(cn + 32, live - 1)) * p.K + 16 * cc;
+    const uint32_t dst0 = sm0 + T::Q + cn * 128 + ((cc ^ (cn & 7)) << 4);
+    const int sn = tid & (TOK - 1);
     const size_t sat = size_t(n0 + min(sn, live - 1)) * ktot;
-    const void* ssrc = tid < 64 ? static_cast<const void*>(p.s + sat) : static_cast<const void*>(p.sum + sat);
-    const uint32_t sdst = sm0 + DT_SX + 4 * (tid & 127);
+    const void* ssrc = tid < TOK ? static_cast<const void*>(p.s + sat) : static_cast<const void*>(p.sum + sat);
+    const uint32_t sdst = sm0 + T::SX + 4 * (tid & (2 * TOK - 1));
     auto fetch = [&](int i) {                  // one commit per call, so groups count uniformly
         if (i < ktot) {
-            const uint32_t st = uint32_t(i % DT_STAGES) * DT_STAGE_BYTES;
-            const uint32_t mine = sm0 + DT_CODES + warp * DN_TILE_BYTES + 16 * lane + st;
+            const uint32_t st = uint32_t(i % DT_STAGES) * T::STAGE;
+            const uint32_t mine = sm0 + warp * DN_TILE_BYTES + 16 * lane + st;
             cp_async16(mine, codes + size_t(i) * DN_TILE_BYTES + 16 * lane, true);
             cp_async16(mine + 512, codes + size_t(i) * DN_TILE_BYTES + 512 + 16 * lane, true);
-            if (lane < 3) cp_async16(sm0 + DT_META + warp * DN_META_BYTES + 16 * lane + st, metas + size_t(i) * DN_META_BYTES + 16 * lane, true);
-            cp_async16(dst0 + st, src0 + size_t(i) * DN_GROUP, live0);
-            cp_async16(dst0 + st + 32 * 128, src1 + size_t(i) * DN_GROUP, live1);
-            if (tid < 128) cp_async4(sdst + st, static_cast<const uint8_t*>(ssrc) + 4 * size_t(i), sn < live);
+            if (lane < 3) cp_async16(sm0 + T::META + warp * DN_META_BYTES + 16 * lane + st, metas + size_t(i) * DN_META_BYTES + 16 * lane, true);
+            if (TOK >= 32 || cn < TOK) cp_async16(dst0 + st, src + size_t(i) * DN_GROUP, cn < live);
+            if (TOK == 64) cp_async16(dst0 + st + 32 * 128, src32 + size_t(i) * DN_GROUP, cn + 32 < live);
+            if (tid < 2 * TOK) cp_async4(sdst + st, static_cast<const uint8_t*>(ssrc) + 4 * size_t(i), sn < live);
         }
         cp_async_commit();
     };
     for (int i = 0; i < DT_STAGES - 1; ++i) fetch(i);
-    // the tile's 64 x 512 bytes of Y into L2: wanted when the last group is folded
+    // the tile's TOK x 512 bytes of Y into L2: wanted when the last group is folded
     if ((tid >> 2) < live) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.Y + size_t(n0 + (tid >> 2)) * p.rows + row0 + 32 * (tid & 3)));
-    // this warp: strips 2 (warp / 2) and + 1, tokens 32 (warp % 2) .. + 31
-    const int sp = 2 * (warp >> 1), tb = 32 * (warp & 1);
-    f32x2 c[2][4][2];                          // per strip and n-tile: rows g and g + 8, tokens tb + 8 nt + 2 t and + 1
+    // this warp: strips 2 (warp / 2) and + 1, tokens TOK / 2 (warp % 2) .. + TOK / 2 - 1
+    const int sp = 2 * (warp >> 1), tb = TOK / 2 * (warp & 1);
+    f32x2 c[2][T::NT][2];                          // per strip and n-tile: rows g and g + 8, tokens tb + 8 nt + 2 t and + 1
 #pragma unroll
-    for (int k = 0; k < 16; ++k) (&c[0][0][0])[k] = 0ull;
+    for (int k = 0; k < 4 * T::NT; ++k) (&c[0][0][0])[k] = 0ull;
     const f32x2 magic = 0xCB400000CB400000ull; // -1.5 * 2^23 twice
 #pragma unroll 1
     for (int i = 0; i < ktot; ++i) {
         cp_async_wait<DT_STAGES - 2>();
         __syncthreads();                       // group i is in for everybody; group i - 1 is done with, its stage can be refilled
         fetch(i + DT_STAGES - 1);
-        const uint8_t* st = dt_smem + (i % DT_STAGES) * DT_STAGE_BYTES;
+        const uint8_t* st = dt_smem + (i % DT_STAGES) * T::STAGE;
         uint32_t w[2][8];                      // the lane's code words of both strips
         float swa[2], swb[2];
         int za[2], zb[2];
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-            const uint8_t* meta = st + DT_META + (sp + u) * DN_META_BYTES;
+            const uint8_t* meta = st + T::META + (sp + u) * DN_META_BYTES;
             const uint32_t sw2 = *reinterpret_cast<const uint32_t*>(meta + 4 * g), z2 = *reinterpret_cast<const uint16_t*>(meta + 32 + 2 * g);
             swa[u] = __half2float(__ushort_as_half(uint16_t(sw2 & 0xffffu))); swb[u] = __half2float(__ushort_as_half(uint16_t(sw2 >> 16)));
             za[u] = int(z2 & 0xffu); zb[u] = int(z2 >> 8);
-            *reinterpret_cast<uint4*>(&w[u][0]) = *reinterpret_cast<const uint4*>(st + DT_CODES + (sp + u) * DN_TILE_BYTES + 16 * lane);
-            *reinterpret_cast<uint4*>(&w[u][4]) = *reinterpret_cast<const uint4*>(st + DT_CODES + (sp + u) * DN_TILE_BYTES + 512 + 16 * lane);
+            *reinterpret_cast<uint4*>(&w[u][0]) = *reinterpret_cast<const uint4*>(st + (sp + u) * DN_TILE_BYTES + 16 * lane);
+            *reinterpret_cast<uint4*>(&w[u][4]) = *reinterpret_cast<const uint4*>(st + (sp + u) * DN_TILE_BYTES + 512 + 16 * lane);
         }
         const uint32_t mk = 0x0F0F0F0Fu;
-        int acc[2][4][4] = {};
+        int acc[2][T::NT][4] = {};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            uint4 b[4];
+            uint4 b[T::NT];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) b[k] = *reinterpret_cast<const uint4*>(st + DT_Q + (tb + 8 * k + g) * 128 + (((2 * t + h) ^ g) << 4));
+            for (int k = 0; k < T::NT; ++k) b[k] = *reinterpret_cast<const uint4*>(st + T::Q + (tb + 8 * k + g) * 128 + (((2 * t + h) ^ g) << 4));
 #pragma unroll
             for (int j = 0; j < 2; ++j)
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     const uint32_t x = w[u][4 * h + 2 * j], y = w[u][4 * h + 2 * j + 1], a0 = x & mk, a1 = (x >> 4) & mk, a2 = y & mk, a3 = (y >> 4) & mk;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) mma_m16n8k32_u8s8(acc[u][k], a0, a1, a2, a3, j ? b[k].z : b[k].x, j ? b[k].w : b[k].y);
+                    for (int k = 0; k < T::NT; ++k) mma_m16n8k32_u8s8(acc[u][k], a0, a1, a2, a3, j ? b[k].z : b[k].x, j ? b[k].w : b[k].y);
                 }
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const f32x2 sx = *reinterpret_cast<const f32x2*>(st + DT_SX + 4 * tb + 8 * t + 32 * k);
-            const int2 sq = *reinterpret_cast<const int2*>(st + DT_SQ + 4 * tb + 8 * t + 32 * k);
+        for (int k = 0; k < T::NT; ++k) {
+            const f32x2 sx = *reinterpret_cast<const f32x2*>(st + T::SX + 4 * tb + 8 * t + 32 * k);
+            const int2 sq = *reinterpret_cast<const int2*>(st + T::SQ + 4 * tb + 8 * t + 32 * k);
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const f32x2 va = add2(pack2(uint32_t(acc[u][k][0] + (0x4B400000 - za[u] * sq.x)), uint32_t(acc[u][k][1] + (0x4B400000 - za[u] * sq.y))), magic);
@@ -264,14 +268,14 @@ __global__ void __launch_bounds__(DT_THREADS, 2) dense_tile_kernel(const DensePa
     float* ybase = p.Y + size_t(n0 + tb + 2 * t) * p.rows + row0 + 16 * sp + g;
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-        float y[4][4];
+        float y[T::NT][4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < T::NT; ++k)
 #pragma unroll
             for (int e = 0; e < 4; ++e)
                 y[k][e] = tb + 8 * k + 2 * t + (e & 1) < live ? __ldcg(ybase + size_t(8 * k + (e & 1)) * p.rows + 16 * u + 8 * (e >> 1)) : 0.f;
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < T::NT; ++k)
 #pragma unroll
             for (int e = 0; e < 4; ++e)
                 if (tb + 8 * k + 2 * t + (e & 1) < live) {

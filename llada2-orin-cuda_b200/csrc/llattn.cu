@@ -203,7 +203,7 @@ int llattn_qkv_prepare_commit(const float* qkv, const int32_t* pos, const float*
 
 namespace {
 // At most this many tokens go to the strip kernel: it reads the weights once per 32 tokens, with every SM, and a call is
-// 3.8 us at 32 tokens and 6.6 at 64; the tile kernel's 16 row tiles at 65 tokens leave most SMs idle (16.3 us).
+// 3.8 us at 32 tokens and 6.6 at 64; the tile kernel's 16 row tiles at 65 tokens still leave most SMs idle at that size (8.1 us).
 constexpr int DENSE_STRIP_MAX_TOKENS = 64;
 }  // namespace
 
@@ -222,14 +222,26 @@ int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int3
     if (dev >= 0 && dev < 64)
         std::call_once(once[dev], [] {
             cudaFuncSetAttribute(llattn::dense_strip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DS_SMEM_BYTES);
-            cudaFuncSetAttribute(llattn::dense_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DT_SMEM_BYTES);
+            cudaFuncSetAttribute(llattn::dense_tile_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseTile<16>::SMEM);
+            cudaFuncSetAttribute(llattn::dense_tile_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseTile<32>::SMEM);
+            cudaFuncSetAttribute(llattn::dense_tile_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseTile<64>::SMEM);
         });
     if (ntokens <= DENSE_STRIP_MAX_TOKENS) {
         const dim3 grid(rows / 16, (ntokens + llattn::DS_TOK - 1) / llattn::DS_TOK);
         llattn::dense_strip_kernel<<<grid, llattn::DS_THREADS, llattn::DS_SMEM_BYTES, as_stream(stream)>>>(p);
     } else {
-        const dim3 grid(rows / llattn::DN_ROWS, (ntokens + llattn::DT_TOK - 1) / llattn::DT_TOK);
-        llattn::dense_tile_kernel<<<grid, llattn::DT_THREADS, llattn::DT_SMEM_BYTES, as_stream(stream)>>>(p);
+        // The largest tile is the cheapest per token, as long as the tiles fill the chip: with smaller ones while they do not.
+        // 2048 x 2048, in a graph: 65 .. 144 tokens 16.2 .. 16.6 us with 64 tokens a tile, 8.1 .. 8.7 with 16; 160 .. 288 tokens 16.7 and
+        // 11.3 .. 11.8 (32); at 512 tokens 16.8 (64) and 17.3 (32), at 1024 26.4 and 30.7.
+        int sms = 0;
+        CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        const long long row_tiles = rows / llattn::DN_ROWS;
+        auto launch = [&](auto* kernel, int tok, int smem) {
+            kernel<<<dim3(rows / llattn::DN_ROWS, (ntokens + tok - 1) / tok), llattn::DT_THREADS, smem, as_stream(stream)>>>(p);
+        };
+        if (row_tiles * ((ntokens + 15) / 16) <= sms) launch(llattn::dense_tile_kernel<16>, 16, llattn::DenseTile<16>::SMEM);
+        else if (row_tiles * ((ntokens + 31) / 32) <= sms) launch(llattn::dense_tile_kernel<32>, 32, llattn::DenseTile<32>::SMEM);
+        else launch(llattn::dense_tile_kernel<64>, 64, llattn::DenseTile<64>::SMEM);
     }
     CU(cudaGetLastError());
     return LLATTN_OK;

@@ -76,7 +76,8 @@ def test_dense_bit_exact_vs_oracle(api, orc, pkg, ntokens, rows, K):
 @pytest.mark.parametrize("ntokens,rows,K,odd", [
     (7, 128, 128, False), (8, 256, 2176, False), (31, 128, 2048, True), (33, 128, 4224, False), (63, 384, 256, False),   # a strip's tokens, one group, more groups than warps
     (65, 128, 128, False), (97, 128, 4224, True), (127, 256, 384, True), (129, 128, 2176, False), (257, 2048, 256, False),
-    (1000, 384, 512, True), (2500, 1024, 128, False)])
+    (1000, 384, 512, True), (2500, 1024, 128, False),
+    (66, 2048, 512, True), (128, 2048, 128, False), (143, 2048, 2176, True), (144, 2048, 256, False), (145, 2048, 128, False), (288, 2048, 256, True), (290, 2048, 128, False)])     # where the tile size changes
 def test_dense_tile_edges(api, orc, pkg, ntokens, rows, K, odd):
     """Token counts around the tile sizes of both kernels, one to more groups than pipeline stages or warps. `odd`: zero
     points over the whole byte and sums that are not the sums of the codes, which the formula allows."""
