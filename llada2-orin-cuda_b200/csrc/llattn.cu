@@ -9,7 +9,9 @@
 #include <cstdlib>
 #include <cmath>
 #include <mutex>
+#include <functional>
 #include <new>
+#include <queue>
 #include <vector>
 
 #include "llattn.h"

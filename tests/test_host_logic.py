@@ -203,3 +203,14 @@ def test_planner_prefers_whole_tiles_to_short_pieces(api):
         st, items, cta_first = api.plan_preview([nblocks], 148)
         units = items[:, 4] + items[:, 5]
         assert st.nitems == st.nctas and st.nitems <= 148 and units.max() <= 8
+
+
+def test_planner_puts_unequal_whole_tiles_on_the_least_loaded_cta(api):
+    """Four first prompt passes of 13 blocks: 208 tiles of 1 .. 13 units on 148 CTAs. The longest tiles get a CTA each, short ones
+    share; a tile stays with one CTA, and with plenty of work the shares may not differ more than the cuts' would."""
+    st, items, cta_first = api.plan_preview([0] * 4, 148, [13] * 4)
+    assert st.nitems == 208 and st.nctas == 148 and st.max_cta_units <= 14
+    assert sorted(map(tuple, items[:, [0, 1, 2]].tolist())) == [(s, j, h) for s in range(4) for j in range(13) for h in range(4)]
+    assert np.all(items[:, 4] == items[:, 1]) and np.all(items[:, 5] == 1)
+    st, items, cta_first = api.plan_preview([3, 0, 17, 250, 1, 64], 7)        # whole tiles would leave one CTA with 251 of 1364 units
+    assert st.max_cta_units <= 1.02 * st.total_units / 7 + 12
