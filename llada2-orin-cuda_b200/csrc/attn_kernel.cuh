@@ -23,7 +23,7 @@
 // reference maximum (log2 units) and row sum go to a partial slot in the format of the reference's Opart/Mpart/Lpart
 // (engine/attn.cu:291-305) and it counts itself in at the tile's arrival counter. When a CTA has no runs left it returns
 // to its split tiles: it waits (bounded) until every run of the tile is counted, then folds its share of the tile's
-// rows (run k of n takes rows k, k + n, ...; all sixteen warps, a warp per row; merge_kernel.cuh) and writes their
+// rows (run k of n takes rows k, k + n, ...; all sixteen warps, one or several per row; merge_kernel.cuh) and writes their
 // outputs, so a tile cut into n runs is folded by n SMs at once. A CTA only ever waits after all of its own runs are
 // out, so the waits cannot form a cycle; they need every CTA of the launch to be on an SM, which a grid of at most one
 // CTA per SM launched cooperatively guarantees. With the reference-shaped operator pair the caller's attn_combine
@@ -1048,7 +1048,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
 
     // ---- split tiles. Every run of this CTA is stored and counted by now, so nothing this CTA waits for depends on
     // this CTA: for each of its runs that is part of a split tile, wait (bounded) until all of the tile's runs are
-    // counted in, then all sixteen warps finish this run's share of the rows, a warp per row. The last warp to leave a
+    // counted in, then all sixteen warps finish this run's share of the rows. The last warp to leave a
     // tile puts both of its counters back to zero for the next launch. Every thread of the CTA walks this loop the same
     // way (same runs, same outcome), so the CTA barrier inside it is reached by all.
     if (p.fused) {

@@ -215,8 +215,9 @@ int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int3
     if (ntokens < 0 || ntokens > 1 << 22) return fail(LLATTN_EINVAL, "dense_w4a8: ntokens = %d", ntokens);
     if (rows <= 0 || rows % llattn::DN_ROWS || K <= 0 || K % llattn::DN_GROUP || K > 1 << 20 || rows > 1 << 20)
         return fail(LLATTN_EINVAL, "dense_w4a8: rows = %d, K = %d (both multiples of 128)", rows, K);
-    if (!aligned16(W) || !aligned16(q)) return fail(LLATTN_EINVAL, "dense_w4a8: W and q must be 16-byte aligned");
+    (void)err_word;
     if (ntokens == 0) return LLATTN_OK;
+    if (!aligned16(W) || !aligned16(q)) return fail(LLATTN_EINVAL, "dense_w4a8: W and q must be 16-byte aligned");
     const llattn::DenseParams p{static_cast<const uint8_t*>(W), q, s, sum, Y, ntokens, rows, K};
     static std::once_flag once[64];
     int dev = 0;

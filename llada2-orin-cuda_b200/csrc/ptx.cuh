@@ -23,13 +23,6 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
     return t;
 }
 
-__device__ __forceinline__ bool elect_one() {
-    uint32_t pred;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(pred));
-    return pred != 0;
-}
-
 // ---------------------------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -161,42 +154,16 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
 }
 
 // ---------------------------------------------------------------------------------------------- tcgen05 MMA
-// Shared-memory matrix descriptor, no swizzle ("interleaved" canonical layout): the operand is made of 8x16-byte
-// core matrices, each stored as 128 contiguous bytes.
-//   K-major operand (rows = M or N index, 16 bytes = 8 consecutive K elements):
-//       lbo = byte distance between the two core matrices adjacent in K, sbo = between 8-row groups.
-//   MN-major operand (16 bytes = 8 consecutive M/N elements, the 8 rows of a core matrix are 8 K indices):
-//       lbo = byte distance between core matrices adjacent in K, sbo = between groups of 8 in M/N.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-    return uint64_t((saddr & 0x3ffffu) >> 4) | (uint64_t(lbo_bytes >> 4) << 16) | (uint64_t(sbo_bytes >> 4) << 32) |
-           (uint64_t(1) << 46);
-}
-// The same with the 128-byte swizzle: rows of 128 bytes, the 16-byte chunk c of row r stored at chunk position
-// c ^ (r % 8), tile base 1024-byte aligned. K-major operand (row = M/N index, 64 fp16 of K per row): sbo = 1024 (next
-// 8 rows), lbo unused, a K-step of 16 elements advances the start address by 32 bytes. MN-major operand (row = K index,
-// 64 fp16 of N per row): sbo = 1024 (next 8 K rows), lbo = distance between 64-element column blocks of N, a K-step
-// advances by 16 rows. Both conventions were checked against a CPU product on the device.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-    return smem_desc(saddr, lbo_bytes, sbo_bytes) | (uint64_t(2) << 61);
-}
+// Shared-memory operands are described by 64-bit descriptors: start address, LBO and SBO in 16-byte units, a version bit and
+// the swizzle mode (desc_lo, desc_hi below; 2 << 61 = 128-byte swizzle: rows of 128 bytes, the 16-byte chunk c of row r
+// stored at chunk position c ^ (r % 8), tile base 1024-byte aligned). K-major operand (row = M/N index, 64 fp16 of K per
+// row): SBO = 1024 (next 8 rows), LBO unused, a K-step of 16 elements advances the start address by 32 bytes. MN-major
+// operand (row = K index, 64 fp16 of N per row): SBO = 1024 (next 8 K rows), LBO = distance between 64-element column blocks
+// of N, a K-step advances by 16 rows. Both conventions were checked against a CPU product on the device.
 // Instruction descriptor for kind::f16 with fp16 A and B, fp32 accumulate, M x N tile, no negate, dense.
 __host__ __device__ constexpr uint32_t idesc_f16(int M, int N, bool a_mn_major, bool b_mn_major) {
     return (1u << 4) | (uint32_t(a_mn_major) << 15) | (uint32_t(b_mn_major) << 16) | (uint32_t(N >> 3) << 17) |
            (uint32_t(M >> 4) << 24);
-}
-// D[tmem] (+)= A[smem] * B[smem]; issued by one thread.
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]; A is K-major fp16 pairs packed in 32-bit cells, row i in lane i.
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
-        :: "r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // Descriptor words for the fused issue helpers below: the low word carries the start address and LBO, the high word
 // SBO and the version bit; stepping an operand through shared memory is an add on the low word (16-byte units).
@@ -289,10 +256,5 @@ __device__ __forceinline__ void mma_commit_warp(uint32_t bar) {
     asm volatile("{\n\t.reg .pred pe;\n\telect.sync _|pe, 0xffffffff;\n\t"
                  "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(bar) : "memory");
 }
-// Arrive once on `bar` when every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
 }  // namespace ptx
 }  // namespace llattn
