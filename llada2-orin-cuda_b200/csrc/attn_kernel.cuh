@@ -1106,6 +1106,9 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
 
 template <bool PRECISE>
 __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_tile_kernel(const __grid_constant__ KParams p) {
+    // reference-grid mode: the folding launch behind this one may take its place on the SMs this one leaves idle, and wait
+    // there (not in list mode: what follows there may be another cooperative launch, which needs the whole chip)
+    if (!PRECISE && !p.items) ptx::launch_dependents();
     attn_tile_body<PRECISE>(p, blockIdx.x);
 }
 

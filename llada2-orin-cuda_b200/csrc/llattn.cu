@@ -89,6 +89,20 @@ struct DeviceGuard {
     ~DeviceGuard() { if (prev >= 0) cudaSetDevice(prev); }
 };
 
+// A launch that may start before the kernel ahead of it in the stream has run out; its kernel waits with griddepcontrol.wait.
+// Behind a kernel that does not allow it, it is an ordinary launch.
+template <typename... KArgs>
+cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, int threads, cudaStream_t stream, KArgs... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 int ensure_kernel_attrs() {
     static std::mutex mu;
     static bool done[64] = {};
@@ -334,8 +348,9 @@ extern "C" int llattn_attention_static(const void* Q, const void* Kf, const void
     attn_tile_kernel<false><<<NKV * nchunks * nb, ATTN_THREADS, ATTN_SMEM_BYTES, as_stream(stream)>>>(p);
     CU(cudaGetLastError());
     MergeOut o{static_cast<half*>(O16), O32, LSE, q8, s8, sum8};
-    combine_ref_kernel<<<dim3(NKV, QR / MERGE_ROWS, nb), MERGE_THREADS, 0, as_stream(stream)>>>(Opart, Mpart, Lpart, nchunks, nblocks, bpc, o);
-    CU(cudaGetLastError());
+    CU(launch_dependent(
+        combine_ref_kernel, dim3(NKV, QR / MERGE_ROWS, nb), MERGE_THREADS, as_stream(stream),
+        static_cast<const float*>(Opart), static_cast<const float*>(Mpart), static_cast<const float*>(Lpart), nchunks, nblocks, bpc, o));
     return LLATTN_OK;
 }
 

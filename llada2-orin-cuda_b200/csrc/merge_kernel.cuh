@@ -14,6 +14,7 @@
 #pragma once
 #include <cuda_fp16.h>
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace llattn {
 
@@ -282,6 +283,7 @@ __device__ __forceinline__ void fold_rows_few(const float* Opart, const float* M
 __global__ void __launch_bounds__(MERGE_THREADS)
 combine_ref_kernel(const float* __restrict__ Opart, const float* __restrict__ Mpart, const float* __restrict__ Lpart,
                    int nchunks, int nblocks, int bpc, MergeOut o) {
+    ptx::grid_dependency_wait();               // nothing is read or written before the kernel ahead has completed
     const int kvh = blockIdx.x, jb = blockIdx.z, nbl = nblocks + jb;
     const MergeDesc md{jb, kvh, (jb * NKV + kvh) * nchunks, nbl <= 0 ? 1 : (nbl + bpc - 1) / bpc};
     fold_row_warp(Opart, Mpart, Lpart, md, int(blockIdx.y) * MERGE_ROWS + int(threadIdx.x >> 5), int(threadIdx.x & 31), o);

@@ -68,6 +68,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return mbar_wait_limit(bar, parity, abort_flag, WAIT_LIMIT_NS);
 }
 
+// Programmatic dependent launch. A kernel launched with the attribute may start once every CTA of the kernel before it in the
+// stream has said launch_dependents (or is gone); wait returns when that kernel has completed and its writes are visible.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Generic-proxy writes to shared memory (st.shared by threads) must be made visible to the async proxy (the
 // tensor core reading operands through descriptors) before the consumer is signalled.
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
