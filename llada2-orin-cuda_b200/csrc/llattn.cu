@@ -8,10 +8,9 @@
 #include <cstring>
 #include <cstdlib>
 #include <cmath>
+#include <cstdint>
 #include <mutex>
-#include <functional>
 #include <new>
-#include <queue>
 #include <vector>
 
 #include "llattn.h"

@@ -17,173 +17,284 @@ int grow_workspace(llattn_ctx* c, size_t need) {
     return LLATTN_OK;
 }
 
-// Splits the flattened unit sequence (every (sequence, query block, kv head) tile contributes nblocks + j records and
-// one fresh block, in that order) into `nctas` contiguous shares of near-equal size. A share boundary inside a tile
-// falls on a multiple of 4 units from the tile's start so that 128-key MMA tiles stay full, and a run is never
-// shorter than `shortest` unless the tile itself is. Every run gets its own partial slot; the slots of one tile are
-// consecutive. When there are no more output tiles than CTAs the tiles are cut one by one instead (see build_plan).
 struct HostPlan {
     std::vector<llattn::SeqDesc> seqs;
     std::vector<llattn::WorkItem> items;
     std::vector<int32_t> cta_first;
     std::vector<llattn::MergeDesc> merge;
-    int64_t total_units = 0, max_cta_units = 0, max_cta_cost = 0;
+    int64_t total_units = 0, max_cta_units = 0;
     int nq_total = 0, used_ctas = 0;
 };
 
 // What a CTA's list costs, in the time of a unit (about a third of a microsecond): its units, a start-up charge per run
 // (query load, first records, the pipeline filling up, the epilogue), and for a run of a split tile the partial result's
-// round trip through the L2 and its share of the folding.
+// round trip through the L2 and its share of the folding. A plan costs what its most expensive CTA does.
 constexpr int64_t RUN_STARTUP_UNITS = 20, RUN_SPLIT_UNITS = 4;
+
+// A plan is made of output tiles: tile 4 g + h is kv head h of group g, a query block of a sequence, and has nblocks + j
+// records and one fresh block, in that order: `units`.
+struct TileGroup {
+    int32_t seq, qblk, units;
+};
 
 void finish_plan(HostPlan& hp, int nctas) {
     if (hp.cta_first.back() != int32_t(hp.items.size())) hp.cta_first.push_back(int32_t(hp.items.size()));
     hp.used_ctas = int(hp.cta_first.size()) - 1;
-    // the launch always has `nctas` CTAs (a captured graph keeps its grid when the plan is updated): the rest get no items
-    while (int(hp.cta_first.size()) < nctas + 1) hp.cta_first.push_back(int32_t(hp.items.size()));
-    hp.max_cta_units = hp.max_cta_cost = 0;
+    hp.max_cta_units = 0;
     for (size_t c = 0; c + 1 < hp.cta_first.size(); ++c) {
         int64_t u = 0;
         for (int i = hp.cta_first[c]; i < hp.cta_first[c + 1]; ++i) u += hp.items[i].rec_count + hp.items[i].fresh;
         hp.max_cta_units = std::max(hp.max_cta_units, u);
-        int64_t cost = u;
-        for (int i = hp.cta_first[c]; i < hp.cta_first[c + 1]; ++i)
-            cost += RUN_STARTUP_UNITS + (hp.merge[hp.items[i].tile].nslots > 1 ? RUN_SPLIT_UNITS : 0);
-        hp.max_cta_cost = std::max(hp.max_cta_cost, cost);
     }
+    // the launch always has `nctas` CTAs (a captured graph keeps its grid when the plan is updated): the rest get no items
+    while (int(hp.cta_first.size()) < nctas + 1) hp.cta_first.push_back(int32_t(hp.items.size()));
 }
 
-// Contiguous shares of the flattened unit sequence (see above).
-// A piece of a tile shorter than `shortest` gets no run of its own: the cut moves to the tile's end (or start) instead.
-void cut_contiguous(const llattn_seq* seqs, int nseq, int nctas, int64_t total, int64_t MIN_UNITS, int shortest, HostPlan& hp) {
+// Splits the flattened unit sequence into `nctas` contiguous shares of near-equal size. A share boundary inside a tile
+// falls on a multiple of 4 units from the tile's start so that 128-key MMA tiles stay full, and a piece of a tile shorter
+// than `shortest` gets no run of its own: the cut moves to the tile's end (or start) instead. Every run gets its own partial
+// slot; the slots of one tile are consecutive.
+// Visit: run(group, head, first unit, units, units of the tile) for every run in order, or whole(group, units) for the four whole
+// tiles of a group at once, false stops the walk; next_cta().
+// Returns the largest `shortest` for which the walk would have been the same.
+template <typename Visit>
+int walk_contiguous(const std::vector<TileGroup>& groups, int nctas, int64_t total, int64_t min_units, int shortest, Visit& v) {
     using namespace llattn;
     // The share of the CTA being filled is re-derived from what is left (units and CTAs), so rounding a cut down to a
     // tile boundary never pushes work into an extra CTA: the plan uses at most `nctas` CTAs.
     int64_t left = total;
-    int ctas_left = nctas;
+    int ctas_left = nctas, same_up_to = INT32_MAX;
     auto new_share = [&]() -> int64_t {
-        int64_t sh = ctas_left > 1 ? (left + ctas_left - 1) / ctas_left : left;
-        sh = std::max<int64_t>(sh, MIN_UNITS);
+        int64_t sh = left;
+        if (ctas_left > 1) {                       // a division per CTA is half of a walk's time: the short one where it will do
+            sh += ctas_left - 1;
+            sh = sh >> 32 ? sh / ctas_left : int64_t(uint32_t(sh) / uint32_t(ctas_left));
+        }
+        sh = std::max<int64_t>(sh, min_units);
         return (sh + TILE_UNITS - 1) / TILE_UNITS * TILE_UNITS;
     };
-    hp.cta_first.assign(1, 0);
     int64_t room = new_share();      // units the current CTA can still take
-    int slot = 0;
+    bool busy = false;               // it has a run already
     auto next_cta = [&]() {
-        hp.cta_first.push_back(int32_t(hp.items.size()));
+        v.next_cta();
+        busy = false;
         if (ctas_left > 1) --ctas_left;
         room = new_share();
     };
-    for (int s = 0; s < nseq; ++s)
-        for (int j = 0; j < seqs[s].nq; ++j)
-            for (int h = 0; h < NKV; ++h) {
-                const int nrec = seqs[s].nblocks + j;
-                const int U = nrec + 1;
-                int done = 0;
-                const int slot0 = slot, tile = int(hp.merge.size());
-                while (done < U) {
-                    int take = int(std::min<int64_t>(room, U - done));
-                    if (take < U - done) {
-                        take = take / TILE_UNITS * TILE_UNITS;                      // keep the cut on a tile boundary
-                        if (U - done - take < shortest) take = U - done;      // no short tail for the next CTA
-                        else if (take < shortest && int(hp.items.size()) > hp.cta_first.back()) take = 0;   // no short head here
+    for (size_t g = 0; g < groups.size(); ++g) {
+        const int U = groups[g].units;
+        if (room >= NKV * int64_t(U)) {
+            if (!v.whole(int(g), U)) return same_up_to;
+            busy = true;
+            room -= NKV * int64_t(U);
+            left -= NKV * int64_t(U);
+            if (room <= 0 && left > 0) next_cta();
+            continue;
+        }
+        for (int h = 0; h < NKV; ++h)
+            for (int done = 0; done < U;) {
+                int take = int(std::min<int64_t>(room, U - done));
+                if (take < U - done) {
+                    take = take / TILE_UNITS * TILE_UNITS;                      // keep the cut on a tile boundary
+                    const int rest = U - done - take;
+                    if (rest < shortest) {
+                        take = U - done;                                        // no short tail for the next CTA
+                    } else {
+                        same_up_to = std::min(same_up_to, rest);
+                        if (busy && take < shortest) take = 0;                  // no short head here
+                        else if (busy) same_up_to = std::min(same_up_to, take);
                     }
-                    if (take == 0) { next_cta(); continue; }
-                    const int rec_cnt = std::min(take, nrec - done);
-                    hp.items.push_back(WorkItem{s, j, h, done, std::max(rec_cnt, 0), done + take == U ? 1 : 0, slot++, tile});
-                    done += take;
-                    room -= take;
-                    left -= take;
-                    if (room <= 0 && left > 0) next_cta();
                 }
-                hp.merge.push_back(MergeDesc{seqs[s].q_first + j, h, slot0, slot - slot0});
+                if (take == 0) { next_cta(); continue; }
+                if (!v.run(int(g), h, done, take, U)) return same_up_to;
+                busy = true;
+                done += take;
+                room -= take;
+                left -= take;
+                if (room <= 0 && left > 0) next_cta();
             }
-    finish_plan(hp, nctas);
+    }
+    return same_up_to;
 }
+
+// The cost of a walk; it stops as soon as it cannot come out below `best`.
+struct CostVisit {
+    int64_t best, worst = 0, cta = 0;
+    bool run(int, int, int, int units, int tile_units) {
+        cta += units + RUN_STARTUP_UNITS + (units < tile_units ? RUN_SPLIT_UNITS : 0);
+        worst = std::max(worst, cta);
+        return worst < best;
+    }
+    bool whole(int, int units) {
+        cta += llattn::NKV * (units + RUN_STARTUP_UNITS);
+        worst = std::max(worst, cta);
+        return worst < best;
+    }
+    void next_cta() { cta = 0; }
+};
+
+// One more run in a plan, field by field: an aggregate that is put together on the stack and copied in wide words waits for
+// its own narrow stores, five times the time of the stores.
+inline void add_run(HostPlan& hp, const TileGroup& g, int h, int first, int units, int tile) {
+    hp.items.emplace_back();
+    llattn::WorkItem& w = hp.items.back();
+    w.seq = g.seq; w.qblk = g.qblk; w.kvh = h;
+    w.rec_begin = first; w.fresh = first + units == g.units; w.rec_count = units - w.fresh;
+    w.slot = int32_t(hp.items.size()) - 1; w.tile = tile;
+}
+inline void set_tile(llattn::MergeDesc& m, const HostPlan& hp, const TileGroup& g, int h, int slot_begin, int nslots) {
+    m.q_index = hp.seqs[g.seq].q_first + g.qblk; m.kvh = h; m.slot_begin = slot_begin; m.nslots = nslots;
+}
+
+// Appends a walk's runs to a plan.
+struct BuildVisit {
+    HostPlan& hp;
+    const std::vector<TileGroup>& groups;
+    bool run(int g, int h, int first, int units, int) {
+        if (first == 0) {
+            hp.merge.emplace_back();
+            set_tile(hp.merge.back(), hp, groups[g], h, int(hp.items.size()), 0);
+        }
+        ++hp.merge.back().nslots;
+        add_run(hp, groups[g], h, first, units, llattn::NKV * g + h);
+        return true;
+    }
+    bool whole(int g, int units) {
+        for (int h = 0; h < llattn::NKV; ++h) run(g, h, 0, units, units);
+        return true;
+    }
+    void next_cta() { hp.cta_first.push_back(int32_t(hp.items.size())); }
+};
 
 // Every run on a CTA of its own: each output tile is cut into equal runs, their number in proportion to the tile's
 // length (and no run shorter than about 0.75 sqrt(units of the tile)). Possible when there are no more output tiles than CTAs; better
 // than contiguous shares when the step is a latency problem (a handful of sequences), because no CTA then pays the
-// start-up of two runs one after the other.
-void cut_per_tile(const llattn_seq* seqs, int nseq, int nctas, int64_t total, HostPlan& hp) {
+// start-up of two runs one after the other. Returns the units per run of every tile.
+std::vector<int> equal_runs(const std::vector<TileGroup>& groups, int nctas, int64_t total) {
     using namespace llattn;
     std::vector<int> runs;
+    runs.reserve(groups.size() * NKV);
     int64_t given = 0;
-    for (int s = 0; s < nseq; ++s)
-        for (int j = 0; j < seqs[s].nq; ++j)
-            for (int h = 0; h < NKV; ++h) {
-                const int64_t U = seqs[s].nblocks + j + 1;
-                // a run costs about a unit's time per unit plus a bit over half a unit per run of its tile (its partial
-                // result is written, waited for and read back): the sum is smallest near 0.75 sqrt(U) units per run
-                // (measured: 8 units at 2 K tokens, 12 at 8 K)
-                const int64_t shortest = std::max<int64_t>(2 * TILE_UNITS, int64_t(0.75 * std::sqrt(double(U)) + 0.5));
-                const int64_t by_share = U * nctas / total, by_length = (U + shortest - 1) / shortest;
-                runs.push_back(int(std::max<int64_t>(1, std::min(by_share, by_length))));
-                given += runs.back();
-            }
+    for (const TileGroup& g : groups) {
+        const int64_t U = g.units;
+        // a run costs about a unit's time per unit plus a bit over half a unit per run of its tile (its partial
+        // result is written, waited for and read back): the sum is smallest near 0.75 sqrt(U) units per run
+        // (measured: 8 units at 2 K tokens, 12 at 8 K)
+        const int64_t shortest = std::max<int64_t>(2 * TILE_UNITS, int64_t(0.75 * std::sqrt(double(U)) + 0.5));
+        const int64_t by_share = U * nctas / total, by_length = (U + shortest - 1) / shortest;
+        runs.insert(runs.end(), NKV, int(std::max<int64_t>(1, std::min(by_share, by_length))));
+        given += NKV * runs.back();
+    }
     while (given > nctas) {                       // only when many tiles were rounded up to one run
         auto it = std::max_element(runs.begin(), runs.end());
         --*it; --given;
     }
-    hp.cta_first.assign(1, 0);
-    int slot = 0, t = 0;
-    for (int s = 0; s < nseq; ++s)
-        for (int j = 0; j < seqs[s].nq; ++j)
-            for (int h = 0; h < NKV; ++h, ++t) {
-                const int nrec = seqs[s].nblocks + j, U = nrec + 1, slot0 = slot;
-                const int per = std::max(TILE_UNITS, ((U + runs[t] - 1) / runs[t] + TILE_UNITS - 1) / TILE_UNITS * TILE_UNITS);
-                for (int done = 0; done < U; done += per) {
-                    const int take = std::min(per, U - done);
-                    hp.items.push_back(WorkItem{s, j, h, done, std::max(std::min(take, nrec - done), 0), done + take == U ? 1 : 0, slot++, t});
-                    hp.cta_first.push_back(int32_t(hp.items.size()));
-                }
-                hp.merge.push_back(MergeDesc{seqs[s].q_first + j, h, slot0, slot - slot0});
-            }
-    finish_plan(hp, nctas);
+    for (size_t t = 0; t < runs.size(); ++t) {
+        const int U = groups[t / NKV].units;
+        runs[t] = std::max(TILE_UNITS, ((U + runs[t] - 1) / runs[t] + TILE_UNITS - 1) / TILE_UNITS * TILE_UNITS);
+    }
+    return runs;
+}
+template <typename Visit>
+void walk_equal_runs(const std::vector<TileGroup>& groups, const std::vector<int>& per, Visit& v) {
+    for (size_t t = 0; t < per.size(); ++t) {
+        const int g = int(t) / llattn::NKV, U = groups[g].units;
+        for (int done = 0; done < U; done += per[t]) {
+            if (!v.run(g, int(t) % llattn::NKV, done, std::min(per[t], U - done), U)) return;
+            v.next_cta();
+        }
+    }
 }
 
 // Whole tiles only, the longest first, each to the CTA that has the least to do so far (start-ups counted): for more tiles
 // than CTAs of very unequal length, or enough tiles per CTA that they even out without a cut. The first pass over four
 // prompts of 13 blocks (208 tiles of 1 .. 13 units) is 39.0 us in contiguous order, which puts the longest tiles of a prompt side by
 // side, and 16.2 us like this; 200 ragged sequences 403 and 339.
-void cut_whole_tiles(const llattn_seq* seqs, int nseq, int nctas, HostPlan& hp) {
-    using namespace llattn;
-    std::vector<WorkItem> tiles;
-    for (int s = 0; s < nseq; ++s)
-        for (int j = 0; j < seqs[s].nq; ++j)
-            for (int h = 0; h < NKV; ++h) tiles.push_back(WorkItem{s, j, h, 0, seqs[s].nblocks + j, 1, 0, int32_t(tiles.size())});
-    std::vector<int32_t> order(tiles.size());
-    for (size_t i = 0; i < order.size(); ++i) order[i] = int32_t(i);
-    std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return tiles[a].rec_count > tiles[b].rec_count; });
-    typedef std::pair<int64_t, int32_t> Load;                    // cost so far, CTA
-    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
-    for (int c = 0; c < nctas; ++c) least.push(Load{0, c});
-    std::vector<std::vector<int32_t>> lists(nctas);
-    for (int32_t t : order) {
-        Load l = least.top();
-        least.pop();
-        lists[l.second].push_back(t);
-        l.first += tiles[t].rec_count + 1 + RUN_STARTUP_UNITS;
-        least.push(l);
-    }
-    hp.merge.resize(tiles.size());
-    hp.cta_first.assign(1, 0);
-    for (const std::vector<int32_t>& list : lists) {
-        for (int32_t t : list) {
-            WorkItem w = tiles[t];
-            w.slot = int32_t(hp.items.size());
-            hp.items.push_back(w);
-            hp.merge[t] = MergeDesc{seqs[w.seq].q_first + w.qblk, w.kvh, w.slot, 1};
-        }
-        hp.cta_first.push_back(int32_t(hp.items.size()));
-    }
-    finish_plan(hp, nctas);
-}
+struct WholeTiles {
+    std::vector<int32_t> head, tail, next;        // a CTA's tiles as a list
+    int64_t worst = 0, max_units = 0;
 
+    // Groups by length, longest first, those of one length in order: a counting sort per eleven bits of the length.
+    static std::vector<int32_t> by_length(const std::vector<TileGroup>& groups) {
+        std::vector<int32_t> order(groups.size()), other(groups.size());
+        int32_t lo = INT32_MAX, hi = 0;
+        for (size_t g = 0; g < groups.size(); ++g) { order[g] = int32_t(g); lo = std::min(lo, groups[g].units); hi = std::max(hi, groups[g].units); }
+        for (int shift = 0; shift < 31 && uint32_t(hi - lo) >> shift; shift += 11) {
+            uint32_t at[2049] = {};
+            for (int32_t g : order) ++at[((uint32_t(hi - groups[g].units) >> shift) & 2047) + 1];
+            for (int k = 1; k < 2049; ++k) at[k] += at[k - 1];
+            for (int32_t g : order) other[at[(uint32_t(hi - groups[g].units) >> shift) & 2047]++] = g;
+            order.swap(other);
+        }
+        return order;
+    }
+
+    // false: does not come out below `best`
+    bool assign(const std::vector<TileGroup>& groups, int nctas, int64_t best) {
+        // (cost so far, CTA) in one word each, in order, in a window that moves on with every tile: the least loaded CTA leaves at
+        // the front and comes in again further back, at the very end when the tiles are of one length
+        int cta_bits = 1;
+        while (nctas >> cta_bits) ++cta_bits;
+        const uint64_t cta_mask = (uint64_t(1) << cta_bits) - 1;
+        std::vector<uint64_t> loads(4 * size_t(nctas) + 64);
+        for (int c = 0; c < nctas; ++c) loads[c] = uint64_t(c);
+        uint64_t *front = loads.data(), *end = front + nctas;
+        head.assign(nctas, -1); tail.assign(nctas, -1); next.assign(groups.size() * llattn::NKV, -1);
+        std::vector<int32_t> tiles(nctas, 0);
+        for (int32_t g : by_length(groups)) {
+            const uint64_t c = uint64_t(groups[g].units + RUN_STARTUP_UNITS) << cta_bits;
+            for (int h = 0; h < llattn::NKV;) {
+                // the group's four tiles at once where the first CTA's new load is beyond the fourth's old one
+                const int n = h == 0 && nctas >= llattn::NKV && front[0] + c > front[llattn::NKV - 1] ? llattn::NKV : 1;
+                uint64_t w[llattn::NKV];
+                for (int i = 0; i < n; ++i) w[i] = front[i] + c;
+                worst = std::max(worst, int64_t(w[n - 1] >> cta_bits));
+                if (worst >= best) return false;
+                front += n;
+                if (loads.data() + loads.size() - end < n) {                     // the window is at the end of its memory: back to the start
+                    memmove(loads.data(), front, size_t(end - front) * sizeof(uint64_t));
+                    end = loads.data() + (end - front);
+                    front = loads.data();
+                }
+                uint64_t *from = end, *to = end += n;
+                for (int i = n - 1; i >= 0; --i) {
+                    while (from != front && from[-1] > w[i]) *--to = *--from;
+                    *--to = w[i];
+                }
+                for (int i = 0; i < n; ++i, ++h) {
+                    const int32_t cta = int32_t(w[i] & cta_mask), t = llattn::NKV * g + h;
+                    (head[cta] < 0 ? head[cta] : next[tail[cta]]) = t;
+                    tail[cta] = t;
+                    ++tiles[cta];
+                }
+            }
+        }
+        for (; front != end; ++front)
+            max_units = std::max(max_units, int64_t(*front >> cta_bits) - RUN_STARTUP_UNITS * tiles[*front & cta_mask]);
+        return true;
+    }
+
+    void build(const std::vector<TileGroup>& groups, HostPlan& hp) const {
+        hp.merge.resize(next.size());
+        for (int32_t first : head) {
+            for (int32_t t = first; t >= 0; t = next[t]) {
+                const TileGroup& g = groups[t / llattn::NKV];
+                set_tile(hp.merge[t], hp, g, t % llattn::NKV, int(hp.items.size()), 1);
+                add_run(hp, g, t % llattn::NKV, 0, g.units, t);
+            }
+            hp.cta_first.push_back(int32_t(hp.items.size()));
+        }
+    }
+};
+
+// Finds the cheapest way of cutting by cost alone (a walk that builds nothing and stops where it cannot win) and builds that
+// one: a serving loop replans whenever a block is committed. On one core, the first candidate alone / every candidate built /
+// this: 64 x 32 K tokens 8.1 / 49.6 / 8.6 us, 64 x 1 K 7.1 / 43.1 / 8.2, 256 ragged sequences 20.6 / 214 / 34.5, four first
+// passes of 13 blocks 9.1 / 44.5 / 9.2, 16,384 tiles 259 / 3400 / 228.
 int build_plan(const llattn_seq* seqs, int nseq, int nctas, HostPlan& hp) {
     using namespace llattn;
     hp.seqs.resize(nseq);
-    int64_t total = 0, ntile_out = 0;
+    int64_t total = 0, ngroups = 0;
     int nq_total = 0;
     for (int s = 0; s < nseq; ++s) {
         const llattn_seq& q = seqs[s];
@@ -194,46 +305,66 @@ int build_plan(const llattn_seq* seqs, int nseq, int nctas, HostPlan& hp) {
             return fail(LLATTN_EINVAL, "plan: sequence %d reads %d blocks but head_stride is %d", s, q.nblocks + q.nq - 1, q.head_stride);
         if (q.cache && !aligned16(q.cache)) return fail(LLATTN_EINVAL, "plan: sequence %d cache is not 16-byte aligned", s);
         hp.seqs[s] = SeqDesc{static_cast<const uint8_t*>(q.cache), q.pages, q.head_stride, q.nblocks, q.nq, q.q_first};
-        for (int j = 0; j < q.nq; ++j) total += int64_t(NKV) * (q.nblocks + j + 1);
-        ntile_out += int64_t(NKV) * q.nq;
+        ngroups += q.nq;
         nq_total = std::max(nq_total, q.q_first + q.nq);
     }
+    std::vector<TileGroup> groups;
+    groups.reserve(ngroups);
+    int32_t longest = 0;
+    for (int s = 0; s < nseq; ++s)
+        for (int j = 0; j < seqs[s].nq; ++j) {
+            groups.push_back(TileGroup{s, j, seqs[s].nblocks + j + 1});
+            longest = std::max(longest, groups.back().units);
+            total += int64_t(NKV) * groups.back().units;
+        }
+    const int64_t ntiles = NKV * ngroups;
     hp.total_units = total;
     hp.nq_total = nq_total;
-    auto take_if_cheaper = [&](HostPlan& alt) {
-        if (alt.max_cta_cost < hp.max_cta_cost) {
-            hp.items.swap(alt.items); hp.cta_first.swap(alt.cta_first); hp.merge.swap(alt.merge);
-            hp.used_ctas = alt.used_ctas; hp.max_cta_units = alt.max_cta_units; hp.max_cta_cost = alt.max_cta_cost;
-        }
+
+    // The candidates in order of preference: a later one has to be strictly cheaper.
+    int64_t best = INT64_MAX, best_min_units = 0;
+    int best_shortest = 0;
+    std::vector<int> equal;          // the units per run of every tile, where every run on a CTA of its own is the best so far
+    auto try_contiguous = [&](int64_t min_units, int shortest) -> int {
+        CostVisit cost{best};
+        const int same_up_to = walk_contiguous(groups, nctas, total, min_units, shortest, cost);
+        if (cost.worst < best) { best = cost.worst; best_min_units = min_units; best_shortest = shortest; equal.clear(); }
+        return same_up_to;
     };
-    // Contiguous shares, with pieces allowed down to 12, 24, 48 or 96 units: the longer they must be, the fewer runs and
-    // tiles shared between CTAs, and the less equal the shares; the model decides. (64 sequences of 1 K tokens, two and a bit
-    // tiles of 33 units per CTA: 47.6 us with pieces of 12, 35.2 without any; 16 ragged sequences 86 -> 76 us with 24.)
-    cut_contiguous(seqs, nseq, nctas, total, 16, 12, hp);
-    for (int shortest : {24, 48, 96}) {
-        HostPlan alt;
-        cut_contiguous(seqs, nseq, nctas, total, 16, shortest, alt);
-        take_if_cheaper(alt);
+    int same_up_to = try_contiguous(16, 12);
+    // little work: shorter shares on more CTAs may beat several runs per CTA
+    const bool little = total < 16 * int64_t(nctas);
+    if (little) try_contiguous(TILE_UNITS, 12);
+    // Longer pieces at least, 24, 48 or 96 units: fewer runs and tiles shared between CTAs, and less equal shares; the model
+    // decides. (64 sequences of 1 K tokens, two and a bit tiles of 33 units per CTA: 47.6 us with pieces of 12, 35.2 without any;
+    // 16 ragged sequences 86 -> 76 us with 24.)
+    for (int shortest : {24, 48, 96})
+        if (shortest > same_up_to) same_up_to = try_contiguous(16, shortest);
+    // Shares down to a single 128-key tile where the tiles outnumber the CTAs (64 x 128 tokens 22.0 -> 17.9 us) or the units do
+    // not (one sequence at 1 K tokens 14.6 -> 12.1); between the two, equal runs are within 2 us of it with half the slots to fold.
+    if (little && (total <= nctas || ntiles > nctas)) try_contiguous(TILE_UNITS, TILE_UNITS);
+    if (ntiles <= nctas) {
+        std::vector<int> per = equal_runs(groups, nctas, total);
+        CostVisit cost{best};
+        walk_equal_runs(groups, per, cost);
+        if (cost.worst < best) { best = cost.worst; equal.swap(per); }
     }
-    // Little work: shorter shares on more CTAs may beat several runs per CTA. Down to a single 128-key tile where the tiles
-    // outnumber the CTAs (64 x 128 tokens 22.0 -> 17.9 us) or the units do not (one sequence at 1 K tokens 14.6 -> 12.1);
-    // between the two, the runs of about 0.75 sqrt(units) below are within 2 us of it with half the slots to fold.
-    if (total < 16 * int64_t(nctas))
-        for (int shortest : {12, TILE_UNITS}) {
-            if (shortest < 12 && total > nctas && ntile_out <= nctas) break;
-            HostPlan alt;
-            cut_contiguous(seqs, nseq, nctas, total, TILE_UNITS, shortest, alt);
-            take_if_cheaper(alt);
-        }
-    HostPlan alt;
-    if (ntile_out <= nctas) {
-        cut_per_tile(seqs, nseq, nctas, total, alt);
-        take_if_cheaper(alt);
-    } else {
-        cut_whole_tiles(seqs, nseq, nctas, alt);
-        // with plenty of work per CTA the shares stay near equal whatever the start-ups: only tiles that even out by themselves
-        if (total < 64 * int64_t(nctas) || 100 * alt.max_cta_units * nctas <= 102 * total + 1200 * int64_t(nctas)) take_if_cheaper(alt);
-    }
+    WholeTiles whole;
+    // with plenty of work per CTA the shares stay near equal whatever the start-ups: only tiles that even out by themselves
+    const bool whole_tiles =
+        ntiles > nctas && std::max<int64_t>(longest + RUN_STARTUP_UNITS, (total + RUN_STARTUP_UNITS * ntiles + nctas - 1) / nctas) < best &&
+        whole.assign(groups, nctas, best) &&
+        (total < 64 * int64_t(nctas) || 100 * whole.max_units * nctas <= 102 * total + 1200 * int64_t(nctas));
+
+    hp.items.reserve(ntiles + nctas);
+    hp.merge.reserve(ntiles);
+    hp.cta_first.reserve(nctas + 1);
+    hp.cta_first.push_back(0);
+    BuildVisit build{hp, groups};
+    if (whole_tiles) whole.build(groups, hp);
+    else if (!equal.empty()) walk_equal_runs(groups, equal, build);
+    else walk_contiguous(groups, nctas, total, best_min_units, best_shortest, build);
+    finish_plan(hp, nctas);
     return LLATTN_OK;
 }
 

@@ -2,9 +2,11 @@
 as status codes without touching a GPU, the host planner covers every KV unit exactly once within its CTA budget,
 and the request sharding balances. No compute call is made here."""
 import ctypes
+import heapq
 import importlib
 import os
 import re
+import time
 
 import numpy as np
 import pytest
@@ -214,3 +216,55 @@ def test_planner_puts_unequal_whole_tiles_on_the_least_loaded_cta(api):
     assert np.all(items[:, 4] == items[:, 1]) and np.all(items[:, 5] == 1)
     st, items, cta_first = api.plan_preview([3, 0, 17, 250, 1, 64], 7)        # whole tiles would leave one CTA with 251 of 1364 units
     assert st.max_cta_units <= 1.02 * st.total_units / 7 + 12
+
+
+def _preview_us(api, lengths, nq, nctas=148, repeats=30):
+    """Best time of a call of the host planner alone, without the binding's arrays."""
+    n, q0 = len(lengths), 0
+    arr = (api._Seq * n)()
+    for i in range(n):
+        arr[i] = api._Seq(0x1000, None, lengths[i] + nq[i], lengths[i], nq[i], q0)
+        q0 += nq[i]
+    st, best = api.PlanStats(), float("inf")
+    for _ in range(repeats):
+        t = time.perf_counter()
+        assert api.lib().llattn_plan_preview(arr, n, nctas, ctypes.byref(st), None, 0, None, 0) == api.OK
+        best = min(best, time.perf_counter() - t)
+    return 1e6 * best
+
+
+def test_planning_builds_one_plan_only(api):
+    """A serving loop replans per committed block. The limits are three to four times what choosing by cost takes on one
+    2024 server core, and a half to a third of what it took to build every candidate plan and keep one."""
+    g = np.random.default_rng(3)
+    ragged = [int(x) for x in g.integers(4, 1025, 256)]
+    assert _preview_us(api, ragged, [1] * 256) < 110                       # 34 us (every candidate built: 214)
+    assert _preview_us(api, [0] * 16, [16] * 16) < 80                      # 25 (158)
+    assert _preview_us(api, [100] * 256, [16] * 256) < 1000                # 228 (3400)
+
+
+def test_whole_tiles_go_to_the_least_loaded_cta_in_order_of_length(api):
+    """Where the planner keeps tiles whole and out of order, its lists are those of the plain form: tiles by length, longest
+    first, each to the CTA with the least cost so far (20 units a run), the lowest CTA among equals."""
+    g = np.random.default_rng(8)
+    seen = set()
+    for trial in range(400):
+        nctas = int(g.choice([1, 2, 3, 4, 5, 9, 40, 148, 160]))
+        nseq = int(g.integers(1, 90))
+        top = int(g.choice([0, 3, 60, 1000, 5000]))
+        lengths = [top] * nseq if trial % 3 == 0 else [int(x) for x in g.integers(0, top + 1, nseq)]
+        nq = [int(x) for x in g.integers(1, 17, nseq)] if trial % 2 else [1] * nseq
+        st, items, cta_first = api.plan_preview(lengths, nctas, nq)
+        tiles = [n + j + 1 for n, q in zip(lengths, nq) for j in range(q) for _ in range(4)]
+        if st.nitems != len(tiles) or np.array_equal(items[:, 7], np.arange(len(tiles))):
+            continue                                                        # shares in order
+        heap, want = [(0, c) for c in range(nctas)], [[] for _ in range(nctas)]
+        for t in sorted(range(len(tiles)), key=lambda t: (-tiles[t], t)):
+            cost, c = heapq.heappop(heap)
+            want[c].append(t)
+            heapq.heappush(heap, (cost + tiles[t] + 20, c))
+        got = [items[cta_first[c]:cta_first[c + 1], 7].tolist() for c in range(st.nctas)]
+        assert got == want[:st.nctas] and not any(want[st.nctas:])
+        assert np.array_equal(items[:, 3], np.zeros(st.nitems)) and np.array_equal(items[:, 4] + items[:, 5], [tiles[t] for t in items[:, 7]])
+        seen.add(nctas)
+    assert {2, 3, 4, 5, 9, 40, 148, 160} <= seen, seen
