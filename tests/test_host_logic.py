@@ -268,3 +268,12 @@ def test_whole_tiles_go_to_the_least_loaded_cta_in_order_of_length(api):
         assert np.array_equal(items[:, 3], np.zeros(st.nitems)) and np.array_equal(items[:, 4] + items[:, 5], [tiles[t] for t in items[:, 7]])
         seen.add(nctas)
     assert {2, 3, 4, 5, 9, 40, 148, 160} <= seen, seen
+
+
+def test_planner_cuts_no_tile_where_that_shortens_nothing(api):
+    """As many tiles as fit on a CTA each, all about as long: the longest list is a whole tile whatever is cut, and a cut tile
+    only adds partial results (24 x 2 K tokens: 29.2 us whole, 32.4 cut). The same cost, so the plain form stays."""
+    for lengths, nq in (([64] * 24, None), ([64] * 32, None), ([128] * 32, None), ([45] * 36, None), ([60] * 3, [9] * 3), ([60] * 4, [9] * 4)):
+        st, items, cta_first = api.plan_preview(lengths, 148, nq)
+        tiles = 4 * (len(lengths) if nq is None else sum(nq))
+        assert st.nitems == st.nctas == tiles, (lengths[0], st.nitems)
