@@ -494,6 +494,18 @@ __device__ __forceinline__ void copy_fresh(const half* src, uint8_t* tile_unit, 
     }
 }
 
+// Third block of both V tiles: column 128 of V is all ones (O column 128 accumulates sum(P)), 129..143 zero. Written by the warp
+// that issues the MMAs which read it; its first tile is still on its way then.
+__device__ __forceinline__ void write_ones_column(uint8_t* smem, int lane) {
+    for (int idx = lane; idx < 2 * 128 * 8; idx += 32) {
+        const int buf = idx >> 10, key = (idx >> 3) & 127, pos = idx & 7;
+        *reinterpret_cast<uint4*>(smem + SM_V + buf * VTILE_BYTES + 2 * KBLOCK + key * 128 + pos * 16) =
+            make_uint4(pos == (key & 7) ? 0x00003C00u : 0u, 0u, 0u, 0u);
+    }
+    ptx::fence_proxy_async_smem();
+    __syncwarp();
+}
+
 // The whole CTA's work. `cta` is the CTA's index in the plan (list mode) or in the flattened reference grid
 // (kv head fastest, then chunk, then query block).
 // PRECISE: P is carried as fp16 value + fp16 remainder (two PV chains per tile), for callers that need the result to
@@ -885,6 +897,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
         const uint32_t tmem = uniform_u32(tmem_any);
         const int i0 = uniform_i32(i0_any), i1 = uniform_i32(i1_any);
 #if LLATTN_SINGLE_ISSUER
+        write_ones_column(smem, lane);
         // This warp issues everything, per tile t in the order PV(t), S(t+2). S(t+2) overwrites the buffer that holds P(t);
         // the tensor pipe executes the MMAs of one thread in issue order, so no wait for PV(t) to complete is needed.
         const uint32_t v_s = ptx::smem_u32(smem + SM_V);
@@ -981,15 +994,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
         // ================================================================== O += P V issue
         uint32_t t = 0, itc = 0;
         bool alive = true;
-        // third block of both V tiles: column 128 of V is all ones (O column 128 accumulates sum(P)), 129..143 zero. Written by
-        // the warp whose MMAs read it, which has nothing else to do while the first tile is on its way.
-        for (int idx = lane; idx < 2 * 128 * 8; idx += 32) {
-            const int buf = idx >> 10, key = (idx >> 3) & 127, pos = idx & 7;
-            *reinterpret_cast<uint4*>(smem + SM_V + buf * VTILE_BYTES + 2 * KBLOCK + key * 128 + pos * 16) =
-                make_uint4(pos == (key & 7) ? 0x00003C00u : 0u, 0u, 0u, 0u);
-        }
-        ptx::fence_proxy_async_smem();
-        __syncwarp();
+        write_ones_column(smem, lane);
         const uint32_t v_s = ptx::smem_u32(smem + SM_V);
         const uint32_t idO = ptx::idesc_f16(128, PV_N, false, true);
         // one base descriptor per V buffer (MN-major, 128-byte swizzle: 8-key groups 1024 B apart, 64-dim blocks KBLOCK apart)

@@ -1,0 +1,60 @@
+"""The attention kernel's build option LLATTN_SINGLE_ISSUER (one warp issues both MMA chains) gives the default build's
+numbers: whatever a role sets up in shared memory, it sets up in either form. The option's library is compiled here."""
+import importlib
+import importlib.util
+import os
+import shutil
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def single(pkg, tmp_path_factory):
+    nvcc = os.environ.get("NVCC") or shutil.which("nvcc")
+    if nvcc is None:
+        pytest.skip("needs nvcc: the option is a compile-time one")
+    bld = importlib.import_module(pkg.__name__ + ".build")
+    lib = str(tmp_path_factory.mktemp("single") / "libllattn_single.so")
+    subprocess.check_call([nvcc] + bld.NVCC_FLAGS + ["-DLLATTN_SINGLE_ISSUER=1", os.path.join(bld.CSRC, "llattn.cu"), "-o", lib])
+    old = os.environ.get("LLATTN_LIB")
+    os.environ["LLATTN_LIB"] = lib                             # read when the module is loaded
+    try:
+        spec = importlib.util.spec_from_file_location("llattn_api_single", os.path.join(bld.HERE, "api.py"))
+        api = sys.modules[spec.name] = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(api)
+    finally:
+        os.environ.pop("LLATTN_LIB")
+        if old is not None:
+            os.environ["LLATTN_LIB"] = old
+    assert api.lib()._name == lib
+    return api
+
+
+@pytest.mark.parametrize("nblocks,nctas", [(0, 0), (3, 4), (5, 8), (33, 3), (130, 0)])
+@pytest.mark.parametrize("precise", [False, True])
+def test_single_issuer_matches_the_oracle(single, pkg, orc, nblocks, nctas, precise):
+    wl = pkg.workload
+    Q, Kf, Vf = wl.query_blocks(1, seq=nblocks)
+    cache = np.zeros((4, nblocks + 1, orc.REC_BYTES), np.uint8)
+    if nblocks:
+        Kc, Vc = wl.context_blocks(nblocks, seq=nblocks)
+        orc.kv_commit(Kc, Vc, cache, nblocks + 1, 0)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    want, lse = orc.attention(Q, Kf, Vf, cache, nblocks + 1, nblocks, dq_mode=1)
+    ctx = single.Context(0)
+    cached = dev(cache)
+    plan = ctx.plan([single.Seq(cache=cached, nblocks=nblocks)], nctas)
+    O, L = torch.zeros((32, 16, 128), device="cuda"), torch.zeros((32, 16), device="cuda")
+    ctx.attention(plan, dev(Q), dev(Kf), dev(Vf), O32=O, LSE=L, precise=precise)
+    assert ctx.device_status() == 0
+    rms = np.sqrt((want.astype(np.float64) ** 2).mean())
+    # the bounds of the default build's tests: 2e-3 up to 8 blocks and with precise, 5e-3 above (fp16 rounding of P); LSE 1e-3
+    assert np.abs(O.cpu().numpy() - want).max() <= (2e-3 if precise or nblocks <= 8 else 5e-3) * rms
+    assert np.abs(L.cpu().numpy() - lse).max() <= 1e-3
+    plan.close(); ctx.close()
