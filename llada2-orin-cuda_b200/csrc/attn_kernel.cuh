@@ -1080,7 +1080,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
             }
             constexpr int NW = ATTN_THREADS / 32;
             const int r0 = (w.slot - md.slot_begin) + md.nslots * warp, step = md.nslots * NW;
-            if (md.nslots > FOLD_PART) {
+            if (md.nslots > FOLD_PART && md.nslots <= FOLD_SHARED_SLOTS) {
                 fold_rows_shared(p.Opart, p.Mpart, p.Lpart, md, w.slot - md.slot_begin, warp, lane, smem + SM_K, p.out);      // the tiles are done with
             } else if (md.nslots == 2) {
 #pragma unroll 1

@@ -125,8 +125,9 @@ __device__ __forceinline__ void emit_row_warp(float M, float den, const float4& 
     }
 }
 
-// Up to FOLD_PART slots of one row, by one warp: reference exponent, row sum and weighted dims of those slots. Every load
-// - the slots' scalars and their rows - is on its way before the first is used: one round trip to the L2.
+// Up to FOLD_PART slots of one row, by one warp: reference exponent, row sum and weighted dims of those slots. No load waits for
+// another, so with the registers for it (the attention kernel has them) they take one round trip to the L2; the folding
+// launch has many warps an SM instead and issues them as its 47 registers allow.
 constexpr int FOLD_PART = 16;
 __device__ __forceinline__ void fold_part(const float* Opart, const float* Mpart, const float* Lpart, size_t slot0, int cnt, int r, int lane,
                                           float& M, float& den, float4& acc) {
@@ -205,14 +206,18 @@ __device__ __forceinline__ void fold_row_warp(const float* Opart, const float* M
     emit_row_warp(M, den, acc, md, r, lane, o);
 }
 
-// This CTA's rows k, k + n, ... (n > FOLD_PART slots, so at most 7 rows) of a tile cut into n runs, by 16 warps: W warps share
-// a row, each folds n / W of its slots (at most FOLD_PART), the row's first warp adds their results up in slot order. With a
-// warp per row, most of the warps had none and the others went through their slots in several round trips:
-// 22 runs a tile, 7,000 cycles from the last count-in to the outputs. `scratch`: 16 x 544 bytes of shared memory; every
-// thread of the CTA calls.
-__device__ __noinline__ void fold_rows_shared(const float* Opart, const float* Mpart, const float* Lpart, const MergeDesc& md, int k, int warp,
+// This CTA's rows k, k + n, ... of a tile cut into n runs, FOLD_PART < n <= FOLD_SHARED_SLOTS, by 16 warps: W warps share a
+// row, each folds n / W of its slots, the row's first warp adds their results up in slot order. With a warp per row, most of
+// the warps had none and the others went through their slots in several round trips: 22 runs a tile, 7,000 cycles from the last
+// count-in to the outputs. Two warps a row up to 32 slots (at most 8 rows), four above (at most 4 rows); the planner
+// gives a tile at most 59 runs on 160 CTAs, and more would take the general form. `scratch`: 16 x 544 bytes of shared memory; every
+// thread of the CTA calls. Inlined: as a call it made the attention kernel spill (12 bytes of stores, 20 of loads), which
+// cost 1 .. 3 % everywhere (64 sequences at 32 K tokens 704 -> 688 us, 128 at 1 K 82.3 -> 80.7).
+constexpr int FOLD_SHARED_SLOTS = 4 * FOLD_PART;
+static_assert((QR + FOLD_PART) / (FOLD_PART + 1) <= 16 / 2 && (QR + 2 * FOLD_PART) / (2 * FOLD_PART + 1) <= 16 / 4, "rows of a CTA: one per W warps");
+__device__ __forceinline__ void fold_rows_shared(const float* Opart, const float* Mpart, const float* Lpart, const MergeDesc& md, int k, int warp,
                                                  int lane, uint8_t* scratch, const MergeOut& o) {
-    const int n = md.nslots, W = n <= 32 ? 2 : n <= 64 ? 4 : n <= 128 ? 8 : 16;
+    const int n = md.nslots, W = n <= 2 * FOLD_PART ? 2 : 4;
     const int part = warp & (W - 1), per = (n + W - 1) / W, s0 = part * per, cnt = min(per, n - s0);
     const int r = k + n * (warp / W);
     float M = -INFINITY, den = 0.f;

@@ -285,6 +285,57 @@ def test_tiles_cut_into_n_runs_are_folded_by_their_ctas(api, ctx, orc, pkg, nblo
     assert one["stats"].nitems == 4 and rel_l2(one["O32"], res["O32"]) <= 2 * TOL_L2
 
 
+@pytest.mark.parametrize("nblocks,nctas,per_tile", [(255, 64, 16), (269, 68, 17), (889, 128, 32), (1024, 132, 33), (1024, 148, 37), (235, 148, 57)])
+def test_tiles_cut_into_many_runs(api, ctx, orc, pkg, nblocks, nctas, per_tile):
+    """Where the folding changes form: up to 16 runs a warp folds a row, with 17 two warps share one, with 33 four. Every output
+    form, and the same bits from two launches. (57: the most runs that any tile gets, next to three of 29.)"""
+    Q, Kf, Vf, cache, maxb = make_case(pkg.workload, orc, nblocks, seq=900 + nctas)
+    case = [(Q, Kf, Vf, cache, maxb, nblocks)]
+    st, items, _ = api.plan_preview([nblocks], nctas)
+    assert np.bincount(items[:, 7]).max() == per_tile
+    res = run_batched(api, ctx, case, want=("O32", "O16", "LSE", "q8"), nctas=nctas)
+    assert res["stats"].nitems == st.nitems
+    Ow, Lw = orc.attention(Q, Kf, Vf, cache, maxb, nblocks, dq_mode=1)
+    assert relmax(res["O32"], Ow) <= tol_o(nblocks) and rel_l2(res["O32"], Ow) <= TOL_L2
+    assert np.abs(res["LSE"] - Lw).max() <= TOL_LSE
+    assert np.array_equal(res["O16"], res["O32"].astype(np.float16))
+    q8, s8, sum8 = orc.act_q8(res["O32"])
+    assert np.array_equal(res["q8"], q8) and np.array_equal(res["s8"], s8) and np.array_equal(res["sum8"], sum8)
+    again = run_batched(api, ctx, case, want=("O32", "LSE", "q8"), nctas=nctas)
+    assert all(np.array_equal(again[k], res[k]) for k in ("O32", "LSE", "q8"))
+
+
+@pytest.mark.parametrize("nblocks", [4, 32])
+def test_a_whole_tile_has_the_bits_of_a_lone_run(api, ctx, pkg, nblocks):
+    """64 short sequences: every tile stays with one CTA, next to others or not, in whatever order; the outputs are those of each
+    sequence alone on four CTAs, bit for bit, and repeat."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(nblocks)
+    half = lambda *s: torch.randn(s, generator=g, device="cuda").half()
+    n = 64
+    caches = torch.zeros((n, 4, nblocks, 4736), dtype=torch.uint8, device="cuda")
+    for c in caches:
+        api.kv_commit(half(nblocks, 32, 4, 128), half(nblocks, 32, 4, 128), c, nblocks, 0)
+    Q, Kf, Vf = half(n, 32, 16, 128), half(n, 32, 4, 128), half(n, 32, 4, 128)
+    plan = ctx.plan([api.Seq(cache=caches[i], nblocks=nblocks, q_first=i) for i in range(n)])
+    assert plan.stats.nitems == 4 * n
+    O, L = torch.zeros((n, 32, 16, 128), device="cuda"), torch.zeros((n, 32, 16), device="cuda")
+    ctx.attention(plan, Q, Kf, Vf, O32=O, LSE=L)
+    O2, L2 = torch.zeros_like(O), torch.zeros_like(L)
+    ctx.attention(plan, Q, Kf, Vf, O32=O2, LSE=L2)
+    assert torch.equal(O, O2) and torch.equal(L, L2)
+    for i in range(n):
+        lone = ctx.plan([api.Seq(cache=caches[i], nblocks=nblocks)], 4)
+        assert lone.stats.nitems == 4
+        o, l = torch.zeros((32, 16, 128), device="cuda"), torch.zeros((32, 16), device="cuda")
+        ctx.attention(lone, Q[i:i + 1], Kf[i:i + 1], Vf[i:i + 1], O32=o, LSE=l)
+        torch.cuda.synchronize()
+        assert torch.equal(o, O[i]) and torch.equal(l, L[i])
+        lone.close()
+    assert ctx.device_status() == 0
+    plan.close()
+
+
 def test_random_small_batches_on_random_grids(api, ctx, orc, pkg):
     """Ten seeded random batches (1 .. 9 sequences, 0 .. 90 blocks, one or two query blocks) on 3, 11, 40 or all CTAs:
     whatever mixture of whole tiles, tiles cut in two and tiles cut in many the planner makes of them, every CTA's waits

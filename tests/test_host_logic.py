@@ -277,3 +277,14 @@ def test_planner_cuts_no_tile_where_that_shortens_nothing(api):
         st, items, cta_first = api.plan_preview(lengths, 148, nq)
         tiles = 4 * (len(lengths) if nq is None else sum(nq))
         assert st.nitems == st.nctas == tiles, (lengths[0], st.nitems)
+
+
+def test_no_tile_gets_more_runs_than_the_shared_folding_takes(api):
+    """A tile of 17 .. 64 runs is folded by several warps a row; the planner gives none more than that (most: one sequence of a
+    few thousand tokens, whose last tile is cut finest)."""
+    most = 0
+    for nctas in (148, 160):
+        for n in list(range(0, 1100, 3)) + [235, 243, 4000, 32768]:
+            st, items, _ = api.plan_preview([n], nctas)
+            most = max(most, int(np.bincount(items[:, 7]).max()))
+    assert 37 <= most <= 64, most
