@@ -348,7 +348,7 @@ extern "C" int llattn_attention_static(const void* Q, const void* Kf, const void
     CU(cudaGetLastError());
     MergeOut o{static_cast<half*>(O16), O32, LSE, q8, s8, sum8};
     CU(launch_dependent(
-        combine_ref_kernel, dim3(NKV, QR / MERGE_ROWS, nb), MERGE_THREADS, as_stream(stream),
+        nchunks > FOLD_PART ? combine_ref_kernel<true> : combine_ref_kernel<false>, dim3(NKV, QR / MERGE_ROWS, nb), MERGE_THREADS, as_stream(stream),
         static_cast<const float*>(Opart), static_cast<const float*>(Mpart), static_cast<const float*>(Lpart), nchunks, nblocks, bpc, o));
     return LLATTN_OK;
 }

@@ -420,7 +420,7 @@ int llattn_attn_combine(const float* Opart, const float* Mpart, const float* Lpa
     if (q8) { o.q8 = q8; o.s8 = s8; o.sum8 = sum8; }       // as the reference: int8 form replaces the fp16 output
     else o.O16 = static_cast<half*>(O);
     CU(launch_dependent(
-        combine_ref_kernel, dim3(NKV, QR / MERGE_ROWS, nb), MERGE_THREADS, as_stream(stream), Opart, Mpart, Lpart, nchunks, nblocks, bpc, o));
+        nchunks > FOLD_PART ? combine_ref_kernel<true> : combine_ref_kernel<false>, dim3(NKV, QR / MERGE_ROWS, nb), MERGE_THREADS, as_stream(stream), Opart, Mpart, Lpart, nchunks, nblocks, bpc, o));
     return LLATTN_OK;
 }
 
