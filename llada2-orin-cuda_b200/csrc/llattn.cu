@@ -217,9 +217,22 @@ int llattn_qkv_prepare_commit(const float* qkv, const int32_t* pos, const float*
 // The attention-output projection on the int8 activations the merge kernel writes.
 
 namespace {
-// At most this many tokens go to the strip kernel: it reads the weights once per 32 tokens, with every SM, and a call is
-// 3.8 us at 32 tokens and 6.6 at 64; the tile kernel's 16 row tiles at 65 tokens still leave most SMs idle at that size (8.1 us).
+// Up to this many tokens the strip kernel may be the faster one: it reads the weights once per 32 tokens, with every SM.
 constexpr int DENSE_STRIP_MAX_TOKENS = 64;
+
+// Strip kernel or 16-token tiles. One strip CTA fills an SM (512 threads of 128 registers), so its time goes with the rows too:
+// 2048 rows of K = 2048 are one wave (3.2 us for 16 tokens, 8.0 as tiles), 4096 two (5.3 and 8.3), 16,384 seven (17.5 and 9.7; 64
+// tokens at K = 512 26.0, in 64-token tiles 7.2). Both as measured in a graph over 2048 .. 32,768 rows, K = 256 .. 8192 and 1 .. 64
+// tokens, in hundredths of a microsecond: a wave of strips per sixteen groups and the tokens in it (a partly filled last wave
+// counts half), and the serial groups of a tile. The choice is within 11 % of the faster one everywhere there. (Rows and tokens
+// beyond one wave of 16-token tiles need no case of their own: the strips have lost long before.)
+bool dense_strips_win(int rows, int K, int ntokens, int sms) {
+    const int batches = (ntokens + llattn::DS_TOK - 1) / llattn::DS_TOK, per_cta = (ntokens + batches - 1) / batches;
+    const double groups = K / llattn::DN_GROUP, live = std::min(groups, double(llattn::DS_WARPS));          // live: warps with a group
+    const double ctas = double(rows / 16) * batches, waves = std::max(1.0, (ctas / sms + std::ceil(ctas / sms)) / 2);
+    const double wave = 110 + 2 * live + per_cta * (0.9 + 0.14 * live);
+    return 130 + waves * std::max(1.0, groups / llattn::DS_WARPS) * wave <= 210 + 37 * groups;
+}
 }  // namespace
 
 int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int32_t* sum, float* Y, int ntokens, int rows, int K,
@@ -242,21 +255,22 @@ int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int3
             cudaFuncSetAttribute(llattn::dense_tile_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseTile<32>::SMEM);
             cudaFuncSetAttribute(llattn::dense_tile_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseTile<64>::SMEM);
         });
-    if (ntokens <= DENSE_STRIP_MAX_TOKENS) {
+    int sms = 0;
+    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (ntokens <= DENSE_STRIP_MAX_TOKENS && dense_strips_win(rows, K, ntokens, sms)) {
         const dim3 grid(rows / 16, (ntokens + llattn::DS_TOK - 1) / llattn::DS_TOK);
         llattn::dense_strip_kernel<<<grid, llattn::DS_THREADS, llattn::DS_SMEM_BYTES, as_stream(stream)>>>(p);
     } else {
         // The largest tile is the cheapest per token, as long as the tiles fill the chip: with smaller ones while they do not.
         // 2048 x 2048, in a graph: 65 .. 144 tokens 16.2 .. 16.6 us with 64 tokens a tile, 8.1 .. 8.7 with 16; 160 .. 288 tokens 16.7 and
         // 11.3 .. 11.8 (32); at 512 tokens 16.8 (64) and 17.3 (32), at 1024 26.4 and 30.7.
-        int sms = 0;
-        CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         const long long row_tiles = rows / llattn::DN_ROWS;
         auto launch = [&](auto* kernel, int tok, int smem) {
             kernel<<<dim3(rows / llattn::DN_ROWS, (ntokens + tok - 1) / tok), llattn::DT_THREADS, smem, as_stream(stream)>>>(p);
         };
-        if (row_tiles * ((ntokens + 15) / 16) <= sms) launch(llattn::dense_tile_kernel<16>, 16, llattn::DenseTile<16>::SMEM);
-        else if (row_tiles * ((ntokens + 31) / 32) <= sms) launch(llattn::dense_tile_kernel<32>, 32, llattn::DenseTile<32>::SMEM);
+        // Never a tile larger than the tokens: 32,768 rows of K = 8192 and one token 43 us with 16, 85 with 64.
+        if (ntokens <= 16 || row_tiles * ((ntokens + 15) / 16) <= sms) launch(llattn::dense_tile_kernel<16>, 16, llattn::DenseTile<16>::SMEM);
+        else if (ntokens <= 32 || row_tiles * ((ntokens + 31) / 32) <= sms) launch(llattn::dense_tile_kernel<32>, 32, llattn::DenseTile<32>::SMEM);
         else launch(llattn::dense_tile_kernel<64>, 64, llattn::DenseTile<64>::SMEM);
     }
     CU(cudaGetLastError());

@@ -106,6 +106,51 @@ def test_dense_tile_edges(api, orc, pkg, ntokens, rows, K, odd):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("ntokens,rows,K", [
+    (1, 128, 128), (32, 128, 128), (64, 2048, 128), (1, 4096, 512), (32, 4096, 512), (33, 3072, 2048), (64, 3072, 2048), (24, 6144, 2048), (33, 8192, 256),
+    (16, 12288, 256), (24, 12288, 256), (48, 12288, 256), (1, 16384, 512), (64, 16384, 512), (20, 32768, 256), (64, 32768, 256)])
+def test_dense_few_tokens_many_rows(api, orc, pkg, ntokens, rows, K):
+    """Few tokens on both sides of the line between the strip kernel and the tiles, and between the tile sizes: the same bits."""
+    wl = pkg.workload
+    strips, _, _, _ = wl.dense_weights(rows, K, 51)
+    q, s, qsum = wl.int8_activations(ntokens, K, 52)
+    want = np.random.default_rng(53).normal(size=(ntokens, rows)).astype(np.float32)
+    Y = _dev(want.copy())
+    orc.dense_w4a8(strips, q, s, qsum, want)
+    api.dense_w4a8(_dev(strips), _dev(q), _dev(s), _dev(qsum), Y)
+    assert np.array_equal(Y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,K", [(2048, 2048), (8192, 512), (16384, 512), (16384, 2048)])
+def test_dense_few_tokens_cost_no_more_than_many(api, rows, K):
+    """64 tokens take no longer than 96 of the same weights, whatever the rows, and 32 not longer than 64 (1.25 leaves room for
+    timing; choosing the kernel by the tokens alone, 64 tokens took 1.8 .. 2.7 times as long as 96 at 8192 and 16,384 rows)."""
+    ktot = K // 128
+    W = torch.randint(0, 256, (rows // 16, ktot * 1072), device="cuda", dtype=torch.uint8)
+    W[:, ktot * 1024:] = 0x11
+
+    def us(n):
+        q = torch.randint(-127, 128, (n, K), device="cuda", dtype=torch.int8)
+        s, qsum = torch.rand((n, ktot), device="cuda"), q.view(n, ktot, 128).sum(2, dtype=torch.int32)
+        Y = torch.zeros((n, rows), device="cuda")
+        api.dense_w4a8(W, q, s, qsum, Y)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(20):
+                api.dense_w4a8(W, q, s, qsum, Y)
+        best = float("inf")
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(); graph.replay(); b.record(); b.synchronize()
+            best = min(best, a.elapsed_time(b) * 1000 / 20)
+        return best
+
+    t32, t64, t96 = us(32), us(64), us(96)
+    assert t64 <= 1.25 * t96 and t32 <= 1.25 * t64, (t32, t64, t96)
+
+
+@pytest.mark.gpu
 def test_dense_bit_exact_vs_reference_kernel(api, pkg):
     import refkernel
     if not refkernel.gemm_available():
