@@ -145,14 +145,19 @@ int llattn_tile_units(void) { return llattn::TILE_UNITS; }
 // ------------------------------------------------------------------------------------------------------ commit
 
 namespace {
-// Few blocks: 512 threads a record, for the shortest chain. From the number of blocks on whose records no longer fit on the
-// chip at four of those CTAs an SM: 256 threads, eight records an SM in flight (2048 blocks 75 -> 68 us; 64
-// blocks 4.3 us with 512).
+// Few blocks: 512 threads a record, for the shortest chain. They fit on an SM three at a time (40 registers), CTAs of 256 threads
+// four at a time (56), so records pass faster through the latter once there are many waves of them: from two waves of the
+// 256-thread form on, twice as many blocks as there are SMs (a block is four CTAs). 512 / 256 threads in a graph: 1 block 3.1 /
+// 3.8 us, 64 4.4 / 4.6, 111 and 112 (the second wave of 512) 5.7 and 6.7 / 5.7 and 6.8, 128 6.9 / 7.0, 149 7.9 / 8.2, 222 9.4 / 9.6,
+// 296 11.8 / 12.0, 384 15.3 / 14.9, 1024 37.5 / 34.8, 2048 74.7 / 67.9.
 int launch_commit(const void* Kf, const void* Vf, void* records, const int32_t* pages, int max_blocks, int blk, int nb, void* stream) {
+    int dev = 0, sms = 0;
+    CU(cudaGetDevice(&dev));
+    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const dim3 grid(llattn::NKV, nb);
     const half *k = static_cast<const half*>(Kf), *v = static_cast<const half*>(Vf);
     uint8_t* r = static_cast<uint8_t*>(records);
-    if (nb <= 128) llattn::kv_commit_kernel<512><<<grid, 512, 0, as_stream(stream)>>>(k, v, r, pages, max_blocks, blk);
+    if (nb <= 2 * sms) llattn::kv_commit_kernel<512><<<grid, 512, 0, as_stream(stream)>>>(k, v, r, pages, max_blocks, blk);
     else llattn::kv_commit_kernel<256><<<grid, 256, 0, as_stream(stream)>>>(k, v, r, pages, max_blocks, blk);
     CU(cudaGetLastError());
     return LLATTN_OK;
