@@ -247,18 +247,6 @@ __device__ __forceinline__ float rowmax32(const uint32_t (&r)[32]) {
     }
     return max3(max3(a, b, __uint_as_float(r[15])), __uint_as_float(r[31]), __uint_as_float(r[31]));
 }
-// Score pairs J0 .. J1-1 of a chunk -> p = 2^(s * sl2 - mref) as packed fp16 (the multiply-add on two scores at a time).
-template <int J0, int J1>
-__device__ __forceinline__ void exp_pairs(const uint32_t (&r)[32], uint32_t (&pk)[16], unsigned long long sl2x2, unsigned long long nm2) {
-#pragma unroll
-    for (int j = J0; j < J1; ++j) {
-        if (LLATTN_SKIP & 2) { pk[j] = r[2 * j] & 0x03ff03ffu; continue; }
-        float x0, x1;
-        fma2(r[2 * j], r[2 * j + 1], sl2x2, nm2, x0, x1);
-        const half2 h = __floats2half2_rn(ex2(x0), ex2(x1));
-        pk[j] = *reinterpret_cast<const uint32_t*>(&h);
-    }
-}
 
 // Maximum of 16 scores.
 __device__ __forceinline__ float rowmax16(const uint32_t (&r)[16]) {
@@ -1111,8 +1099,8 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
 
 template <bool PRECISE>
 __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_tile_kernel(const __grid_constant__ KParams p) {
-    // reference-grid mode: the folding launch behind this one may take its place on the SMs this one leaves idle, and wait
-    // there (not in list mode: what follows there may be another cooperative launch, which needs the whole chip)
+    // reference-grid mode: the folding launch behind this one carries the attribute of a dependent launch, may take its place
+    // on the SMs this one leaves idle, and waits there (nothing behind a list-mode launch carries it)
     if (!PRECISE && !p.items) ptx::launch_dependents();
     attn_tile_body<PRECISE>(p, blockIdx.x);
 }
