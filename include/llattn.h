@@ -120,7 +120,9 @@ int llattn_attn_partial(const llattn_args* args, int nb, int* err_word, void* st
 
 /* Stands in for attn::attn_combine<<<dim3(4, 16, nb), 256, 0, st>>>(Opart, Mpart, Lpart, nchunks, nblocks, bpc,
  * O, q8, s8, sum8) (engine/attn.cu:319; call sites engine/engine.cu:432 and :598). With q8 non-null the int8
- * activation form (fragment order, per-head scale, integer sum) is written and O is not, as in the reference. */
+ * activation form (fragment order, per-head scale, integer sum) is written and O is not, as in the reference.
+ * A programmatic dependent launch: behind llattn_attn_partial it may take its place on the chip early, and it waits for all
+ * that is ahead of it before it reads or writes. In a captured graph the edge in front of it has that type. */
 int llattn_attn_combine(const float* Opart, const float* Mpart, const float* Lpart, int nchunks, int nblocks,
                         int blocks_per_chunk, void* O, int8_t* q8, float* s8, int32_t* sum8, int nb, void* stream);
 

@@ -56,8 +56,8 @@ __device__ __forceinline__ float small_int_to_float(int v) { return __int_as_flo
 // the length of the dependent chain and how many SMs pull on the weights: one CTA per (strip, 32 tokens), 128 CTAs at
 // 2048 rows, warp w on group w (w + 16, ... when K > 2048). Each warp leaves the two factors of its group's multiply-add
 // in shared memory; then thread = output element runs the sixteen in order.
-// Measured, 2048 x 2048, launches in a graph over 20 different weights: 32 tokens 3.8 us (a 128-row tile per CTA, group after group: 18.7),
-// 1 token 2.4 us.
+// Measured, 2048 x 2048, launches in a graph over 20 different weights: 32 tokens 4.0 us (a 128-row tile per CTA, group after group: 17.7),
+// 1 token 2.7 us (17.3).
 constexpr int DS_WARPS = 16, DS_THREADS = 32 * DS_WARPS, DS_TOK = 32;
 constexpr int DS_LD = 18;                          // (value, scale) pairs per token row of 16: keeps the fragment writes conflict-free
 constexpr int DS_SMEM_BYTES = DS_WARPS * DS_TOK * DS_LD * 8;
@@ -149,9 +149,9 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dense_strip_kernel(const DenseP
 // What bounds it: about 200 issue slots and 32 MMAs (8.8 cycles each on a scheduler) per warp and group of 1,024 outputs -
 // 2048 tokens x 2048 x 2048: 17 us of tensor pipe over 148 SMs - then reading and writing Y (33.6 MB, 5.1 us; brought
 // into L2 while the groups run).
-// Measured, 2048 x 2048, launches in a graph: 2048 tokens 49.4 us (a warp per strip and 64 tokens, whose
-// fragment loads took half of the shared-memory bandwidth: 54; the tcgen05 form it replaces: 61), 128 tokens 8.6 us (16-token
-// tiles; 16.6 with 64).
+// Measured, 2048 x 2048, launches in a graph: 2048 tokens 51 us (a warp per strip and 64 tokens, whose
+// fragment loads took half of the shared-memory bandwidth: 4 more; the tcgen05 form it replaces: 60), 128 tokens 8.5 us (16-token
+// tiles; 16.4 with 64).
 constexpr int DT_THREADS = 256, DT_STAGES = 4;
 template <int TOK> struct DenseTile {                              // shared-memory layout of a stage: codes, q, scales, sums, metas
     static constexpr int Q = 8 * DN_TILE_BYTES, SX = Q + TOK * 128, SQ = SX + TOK * 4, META = SQ + TOK * 4, STAGE = META + 8 * DN_META_BYTES;
