@@ -213,12 +213,13 @@ __device__ __forceinline__ void fold_row_warp(const float* Opart, const float* M
 // the warps had none and the others went through their slots in several round trips: 22 runs a tile, 7,000 cycles from the last
 // count-in to the outputs. Two warps a row up to 32 slots (at most 8 rows), four above (at most 4 rows); the planner
 // gives a tile at most 59 runs on 160 CTAs, and more would take the general form. `scratch`: 16 x 544 bytes of shared memory; every
-// thread of the CTA calls. Inlined: as a call it made the attention kernel spill (12 bytes of stores, 20 of loads), which
-// cost 1 .. 3 % everywhere (64 sequences at 32 K tokens 704 -> 688 us, 128 at 1 K 82.3 -> 80.7).
+// thread of the CTA calls. A call, with the descriptors by value: by reference they lived on the stack and the
+// attention kernel spilled around it (12 bytes of stores, 20 of loads; 64 sequences at 32 K tokens 714 us, now 698), and inlined
+// it cost the precise form up to 5 % (four passes of 9 blocks on 300 162 -> 171 us, now 158).
 constexpr int FOLD_SHARED_SLOTS = 4 * FOLD_PART;
 static_assert((QR + FOLD_PART) / (FOLD_PART + 1) <= 16 / 2 && (QR + 2 * FOLD_PART) / (2 * FOLD_PART + 1) <= 16 / 4, "rows of a CTA: one per W warps");
-__device__ __forceinline__ void fold_rows_shared(const float* Opart, const float* Mpart, const float* Lpart, const MergeDesc& md, int k, int warp,
-                                                 int lane, uint8_t* scratch, const MergeOut& o) {
+__device__ __noinline__ void fold_rows_shared(const float* Opart, const float* Mpart, const float* Lpart, const MergeDesc md, int k, int warp,
+                                              int lane, uint8_t* scratch, const MergeOut o) {
     const int n = md.nslots, W = n <= 2 * FOLD_PART ? 2 : 4;
     const int part = warp & (W - 1), per = (n + W - 1) / W, s0 = part * per, cnt = min(per, n - s0);
     const int r = k + n * (warp / W);
