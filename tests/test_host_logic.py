@@ -233,14 +233,24 @@ def _preview_us(api, lengths, nq, nctas=148, repeats=30):
     return 1e6 * best
 
 
+def _loop_us():
+    """Best time of 10,000 turns of a plain Python loop: the speed of this core, 350 us where the planner's times were taken."""
+    best = float("inf")
+    for _ in range(30):
+        t, x = time.perf_counter(), 0
+        for i in range(10000):
+            x += i
+        best = min(best, time.perf_counter() - t)
+    return 1e6 * best
+
+
 def test_planning_builds_one_plan_only(api):
-    """A serving loop replans per committed block. The limits are three to four times what choosing by cost takes on one
-    2024 server core, and a half to a third of what it took to build every candidate plan and keep one."""
+    """A serving loop replans per committed block. Choosing the way of cutting by cost takes 34, 25 and 228 us for these batches, building
+    every candidate plan and keeping one took 214, 158 and 3400; the limits lie between, for a core of this one's speed."""
     g = np.random.default_rng(3)
     ragged = [int(x) for x in g.integers(4, 1025, 256)]
-    assert _preview_us(api, ragged, [1] * 256) < 110                       # 34 us (every candidate built: 214)
-    assert _preview_us(api, [0] * 16, [16] * 16) < 80                      # 25 (158)
-    assert _preview_us(api, [100] * 256, [16] * 256) < 1000                # 228 (3400)
+    for lengths, nq, limit in ((ragged, [1] * 256, 100), ([0] * 16, [16] * 16, 75), ([100] * 256, [16] * 256, 1000)):
+        assert _preview_us(api, lengths, nq) < limit * max(1.0, _loop_us() / 350)
 
 
 def test_whole_tiles_go_to_the_least_loaded_cta_in_order_of_length(api):
