@@ -15,15 +15,15 @@
 // 16 h + 4 t + e (e = byte index), the code of row g in the low nibble and of row g + 8 in the high nibble
 // (engine/moe_i8.cu:127-160). A meta holds fp16 scale pairs (rows g | g + 8) at 4 g and zero-point pairs at 32 + 2 g.
 //
-// Both kernels use mma.sync m16n8k32 (u8 x s8 -> s32), whose fragments these layouts are: a lane's eight code words ARE its
+// The first two kernels use mma.sync m16n8k32 (u8 x s8 -> s32), whose fragments these layouts are: a lane's eight code words ARE its
 // A fragments (one nibble mask per register) and a token's B fragments are 32 contiguous bytes per lane, so operands go
 // from memory to the tensor core without being unpacked into shared memory, and the integers come out in registers,
 // where the fold into fp32 needs them. What the path costs is that fold, 16 float steps per output which cannot be
-// reordered, not the products: the tcgen05 form (unpack to shared memory, proxy fence, MMA, commit, tensor-memory load)
-// took 1.2 us for every group at any number of tokens, a chain longer than the group's arithmetic.
+// reordered, not the products.
 //   dense_strip_kernel  a decode step's few tokens: a CTA takes ONE strip and one warp per 128-group works on it; the
 //                       integers of all groups exist at once, only the multiply-adds run in group order.
 //   dense_tile_kernel   many tokens: 128 rows x 16, 32 or 64 tokens per CTA.
+//   dense_wide_kernel   more tokens, or more groups: 128 rows x 32, 64 or 128 tokens per CTA, the products on tcgen05 (kind::i8).
 #pragma once
 #include <cuda_fp16.h>
 #include "common.cuh"
@@ -41,6 +41,7 @@ struct DenseParams {
     const int32_t* sum;    // [ntokens][K / 128]
     float* Y;              // [ntokens][rows], accumulated into
     int ntokens, rows, K;
+    int* err;              // device error word, or null
 };
 
 __device__ __forceinline__ void mma_m16n8k32_u8s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -283,6 +284,311 @@ __global__ void __launch_bounds__(DT_THREADS, TOK == 64 ? 2 : 3) dense_tile_kern
                     __stcg(ybase + size_t(8 * k + (e & 1)) * p.rows + 16 * u + 8 * (e >> 1), y[k][e] + __uint_as_float(uint32_t(e & 1 ? v >> 32 : v)));
                 }
     }
+}
+
+// ------------------------------------------------------------------------------------------------------- very many tokens
+// CTA = 128 rows x N tokens, one per SM, the products on tcgen05 kind::i8 (u8 x s8, M = 128), four times as fast as mma.sync
+// here, so that the fold is what is left: sixteen warps, six instructions per two outputs and group. The other roles run ahead of them through rings whose slots hold TWO groups: a warp by itself issues an instruction
+// every five cycles or so, and with a slot per group the barriers' instructions alone took a role 1,500 cycles a group.
+//   producer warp  bulk copies of the strips' codes into a ring, 2 KB a copy
+//   unpack warps   codes -> u8 rows in the 128-byte-swizzle operand layout
+//   load warps     activations, cp.async straight into the operand layout (completion by mbarrier, no waiting)
+//   MMA warp       four K-steps a group into one of four accumulators
+// The factors of the fold (token scales and sums, row scales and zero points) of sixteen groups lie in shared memory as floats.
+// Measured, 2048 x 2048, launches in a graph, mma.sync tiles / this: 320 tokens 16.7 / 12.3 us, 640 26.5 / 17.9, 1024 26.0 / 17.6, 2048
+// 49.2 / 34.3. 1024 tokens are one CTA on 128 SMs: 0.66 us a group, half of the issue slots (16 folding warps x 110 instructions and the
+// unpacking), and 7 us before the first and behind the last.
+constexpr int DW_FOLD_WARPS = 16, DW_UNPACK_WARPS = 4, DW_LOAD_WARPS = 1;
+constexpr int DW_WARP_UNPACK = DW_FOLD_WARPS, DW_WARP_LOAD = DW_WARP_UNPACK + DW_UNPACK_WARPS, DW_WARP_PRODUCER = DW_WARP_LOAD + DW_LOAD_WARPS,
+              DW_WARP_MMA = DW_WARP_PRODUCER + 1, DW_THREADS = 32 * (DW_WARP_MMA + 1);
+constexpr int DW_RAW = 2, DW_A = 2, DW_B = 2, DW_ACC = 4, DW_SC = 16;      // ring slots; groups of factors held
+template <int N> struct DenseWide {
+    static constexpr int A_GROUP = DN_ROWS * DN_GROUP, B_GROUP = N * DN_GROUP, RAW_GROUP = 8 * DN_TILE_BYTES;
+    static constexpr int A = 0, B = A + DW_A * 2 * A_GROUP, RAW = B + DW_B * 2 * B_GROUP;
+    static constexpr int LD_T = N + 4, LD_R = DN_ROWS + 1;                 // a group's token factors and rows, padded for the transposing stores
+    static constexpr int SX = RAW + DW_RAW * 2 * RAW_GROUP, SQ = SX + DW_SC * LD_T * 4, WZ = SQ + DW_SC * LD_T * 4;
+    static constexpr int BAR = WZ + DW_SC * LD_R * 8, SMEM = BAR + 8 * 32;
+    static constexpr int COLS = N / 4;                                     // a fold warp's tokens
+    static constexpr int TMEM = DW_ACC * N;
+};
+enum { WB_RAW_FULL = 0, WB_RAW_EMPTY = WB_RAW_FULL + DW_RAW, WB_A_FULL = WB_RAW_EMPTY + DW_RAW, WB_A_EMPTY = WB_A_FULL + DW_A,
+       WB_B_FULL = WB_A_EMPTY + DW_A, WB_B_EMPTY = WB_B_FULL + DW_B, WB_ACC_FULL = WB_B_EMPTY + DW_B, WB_ACC_EMPTY = WB_ACC_FULL + DW_ACC,
+       WB_SC_FULL = WB_ACC_EMPTY + DW_ACC, WB_SC_EMPTY, WB_SPARE, WB_COUNT };
+static_assert(WB_COUNT <= 32, "barrier area");
+
+// kind::i8 instruction descriptor: s32 accumulator, A u8 (format 0), B s8 (format 1), both K-major.
+__host__ __device__ constexpr uint32_t idesc_i8_u8s8(int M, int N) {
+    return (2u << 4) | (0u << 7) | (1u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
+}
+// A group: four K-steps of 32 over 128-byte-swizzle tiles, the first overwriting the accumulator, and a commit.
+__device__ __forceinline__ void mma_i8_group_warp(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred pe, pf, pt;\n\t.reg .b32 x, y;\n\t.reg .b64 da, db;\n\t"
+        "elect.sync _|pe, 0xffffffff;\n\t"
+        "setp.ne.b32 pf, 0, 0;\n\t setp.eq.b32 pt, 0, 0;\n\t"
+        "mov.b64 da, {%1, %3};\n\t mov.b64 db, {%2, %3};\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, pf;\n\t"
+        "add.u32 x, %1, 2;\n\t add.u32 y, %2, 2;\n\t mov.b64 da, {x, %3};\n\t mov.b64 db, {y, %3};\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, pt;\n\t"
+        "add.u32 x, %1, 4;\n\t add.u32 y, %2, 4;\n\t mov.b64 da, {x, %3};\n\t mov.b64 db, {y, %3};\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, pt;\n\t"
+        "add.u32 x, %1, 6;\n\t add.u32 y, %2, 6;\n\t mov.b64 da, {x, %3};\n\t mov.b64 db, {y, %3};\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, pt;\n\t"
+        "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
+        "}\n" :: "r"(d), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(bar) : "memory");
+}
+// An arrival on `bar` once this thread's cp.async so far have landed.
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory"); }
+
+template <int N>
+__global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DenseParams p) {
+    using T = DenseWide<N>;
+    extern __shared__ __align__(1024) uint8_t dw_smem[];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_word;
+    volatile int* const abort_flag = &abort_word;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row0 = blockIdx.x * DN_ROWS, n0 = blockIdx.y * N, live = min(N, p.ntokens - n0);
+    const int ktot = p.K / DN_GROUP, nst = (ktot + 1) / 2;       // stages: two groups each, the last one perhaps a single one
+    const uint32_t sm0 = ptx::smem_u32(dw_smem), bar0 = sm0 + T::BAR;
+    auto BAR = [&](int i) -> uint32_t { return bar0 + 8u * uint32_t(i); };
+    if (sm0 & 1023u) {                         // the swizzled tiles need a 1024-byte aligned base: report, do nothing
+        if (tid == 0 && p.err) atomicOr(p.err, ERR_SMEM_ALIGN);
+        return;
+    }
+    if (tid == 0) {
+        for (int i = 0; i < DW_RAW; ++i) { ptx::mbar_init(BAR(WB_RAW_FULL + i), 1); ptx::mbar_init(BAR(WB_RAW_EMPTY + i), 32 * DW_UNPACK_WARPS); }
+        for (int i = 0; i < DW_A; ++i) { ptx::mbar_init(BAR(WB_A_FULL + i), 32 * DW_UNPACK_WARPS); ptx::mbar_init(BAR(WB_A_EMPTY + i), 1); }
+        for (int i = 0; i < DW_B; ++i) { ptx::mbar_init(BAR(WB_B_FULL + i), 32 * DW_LOAD_WARPS); ptx::mbar_init(BAR(WB_B_EMPTY + i), 1); }
+        for (int i = 0; i < DW_ACC; ++i) { ptx::mbar_init(BAR(WB_ACC_FULL + i), 1); ptx::mbar_init(BAR(WB_ACC_EMPTY + i), 32 * DW_FOLD_WARPS); }
+        ptx::mbar_init(BAR(WB_SC_FULL), 32 * DW_FOLD_WARPS); ptx::mbar_init(BAR(WB_SC_EMPTY), 32 * DW_FOLD_WARPS);
+        ptx::mbar_init(BAR(WB_SPARE), 1);
+        ptx::fence_mbar_init();
+        abort_word = 0;
+    }
+    if (warp == DW_WARP_MMA) { ptx::tmem_alloc(ptx::smem_u32(&tmem_slot), T::TMEM); ptx::tmem_relinquish(); }
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    const size_t strip_bytes = size_t(ktot) * (DN_TILE_BYTES + DN_META_BYTES);
+    const uint8_t* strips = p.W + size_t(row0 >> 4) * strip_bytes;
+    int errbits = 0;
+    // wait for use `u` of a slot to be filled / for the previous use of a slot to be over (the first needs no wait)
+    auto filled = [&](int bar, int u, int err) -> bool {
+        if (ptx::mbar_wait(BAR(bar), u & 1, abort_flag)) return true;
+        errbits |= err;
+        return false;
+    };
+    auto emptied = [&](int bar, int u, int err) -> bool { return u == 0 || filled(bar, u - 1, err); };
+
+    if (warp < DW_FOLD_WARPS) {
+        // ---- fold: a warp has 32 rows and COLS tokens, as an mma fragment: lane l rows l / 4 + 8 k, tokens 8 i + 2 (l % 4) and + 1. Two token
+        // factors then serve eight outputs (with a row a lane: two), and 80 registers a thread do without spills.
+        constexpr int C = T::COLS;
+        const int row = 32 * (warp & 3) + (lane >> 2), col = C * (warp >> 2) + 2 * (lane & 3);
+        const uint32_t tacc = tmem + (uint32_t(32 * (warp & 3)) << 16) + C * (warp >> 2);
+        float* const sx = reinterpret_cast<float*>(dw_smem + T::SX);
+        float* const sq = reinterpret_cast<float*>(dw_smem + T::SQ);
+        float2* const wz = reinterpret_cast<float2*>(dw_smem + T::WZ);
+        f32x2 c[C / 8][4];                             // per eight tokens: rows row, + 8, + 16, + 24
+#pragma unroll
+        for (int j = 0; j < C / 2; ++j) (&c[0][0])[j] = 0ull;
+        const f32x2 magic = 0xCB400000CB400000ull;     // -1.5 * 2^23 twice
+        bool alive = true;
+#pragma unroll 1
+        for (int g0 = 0, u = 0; g0 < ktot && alive; g0 += DW_SC, ++u) {
+            // the factors of the next sixteen groups: thread = (token or row, group)
+            if (!emptied(WB_SC_EMPTY, u, ERR_WAIT_SOFTMAX)) { alive = false; break; }
+            const int g = tid & 15, gi = min(g0 + g, ktot - 1);
+#pragma unroll
+            for (int k = 0; k < (N + 31) / 32; ++k) {
+                const int n = (tid >> 4) + 32 * k;
+                const size_t at = size_t(n0 + min(n, live - 1)) * ktot + gi;
+                sx[g * T::LD_T + n] = __ldg(p.s + at);
+                sq[g * T::LD_T + n] = float(__ldg(p.sum + at));
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int r = (tid >> 4) + 32 * k, rr = r & 15;
+                const uint8_t* mt = strips + size_t(r >> 4) * strip_bytes + size_t(ktot) * DN_TILE_BYTES + size_t(gi) * DN_META_BYTES;
+                wz[g * T::LD_R + r] = make_float2(__half2float(__ushort_as_half(__ldg(reinterpret_cast<const uint16_t*>(mt + 4 * (rr & 7) + 2 * (rr >> 3))))),
+                                                  -float(__ldg(mt + 32 + 2 * (rr & 7) + (rr >> 3))));
+            }
+            ptx::mbar_arrive(BAR(WB_SC_FULL));
+            if (!filled(WB_SC_FULL, u, ERR_WAIT_SOFTMAX)) { alive = false; break; }
+            const int ng = min(DW_SC, ktot - g0);
+#pragma unroll 1
+            for (int i = 0; i < ng; ++i) {
+                const int slot = i % DW_ACC;           // DW_SC is a multiple of DW_ACC
+                f32x2 sw[4], nz[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float2 f = wz[i * T::LD_R + row + 8 * k];
+                    sw[k] = pack2(__float_as_uint(f.x), __float_as_uint(f.x)); nz[k] = pack2(__float_as_uint(f.y), __float_as_uint(f.y));
+                }
+                if (!filled(WB_ACC_FULL + slot, (g0 + i) / DW_ACC, ERR_WAIT_SOFTMAX)) { alive = false; break; }
+                ptx::tc_fence_after();
+                constexpr int H = C < 16 ? C : 16;     // tokens a round
+#pragma unroll
+                for (int h = 0; h < C; h += H) {
+                    uint32_t d0[H / 2], d1[H / 2];     // rows + 0, + 8 and rows + 16, + 24
+                    ptx::tmem_ld16x256_cols(tacc + slot * N + h, d0);
+                    ptx::tmem_ld16x256_cols(tacc + slot * N + h + (16u << 16), d1);
+                    ptx::tmem_wait_ld_tied(d0);
+                    ptx::tmem_wait_ld_tied(d1);
+                    if (h + H == C) {
+                        ptx::tc_fence_before();
+                        ptx::mbar_arrive(BAR(WB_ACC_EMPTY + slot));
+                    }
+#pragma unroll
+                    for (int j = 0; j < H / 8; ++j) {
+                        const f32x2 x = *reinterpret_cast<const f32x2*>(sx + i * T::LD_T + col + h + 8 * j), q = *reinterpret_cast<const f32x2*>(sq + i * T::LD_T + col + h + 8 * j);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const uint32_t *d = (k < 2 ? d0 : d1) + 4 * j + 2 * (k & 1);
+                            // float(P - z sq) = (1.5 * 2^23 + P) + (-z sq - 1.5 * 2^23): both terms are whole numbers below 2^24 in
+                            // magnitude (|P|, |z sq| <= 255 * 128 * 128 = 4,177,920), so every step is exact
+                            const f32x2 v = add2(pack2(d[0] + 0x4B400000u, d[1] + 0x4B400000u), fma2v(nz[k], q, magic));
+                            f32x2& o = c[h / 8 + j][k];
+                            o = fma2v(mul2(sw[k], x), v, o);
+                        }
+                    }
+                }
+            }
+            if (g0 + DW_SC < ktot) ptx::mbar_arrive(BAR(WB_SC_EMPTY));
+        }
+        if (alive) {
+            // Y += c: a warp's access is eight rows of four tokens, whole sectors; all loads of eight tokens before the first add
+            float* y0 = p.Y + size_t(n0 + col) * p.rows + row0 + row;
+#pragma unroll
+            for (int j = 0; j < C / 8; ++j) {
+                float y[4][2];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) y[k][e] = col + 8 * j + e < live ? __ldcg(y0 + size_t(8 * j + e) * p.rows + 8 * k) : 0.f;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        if (col + 8 * j + e < live)
+                            __stcg(y0 + size_t(8 * j + e) * p.rows + 8 * k, y[k][e] + __uint_as_float(uint32_t(e ? c[j][k] >> 32 : c[j][k])));
+            }
+        }
+    } else if (warp < DW_WARP_LOAD) {
+        // ---- unpack: this warp's two strips of every group. Word k of lane l = 4 g + t holds the codes at fragment positions
+        // 32 t + 4 k .. + 3, of row g in the low nibbles and of row g + 8 in the high ones: words 0-3 are the 16-byte chunk 2 t of these
+        // rows, words 4-7 chunk 2 t + 1. A quarter warp's stores cover eight chunk positions.
+        const int g = lane >> 2, t = lane & 3, s0 = 2 * (warp - DW_WARP_UNPACK);
+        const uint32_t m = 0x0F0F0F0Fu;
+        const uint8_t* const src = dw_smem + T::RAW + s0 * 2 * DN_TILE_BYTES + 16 * lane;
+        uint8_t* const dst0 = dw_smem + T::A + (16 * s0 + g) * 128 + (((2 * t) ^ g) << 4);
+        uint8_t* const dst1 = dw_smem + T::A + (16 * s0 + g) * 128 + (((2 * t + 1) ^ g) << 4);
+#pragma unroll 1
+        for (int i = 0; i < nst; ++i) {
+            const int b = i & 1, u = i >> 1;
+            static_assert(DW_RAW == 2 && DW_A == 2 && DW_B == 2, "slot = stage % 2");
+            if (!filled(WB_RAW_FULL + b, u, ERR_WAIT_DEQUANT) || !emptied(WB_A_EMPTY + b, u, ERR_WAIT_DEQUANT)) break;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {              // the stage's groups (a missing one is whatever the slot held: no MMA reads it)
+                uint4 w[2][2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        w[k][h] = *reinterpret_cast<const uint4*>(src + b * 2 * T::RAW_GROUP + k * 2 * DN_TILE_BYTES + e * DN_TILE_BYTES + 512 * h);
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        uint8_t* a = (h ? dst1 : dst0) + (2 * b + e) * T::A_GROUP + 16 * k * 128;
+                        const uint4 x = w[k][h];
+                        *reinterpret_cast<uint4*>(a) = make_uint4(x.x & m, x.y & m, x.z & m, x.w & m);
+                        *reinterpret_cast<uint4*>(a + 8 * 128) = make_uint4((x.x >> 4) & m, (x.y >> 4) & m, (x.z >> 4) & m, (x.w >> 4) & m);
+                    }
+            }
+            ptx::mbar_arrive(BAR(WB_RAW_EMPTY + b));
+            ptx::fence_proxy_async_smem();
+            ptx::mbar_arrive(BAR(WB_A_FULL + b));
+        }
+    } else if (warp < DW_WARP_PRODUCER) {
+        // ---- activations: 16-byte chunk c of token n at chunk position c ^ (n % 8), zeros for tokens past the end
+        const int lt = tid - 32 * DW_WARP_LOAD, n = lt >> 3, cc = lt & 7;
+        constexpr int STEP = 32 * DW_LOAD_WARPS / 8;   // tokens a round
+        const uint32_t dst = sm0 + T::B + n * 128 + ((cc ^ (n & 7)) << 4);
+        const int8_t* const src = p.q + size_t(n0) * p.K + 16 * cc;
+        const size_t step = size_t(STEP) * p.K;
+#pragma unroll 1
+        for (int i = 0; i < nst; ++i) {
+            const int b = i & 1;
+            if (!emptied(WB_B_EMPTY + b, i >> 1, ERR_WAIT_PRODUCER)) break;
+            const bool two = 2 * i + 1 < ktot;
+            const int8_t* at = src + size_t(n) * p.K + size_t(2 * i) * DN_GROUP;
+#pragma unroll
+            for (int k = 0; k < N / STEP; ++k, at += step) {
+                const bool on = n + STEP * k < live;
+                const int8_t* from = on ? at : src;
+                const uint32_t to = (dst ^ (STEP == 4 ? 64 * (k & 1) : 0)) + b * 2 * T::B_GROUP + k * STEP * 128;      // token n + 4: the other half of the chunks
+                cp_async16(to, from, on);
+                if (two) cp_async16(to + T::B_GROUP, from + (on ? DN_GROUP : 0), on);
+            }
+            cp_async_arrive(BAR(WB_B_FULL + b));
+            // the tile's part of Y into L2, wanted when the last group is folded
+            if (i == 0)
+                for (int k = lt; k < live * 4; k += 32 * DW_LOAD_WARPS) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.Y + size_t(n0 + (k >> 2)) * p.rows + row0 + 32 * (k & 3)));
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+    } else if (warp == DW_WARP_PRODUCER) {
+        // ---- codes by bulk copy, one strip a lane
+        int issued = 0;
+#pragma unroll 1
+        for (int i = 0; i < nst; ++i) {
+            const int b = i & 1;
+            if (!emptied(WB_RAW_EMPTY + b, i >> 1, ERR_WAIT_PRODUCER)) break;
+            const uint32_t bytes = 2 * i + 1 < ktot ? 2 * DN_TILE_BYTES : DN_TILE_BYTES;
+            if (lane == 0) ptx::mbar_arrive_expect_tx(BAR(WB_RAW_FULL + b), 8 * bytes);
+            __syncwarp();
+            if (lane < 8)
+                ptx::bulk_g2s(sm0 + T::RAW + b * 2 * T::RAW_GROUP + lane * 2 * DN_TILE_BYTES, strips + lane * strip_bytes + size_t(2 * i) * DN_TILE_BYTES, bytes, BAR(WB_RAW_FULL + b));
+            issued = i + 1;
+        }
+        // copies still in flight must land before the shared memory is given back
+        if (*abort_flag)
+            for (int k = max(0, issued - DW_RAW); k < issued; ++k) {
+                volatile int never = 0;
+                ptx::mbar_wait(BAR(WB_RAW_FULL + (k & 1)), (k >> 1) & 1, &never);
+            }
+    } else {
+        // ---- MMA issue (one elected lane issues, the warp stays together)
+        const uint32_t hi = ptx::desc_hi(1024) | (2u << 29), idesc = idesc_i8_u8s8(DN_ROWS, N);
+        const uint32_t a_lo = ptx::desc_lo(sm0 + T::A, 16), b_lo = ptx::desc_lo(sm0 + T::B, 16);
+        bool alive = true;
+#pragma unroll 1
+        for (int i = 0; i < nst && alive; ++i) {
+            const int b = i & 1, u = i >> 1;
+            if (!filled(WB_B_FULL + b, u, ERR_WAIT_MMA) || !filled(WB_A_FULL + b, u, ERR_WAIT_MMA)) break;
+            ptx::fence_proxy_async_smem();             // the activations, written by other threads' cp.async and seen through the barrier
+#pragma unroll 1
+            for (int e = 0; e < 2; ++e) {
+                const int gi = 2 * i + e, slot = gi % DW_ACC;
+                if (gi >= ktot) break;
+                if (!emptied(WB_ACC_EMPTY + slot, gi / DW_ACC, ERR_WAIT_MMA)) { alive = false; break; }
+                ptx::tc_fence_after();
+                mma_i8_group_warp(tmem + slot * N, a_lo + (2 * b + e) * (T::A_GROUP / 16), b_lo + (2 * b + e) * (T::B_GROUP / 16), hi, idesc, BAR(WB_ACC_FULL + slot));
+            }
+            ptx::mma_commit_warp(BAR(WB_A_EMPTY + b));
+            ptx::mma_commit_warp(BAR(WB_B_EMPTY + b));
+        }
+        ptx::mma_commit_warp(BAR(WB_SPARE));           // every MMA issued must have retired before tensor memory is released
+        volatile int never = 0;
+        if (!ptx::mbar_wait(BAR(WB_SPARE), 0, &never)) errbits |= ERR_WAIT_TEARDOWN;
+    }
+    if (errbits && p.err) atomicOr(p.err, errbits);
+    ptx::tc_fence_before();
+    __syncthreads();
+    if (warp == DW_WARP_MMA) ptx::tmem_dealloc(tmem, T::TMEM);
 }
 
 }  // namespace llattn

@@ -238,6 +238,34 @@ bool dense_strips_win(int rows, int K, int ntokens, int sms) {
     const double wave = 110 + 2 * live + per_cta * (0.9 + 0.14 * live);
     return 130 + waves * std::max(1.0, groups / llattn::DS_WARPS) * wave <= 210 + 37 * groups;
 }
+
+// Tokens per CTA of the tcgen05 form, or 0 where the mma.sync tiles are the faster ones. A CTA of the former fills an SM and has a
+// long start (tensor memory, four roles, sixteen groups' factors), so it wins with the groups and with the tokens; the line follows
+// both sides' measured costs in microseconds, in a graph over 1024 .. 8192 rows, K = 128 .. 8192 and 80 .. 2560 tokens. 2048 rows,
+// tiles / tcgen05 with 32, 64 and 128 tokens: K = 2048, 80 tokens 8.4 / 10.4, 12.2, 17.1, 160 11.0 / 10.5, 12.2, 17.8, 320 16.7 / 19.1,
+// 12.3, 17.6, 640 26.5 / 28.3, 23.0, 17.9, 2560 62 / 82, 56, 51; K = 512, 320 tokens 6.7 / 10.4, 7.1, 9.6, 2560 22.7 / 43, 30, 26.5.
+int dense_wide_tokens(int rows, int K, int ntokens, int sms) {
+    if (ntokens <= 32) return 0;
+    const double groups = K / llattn::DN_GROUP, row_tiles = rows / llattn::DN_ROWS;
+    auto ctas = [&](int tok) { return row_tiles * ((ntokens + tok - 1) / tok); };
+    double best;
+    if (ctas(16) <= sms) best = 2.1 + 0.38 * groups;
+    else if (ctas(32) <= sms) best = 2.3 + 0.54 * groups;
+    else if (ctas(64) <= sms) best = 2.6 + 0.88 * groups;
+    else {                                     // two CTAs an SM; a partly filled last wave counts half
+        const double waves = ctas(64) / (2 * sms);
+        best = std::max(1.0, (waves + std::ceil(waves)) / 2) * (2.9 + 1.42 * groups);
+    }
+    int wide = 0;
+    auto consider = [&](int tok, double start, double group) {
+        const double cost = std::ceil(ctas(tok) / sms) * (start + group * groups);
+        if (cost < best) { best = cost; wide = tok; }
+    };
+    consider(32, 4.7, 0.355);
+    consider(64, 5.4, 0.42);
+    consider(128, 6.9, 0.67);
+    return wide;
+}
 }  // namespace
 
 int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int32_t* sum, float* Y, int ntokens, int rows, int K,
@@ -246,10 +274,9 @@ int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int3
     if (ntokens < 0 || ntokens > 1 << 22) return fail(LLATTN_EINVAL, "dense_w4a8: ntokens = %d", ntokens);
     if (rows <= 0 || rows % llattn::DN_ROWS || K <= 0 || K % llattn::DN_GROUP || K > 1 << 20 || rows > 1 << 20)
         return fail(LLATTN_EINVAL, "dense_w4a8: rows = %d, K = %d (both multiples of 128)", rows, K);
-    (void)err_word;
     if (ntokens == 0) return LLATTN_OK;
     if (!aligned16(W) || !aligned16(q)) return fail(LLATTN_EINVAL, "dense_w4a8: W and q must be 16-byte aligned");
-    const llattn::DenseParams p{static_cast<const uint8_t*>(W), q, s, sum, Y, ntokens, rows, K};
+    const llattn::DenseParams p{static_cast<const uint8_t*>(W), q, s, sum, Y, ntokens, rows, K, err_word};
     static std::once_flag once[64];
     int dev = 0;
     CU(cudaGetDevice(&dev));
@@ -259,12 +286,20 @@ int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int3
             cudaFuncSetAttribute(llattn::dense_tile_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseTile<16>::SMEM);
             cudaFuncSetAttribute(llattn::dense_tile_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseTile<32>::SMEM);
             cudaFuncSetAttribute(llattn::dense_tile_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseTile<64>::SMEM);
+            cudaFuncSetAttribute(llattn::dense_wide_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseWide<32>::SMEM);
+            cudaFuncSetAttribute(llattn::dense_wide_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseWide<64>::SMEM);
+            cudaFuncSetAttribute(llattn::dense_wide_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseWide<128>::SMEM);
         });
     int sms = 0;
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (ntokens <= DENSE_STRIP_MAX_TOKENS && dense_strips_win(rows, K, ntokens, sms)) {
         const dim3 grid(rows / 16, (ntokens + llattn::DS_TOK - 1) / llattn::DS_TOK);
         llattn::dense_strip_kernel<<<grid, llattn::DS_THREADS, llattn::DS_SMEM_BYTES, as_stream(stream)>>>(p);
+    } else if (const int wide = dense_wide_tokens(rows, K, ntokens, sms)) {
+        const dim3 grid(rows / llattn::DN_ROWS, (ntokens + wide - 1) / wide);
+        if (wide == 32) llattn::dense_wide_kernel<32><<<grid, llattn::DW_THREADS, llattn::DenseWide<32>::SMEM, as_stream(stream)>>>(p);
+        else if (wide == 64) llattn::dense_wide_kernel<64><<<grid, llattn::DW_THREADS, llattn::DenseWide<64>::SMEM, as_stream(stream)>>>(p);
+        else llattn::dense_wide_kernel<128><<<grid, llattn::DW_THREADS, llattn::DenseWide<128>::SMEM, as_stream(stream)>>>(p);
     } else {
         // The largest tile is the cheapest per token, as long as the tiles fill the chip: with smaller ones while they do not.
         // 2048 x 2048, in a graph: 65 .. 144 tokens 16.2 .. 16.6 us with 64 tokens a tile, 8.1 .. 8.7 with 16; 160 .. 288 tokens 16.7 and

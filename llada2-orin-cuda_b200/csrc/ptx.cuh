@@ -157,6 +157,22 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
                  :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
+// 16 lanes (lane field of taddr: the warp's quarter, + 16 for its second half) as an mma C fragment: thread t has columns 8 i + 2 (t % 4)
+// and + 1 of lane t / 4 in r[4 i], r[4 i + 1] and of lane t / 4 + 8 in r[4 i + 2], r[4 i + 3]. 8 or 16 columns.
+__device__ __forceinline__ void tmem_ld16x256_cols(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16x256_cols(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld_tied(uint32_t (&r)[4]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]) :: "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld_tied(uint32_t (&r)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]) :: "memory");
+}
+
 // ---------------------------------------------------------------------------------------------- tcgen05 MMA
 // Shared-memory operands are described by 64-bit descriptors: start address, LBO and SBO in 16-byte units, a version bit and
 // the swizzle mode (desc_lo, desc_hi below; 2 << 61 = 128-byte swizzle: rows of 128 bytes, the 16-byte chunk c of row r

@@ -203,3 +203,27 @@ def test_dense_argument_errors(api):
         api.lib().llattn_dense_w4a8  # symbol exists
         api._check(api.lib().llattn_dense_w4a8(t.data_ptr(), t.data_ptr(), t.data_ptr(), t.data_ptr(), t.data_ptr(), 32, 100, 128, None, None))
     assert e.value.code == api.EINVAL
+
+
+# Where the tcgen05 form takes over: 32, 64 and 128 tokens a CTA, with a ragged last tile, one and several waves, an odd number of
+# groups (a stage of one), and more groups than factors held at a time (16)
+@pytest.mark.gpu
+@pytest.mark.parametrize("ntokens,rows,K", [
+    (149, 2048, 2048), (160, 2048, 2176), (289, 2048, 2048), (321, 2048, 2176), (577, 2048, 2048), (641, 2048, 1152), (1153, 2048, 2048),
+    (2049, 1024, 4224), (65, 8192, 2048), (200, 8192, 4224)])
+def test_dense_tcgen05_form(api, orc, pkg, ntokens, rows, K):
+    wl = pkg.workload
+    strips, _, _, _ = wl.dense_weights(rows, K, 41)
+    strips = strips.copy()
+    strips[:, K // 128 * 1024:].reshape(-1, K // 128, 48)[:, ::3, 32:] = 255          # zero points up to the largest
+    q, s, qsum = wl.int8_activations(ntokens, K, 42)
+    q, qsum = q.copy(), qsum.copy()
+    q.reshape(ntokens, -1, 128)[::5, ::2] = -127                                     # and sums down to the smallest
+    qsum.reshape(ntokens, -1)[::5, ::2] = -127 * 128
+    Y0 = np.random.default_rng(43).normal(size=(ntokens, rows)).astype(np.float32)
+    want = Y0.copy()
+    orc.dense_w4a8(strips, q, s, qsum, want)
+    Y, err = _dev(Y0), torch.zeros(1, dtype=torch.int32, device="cuda")
+    api.dense_w4a8(_dev(strips), _dev(q), _dev(s), _dev(qsum), Y, err_word=err)
+    assert int(err.item()) == 0
+    assert np.array_equal(Y.cpu().numpy().view(np.uint32), want.view(np.uint32))
