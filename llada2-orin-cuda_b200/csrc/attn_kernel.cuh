@@ -12,7 +12,8 @@
 //                   O += P V   (A = P read from TMEM as packed fp16, B = V MN-major in shared memory, fp32 O in TMEM);
 //                   V carries one extra column of ones, so the same MMA also accumulates the softmax row sum from
 //                   exactly the fp16 P the numerator uses (numerator and denominator then share their rounding)
-//   softmax warps : four warps, one thread per query row (TMEM lane), all keys of the row: no exchange between warps.
+//   softmax warps : four warps, one thread per query row (TMEM lane), all keys of the row: no exchange between warps (the
+//                   precise form: eight warps, four threads per row, see softmax_tile_rows16).
 //                   One pass per tile: p = 2^(s*scale*log2e - mref) for 16 scores at a time while the next 16 arrive
 //                   from tensor memory, the chunk maximum taken on the way; P goes back over S in TMEM as fp16 pairs
 //                   (the 32 keys of chunk g at columns 32 g .. 32 g + 15, the first half of the S columns they were
@@ -88,7 +89,9 @@ constexpr int SM_FIRST = SM_MISC + 16;             // the CTA's first run descri
 // A softmax warp's way between its row-per-thread tensor memory and row-major global memory: 32 rows x 128 bytes, the 16-byte
 // chunk c of row r at chunk position c ^ (r % 8). Without it a warp's 16-byte accesses touch 32 lines each.
 constexpr int SM_STAGE = (SM_FIRST + int(sizeof(RunDesc)) + 127) / 128 * 128, STAGE_BYTES = 32 * 128;
-constexpr int ATTN_SMEM_BYTES = SM_STAGE + 4 * STAGE_BYTES;
+constexpr int SM_ROWREF = SM_STAGE + 4 * STAGE_BYTES;    // precise form: the run's final reference exponents, one per query row,
+constexpr int SM_QSUM = SM_ROWREF + QR * 4;              // and for the int8 output the code sums of dims 64 .. 127
+constexpr int ATTN_SMEM_BYTES = SM_QSUM + QR * 4;
 // warps 0-3 softmax (warp w: TMEM lanes 32 w .. 32 w + 31, one query row per thread), 4-11 dequant (four groups of two
 // warps, group g takes unit g of every tile: a thread's scale / minimum words then serve eight passes over the record),
 // then the service warps. Every scheduler carries one softmax warp, two dequantising warps and one service warp.
@@ -104,14 +107,14 @@ constexpr int ATTN_SMEM_BYTES = SM_STAGE + 4 * STAGE_BYTES;
 #ifndef LLATTN_WARP_ARRIVE
 #define LLATTN_WARP_ARRIVE 0       // 1: one arrival per softmax warp on the P barrier instead of one per thread
 #endif
-constexpr int SOFTMAX_WARPS = 4, DEQUANT_WARPS = LLATTN_DEQUANT_WARPS, GROUP_WARPS = LLATTN_GROUP_WARPS, DEQUANT_GROUPS = DEQUANT_WARPS / GROUP_WARPS;
+__host__ __device__ constexpr int softmax_warps(bool precise) { return precise ? 8 : 4; }
+constexpr int DEQUANT_WARPS = LLATTN_DEQUANT_WARPS, GROUP_WARPS = LLATTN_GROUP_WARPS, DEQUANT_GROUPS = DEQUANT_WARPS / GROUP_WARPS;
 constexpr int GROUP_THREADS = 32 * GROUP_WARPS, DQ_PASSES = 16 / GROUP_WARPS;      // a group converts one record: 32 keys, two per warp and pass
-constexpr int WARP_SERVICE = SOFTMAX_WARPS + DEQUANT_WARPS;
 // Service warps, one per scheduler (a warp runs on scheduler warp % 4 and the softmax warps cannot move): PV issue, S
 // issue and two copy producers that take alternate records, so that no scheduler carries much more than the others.
-constexpr int WARP_MMA_PV = WARP_SERVICE, WARP_MMA = WARP_SERVICE + 1, WARP_PRODUCER = WARP_SERVICE + 2, PRODUCERS = 2;
-constexpr int ATTN_THREADS = 32 * (WARP_SERVICE + 2 + PRODUCERS);  // 512
-constexpr int P_ARRIVALS = LLATTN_WARP_ARRIVE ? SOFTMAX_WARPS : 32 * SOFTMAX_WARPS;
+constexpr int PRODUCERS = 2;
+__host__ __device__ constexpr int attn_threads(bool precise) { return 32 * (softmax_warps(precise) + DEQUANT_WARPS + 2 + PRODUCERS); }
+constexpr int ATTN_THREADS = attn_threads(false);  // 512; 640 in the precise form
 constexpr int TMEM_COLS = 512;
 constexpr int TM_S = 0, TM_O = 256, TM_L = TM_O + 128, TM_Q = 400;   // S at columns 0 and 128, O at 256..383, row sum at 384, Q at 400..463
 // The reference exponent of a row moves when a score exceeds it by more than this many powers of two, the reference's own
@@ -122,7 +125,7 @@ constexpr float RESCALE_SLACK = 8.f;
 // barrier indices
 enum { B_RAW_FULL = 0, B_RAW_EMPTY = B_RAW_FULL + NRAW, B_K_FULL = B_RAW_EMPTY + NRAW, B_V_FULL = B_K_FULL + 2,
        B_K_FREE = B_V_FULL + 2, B_PV_DONE = B_K_FREE + 2, B_S_FULL = B_PV_DONE + 2, B_P_FULL = B_S_FULL + 2,
-       B_Q_FULL = B_P_FULL + 2, B_O_FREE, B_SPARE, B_COUNT = B_SPARE + 2 };
+       B_Q_FULL = B_P_FULL + 2, B_O_FREE, B_QSUM, B_SPARE, B_COUNT = B_SPARE + 2 };
 static_assert(B_COUNT * 8 <= 512, "barrier area");
 static_assert(ATTN_SMEM_BYTES <= 232448, "shared memory budget");
 static_assert((GROUP_WARPS == 2 || GROUP_WARPS == 4) && DEQUANT_WARPS % GROUP_WARPS == 0 && DEQUANT_GROUPS >= 1 && TILE_UNITS % DEQUANT_GROUPS == 0,
@@ -283,10 +286,9 @@ __device__ __forceinline__ void exp2_pair_poly(float x0, float x1, float& e0, fl
     e1 = __uint_as_float(q1 + (t1 << 23));
 }
 
-// Score pairs J0 .. J1-1 of 16 scores -> packed fp16 p. PRECISE: also the fp16 remainder p - fp16(p) (exact in fp32, then
-// rounded once more: together the pair carries p to about 22 bits).
-template <int J0, int J1, bool PRECISE>
-__device__ __forceinline__ void exp_pairs16(const uint32_t (&r)[16], uint32_t* pk, uint32_t* pkl, unsigned long long sl2x2, unsigned long long nm2) {
+// Score pairs J0 .. J1-1 of 16 scores -> packed fp16 p.
+template <int J0, int J1>
+__device__ __forceinline__ void exp_pairs16(const uint32_t (&r)[16], uint32_t* pk, unsigned long long sl2x2, unsigned long long nm2) {
 #pragma unroll
     for (int j = J0; j < J1; ++j) {
         if (LLATTN_SKIP & 2) { pk[j] = r[2 * j] & 0x03ff03ffu; continue; }
@@ -297,11 +299,6 @@ __device__ __forceinline__ void exp_pairs16(const uint32_t (&r)[16], uint32_t* p
         else { e0 = ex2(x0); e1 = ex2(x1); }
         const half2 h = __floats2half2_rn(e0, e1);
         pk[j] = *reinterpret_cast<const uint32_t*>(&h);
-        if (PRECISE) {
-            const float2 hf = __half22float2(h);
-            const half2 l = __floats2half2_rn(e0 - hf.x, e1 - hf.y);
-            pkl[j] = *reinterpret_cast<const uint32_t*>(&l);
-        }
     }
 }
 
@@ -312,7 +309,7 @@ __device__ __forceinline__ void exp_pairs16(const uint32_t (&r)[16], uint32_t* p
 // of line so that the common path stays small.
 // tlane: tensor-memory address of the warp's lanes at column 0; ts: the tile's S / P buffer; bar_pv, par_pv: barrier and
 // parity of "PV of the previous tile has completed". Returns the row's new reference, NaN when that wait ran out.
-__device__ __noinline__ float raise_reference(float mref, float cs, bool over, int chunks_done, bool have_acc, bool precise, uint32_t tlane,
+__device__ __noinline__ float raise_reference(float mref, float cs, bool over, int chunks_done, bool have_acc, uint32_t tlane,
                                               uint32_t ts, uint32_t bar_pv, uint32_t par_pv, volatile int* abort_flag) {
     const float mnew = over ? cs : mref;
     const float corr = over ? ex2(mref - mnew) : 1.f;      // 0 for a row that had no reference yet
@@ -335,11 +332,11 @@ __device__ __noinline__ float raise_reference(float mref, float cs, bool over, i
         ptx::tmem_st16(tlane + TM_L, r);
     }
     const half2 ch = __float2half2_rn(corr);
-    // P chunk pc sits in columns 32 pc .. 32 pc + 15, its remainder (precise mode) in the 16 columns after them
+    // P chunk pc sits in columns 32 pc .. 32 pc + 15
 #pragma unroll 1
-    for (int pc = 0; pc < (precise ? 2 : 1) * chunks_done; ++pc) {
+    for (int pc = 0; pc < chunks_done; ++pc) {
         uint32_t r[16];
-        const uint32_t col = precise ? 16 * pc : 32 * pc;
+        const uint32_t col = 32 * pc;
         ptx::tmem_ld16(ts + col, r);
         ptx::tmem_wait_ld_tied(r);
 #pragma unroll
@@ -359,7 +356,7 @@ __device__ __noinline__ float raise_reference(float mref, float cs, bool over, i
 // goes back over the first 16 of the 32 S columns it came from. Before the last chunk's exponentials the barrier of the
 // next tile's S is tested (next_bar != 0), so that the test's latency is covered and the next tile starts without a wait
 // when its S is already there. Returns false when a wait of the rare path ran out.
-template <int NU, bool PRECISE>
+template <int NU>
 __device__ __forceinline__ bool softmax_tile(float& mref, float sl2, unsigned long long sl2x2, uint32_t tlane, uint32_t ts, bool have_acc,
                                              uint32_t bar_pv, uint32_t par_pv, volatile int* abort_flag, uint32_t next_bar, uint32_t next_par,
                                              bool& next_ready) {
@@ -378,22 +375,170 @@ __device__ __forceinline__ bool softmax_tile(float& mref, float sl2, unsigned lo
         const float cs = cm * sl2;
         const bool over = cs > mref + RESCALE_SLACK;
         if (__any_sync(0xffffffffu, over)) {
-            mref = raise_reference(mref, cs, over, c, have_acc, PRECISE, tlane, ts, bar_pv, par_pv, abort_flag);
+            mref = raise_reference(mref, cs, over, c, have_acc, tlane, ts, bar_pv, par_pv, abort_flag);
             if (__any_sync(0xffffffffu, mref != mref)) return false;
             nm2 = dup2(-mref);
         }
-        uint32_t pk[16], pkl[PRECISE ? 16 : 1];
+        uint32_t pk[16];
         if (c + 1 < NU) ptx::tmem_ld16(ts + 32 * (c + 1), n0);
         else next_ready = next_bar != 0 && ptx::mbar_try_wait(next_bar, next_par);
-        exp_pairs16<0, 8, PRECISE>(c0, pk, pkl, sl2x2, nm2);
+        exp_pairs16<0, 8>(c0, pk, sl2x2, nm2);
         ptx::tmem_st8(ts + 32 * c, pk);
         if (c + 1 < NU) ptx::tmem_ld16(ts + 32 * (c + 1) + 16, n1);
-        exp_pairs16<0, 5, PRECISE>(c1, pk + 8, pkl + (PRECISE ? 8 : 0), sl2x2, nm2);
+        exp_pairs16<0, 5>(c1, pk + 8, sl2x2, nm2);
         if (c + 1 < NU) { ptx::tmem_wait_ld_tied(n0, n1); cm = fmaxf(rowmax16(n0), rowmax16(n1)); }
-        exp_pairs16<5, 8, PRECISE>(c1, pk + 8, pkl + (PRECISE ? 8 : 0), sl2x2, nm2);
+        exp_pairs16<5, 8>(c1, pk + 8, sl2x2, nm2);
         ptx::tmem_st8(ts + 32 * c + 8, pk + 8);
-        // the remainders go over the second half of the chunk's S columns: all 32 have been read by now
-        if (PRECISE) { ptx::tmem_st8(ts + 32 * c + 16, pkl); ptx::tmem_st8(ts + 32 * c + 24, pkl + 8); }
+    }
+    return true;
+}
+
+// ---- The precise form's softmax: eight warps, two per lane quarter, sixteen rows each. It has half as much again to do per score (the
+// remainders: two conversions, two subtractions and a pack per pair), and with one warp on a scheduler that chain was the bound: 64
+// ragged sequences of up to 8 K tokens 169.5 us with four warps, 141 with eight, 9 x 201 blocks 41.1 and 38.2. The default form gains 1 % at
+// large batches from the same split and loses 4 % at a step of one sequence, whose run ends it lengthens (96 registers a thread instead
+// of 128; 20 layers 466 and 486 us), and keeps four. Votes are taken on P, two chunks at a time: a vote per chunk cost 3 %.
+// The 16 scores that a thread holds of a 32-key chunk (16x256b fragment: two rows, eight keys each) -> packed fp16 p in the 16x128b
+// fragment. nmA, nmB: minus the rows' reference exponents. Also the fp16 remainder p - fp16(p) (exact in fp32, then
+// rounded once more: together the pair carries p to about 22 bits).
+__device__ __forceinline__ void exp_chunk(const uint32_t (&r)[16], uint32_t (&pk)[8], uint32_t (&pkl)[8], unsigned long long sl2x2, unsigned long long nmA,
+                                          unsigned long long nmB) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        float x0, x1;
+        fma2(r[2 * j], r[2 * j + 1], sl2x2, j & 1 ? nmB : nmA, x0, x1);
+        const float e0 = ex2(x0), e1 = ex2(x1);
+        const half2 h = __floats2half2_rn(e0, e1);
+        pk[j] = *reinterpret_cast<const uint32_t*>(&h);
+        const float2 hf = __half22float2(h);
+        const half2 l = __floats2half2_rn(e0 - hf.x, e1 - hf.y);
+        pkl[j] = *reinterpret_cast<const uint32_t*>(&l);
+    }
+}
+// Maxima of the fragment's two rows over the quads that hold them.
+__device__ __forceinline__ void row_maxima(const uint32_t (&r)[16], float& mA, float& mB) {
+    auto f = [&](int j) { return __uint_as_float(r[j]); };
+    mA = max3(max3(f(0), f(1), f(4)), max3(f(5), f(8), f(9)), fmaxf(f(12), f(13)));
+    mB = max3(max3(f(2), f(3), f(6)), max3(f(7), f(10), f(11)), fmaxf(f(14), f(15)));
+}
+__device__ __forceinline__ float quad_max(float m) {
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    return fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+}
+// Largest of eight pairs of p, per half: non-negative fp16 numbers are in the order of their bits, and not-a-number is above all.
+__device__ __forceinline__ uint32_t pair_maxima(const uint32_t (&pk)[8]) {
+    const uint32_t a = __vimax3_u16x2(pk[0], pk[1], pk[2]), b = __vimax3_u16x2(pk[3], pk[4], pk[5]);
+    return __vimax3_u16x2(__vimax3_u16x2(a, b, pk[6]), pk[7], pk[7]);
+}
+// Is either half above 2^RESCALE_SLACK, or not a number?
+__device__ __forceinline__ bool above_slack(uint32_t m) {
+    uint32_t r;
+    asm("{\n\t.reg .pred p, q;\n\tsetp.gtu.f16x2 p|q, %1, %2;\n\tor.pred p, p, q;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r) : "r"(m), "r"(((uint32_t(RESCALE_SLACK) + 15u) << 10) * 0x10001u));
+    return r != 0;
+}
+
+// A chunk with a p above 2^RESCALE_SLACK, S still in place: rows whose chunk maximum is more than RESCALE_SLACK above their reference
+// move it to that maximum; what was accumulated under the old reference - O and the row sum of earlier tiles (`have_acc`), and
+// the `chunk` chunks of this tile already turned into P - is rescaled; then the chunk's P is computed and stored. Warp-uniform call, rare
+// (a key 2^8 times heavier than everything before it in the run), kept out of line so that the common path stays small.
+// mref: the references of the thread's two rows; tlane: tensor-memory address of the warp's 16 lanes at column 0; ts: the tile's
+// S / P buffer; bar_pv, par_pv: barrier and parity of "PV of the previous tile has completed". Returns the new references, NaN
+// when that wait ran out.
+__device__ __noinline__ float2 raise_reference_rows16(float2 mref, float sl2, int chunk, bool have_acc, uint32_t tlane, uint32_t ts, uint32_t bar_pv,
+                                               uint32_t par_pv, volatile int* abort_flag) {
+    uint32_t r[16];
+    ptx::tmem_wait_st();                       // the earlier chunks' P is read back below
+    ptx::tmem_ld16x256_x4(ts + 32 * chunk, r);
+    ptx::tmem_wait_ld_tied(r);
+    float cA, cB;
+    row_maxima(r, cA, cB);
+    cA = quad_max(cA) * sl2; cB = quad_max(cB) * sl2;
+    const float2 mnew = make_float2(cA > mref.x + RESCALE_SLACK ? cA : mref.x, cB > mref.y + RESCALE_SLACK ? cB : mref.y);
+    const float fA = mnew.x != mref.x ? ex2(mref.x - mnew.x) : 1.f, fB = mnew.y != mref.y ? ex2(mref.y - mnew.y) : 1.f;
+    if (have_acc) {
+        if (!ptx::mbar_wait(bar_pv, par_pv, abort_flag)) return make_float2(__int_as_float(0x7fc00000), 0.f);
+        ptx::tc_fence_after();
+        // 128 dims, then the row sum in the first of the 16 columns behind them (32 columns from 16 before the end take it in)
+#pragma unroll 1
+        for (int oc = 0; oc < 5; ++oc) {
+            const uint32_t at = tlane + TM_O + (oc < 4 ? 32 * oc : PV_N - 32);
+            uint32_t v[16];
+            ptx::tmem_ld16x256_x4(at, v);
+            ptx::tmem_wait_ld_tied(v);
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (oc < 4 || j >= 8) v[j] = __float_as_uint(__uint_as_float(v[j]) * (j & 2 ? fB : fA));
+            ptx::tmem_st16x256_x4(at, v);
+            ptx::tmem_wait_st();
+        }
+    }
+    const half2 hA = __float2half2_rn(fA), hB = __float2half2_rn(fB);
+    // P chunk pc sits in columns 32 pc .. 32 pc + 15, its remainder in the 16 columns after them
+#pragma unroll 1
+    for (int pc = 0; pc < 2 * chunk; ++pc) {
+        uint32_t v[8];
+        const uint32_t col = 16 * pc;
+        ptx::tmem_ld16x128_x4(ts + col, v);
+        ptx::tmem_wait_ld_tied(v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const half2 h = __hmul2(*reinterpret_cast<const half2*>(&v[j]), j & 1 ? hB : hA);
+            v[j] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        ptx::tmem_st16x128_x4(ts + col, v);
+    }
+    uint32_t pk[8], pkl[8];
+    exp_chunk(r, pk, pkl, dup2(sl2), dup2(-mnew.x), dup2(-mnew.y));
+    ptx::tmem_st16x128_x4(ts + 32 * chunk, pk);
+    ptx::tmem_st16x128_x4(ts + 32 * chunk + 16, pkl);
+    return mnew;
+}
+
+// One tile of NU 32-key chunks for a warp's sixteen query rows: S -> P in a single pass, branch-free except for the vote that
+// guards the rare path. The next chunk's scores are on their way while one chunk's exponentials run, and P goes back over the first
+// 16 of the 32 S columns it came from. Before the last chunk's exponentials the barrier of the
+// next tile's S is tested (next_bar != 0), so that the test's latency is covered and the next tile starts without a wait
+// when its S is already there. Returns false when a wait of the rare path ran out.
+template <int NU>
+__device__ __forceinline__ bool softmax_tile_rows16(float2& mref, float sl2, unsigned long long sl2x2, uint32_t tlane, uint32_t ts, bool have_acc,
+                                             uint32_t bar_pv, uint32_t par_pv, volatile int* abort_flag, uint32_t next_bar, uint32_t next_par,
+                                             bool& next_ready) {
+    unsigned long long nmA = dup2(-mref.x), nmB = dup2(-mref.y);
+    uint32_t s0[16], s1[16];
+    ptx::tmem_ld16x256_x4(ts, s0);
+    ptx::tmem_wait_ld_tied(s0);
+#pragma unroll
+    for (int c = 0; c < NU; c += 2) {          // two chunks between votes
+        const bool two = c + 1 < NU, more = c + 2 < NU;
+        uint32_t p0[8], l0[8], p1[8], l1[8];
+        if (two) ptx::tmem_ld16x256_x4(ts + 32 * (c + 1), s1);
+        if (!more) next_ready = next_bar != 0 && ptx::mbar_try_wait(next_bar, next_par);
+        exp_chunk(s0, p0, l0, sl2x2, nmA, nmB);
+        uint32_t m = pair_maxima(p0);
+        if (two) {
+            ptx::tmem_wait_ld_tied(s1);
+            if (more) ptx::tmem_ld16x256_x4(ts + 32 * (c + 2), s0);
+            exp_chunk(s1, p1, l1, sl2x2, nmA, nmB);
+            m = __vmaxu2(m, pair_maxima(p1));
+        }
+        if (__any_sync(0xffffffffu, above_slack(m))) {
+            if (more) ptx::tmem_wait_ld_tied(s0);      // no load may be in flight to registers that a call saves
+#pragma unroll 1
+            for (int k = c; k < (two ? c + 2 : c + 1); ++k) {
+                mref = raise_reference_rows16(mref, sl2, k, have_acc, tlane, ts, bar_pv, par_pv, abort_flag);
+                if (__any_sync(0xffffffffu, mref.x != mref.x)) return false;
+            }
+            nmA = dup2(-mref.x); nmB = dup2(-mref.y);
+        } else {
+            ptx::tmem_st16x128_x4(ts + 32 * c, p0);
+            // the remainders go over the second half of the chunk's S columns: all 32 have been read by now
+            ptx::tmem_st16x128_x4(ts + 32 * c + 16, l0);
+            if (two) {
+                ptx::tmem_st16x128_x4(ts + 32 * c + 32, p1);
+                ptx::tmem_st16x128_x4(ts + 32 * c + 48, l1);
+            }
+        }
+        if (more) ptx::tmem_wait_ld_tied(s0);
     }
     return true;
 }
@@ -507,6 +652,9 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM_BAR);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM_MISC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM_MISC + 4);
+    constexpr int SOFTMAX_WARPS = softmax_warps(PRECISE), WARP_SERVICE = SOFTMAX_WARPS + DEQUANT_WARPS, WARP_MMA_PV = WARP_SERVICE;
+    constexpr int WARP_MMA = WARP_MMA_PV + 1, WARP_PRODUCER = WARP_MMA + 1, ATTN_THREADS = attn_threads(PRECISE);
+    constexpr int P_ARRIVALS = LLATTN_WARP_ARRIVE ? SOFTMAX_WARPS : 32 * SOFTMAX_WARPS;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar0 = ptx::smem_u32(bars);
     auto BAR = [&](int i) -> uint32_t { return bar0 + 8u * uint32_t(i); };
@@ -528,6 +676,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
             ptx::mbar_init(BAR(B_S_FULL + i), 1); ptx::mbar_init(BAR(B_P_FULL + i), P_ARRIVALS);
         }
         ptx::mbar_init(BAR(B_Q_FULL), 32 * SOFTMAX_WARPS); ptx::mbar_init(BAR(B_O_FREE), 32 * SOFTMAX_WARPS);
+        ptx::mbar_init(BAR(B_QSUM), 128);
         ptx::mbar_init(BAR(B_SPARE), 1);
         ptx::mbar_init(BAR(B_SPARE + 1), 1);
         ptx::fence_mbar_init();
@@ -551,6 +700,227 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
 
     if (warp < SOFTMAX_WARPS) {
         // ================================================================== softmax + epilogue
+        if constexpr (PRECISE) {
+        // Warps w and w + 4 may access lanes 32 w .. 32 w + 31 of tensor memory. In the tile loop each takes sixteen of these rows
+        // with all their keys, a row spread over four threads as in an mma fragment: nothing is exchanged between warps. At the two
+        // ends of a run a thread is a row (lane) and each of the two warps takes half of the channels.
+        const int quarter = warp & 3, hf = warp >> 2, row = quarter * 32 + lane;
+        const uint32_t tlane = tmem + (uint32_t(quarter * 32) << 16), trow = tlane + (uint32_t(16 * hf) << 16);
+        const unsigned long long sl2x2 = dup2(p.sl2);
+        uint8_t* const stage = smem + SM_STAGE + warp * (STAGE_BYTES / 2);
+        // staging rows of 64 bytes, the 16-byte chunk c of row r at chunk position c ^ (r / 2 % 4)
+        auto stage_in = [&](int r, int c) -> uint8_t* { return stage + r * 64 + ((c ^ ((r >> 1) & 3)) << 4); };
+        volatile float* const rowref = reinterpret_cast<volatile float*>(smem + SM_ROWREF);
+        uint32_t q8_runs = 0;
+        uint32_t t = 0;
+        bool alive = true;
+#pragma unroll 1
+        for (int ii = i0; ii < i1 && alive; ++ii) {
+            WorkItem w; SeqDesc s; MergeDesc md{0, 0, 0, 1};
+            if (!fetch_item(p, ii, w, s, first_run, i0_any)) continue;
+            const int U = w.rec_count + w.fresh, ntiles = (U + TILE_UNITS - 1) / TILE_UNITS;
+            // Reference exponent of the row, log2 units: the exact maximum of the run's first tile (a row dominated by a
+            // key of that tile then has p = 1 for it, without rounding); it moves only when a later score exceeds it by
+            // more than RESCALE_SLACK (engine/attn.cu:237-255 moves its reference lazily in the same way).
+            float2 mref = make_float2(-INFINITY, -INFINITY);      // rows lane / 4 and lane / 4 + 8 of the warp's sixteen
+            bool s_ready = false;              // the tile's S has been seen complete already (tested during the previous tile)
+            {   // half the channels of the quarter's 32 query rows into tensor memory as fp16 pairs, row = lane. Every S MMA of the
+                // previous item has completed: this warp has seen the S of its last tile. The rows come in as whole sectors (4 lanes
+                // per 64 bytes), all of them on their way at once, and change hands through the staging rows.
+                const half* src = p.Q + ((size_t(s.q_first + w.qblk) * BLK + 8 * quarter) * NQH + 4 * w.kvh) * D + 64 * hf +
+                                  (size_t(lane >> 4) * NQH + ((lane >> 2) & 3)) * D + (lane & 3) * 8;
+                uint4 v[8];
+#pragma unroll
+                for (int g = 0; g < 8; ++g) v[g] = __ldg(reinterpret_cast<const uint4*>(src + size_t(2 * (g & 3)) * NQH * D + 32 * (g >> 2)));   // rows 8 (g % 4) .., channels 32 (g / 4) ..
+#pragma unroll
+                for (int c2 = 0; c2 < 2; ++c2) {
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) *reinterpret_cast<uint4*>(stage_in(8 * g + (lane >> 2), lane & 3)) = permute8(v[4 * c2 + g]);
+                    __syncwarp();
+                    uint32_t r[16];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint4 x = *reinterpret_cast<const uint4*>(stage_in(lane, c));
+                        r[4 * c] = x.x; r[4 * c + 1] = x.y; r[4 * c + 2] = x.z; r[4 * c + 3] = x.w;
+                    }
+                    ptx::tmem_st16(tlane + TM_Q + 32 * hf + 16 * c2, r);
+                    __syncwarp();
+                }
+                ptx::tmem_wait_st();
+                ptx::tc_fence_before();
+                ptx::mbar_arrive(BAR(B_Q_FULL));
+            }
+#pragma unroll 1
+            for (int i = 0; i < ntiles && alive; ++i, ++t) {
+                const int b = t & 1, nu = min(TILE_UNITS, U - TILE_UNITS * i);
+                LLATTN_TR(1, t);
+                if (!s_ready && !ptx::mbar_wait(BAR(B_S_FULL + b), (t >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; break; }
+                LLATTN_TR(2, t);
+                ptx::tc_fence_after();
+                const uint32_t ts = trow + TM_S + b * 128, bar_pv = BAR(B_PV_DONE + (b ^ 1)), par_pv = ((t - 1) >> 1) & 1;
+                // the next tile's S (other buffer) is tested for during this tile's last chunk, except across runs
+                const uint32_t next_bar = i + 1 < ntiles ? BAR(B_S_FULL + (b ^ 1)) : 0u, next_par = ((t + 1) >> 1) & 1;
+                if (i == 0) {
+                    float mA = -INFINITY, mB = -INFINITY;
+#pragma unroll 1
+                    for (int c = 0; c < nu; ++c) {
+                        uint32_t r[16];
+                        ptx::tmem_ld16x256_x4(ts + 32 * c, r);
+                        ptx::tmem_wait_ld_tied(r);
+                        float a, b2;
+                        row_maxima(r, a, b2);
+                        mA = fmaxf(mA, a); mB = fmaxf(mB, b2);
+                    }
+                    mref = make_float2(quad_max(mA) * p.sl2, quad_max(mB) * p.sl2);
+                }
+                bool ok;
+                if (nu == TILE_UNITS) ok = softmax_tile_rows16<TILE_UNITS>(mref, p.sl2, sl2x2, trow, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);      // every tile of a run but its last
+                else if (nu == 3) ok = softmax_tile_rows16<3>(mref, p.sl2, sl2x2, trow, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
+                else if (nu == 2) ok = softmax_tile_rows16<2>(mref, p.sl2, sl2x2, trow, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
+                else ok = softmax_tile_rows16<1>(mref, p.sl2, sl2x2, trow, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
+                // for the epilogue, where a lane is a row: published by the arrival on P, read behind the tile's PV. The next run's are
+                // written after its query rows are in, by both warps of the quarter.
+                if (i + 1 == ntiles && (lane & 3) == 0) { rowref[quarter * 32 + 16 * hf + (lane >> 2)] = mref.x; rowref[quarter * 32 + 16 * hf + 8 + (lane >> 2)] = mref.y; }
+                if (!ok) { alive = false; errbits |= ERR_WAIT_SOFTMAX; }
+                if (!alive) break;
+                ptx::tmem_wait_st();
+                ptx::tc_fence_before();
+#if LLATTN_WARP_ARRIVE
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(BAR(B_P_FULL + b));
+#else
+                ptx::mbar_arrive(BAR(B_P_FULL + b));
+#endif
+                LLATTN_TR(4, t);
+            }
+            if (!alive) break;
+            // ---- epilogue. A run that is its tile's only one writes the outputs straight from tensor memory. Otherwise
+            // it stores its un-normalised O, reference exponent and row sum as a partial result and counts itself in at
+            // the tile's arrival counter; the tile's runs fold it together once the CTAs have no runs left (end of this
+            // function).
+            const uint32_t tl = t - 1;
+            fetch_item(p, ii, w, s, first_run, i0_any, &md);     // again: cheaper than a dozen registers through the loop above
+            if (!ptx::mbar_wait(BAR(B_PV_DONE + (tl & 1)), (tl >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; break; }
+            ptx::tc_fence_after();
+            float lsum;
+            {
+                uint32_t r[16];
+                ptx::tmem_ld16(tlane + TM_L, r);
+                ptx::tmem_wait_ld_tied(r);
+                lsum = __uint_as_float(r[0]);
+            }
+            const bool fused = p.fused, finish = fused && md.nslots == 1;
+            const float M = rowref[row], den = lsum;
+            const uint32_t tO = tlane + TM_O + 64 * hf;
+            if (!finish) {
+                float* out = p.Opart + (size_t(w.slot) * QR + 32 * quarter + (lane >> 2)) * D + 64 * hf + 4 * (lane & 3);
+#pragma unroll 1
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t r[16];
+                    ptx::tmem_ld16(tO + 16 * c, r);
+                    ptx::tmem_wait_ld_tied(r);
+#pragma unroll
+                    for (int g = 0; g < 2; ++g) {      // positions (0..7) hold dims (0,4,1,5,2,6,3,7)
+                        *reinterpret_cast<uint4*>(stage_in(lane, 2 * g)) = make_uint4(r[8 * g], r[8 * g + 2], r[8 * g + 4], r[8 * g + 6]);
+                        *reinterpret_cast<uint4*>(stage_in(lane, 2 * g + 1)) = make_uint4(r[8 * g + 1], r[8 * g + 3], r[8 * g + 5], r[8 * g + 7]);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)        // eight rows x 64 bytes
+                        *reinterpret_cast<uint4*>(out + 8 * i * D + 16 * c) = *reinterpret_cast<const uint4*>(stage_in(8 * i + (lane >> 2), lane & 3));
+                    __syncwarp();
+                }
+                // the accumulator has been read: the next run's PV may start while the stores below drain
+                ptx::tc_fence_before();
+                ptx::mbar_arrive(BAR(B_O_FREE));
+                if (hf == 0) {
+                    p.Lpart[size_t(w.slot) * QR + row] = lsum;
+                    p.Mpart[size_t(w.slot) * QR + row] = M;
+                }
+                if (fused) {                   // this warp's half of the run's 32 rows is out: count it in
+                    __threadfence();
+                    __syncwarp();
+                    if (lane == 0) atomicAdd(p.tile_counters + 4 * w.tile, 1);
+                }
+            }
+            if (finish) {
+                const float inv = 1.f / den;
+                RowOut ro{size_t(md.q_index) * BLK + (row >> 2), 4 * md.kvh + (row & 3), 0.f, 0};
+                if (p.out.q8) {        // the int8 form needs the row's largest magnitude first
+                    float m = 0.f;
+#pragma unroll 1
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t r[32];
+                        ptx::tmem_ld32(tlane + TM_O + 32 * c, r);
+                        ptx::tmem_wait_ld_tied(r);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) m = fmaxf(m, fabsf(__uint_as_float(r[j]) * inv));
+                    }
+                    ro.qscale = fmaxf(__fdiv_rn(m, 127.f), 1e-30f);
+                }
+#pragma unroll 1
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t r[32];
+                    float v[32];
+                    ptx::tmem_ld32(tO + 32 * c, r);
+                    ptx::tmem_wait_ld_tied(r);
+#pragma unroll
+                    for (int g = 0; g < 4; ++g)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            v[8 * g + k] = __uint_as_float(r[8 * g + 2 * k]) * inv;
+                            v[8 * g + 4 + k] = __uint_as_float(r[8 * g + 2 * k + 1]) * inv;
+                        }
+                    if (p.out.O32) {
+                        float* out = p.out.O32 + ((size_t(md.q_index) * BLK + 8 * quarter + (lane >> 4)) * NQH + 4 * md.kvh + ((lane >> 2) & 3)) * D + 64 * hf + 32 * c + 4 * (lane & 3);
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {  // 16 dims at a time
+#pragma unroll
+                            for (int g = 0; g < 4; ++g)
+                                *reinterpret_cast<float4*>(stage_in(lane, g)) = make_float4(v[16 * k + 4 * g], v[16 * k + 4 * g + 1], v[16 * k + 4 * g + 2], v[16 * k + 4 * g + 3]);
+                            __syncwarp();
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)    // the four heads of two tokens
+                                *reinterpret_cast<uint4*>(out + size_t(2 * i) * NQH * D + 16 * k) = *reinterpret_cast<const uint4*>(stage_in(8 * i + (lane >> 2), lane & 3));
+                            __syncwarp();
+                        }
+                    }
+                    if (p.out.O16) {
+#pragma unroll
+                        for (int g = 0; g < 4; ++g) {
+                            const half2 h0 = __floats2half2_rn(v[8 * g], v[8 * g + 1]), h1 = __floats2half2_rn(v[8 * g + 2], v[8 * g + 3]);
+                            const half2 h2 = __floats2half2_rn(v[8 * g + 4], v[8 * g + 5]), h3 = __floats2half2_rn(v[8 * g + 6], v[8 * g + 7]);
+                            *reinterpret_cast<uint4*>(stage_in(lane, g)) = make_uint4(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1),
+                                                                                      *reinterpret_cast<const uint32_t*>(&h2), *reinterpret_cast<const uint32_t*>(&h3));
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {  // eight rows x 64 bytes
+                            const int rr = 8 * i + (lane >> 2);
+                            half* out = p.out.O16 + ((size_t(md.q_index) * BLK + 8 * quarter + (rr >> 2)) * NQH + 4 * md.kvh + (rr & 3)) * D + 64 * hf + 32 * c + 8 * (lane & 3);
+                            *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(stage_in(rr, lane & 3));
+                        }
+                        __syncwarp();
+                    }
+                    if (p.out.q8) row_store_q8(p.out, ro, 2 * hf + c, v);
+                }
+                if (p.out.q8) {        // the row's code sum: the second warp hands its half over
+                    volatile int* const qsum = reinterpret_cast<volatile int*>(smem + SM_QSUM);
+                    if (hf) {
+                        qsum[row] = ro.qsum;
+                        ptx::mbar_arrive(BAR(B_QSUM));
+                    } else {
+                        if (!ptx::mbar_wait(BAR(B_QSUM), q8_runs & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; break; }
+                        ro.qsum += qsum[row];
+                    }
+                    ++q8_runs;
+                }
+                if (hf == 0) row_finish(p.out, ro, M, den);
+                ptx::tc_fence_before();
+                ptx::mbar_arrive(BAR(B_O_FREE));
+            }
+        }
+        } else {
         // thread = query row = TMEM lane (warp w owns lanes 32 w .. 32 w + 31): it sees all keys of its row, so the row
         // maximum needs no exchange with other warps. One pass per tile: a 32-key chunk of S is loaded while the previous
         // chunk's exponentials run, its maximum is taken between them, and P goes back over the first 16 of the S columns
@@ -619,10 +989,10 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                     mref = mx * p.sl2;
                 }
                 bool ok;
-                if (nu == TILE_UNITS) ok = softmax_tile<TILE_UNITS, PRECISE>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);      // every tile of a run but its last
-                else if (nu == 3) ok = softmax_tile<3, PRECISE>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
-                else if (nu == 2) ok = softmax_tile<2, PRECISE>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
-                else ok = softmax_tile<1, PRECISE>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
+                if (nu == TILE_UNITS) ok = softmax_tile<TILE_UNITS>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);      // every tile of a run but its last
+                else if (nu == 3) ok = softmax_tile<3>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
+                else if (nu == 2) ok = softmax_tile<2>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
+                else ok = softmax_tile<1>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
                 if (!ok) { alive = false; errbits |= ERR_WAIT_SOFTMAX; }
                 if (!alive) break;
                 ptx::tmem_wait_st();
@@ -744,6 +1114,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                 ptx::tc_fence_before();
                 ptx::mbar_arrive(BAR(B_O_FREE));
             }
+        }
         }
     } else if (warp < WARP_SERVICE) {
         // ================================================================== dequant: records -> fp16 operand tiles
@@ -1075,9 +1446,11 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                 fold_rows_shared(p.Opart, p.Mpart, p.Lpart, md, w.slot - md.slot_begin, warp, lane, smem + SM_K, p.out);      // the tiles are done with
             } else if (md.nslots == 2) {
 #pragma unroll 1
-                for (int r = r0; r < QR; r += 4 * step) {
-                    const int rows[4] = {r, r + step < QR ? r + step : -1, r + 2 * step < QR ? r + 2 * step : -1, r + 3 * step < QR ? r + 3 * step : -1};
-                    fold_rows_few<4, 2>(p.Opart, p.Mpart, p.Lpart, md, rows, lane, p.out);
+                for (int r = r0; r < QR; r += (PRECISE ? 2 : 4) * step) {      // the precise form has not the registers for four rows
+                    int rows[PRECISE ? 2 : 4];
+#pragma unroll
+                    for (int q = 0; q < (PRECISE ? 2 : 4); ++q) rows[q] = r + q * step < QR ? r + q * step : -1;
+                    fold_rows_few<PRECISE ? 2 : 4, 2>(p.Opart, p.Mpart, p.Lpart, md, rows, lane, p.out);
                 }
             } else if (md.nslots <= 4) {
 #pragma unroll 1
@@ -1101,7 +1474,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
 }
 
 template <bool PRECISE>
-__global__ void __launch_bounds__(ATTN_THREADS, 1) attn_tile_kernel(const __grid_constant__ KParams p) {
+__global__ void __launch_bounds__(attn_threads(PRECISE), 1) attn_tile_kernel(const __grid_constant__ KParams p) {
     // reference-grid mode: the folding launch behind this one carries the attribute of a dependent launch, may take its place
     // on the SMs this one leaves idle, and waits there (nothing behind a list-mode launch carries it)
     if (!PRECISE && !p.items) ptx::launch_dependents();

@@ -450,7 +450,7 @@ int llattn_create(int device, llattn_ctx** out) {
     // the largest grid a cooperative launch of the attention kernel accepts here: what fits on the device at once (fewer
     // than one CTA per SM when the process was given only a part of the GPU)
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, llattn::attn_tile_kernel<true>, llattn::ATTN_THREADS, llattn::ATTN_SMEM_BYTES) != cudaSuccess || per_sm < 1) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, llattn::attn_tile_kernel<true>, llattn::attn_threads(true), llattn::ATTN_SMEM_BYTES) != cudaSuccess || per_sm < 1) {
         cudaGetLastError();
         cudaFree(c->err_word);
         delete c;
@@ -650,9 +650,10 @@ int llattn_attention(llattn_ctx* c, const llattn_plan* pl, const llattn_io* io, 
     p.cache_offset = io->cache_offset;
     // cooperative: the driver starts the grid only when all of its CTAs can be resident together (see plan_create)
     void* args[] = {&p};
-    const void* fn = (io->flags & LLATTN_IO_PRECISE_P) ? reinterpret_cast<const void*>(attn_tile_kernel<true>)
+    const bool precise = io->flags & LLATTN_IO_PRECISE_P;
+    const void* fn = precise ? reinterpret_cast<const void*>(attn_tile_kernel<true>)
                                                        : reinterpret_cast<const void*>(attn_tile_kernel<false>);
-    CU(cudaLaunchCooperativeKernel(fn, dim3(pl->launch_ctas), dim3(ATTN_THREADS), args, ATTN_SMEM_BYTES, as_stream(stream)));
+    CU(cudaLaunchCooperativeKernel(fn, dim3(pl->launch_ctas), dim3(attn_threads(precise)), args, ATTN_SMEM_BYTES, as_stream(stream)));
     return LLATTN_OK;
 }
 

@@ -208,11 +208,11 @@ __device__ __forceinline__ void fold_row_warp(const float* Opart, const float* M
     emit_row_warp(M, den, acc, md, r, lane, o);
 }
 
-// This CTA's rows k, k + n, ... of a tile cut into n runs, FOLD_PART < n <= FOLD_SHARED_SLOTS, by 16 warps: W warps share a
+// This CTA's rows k, k + n, ... of a tile cut into n runs, FOLD_PART < n <= FOLD_SHARED_SLOTS, by 16 warps (20 in the precise form): W warps share a
 // row, each folds n / W of its slots, the row's first warp adds their results up in slot order. With a warp per row, most of
 // the warps had none and the others went through their slots in several round trips: 22 runs a tile, 7,000 cycles from the last
 // count-in to the outputs. Two warps a row up to 32 slots (at most 8 rows), four above (at most 4 rows); the planner
-// gives a tile at most 59 runs on 160 CTAs, and more would take the general form. `scratch`: 16 x 544 bytes of shared memory; every
+// gives a tile at most 59 runs on 160 CTAs, and more would take the general form. `scratch`: 544 bytes of shared memory per warp; every
 // thread of the CTA calls. A call, with the descriptors by value: by reference they lived on the stack and the
 // attention kernel spilled around it (12 bytes of stores, 20 of loads; 64 sequences at 32 K tokens 714 us, now 698), and inlined
 // it cost the precise form up to 5 % (four passes of 9 blocks on 300 162 -> 171 us, now 158).
@@ -227,7 +227,7 @@ __device__ __noinline__ void fold_rows_shared(const float* Opart, const float* M
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (r < QR && cnt > 0) fold_part(Opart, Mpart, Lpart, size_t(md.slot_begin) + s0, cnt, r, lane, M, den, acc);
     float4* rows = reinterpret_cast<float4*>(scratch);
-    float2* ml = reinterpret_cast<float2*>(scratch + 16 * 512);
+    float2* ml = reinterpret_cast<float2*>(scratch + (blockDim.x >> 5) * 512);
     __syncthreads();                                   // the scratch of a previous tile has been read
     rows[warp * 32 + lane] = acc;
     if (lane == 0) ml[warp] = make_float2(M, den);

@@ -151,3 +151,41 @@ def test_kernel_error_is_the_emulated_fp16_rounding_of_p(api, ctx, orc, pkg, nbl
             # one run of 257 units per kv head: the tensor core's own fp32 accumulation over a chain that long shows
             # (4e-4 x RMS here, 1.6e-3 for a 1025-unit run); in the planner's usual cuts it is below 1e-4
             assert e_k <= 1e-3 and e_e <= 5e-5
+
+
+# The precise form's own softmax role: the int8 output of whole tiles (two warps share a row and add their code sums up), several
+# per CTA, tails of one to four chunks, split tiles, and a reference exponent that moves in the middle of a tile
+@pytest.mark.parametrize("nseq,nblocks,nctas", [(1, 0, 4), (1, 1, 4), (1, 2, 4), (1, 3, 4), (5, 6, 3), (9, 20, 7), (2, 37, 0), (3, 260, 0)])
+def test_precise_int8_output_and_tails(api, pkg, orc, nseq, nblocks, nctas):
+    wl = pkg.workload
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    Q, Kf, Vf, caches, want = [], [], [], [], []
+    for i in range(nseq):
+        q, kf, vf = wl.query_blocks(1, seq=50 + i)
+        cache = np.zeros((4, nblocks + 1, orc.REC_BYTES), np.uint8)
+        if nblocks:
+            Kc, Vc = wl.context_blocks(nblocks, seq=50 + i)
+            if i % 2 == 0 and nblocks > 4:
+                Kc = Kc.copy()
+                Kc[nblocks // 2, 9] *= 6          # one token of the context far above everything before it
+            orc.kv_commit(Kc, Vc, cache, nblocks + 1, 0)
+        o, _ = orc.attention(q, kf, vf, cache, nblocks + 1, nblocks, dq_mode=1)
+        Q.append(q); Kf.append(kf); Vf.append(vf); caches.append(dev(cache)); want.append(o.reshape(32, 16, 128))
+    cat = lambda x: dev(np.concatenate([a.reshape(1, 32, -1, 128) for a in x]))
+    ctx = api.Context(0)
+    plan = ctx.plan([api.Seq(cache=caches[i], nblocks=nblocks, nq=1, q_first=i) for i in range(nseq)], nctas)
+    n = 32 * nseq
+    O = torch.zeros((n, 16, 128), device="cuda")
+    q8, s8, sum8 = torch.zeros((n, 2048), dtype=torch.int8, device="cuda"), torch.zeros((n, 16), device="cuda"), torch.zeros((n, 16), dtype=torch.int32, device="cuda")
+    ctx.attention(plan, cat(Q), cat(Kf), cat(Vf), O32=O, q8=q8, s8=s8, sum8=sum8, precise=True)
+    assert ctx.device_status() == 0
+    got, ref = O.cpu().numpy(), np.concatenate(want)
+    assert np.abs(got - ref).max() <= 2e-3 * np.sqrt((ref.astype(np.float64) ** 2).mean())
+    scale = np.maximum(np.abs(got).max(2) / np.float32(127), np.float32(1e-30))
+    codes = np.clip(np.rint(got / scale[..., None]), -127, 127).astype(np.int8)
+    order = np.array([orc.frag_pos(c) for c in range(2048)])
+    frag = np.zeros((n, 2048), np.int8)
+    frag[:, order] = codes.reshape(n, 2048)
+    assert np.array_equal(s8.cpu().numpy(), scale) and np.array_equal(q8.cpu().numpy(), frag)
+    assert np.array_equal(sum8.cpu().numpy(), codes.astype(np.int32).sum(2))
+    plan.close(); ctx.close()
