@@ -92,7 +92,8 @@ int llattn_qkv_prepare_commit(const float* qkv, const int32_t* pos, const float*
  * engine/moe_i8.cu:34-41 after relayout_strips); q [ntokens][K] int8 in fragment order inside every 128-group,
  * s and sum [ntokens][K/128] (the moe8::Act triple, engine/moe_i8.cu:55-66); Y [ntokens][rows] fp32. rows and K are
  * multiples of 128. Same float operations in the same order as the reference kernel: bit-identical results.
- * W and q must be 16-byte aligned. err_word is not written (the kernels wait for nothing); NULL will do. */
+ * W and q must be 16-byte aligned. err_word is a device int that the kernel for many tokens ORs an error code into when
+ * a bounded wait runs out (Y is then incomplete); may be NULL. */
 int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int32_t* sum, float* Y, int ntokens, int rows, int K,
                       int* err_word, void* stream);
 
