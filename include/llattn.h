@@ -279,7 +279,8 @@ int llattn_kvpool_stats(llattn_kvpool* pool, int64_t* out6);
  * next poll; the fifth warp then waits on its counter once more with `limit_ns` and lets that run out too. The kernel
  * returns normally; `err_word` (device int, zeroed by the caller) then holds bits 1|2|4|8|128 (one per warp: the
  * producer / dequant / MMA / softmax / fold codes of llattn_device_status) and waited_ns6 (device, 6 x uint64) how long
- * each of the five warps waited, then how long the counter wait took to run out alone. No counterpart in the
+ * each of the five warps waited, then how long the counter wait took to run out alone. Of a sixth warp half of the lanes
+ * wait on a barrier that is complete: bit 32 is set if a warp can leave a wait with two answers. No counterpart in the
  * reference, whose kernels have no waits that can fail. */
 int llattn_wait_selftest(unsigned long long limit_ns, int* err_word, unsigned long long* waited_ns6, void* stream);
 

@@ -413,27 +413,32 @@ extern "C" int llattn_attention_static(const void* Q, const void* Kf, const void
 // the other runs of a split tile). Warp 0 has `limit_ns` (a millisecond in the test); when its wait runs out it raises
 // the CTA's abort flag, as every role of the attention kernel does, and the other warps - whose own limit is the
 // kernels' two seconds - see the flag at their next poll and leave too. Then the fifth warp waits on its counter once
-// more, alone and with the short limit, to show that wait running out by itself. Every warp reports through the error
-// word, the kernel returns normally and the context stays usable.
+// more, alone and with the short limit, to show that wait running out by itself. Of a sixth warp half of the lanes wait on a barrier
+// whose phase is complete and half on one that nobody arrives on: it has to leave its wait with one answer, no, in all lanes.
+// Every warp reports through the error word, the kernel returns normally and the context stays usable.
 namespace llattn {
 __device__ int selftest_counter;       // nothing ever counts in here
 
-__global__ void __launch_bounds__(160) wait_selftest_kernel(unsigned long long limit_ns, int* err, unsigned long long* waited_ns) {
-    __shared__ uint64_t bars[4];
+__global__ void __launch_bounds__(192) wait_selftest_kernel(unsigned long long limit_ns, int* err, unsigned long long* waited_ns) {
+    __shared__ uint64_t bars[5];
     __shared__ int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 4; ++i) ptx::mbar_init(ptx::smem_u32(&bars[i]), 1);
+        for (int i = 0; i < 5; ++i) ptx::mbar_init(ptx::smem_u32(&bars[i]), 1);
         ptx::fence_mbar_init();
+        ptx::mbar_arrive(ptx::smem_u32(&bars[4]));
         abort_flag = 0;
     }
     __syncthreads();
     const unsigned long long t0 = ptx::globaltimer_ns();
     bool ok;
     if (warp < 4) ok = ptx::mbar_wait_limit(ptx::smem_u32(&bars[warp]), 0, &abort_flag, warp == 0 ? limit_ns : ptx::WAIT_LIMIT_NS);
-    else ok = wait_count(&selftest_counter, 1, &abort_flag, ptx::WAIT_LIMIT_NS);      // the wait of the tile folding: released by the flag
+    else if (warp == 4) ok = wait_count(&selftest_counter, 1, &abort_flag, ptx::WAIT_LIMIT_NS);      // the wait of the tile folding: released by the flag
+    else ok = ptx::mbar_wait_warp(ptx::smem_u32(&bars[lane & 1 ? 3 : 4]), 0, &abort_flag);
     const unsigned long long t1 = ptx::globaltimer_ns();
-    if (!ok && lane == 0) {
+    if (warp == 5) {
+        if (ok) atomicOr(err, ERR_BAD_ITEM);
+    } else if (!ok && lane == 0) {
         atomicOr(err, warp == 0 ? ERR_WAIT_PRODUCER : warp == 1 ? ERR_WAIT_DEQUANT : warp == 2 ? ERR_WAIT_MMA : warp == 3 ? ERR_WAIT_SOFTMAX : ERR_WAIT_FOLD);
         waited_ns[warp] = t1 - t0;
     }
@@ -452,7 +457,7 @@ __global__ void __launch_bounds__(160) wait_selftest_kernel(unsigned long long l
 extern "C" int llattn_wait_selftest(unsigned long long limit_ns, int* err_word, unsigned long long* waited_ns6, void* stream) {
     if (!err_word || !waited_ns6) return fail(LLATTN_EINVAL, "wait_selftest: null pointer");
     if (limit_ns == 0 || limit_ns > 100000000ull) return fail(LLATTN_EINVAL, "wait_selftest: limit of %llu ns; 1 ns .. 100 ms", limit_ns);
-    llattn::wait_selftest_kernel<<<1, 160, 0, as_stream(stream)>>>(limit_ns, err_word, waited_ns6);
+    llattn::wait_selftest_kernel<<<1, 192, 0, as_stream(stream)>>>(limit_ns, err_word, waited_ns6);
     CU(cudaGetLastError());
     return LLATTN_OK;
 }

@@ -67,6 +67,12 @@ __device__ __forceinline__ bool mbar_wait_limit(uint32_t bar, uint32_t parity, v
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     return mbar_wait_limit(bar, parity, abort_flag, WAIT_LIMIT_NS);
 }
+// The same with one answer for the whole warp: false as soon as one lane gave up. Once the abort flag is up, some lanes of a waiting
+// warp may still see the phase complete while others see the flag; a role whose next step is a warp-wide instruction (elect.sync,
+// tcgen05.ld / st, a vote, __syncwarp) has to reach it with all lanes or leave with all lanes, else it hangs where it should end.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
 
 // Programmatic dependent launch. A kernel launched with the attribute may start once every CTA of the kernel before it in the
 // stream has said launch_dependents (or is gone); wait returns when that kernel has completed and its writes are visible.
