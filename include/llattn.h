@@ -92,10 +92,21 @@ int llattn_qkv_prepare_commit(const float* qkv, const int32_t* pos, const float*
  * engine/moe_i8.cu:34-41 after relayout_strips); q [ntokens][K] int8 in fragment order inside every 128-group,
  * s and sum [ntokens][K/128] (the moe8::Act triple, engine/moe_i8.cu:55-66); Y [ntokens][rows] fp32. rows and K are
  * multiples of 128. Same float operations in the same order as the reference kernel: bit-identical results.
- * W and q must be 16-byte aligned. err_word is a device int that the kernel for many tokens ORs an error code into when
- * a bounded wait runs out (Y is then incomplete); may be NULL. */
+ * W and q must be 16-byte aligned. err_word is a device int, zeroed by the caller, that the kernel for many tokens ORs the
+ * codes of llattn_device_status into when a bounded wait runs out; with NULL they go to a word of the library's own, which
+ * llattn_dense_status reads. After an error some of Y has its sums added and some has not: restore Y before trying again. */
 int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int32_t* sum, float* Y, int ntokens, int rows, int K,
                       int* err_word, void* stream);
+
+/* Reads (and clears) the current device's word for llattn_dense_w4a8 calls without one of their own; synchronises `stream`.
+ * LLATTN_EDEVICE and the bits in *code when a wait of any such call on the device ran out since the word was last read: call
+ * it where the results of a step are read, behind the work of every stream that ran such calls. No counterpart in the
+ * reference, whose kernels have no waits that can fail. */
+int llattn_dense_status(void* stream, int* code);
+
+/* The device address of that word on the current device, for a caller that copies it out with its results (a captured
+ * graph has no place for llattn_dense_status). */
+int llattn_dense_error_word(int** word);
 
 /* ---- the reference operator pair on caller-owned buffers.
  * llattn_args mirrors attn::Args (engine/attn.cu:51-64) field for field. */

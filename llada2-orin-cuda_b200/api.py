@@ -28,7 +28,7 @@ EXPORTS = (
     "llattn_kv_commit_paged", "llattn_qk_norm_rope", "llattn_qkv_prepare_commit", "llattn_attn_partial", "llattn_attn_combine", "llattn_create", "llattn_destroy",
     "llattn_plan_create", "llattn_plan_destroy", "llattn_plan_get_stats", "llattn_plan_preview", "llattn_attention",
     "llattn_plan_update", "llattn_attention_host", "llattn_host_flush", "llattn_device_status",
-    "llattn_dense_w4a8", "llattn_kvpool_create", "llattn_kvpool_destroy", "llattn_kvpool_open", "llattn_kvpool_append", "llattn_kvpool_pages", "llattn_kvpool_mark_committed",
+    "llattn_dense_w4a8", "llattn_dense_status", "llattn_dense_error_word", "llattn_kvpool_create", "llattn_kvpool_destroy", "llattn_kvpool_open", "llattn_kvpool_append", "llattn_kvpool_pages", "llattn_kvpool_mark_committed",
     "llattn_kvpool_close", "llattn_kvpool_stats", "llattn_attention_static", "llattn_wait_selftest",
 )
 
@@ -97,6 +97,8 @@ def lib() -> ctypes.CDLL:
         L.llattn_attention_host.argtypes = [c_void_p, c_void_p, POINTER(_IO), c_void_p]
         L.llattn_host_flush.argtypes = [c_void_p, c_void_p]
         L.llattn_dense_w4a8.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]
+        L.llattn_dense_status.argtypes = [c_void_p, POINTER(c_int)]
+        L.llattn_dense_error_word.argtypes = [POINTER(c_void_p)]
         L.llattn_kvpool_create.argtypes = [c_int, POINTER(c_void_p)]
         L.llattn_kvpool_destroy.argtypes = [c_void_p]
         L.llattn_kvpool_destroy.restype = None
@@ -217,11 +219,29 @@ def commit_block(final_ids, last_forward_ids, Kf, Vf, cache, max_blocks: int, bl
 def dense_w4a8(W, q, s, qsum, Y, err_word=None, stream=None) -> None:
     """Engine::gemm<4, 2>(Ly.dense, ..., oA.a, ones, HID, HID, nullptr, h, 1, 2) (engine/engine.cu:434) for any number of
     tokens: Y [ntokens][rows] fp32 += W4.A8 projection of the int8 activations (q [ntokens][K] in fragment order, s and
-    qsum [ntokens][K/128]) with the weight strips W in the engine's device layout. Bit-identical to the reference."""
+    qsum [ntokens][K/128]) with the weight strips W in the engine's device layout. Bit-identical to the reference.
+    err_word: an int32 device tensor [1], zeroed by the caller, that the kernel for many tokens ORs an error code into when one of
+    its bounded waits runs out; without one the code goes to the library's own word, see dense_status. Y is then
+    partly added to: restore it before trying again."""
     ntokens, K = q.shape
     rows = Y.shape[1]
     _check(lib().llattn_dense_w4a8(_ptr(W), _ptr(q), _ptr(s), _ptr(qsum), _ptr(Y), ntokens, rows, K,
                                    _ptr(err_word) if err_word is not None else None, _stream(stream)))
+
+
+def dense_status(stream=None) -> int:
+    """0, or LlattnError (EDEVICE) when a wait of a dense_w4a8 call without an err_word ran out on the current device since the
+    last dense_status. Synchronises `stream`; call it where a step's results are read."""
+    code = c_int(0)
+    _check(lib().llattn_dense_status(_stream(stream), byref(code)))
+    return code.value
+
+
+def dense_error_word() -> int:
+    """Device address of the word that dense_status reads (current device)."""
+    word = c_void_p()
+    _check(lib().llattn_dense_error_word(byref(word)))
+    return word.value
 
 
 # ------------------------------------------------------------------ producer

@@ -41,8 +41,13 @@ struct DenseParams {
     const int32_t* sum;    // [ntokens][K / 128]
     float* Y;              // [ntokens][rows], accumulated into
     int ntokens, rows, K;
-    int* err;              // device error word, or null
+    int* err;              // the caller's device error word, or null: the library's own
 };
+
+// What calls without an error word of their own report in: one word per device, part of the library image, read and cleared by
+// llattn_dense_status. (Not in an allocation: a first call may be under stream capture.)
+static __device__ int g_dense_err;
+__device__ __forceinline__ void report_error(const DenseParams& p, int bits) { atomicOr(p.err ? p.err : &g_dense_err, bits); }
 
 __device__ __forceinline__ void mma_m16n8k32_u8s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -353,7 +358,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DensePa
     const uint32_t sm0 = ptx::smem_u32(dw_smem), bar0 = sm0 + T::BAR;
     auto BAR = [&](int i) -> uint32_t { return bar0 + 8u * uint32_t(i); };
     if (sm0 & 1023u) {                         // the swizzled tiles need a 1024-byte aligned base: report, do nothing
-        if (tid == 0 && p.err) atomicOr(p.err, ERR_SMEM_ALIGN);
+        if (tid == 0) report_error(p, ERR_SMEM_ALIGN);
         return;
     }
     if (tid == 0) {
@@ -593,7 +598,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DensePa
         volatile int never = 0;
         if (!ptx::mbar_wait(BAR(WB_SPARE), 0, &never)) errbits |= ERR_WAIT_TEARDOWN;
     }
-    if (errbits && p.err) atomicOr(p.err, errbits);
+    if (errbits) report_error(p, errbits);
     ptx::tc_fence_before();
     __syncthreads();
     if (warp == DW_WARP_MMA) ptx::tmem_dealloc(tmem, T::TMEM);

@@ -317,6 +317,28 @@ int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int3
     return LLATTN_OK;
 }
 
+int llattn_dense_error_word(int** word) {
+    if (!word) return fail(LLATTN_EINVAL, "dense_error_word: null pointer");
+    *word = nullptr;
+    void* p = nullptr;
+    CU(cudaGetSymbolAddress(&p, llattn::g_dense_err));
+    *word = static_cast<int*>(p);
+    return LLATTN_OK;
+}
+
+int llattn_dense_status(void* stream, int* code) {
+    if (!code) return fail(LLATTN_EINVAL, "dense_status: null pointer");
+    *code = 0;
+    CU(cudaStreamSynchronize(as_stream(stream)));
+    CU(cudaMemcpyFromSymbol(code, llattn::g_dense_err, sizeof(int)));
+    if (*code) {
+        const int zero = 0;
+        CU(cudaMemcpyToSymbol(llattn::g_dense_err, &zero, sizeof(int)));
+        return fail(LLATTN_EDEVICE, "a projection's wait ran out (error bits 0x%x): its Y is incomplete", *code);
+    }
+    return LLATTN_OK;
+}
+
 }  // extern "C"
 
 #include "llattn_attention.inl"

@@ -205,6 +205,33 @@ def test_dense_argument_errors(api):
     assert e.value.code == api.EINVAL
 
 
+# A call without an error word of its own still has a place where an expired wait is read. (The codes come from the wait
+# self-test, which no projection takes part in: nothing here fails.)
+@pytest.mark.gpu
+def test_dense_reports_without_an_error_word(api, orc, pkg):
+    assert api.dense_status() == 0
+    waited = torch.zeros(6, dtype=torch.int64, device="cuda")
+    api._check(api.lib().llattn_wait_selftest(1_000_000, api.dense_error_word(), waited.data_ptr(), None))
+    torch.cuda.synchronize()
+    with pytest.raises(api.LlattnError) as e:
+        api.dense_status()
+    assert e.value.code == api.EDEVICE and "0x8f" in str(e.value)                    # every role's code
+    assert api.dense_status() == 0                                                   # read once, cleared
+    wl, n = pkg.workload, 300
+    strips, _, _, _ = wl.dense_weights(2048, 2048, 61)
+    q, s, qsum = wl.int8_activations(n, 2048, 62)
+    want = np.zeros((n, 2048), np.float32)
+    orc.dense_w4a8(strips, q, s, qsum, want)
+    Y = torch.zeros((n, 2048), device="cuda")
+    api.dense_w4a8(_dev(strips), _dev(q), _dev(s), _dev(qsum), Y)
+    assert api.dense_status() == 0 and np.array_equal(Y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+def test_dense_status_argument_errors(api):
+    assert api.lib().llattn_dense_status(None, None) == api.EINVAL
+    assert api.lib().llattn_dense_error_word(None) == api.EINVAL
+
+
 # Where the tcgen05 form takes over: 32, 64 and 128 tokens a CTA, with a ragged last tile, one and several waves, an odd number of
 # groups (a stage of one), and more groups than factors held at a time (16)
 @pytest.mark.gpu
