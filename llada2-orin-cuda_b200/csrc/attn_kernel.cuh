@@ -313,8 +313,9 @@ __device__ __noinline__ float raise_reference(float mref, float cs, bool over, i
                                               uint32_t ts, uint32_t bar_pv, uint32_t par_pv, volatile int* abort_flag) {
     const float mnew = over ? cs : mref;
     const float corr = over ? ex2(mref - mnew) : 1.f;      // 0 for a row that had no reference yet
+    bool ok = true;                            // a lane whose wait ran out walks on: the accesses to tensor memory want the whole warp
     if (have_acc) {
-        if (!ptx::mbar_wait(bar_pv, par_pv, abort_flag)) return __int_as_float(0x7fc00000);
+        ok = ptx::mbar_wait(bar_pv, par_pv, abort_flag);
         ptx::tc_fence_after();
 #pragma unroll 1
         for (int oc = 0; oc < 4; ++oc) {
@@ -347,7 +348,7 @@ __device__ __noinline__ float raise_reference(float mref, float cs, bool over, i
         ptx::tmem_st16(ts + col, r);
     }
     ptx::tmem_wait_st();
-    return mnew;
+    return ok ? mnew : __int_as_float(0x7fc00000);
 }
 
 // One tile of NU 32-key chunks for one query row: S -> P in a single pass, branch-free except for the vote that guards
@@ -455,8 +456,9 @@ __device__ __noinline__ float2 raise_reference_rows16(float2 mref, float sl2, in
     cA = quad_max(cA) * sl2; cB = quad_max(cB) * sl2;
     const float2 mnew = make_float2(cA > mref.x + RESCALE_SLACK ? cA : mref.x, cB > mref.y + RESCALE_SLACK ? cB : mref.y);
     const float fA = mnew.x != mref.x ? ex2(mref.x - mnew.x) : 1.f, fB = mnew.y != mref.y ? ex2(mref.y - mnew.y) : 1.f;
+    bool ok = true;                            // as in raise_reference
     if (have_acc) {
-        if (!ptx::mbar_wait(bar_pv, par_pv, abort_flag)) return make_float2(__int_as_float(0x7fc00000), 0.f);
+        ok = ptx::mbar_wait(bar_pv, par_pv, abort_flag);
         ptx::tc_fence_after();
         // 128 dims, then the row sum in the first of the 16 columns behind them (32 columns from 16 before the end take it in)
 #pragma unroll 1
@@ -491,7 +493,7 @@ __device__ __noinline__ float2 raise_reference_rows16(float2 mref, float sl2, in
     exp_chunk(r, pk, pkl, dup2(sl2), dup2(-mnew.x), dup2(-mnew.y));
     ptx::tmem_st16x128_x4(ts + 32 * chunk, pk);
     ptx::tmem_st16x128_x4(ts + 32 * chunk + 16, pkl);
-    return mnew;
+    return ok ? mnew : make_float2(__int_as_float(0x7fc00000), 0.f);
 }
 
 // One tile of NU 32-key chunks for a warp's sixteen query rows: S -> P in a single pass, branch-free except for the vote that
@@ -700,6 +702,9 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
 
     if (warp < SOFTMAX_WARPS) {
         // ================================================================== softmax + epilogue
+        // This role's next steps are warp-wide (tensor memory, staging), so no lane parts from its warp at a wait that ran out: the wait for S
+        // gives one answer per warp, and a lane that gave up on the run's last PV writes what there is with the others and is
+        // missed by the vote in front of the next run. A vote at that wait as well costs 1 % at 64 x 32 K, these nothing that shows.
         if constexpr (PRECISE) {
         // Warps w and w + 4 may access lanes 32 w .. 32 w + 31 of tensor memory. In the tile loop each takes sixteen of these rows
         // with all their keys, a row spread over four threads as in an mma fragment: nothing is exchanged between warps. At the two
@@ -715,7 +720,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
         uint32_t t = 0;
         bool alive = true;
 #pragma unroll 1
-        for (int ii = i0; ii < i1 && alive; ++ii) {
+        for (int ii = i0; ii < i1 && __all_sync(0xffffffffu, alive); ++ii) {
             WorkItem w; SeqDesc s; MergeDesc md{0, 0, 0, 1};
             if (!fetch_item(p, ii, w, s, first_run, i0_any)) continue;
             const int U = w.rec_count + w.fresh, ntiles = (U + TILE_UNITS - 1) / TILE_UNITS;
@@ -754,7 +759,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
             for (int i = 0; i < ntiles && alive; ++i, ++t) {
                 const int b = t & 1, nu = min(TILE_UNITS, U - TILE_UNITS * i);
                 LLATTN_TR(1, t);
-                if (!s_ready && !ptx::mbar_wait(BAR(B_S_FULL + b), (t >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; break; }
+                if (!__all_sync(0xffffffffu, s_ready) && !ptx::mbar_wait_warp(BAR(B_S_FULL + b), (t >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; break; }
                 LLATTN_TR(2, t);
                 ptx::tc_fence_after();
                 const uint32_t ts = trow + TM_S + b * 128, bar_pv = BAR(B_PV_DONE + (b ^ 1)), par_pv = ((t - 1) >> 1) & 1;
@@ -800,7 +805,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
             // function).
             const uint32_t tl = t - 1;
             fetch_item(p, ii, w, s, first_run, i0_any, &md);     // again: cheaper than a dozen registers through the loop above
-            if (!ptx::mbar_wait(BAR(B_PV_DONE + (tl & 1)), (tl >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; break; }
+            if (!ptx::mbar_wait(BAR(B_PV_DONE + (tl & 1)), (tl >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; }
             ptx::tc_fence_after();
             float lsum;
             {
@@ -910,7 +915,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                         qsum[row] = ro.qsum;
                         ptx::mbar_arrive(BAR(B_QSUM));
                     } else {
-                        if (!ptx::mbar_wait(BAR(B_QSUM), q8_runs & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; break; }
+                        if (!ptx::mbar_wait_warp(BAR(B_QSUM), q8_runs & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; break; }
                         ro.qsum += qsum[row];
                     }
                     ++q8_runs;
@@ -933,7 +938,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
         uint32_t t = 0;
         bool alive = true;
 #pragma unroll 1
-        for (int ii = i0; ii < i1 && alive; ++ii) {
+        for (int ii = i0; ii < i1 && __all_sync(0xffffffffu, alive); ++ii) {
             WorkItem w; SeqDesc s; MergeDesc md{0, 0, 0, 1};
             if (!fetch_item(p, ii, w, s, first_run, i0_any)) continue;
             const int U = w.rec_count + w.fresh, ntiles = (U + TILE_UNITS - 1) / TILE_UNITS;
@@ -971,7 +976,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
             for (int i = 0; i < ntiles && alive; ++i, ++t) {
                 const int b = t & 1, nu = min(TILE_UNITS, U - TILE_UNITS * i);
                 LLATTN_TR(1, t);
-                if (!s_ready && !ptx::mbar_wait(BAR(B_S_FULL + b), (t >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; break; }
+                if (!__all_sync(0xffffffffu, s_ready) && !ptx::mbar_wait_warp(BAR(B_S_FULL + b), (t >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; break; }
                 LLATTN_TR(2, t);
                 ptx::tc_fence_after();
                 const uint32_t ts = tlane + TM_S + b * 128, bar_pv = BAR(B_PV_DONE + (b ^ 1)), par_pv = ((t - 1) >> 1) & 1;
@@ -1012,7 +1017,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
             // function).
             const uint32_t tl = t - 1;
             fetch_item(p, ii, w, s, first_run, i0_any, &md);     // again: cheaper than a dozen registers through the loop above
-            if (!ptx::mbar_wait(BAR(B_PV_DONE + (tl & 1)), (tl >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; break; }
+            if (!ptx::mbar_wait(BAR(B_PV_DONE + (tl & 1)), (tl >> 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; }
             ptx::tc_fence_after();
             float lsum;
             {
@@ -1226,7 +1231,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
 #pragma unroll 1
             for (uint32_t u = (pk - r0) % PRODUCERS; u < uint32_t(w.rec_count); u += PRODUCERS) {
                 const uint32_t r = r0 + u, slot = r % NRAW;
-                if (r >= NRAW && !ptx::mbar_wait(BAR(B_RAW_EMPTY + slot), ((r / NRAW) - 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_PRODUCER; break; }
+                if (r >= NRAW && !ptx::mbar_wait_warp(BAR(B_RAW_EMPTY + slot), ((r / NRAW) - 1) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_PRODUCER; break; }
                 if (lane == 0) {
                     const size_t ridx = s.pages ? size_t(s.pages[hbase + w.rec_begin + u]) : hbase + w.rec_begin + u;
                     ptx::mbar_arrive_expect_tx(BAR(B_RAW_FULL + slot), REC_BYTES);

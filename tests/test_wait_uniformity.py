@@ -4,8 +4,9 @@ The kernels' waits are bounded and an abort flag releases them. Evaluated lane b
 lanes of a warp and "give up" in others; if the next step is a warp-wide instruction (elect.sync in front of an MMA or a commit, a
 tensor-memory load or store, __syncwarp, a vote) the lanes would meet at different ones, which may hang. Running such a case needs
 a kernel that fails, so the rule is checked on the sources: in every role (and every function called by one) that has a warp-wide
-instruction, each wait is a warp's, made uniform at once, or one that no flag releases (its flag is `never`). That the warp's wait
-itself has one answer is shown on the device by llattn_wait_selftest."""
+instruction, each wait is a warp's, made uniform at once, one that no flag releases (its flag is `never`), or one that no lane leaves
+by: the lane notes its answer (`ok = wait`, or `alive = false` where the loop around it votes on `alive`) and walks on. That the warp's
+wait itself has one answer is shown on the device by llattn_wait_selftest."""
 import importlib
 import os
 import re
@@ -53,7 +54,10 @@ def _lane_waits(block):
         call = block[m.start():block.index(";", m.start())]
         before = block[:m.start()].rstrip()
         uniform = before.endswith(("uniform_i32(ptx::", "__all_sync(0xffffffffu, ptx::"))
-        if not uniform and "&never" not in call:
+        rest = block[m.start():block.index("\n", m.start())]
+        votes = "for (int ii = i0; ii < i1 && __all_sync(0xffffffffu, alive); ++ii)" in block
+        stays = before.endswith("    ok = ptx::") or (votes and rest.endswith("{ alive = false; errbits |= ERR_WAIT_SOFTMAX; }"))
+        if not uniform and not stays and "&never" not in call:
             bad.append(call[:100])
     return bad
 
@@ -64,8 +68,17 @@ def test_projection_roles(pkg):
     assert [w for r in roles for w in _lane_waits(r)] == []
 
 
+def test_attention_roles(pkg):
+    text = _source(pkg, "attn_kernel.cuh")
+    roles = _roles(text, "if (warp < SOFTMAX_WARPS)")
+    assert len(roles) == 5 and sum(bool(WARP_WIDE.search(r)) for r in roles) == 4          # all but the dequantising warps
+    called = [_block(text, text.index(f))[0] for f in ("float raise_reference(", "float2 raise_reference_rows16(")]
+    assert [w for r in roles + called for w in _lane_waits(r)] == []
+
+
 def test_the_check_itself():
-    lane = "{ if (!ptx::mbar_wait(BAR(0), 0, abort_flag)) break; ptx::tmem_ld16(t, r); }"
+    lane = "{ if (!ptx::mbar_wait(BAR(0), 0, abort_flag)) break;\n ptx::tmem_ld16(t, r); }"
     assert len(_lane_waits(lane)) == 1
     assert _lane_waits(lane.replace("mbar_wait(", "mbar_wait_warp(")) == []
     assert _lane_waits(lane.replace("ptx::tmem_ld16(t, r);", "")) == []
+    assert len(_lane_waits("{ if (!ptx::mbar_wait(B, 0, f)) { alive = false; errbits |= ERR_WAIT_SOFTMAX; }\n ptx::tmem_ld16(t, r); }")) == 1
