@@ -200,6 +200,9 @@ void llattn_destroy(llattn_ctx* ctx);
 int llattn_plan_create(llattn_ctx* ctx, const llattn_seq* seqs_host, int nseq, int nctas, llattn_plan** out);
 void llattn_plan_destroy(llattn_plan* plan);
 int llattn_plan_get_stats(const llattn_plan* plan, llattn_plan_stats* out);
+/* The softmax warps that a LLATTN_IO_PRECISE_P call of this plan gets as the plan is now, 4 or 8, with an fp32 output (o32 != 0) or
+ * without. The two forms' results may differ in the last bits; a captured call keeps the form it was captured with. */
+int llattn_plan_precise_warps(const llattn_plan* plan, int o32, int* warps);
 
 /* New lengths (and cache / page-table pointers) for an existing plan, without allocation or device synchronisation:
  * the work list is rebuilt on the host into the plan's pinned mirror and copied over the plan's device blob with one

@@ -26,7 +26,7 @@ IO_PRECISE_P = 1  # llattn_io.flags
 EXPORTS = (
     "llattn_version", "llattn_last_error", "llattn_pick_bpc", "llattn_chunks_for", "llattn_tile_units", "llattn_kv_commit",
     "llattn_kv_commit_paged", "llattn_qk_norm_rope", "llattn_qkv_prepare_commit", "llattn_attn_partial", "llattn_attn_combine", "llattn_create", "llattn_destroy",
-    "llattn_plan_create", "llattn_plan_destroy", "llattn_plan_get_stats", "llattn_plan_preview", "llattn_attention",
+    "llattn_plan_create", "llattn_plan_destroy", "llattn_plan_get_stats", "llattn_plan_precise_warps", "llattn_plan_preview", "llattn_attention",
     "llattn_plan_update", "llattn_attention_host", "llattn_host_flush", "llattn_device_status",
     "llattn_dense_w4a8", "llattn_dense_status", "llattn_dense_error_word", "llattn_kvpool_create", "llattn_kvpool_destroy", "llattn_kvpool_open", "llattn_kvpool_append", "llattn_kvpool_pages", "llattn_kvpool_mark_committed",
     "llattn_kvpool_close", "llattn_kvpool_stats", "llattn_attention_static", "llattn_wait_selftest",
@@ -91,6 +91,7 @@ def lib() -> ctypes.CDLL:
         L.llattn_plan_destroy.argtypes = [c_void_p]
         L.llattn_plan_destroy.restype = None
         L.llattn_plan_get_stats.argtypes = [c_void_p, POINTER(PlanStats)]
+        L.llattn_plan_precise_warps.argtypes = [c_void_p, c_int, POINTER(c_int)]
         L.llattn_plan_preview.argtypes = [POINTER(_Seq), c_int, c_int, POINTER(PlanStats), c_void_p, c_int, c_void_p, c_int]
         L.llattn_attention.argtypes = [c_void_p, c_void_p, POINTER(_IO), c_void_p]
         L.llattn_plan_update.argtypes = [c_void_p, POINTER(_Seq), c_int, c_void_p]
@@ -420,6 +421,12 @@ class Plan:
         st = PlanStats()
         _check(lib().llattn_plan_get_stats(self._h, byref(st)))
         self.stats = st
+
+    def precise_warps(self, o32: bool) -> int:
+        """Softmax warps (4 or 8) of a precise call of this plan as it is now, with or without an fp32 output."""
+        warps = c_int(0)
+        _check(lib().llattn_plan_precise_warps(self._h, int(o32), byref(warps)))
+        return warps.value
 
     def close(self) -> None:
         if self._h:

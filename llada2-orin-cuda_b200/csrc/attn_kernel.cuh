@@ -107,13 +107,13 @@ constexpr int ATTN_SMEM_BYTES = SM_QSUM + QR * 4;
 #ifndef LLATTN_WARP_ARRIVE
 #define LLATTN_WARP_ARRIVE 0       // 1: one arrival per softmax warp on the P barrier instead of one per thread
 #endif
-__host__ __device__ constexpr int softmax_warps(bool precise) { return precise ? 8 : 4; }
+__host__ __device__ constexpr int softmax_warps(bool rows16) { return rows16 ? 8 : 4; }
 constexpr int DEQUANT_WARPS = LLATTN_DEQUANT_WARPS, GROUP_WARPS = LLATTN_GROUP_WARPS, DEQUANT_GROUPS = DEQUANT_WARPS / GROUP_WARPS;
 constexpr int GROUP_THREADS = 32 * GROUP_WARPS, DQ_PASSES = 16 / GROUP_WARPS;      // a group converts one record: 32 keys, two per warp and pass
 // Service warps, one per scheduler (a warp runs on scheduler warp % 4 and the softmax warps cannot move): PV issue, S
 // issue and two copy producers that take alternate records, so that no scheduler carries much more than the others.
 constexpr int PRODUCERS = 2;
-__host__ __device__ constexpr int attn_threads(bool precise) { return 32 * (softmax_warps(precise) + DEQUANT_WARPS + 2 + PRODUCERS); }
+__host__ __device__ constexpr int attn_threads(bool rows16) { return 32 * (softmax_warps(rows16) + DEQUANT_WARPS + 2 + PRODUCERS); }
 constexpr int ATTN_THREADS = attn_threads(false);  // 512; 640 in the precise form
 constexpr int TMEM_COLS = 512;
 constexpr int TM_S = 0, TM_O = 256, TM_L = TM_O + 128, TM_Q = 400;   // S at columns 0 and 128, O at 256..383, row sum at 384, Q at 400..463
@@ -286,9 +286,10 @@ __device__ __forceinline__ void exp2_pair_poly(float x0, float x1, float& e0, fl
     e1 = __uint_as_float(q1 + (t1 << 23));
 }
 
-// Score pairs J0 .. J1-1 of 16 scores -> packed fp16 p.
-template <int J0, int J1>
-__device__ __forceinline__ void exp_pairs16(const uint32_t (&r)[16], uint32_t* pk, unsigned long long sl2x2, unsigned long long nm2) {
+// Score pairs J0 .. J1-1 of 16 scores -> packed fp16 p. PRECISE: also the fp16 remainder p - fp16(p) (exact in fp32, then
+// rounded once more: together the pair carries p to about 22 bits).
+template <int J0, int J1, bool PRECISE>
+__device__ __forceinline__ void exp_pairs16(const uint32_t (&r)[16], uint32_t* pk, uint32_t* pkl, unsigned long long sl2x2, unsigned long long nm2) {
 #pragma unroll
     for (int j = J0; j < J1; ++j) {
         if (LLATTN_SKIP & 2) { pk[j] = r[2 * j] & 0x03ff03ffu; continue; }
@@ -299,6 +300,11 @@ __device__ __forceinline__ void exp_pairs16(const uint32_t (&r)[16], uint32_t* p
         else { e0 = ex2(x0); e1 = ex2(x1); }
         const half2 h = __floats2half2_rn(e0, e1);
         pk[j] = *reinterpret_cast<const uint32_t*>(&h);
+        if (PRECISE) {
+            const float2 hf = __half22float2(h);
+            const half2 l = __floats2half2_rn(e0 - hf.x, e1 - hf.y);
+            pkl[j] = *reinterpret_cast<const uint32_t*>(&l);
+        }
     }
 }
 
@@ -309,7 +315,7 @@ __device__ __forceinline__ void exp_pairs16(const uint32_t (&r)[16], uint32_t* p
 // of line so that the common path stays small.
 // tlane: tensor-memory address of the warp's lanes at column 0; ts: the tile's S / P buffer; bar_pv, par_pv: barrier and
 // parity of "PV of the previous tile has completed". Returns the row's new reference, NaN when that wait ran out.
-__device__ __noinline__ float raise_reference(float mref, float cs, bool over, int chunks_done, bool have_acc, uint32_t tlane,
+__device__ __noinline__ float raise_reference(float mref, float cs, bool over, int chunks_done, bool have_acc, bool precise, uint32_t tlane,
                                               uint32_t ts, uint32_t bar_pv, uint32_t par_pv, volatile int* abort_flag) {
     const float mnew = over ? cs : mref;
     const float corr = over ? ex2(mref - mnew) : 1.f;      // 0 for a row that had no reference yet
@@ -333,11 +339,11 @@ __device__ __noinline__ float raise_reference(float mref, float cs, bool over, i
         ptx::tmem_st16(tlane + TM_L, r);
     }
     const half2 ch = __float2half2_rn(corr);
-    // P chunk pc sits in columns 32 pc .. 32 pc + 15
+    // P chunk pc sits in columns 32 pc .. 32 pc + 15, its remainder (precise mode) in the 16 columns after them
 #pragma unroll 1
-    for (int pc = 0; pc < chunks_done; ++pc) {
+    for (int pc = 0; pc < (precise ? 2 : 1) * chunks_done; ++pc) {
         uint32_t r[16];
-        const uint32_t col = 32 * pc;
+        const uint32_t col = precise ? 16 * pc : 32 * pc;
         ptx::tmem_ld16(ts + col, r);
         ptx::tmem_wait_ld_tied(r);
 #pragma unroll
@@ -357,7 +363,7 @@ __device__ __noinline__ float raise_reference(float mref, float cs, bool over, i
 // goes back over the first 16 of the 32 S columns it came from. Before the last chunk's exponentials the barrier of the
 // next tile's S is tested (next_bar != 0), so that the test's latency is covered and the next tile starts without a wait
 // when its S is already there. Returns false when a wait of the rare path ran out.
-template <int NU>
+template <int NU, bool PRECISE>
 __device__ __forceinline__ bool softmax_tile(float& mref, float sl2, unsigned long long sl2x2, uint32_t tlane, uint32_t ts, bool have_acc,
                                              uint32_t bar_pv, uint32_t par_pv, volatile int* abort_flag, uint32_t next_bar, uint32_t next_par,
                                              bool& next_ready) {
@@ -376,20 +382,22 @@ __device__ __forceinline__ bool softmax_tile(float& mref, float sl2, unsigned lo
         const float cs = cm * sl2;
         const bool over = cs > mref + RESCALE_SLACK;
         if (__any_sync(0xffffffffu, over)) {
-            mref = raise_reference(mref, cs, over, c, have_acc, tlane, ts, bar_pv, par_pv, abort_flag);
+            mref = raise_reference(mref, cs, over, c, have_acc, PRECISE, tlane, ts, bar_pv, par_pv, abort_flag);
             if (__any_sync(0xffffffffu, mref != mref)) return false;
             nm2 = dup2(-mref);
         }
-        uint32_t pk[16];
+        uint32_t pk[16], pkl[PRECISE ? 16 : 1];
         if (c + 1 < NU) ptx::tmem_ld16(ts + 32 * (c + 1), n0);
         else next_ready = next_bar != 0 && ptx::mbar_try_wait(next_bar, next_par);
-        exp_pairs16<0, 8>(c0, pk, sl2x2, nm2);
+        exp_pairs16<0, 8, PRECISE>(c0, pk, pkl, sl2x2, nm2);
         ptx::tmem_st8(ts + 32 * c, pk);
         if (c + 1 < NU) ptx::tmem_ld16(ts + 32 * (c + 1) + 16, n1);
-        exp_pairs16<0, 5>(c1, pk + 8, sl2x2, nm2);
+        exp_pairs16<0, 5, PRECISE>(c1, pk + 8, pkl + (PRECISE ? 8 : 0), sl2x2, nm2);
         if (c + 1 < NU) { ptx::tmem_wait_ld_tied(n0, n1); cm = fmaxf(rowmax16(n0), rowmax16(n1)); }
-        exp_pairs16<5, 8>(c1, pk + 8, sl2x2, nm2);
+        exp_pairs16<5, 8, PRECISE>(c1, pk + 8, pkl + (PRECISE ? 8 : 0), sl2x2, nm2);
         ptx::tmem_st8(ts + 32 * c + 8, pk + 8);
+        // the remainders go over the second half of the chunk's S columns: all 32 have been read by now
+        if (PRECISE) { ptx::tmem_st8(ts + 32 * c + 16, pkl); ptx::tmem_st8(ts + 32 * c + 24, pkl + 8); }
     }
     return true;
 }
@@ -648,14 +656,14 @@ __device__ __forceinline__ void write_ones_column(uint8_t* smem, int lane) {
 // (kv head fastest, then chunk, then query block).
 // PRECISE: P is carried as fp16 value + fp16 remainder (two PV chains per tile), for callers that need the result to
 // within 2e-3 of the output RMS at long contexts and accept about half the throughput.
-template <bool PRECISE>
+template <bool PRECISE, bool ROWS16 = false>
 __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM_BAR);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM_MISC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM_MISC + 4);
-    constexpr int SOFTMAX_WARPS = softmax_warps(PRECISE), WARP_SERVICE = SOFTMAX_WARPS + DEQUANT_WARPS, WARP_MMA_PV = WARP_SERVICE;
-    constexpr int WARP_MMA = WARP_MMA_PV + 1, WARP_PRODUCER = WARP_MMA + 1, ATTN_THREADS = attn_threads(PRECISE);
+    constexpr int SOFTMAX_WARPS = softmax_warps(ROWS16), WARP_SERVICE = SOFTMAX_WARPS + DEQUANT_WARPS, WARP_MMA_PV = WARP_SERVICE;
+    constexpr int WARP_MMA = WARP_MMA_PV + 1, WARP_PRODUCER = WARP_MMA + 1, ATTN_THREADS = attn_threads(ROWS16);
     constexpr int P_ARRIVALS = LLATTN_WARP_ARRIVE ? SOFTMAX_WARPS : 32 * SOFTMAX_WARPS;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar0 = ptx::smem_u32(bars);
@@ -705,7 +713,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
         // This role's next steps are warp-wide (tensor memory, staging), so no lane parts from its warp at a wait that ran out: the wait for S
         // gives one answer per warp, and a lane that gave up on the run's last PV writes what there is with the others and is
         // missed by the vote in front of the next run. A vote at that wait as well costs 1 % at 64 x 32 K, these nothing that shows.
-        if constexpr (PRECISE) {
+        if constexpr (ROWS16) {
         // Warps w and w + 4 may access lanes 32 w .. 32 w + 31 of tensor memory. In the tile loop each takes sixteen of these rows
         // with all their keys, a row spread over four threads as in an mma fragment: nothing is exchanged between warps. At the two
         // ends of a run a thread is a row (lane) and each of the two warps takes half of the channels.
@@ -994,10 +1002,10 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                     mref = mx * p.sl2;
                 }
                 bool ok;
-                if (nu == TILE_UNITS) ok = softmax_tile<TILE_UNITS>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);      // every tile of a run but its last
-                else if (nu == 3) ok = softmax_tile<3>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
-                else if (nu == 2) ok = softmax_tile<2>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
-                else ok = softmax_tile<1>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
+                if (nu == TILE_UNITS) ok = softmax_tile<TILE_UNITS, PRECISE>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);      // every tile of a run but its last
+                else if (nu == 3) ok = softmax_tile<3, PRECISE>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
+                else if (nu == 2) ok = softmax_tile<2, PRECISE>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
+                else ok = softmax_tile<1, PRECISE>(mref, p.sl2, sl2x2, tlane, ts, i > 0, bar_pv, par_pv, abort_flag, next_bar, next_par, s_ready);
                 if (!ok) { alive = false; errbits |= ERR_WAIT_SOFTMAX; }
                 if (!alive) break;
                 ptx::tmem_wait_st();
@@ -1451,11 +1459,11 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                 fold_rows_shared(p.Opart, p.Mpart, p.Lpart, md, w.slot - md.slot_begin, warp, lane, smem + SM_K, p.out);      // the tiles are done with
             } else if (md.nslots == 2) {
 #pragma unroll 1
-                for (int r = r0; r < QR; r += (PRECISE ? 2 : 4) * step) {      // the precise form has not the registers for four rows
-                    int rows[PRECISE ? 2 : 4];
+                for (int r = r0; r < QR; r += (ROWS16 ? 2 : 4) * step) {      // with twenty warps the registers for four rows are not there
+                    int rows[ROWS16 ? 2 : 4];
 #pragma unroll
-                    for (int q = 0; q < (PRECISE ? 2 : 4); ++q) rows[q] = r + q * step < QR ? r + q * step : -1;
-                    fold_rows_few<PRECISE ? 2 : 4, 2>(p.Opart, p.Mpart, p.Lpart, md, rows, lane, p.out);
+                    for (int q = 0; q < (ROWS16 ? 2 : 4); ++q) rows[q] = r + q * step < QR ? r + q * step : -1;
+                    fold_rows_few<ROWS16 ? 2 : 4, 2>(p.Opart, p.Mpart, p.Lpart, md, rows, lane, p.out);
                 }
             } else if (md.nslots <= 4) {
 #pragma unroll 1
@@ -1478,12 +1486,12 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
     if (warp == WARP_MMA) ptx::tmem_dealloc(tmem, TMEM_COLS);
 }
 
-template <bool PRECISE>
-__global__ void __launch_bounds__(attn_threads(PRECISE), 1) attn_tile_kernel(const __grid_constant__ KParams p) {
+template <bool PRECISE, bool ROWS16 = false>
+__global__ void __launch_bounds__(attn_threads(ROWS16), 1) attn_tile_kernel(const __grid_constant__ KParams p) {
     // reference-grid mode: the folding launch behind this one carries the attribute of a dependent launch, may take its place
     // on the SMs this one leaves idle, and waits there (nothing behind a list-mode launch carries it)
     if (!PRECISE && !p.items) ptx::launch_dependents();
-    attn_tile_body<PRECISE>(p, blockIdx.x);
+    attn_tile_body<PRECISE, ROWS16>(p, blockIdx.x);
 }
 
 }  // namespace llattn

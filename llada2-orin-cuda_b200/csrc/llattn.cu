@@ -69,6 +69,7 @@ struct llattn_plan {
     size_t blob_bytes = 0, off_items = 0, off_cta = 0, off_first = 0;
     size_t cap_seqs = 0, cap_items = 0, cap_tiles = 0;
     int launch_ctas = 0;              // grid of every launch of this plan (CTAs beyond the used ones find no items)
+    int ntiles = 0;                   // output tiles of the plan as it is now
     cudaEvent_t ev_upload = nullptr;
     bool upload_pending = false;
     const llattn::RunDesc* d_items = nullptr;
@@ -111,6 +112,7 @@ int ensure_kernel_attrs() {
     if (dev < 64 && done[dev]) return LLATTN_OK;
     CU(cudaFuncSetAttribute(llattn::attn_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::ATTN_SMEM_BYTES));
     CU(cudaFuncSetAttribute(llattn::attn_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::ATTN_SMEM_BYTES));
+    CU(cudaFuncSetAttribute(llattn::attn_tile_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::ATTN_SMEM_BYTES));
     if (dev < 64) done[dev] = true;
     return LLATTN_OK;
 }

@@ -450,7 +450,7 @@ int llattn_create(int device, llattn_ctx** out) {
     // the largest grid a cooperative launch of the attention kernel accepts here: what fits on the device at once (fewer
     // than one CTA per SM when the process was given only a part of the GPU)
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, llattn::attn_tile_kernel<true>, llattn::attn_threads(true), llattn::ATTN_SMEM_BYTES) != cudaSuccess || per_sm < 1) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, llattn::attn_tile_kernel<true, true>, llattn::attn_threads(true), llattn::ATTN_SMEM_BYTES) != cudaSuccess || per_sm < 1) {
         cudaGetLastError();
         cudaFree(c->err_word);
         delete c;
@@ -486,6 +486,21 @@ void fill_stats(llattn_plan* pl, const HostPlan& hp, int nseq) {
     pl->stats.nctas = hp.used_ctas;
     pl->stats.total_units = hp.total_units;
     pl->stats.max_cta_units = hp.max_cta_units;
+    pl->ntiles = int(hp.merge.size());
+}
+
+// Does a precise call get eight softmax warps of sixteen rows, or four with a thread per row? Eight go through a tile up to a quarter
+// faster (256 sequences of 128 blocks: four 507 us, eight 417) and take longer over the ends of a run, where partial results and fp32
+// outputs leave in half lines and a thread has 96 registers instead of 128. So the runs have to be long enough to earn that back.
+// Measured in a graph over 612 plans: 1 .. 256 sequences of 0 .. 1024 blocks, equal and ragged, and prefill passes (us, four / eight).
+// Cut tiles, whatever the outputs: 1 x 64 blocks, 8 units a CTA, 14.7 / 15.8; 6 x 64, 12 units, 18.5 / 20.3; 6 x 128, 24 units, 25.5 / 25.1;
+// with two runs a tile earlier: 16 x 16, 12 units, 17.9 / 17.5. Whole tiles with fp32 outputs: 9 units 12.5 / 13.2 (37 x 8 blocks) and 11.8 / 11.5
+// (16 x 8), 17 units 29.4 / 28.3 (64 x 16) and 16.0 / 16.3 (37 x 16); without: one unit 21.2 / 22.0 (148 x 0), three 27.0 / 26.2 (148 x 2).
+// The choice costs 0.14 % over the faster form in the mean and 6 % at most (24 x 8 blocks, fp16 outputs).
+bool precise_rows16(const llattn_plan* pl, bool o32) {
+    const int64_t items = pl->stats.nitems, tiles = pl->ntiles;
+    if (items > tiles) return pl->stats.max_cta_units >= (2 * items <= 5 * tiles ? 12 : 18);
+    return pl->stats.total_units >= (o32 ? 12 : 2.5) * items;
 }
 
 // Lays the host plan out in the plan's pinned mirror (section offsets are fixed by the capacities chosen at creation).
@@ -623,6 +638,12 @@ int llattn_plan_get_stats(const llattn_plan* pl, llattn_plan_stats* out) {
     return LLATTN_OK;
 }
 
+int llattn_plan_precise_warps(const llattn_plan* pl, int o32, int* warps) {
+    if (!pl || !warps) return fail(LLATTN_EINVAL, "plan_precise_warps: null pointer");
+    *warps = llattn::softmax_warps(precise_rows16(pl, o32 != 0));
+    return LLATTN_OK;
+}
+
 int llattn_attention(llattn_ctx* c, const llattn_plan* pl, const llattn_io* io, void* stream) {
     using namespace llattn;
     if (!c || !pl || pl->ctx != c) return fail(LLATTN_EINVAL, "attention: plan does not belong to this context");
@@ -650,10 +671,10 @@ int llattn_attention(llattn_ctx* c, const llattn_plan* pl, const llattn_io* io, 
     p.cache_offset = io->cache_offset;
     // cooperative: the driver starts the grid only when all of its CTAs can be resident together (see plan_create)
     void* args[] = {&p};
-    const bool precise = io->flags & LLATTN_IO_PRECISE_P;
-    const void* fn = precise ? reinterpret_cast<const void*>(attn_tile_kernel<true>)
-                                                       : reinterpret_cast<const void*>(attn_tile_kernel<false>);
-    CU(cudaLaunchCooperativeKernel(fn, dim3(pl->launch_ctas), dim3(attn_threads(precise)), args, ATTN_SMEM_BYTES, as_stream(stream)));
+    const bool precise = io->flags & LLATTN_IO_PRECISE_P, rows16 = precise && precise_rows16(pl, io->O32 != nullptr);
+    const void* fn = rows16 ? reinterpret_cast<const void*>(attn_tile_kernel<true, true>)
+                   : precise ? reinterpret_cast<const void*>(attn_tile_kernel<true>) : reinterpret_cast<const void*>(attn_tile_kernel<false>);
+    CU(cudaLaunchCooperativeKernel(fn, dim3(pl->launch_ctas), dim3(attn_threads(rows16)), args, ATTN_SMEM_BYTES, as_stream(stream)));
     return LLATTN_OK;
 }
 
