@@ -98,6 +98,12 @@ int llattn_qkv_prepare_commit(const float* qkv, const int32_t* pos, const float*
 int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int32_t* sum, float* Y, int ntokens, int rows, int K,
                       int* err_word, void* stream);
 
+/* The kernel that a call of these sizes gets on a device of num_sms SMs, and the tokens of a CTA. Host only. */
+#define LLATTN_DENSE_STRIPS 0  /* a 16-row strip per CTA, a warp per 128-group */
+#define LLATTN_DENSE_TILES 1   /* 128 rows per CTA, mma.sync */
+#define LLATTN_DENSE_TCGEN05 2 /* 128 rows per CTA, tcgen05 */
+int llattn_dense_preview(int rows, int K, int ntokens, int num_sms, int* kernel, int* tokens_per_cta);
+
 /* Reads (and clears) the current device's word for llattn_dense_w4a8 calls without one of their own; synchronises `stream`.
  * LLATTN_EDEVICE and the bits in *code when a wait of any such call on the device ran out since the word was last read: call
  * it where the results of a step are read, behind the work of every stream that ran such calls. No counterpart in the

@@ -22,13 +22,14 @@ SCALE = 0.08838834764831845  # 1/sqrt(128), the constant engine/engine.cu:430 pa
 
 OK, EINVAL, ECUDA, ENOMEM, EDEVICE = 0, 1, 2, 3, 4
 IO_PRECISE_P = 1  # llattn_io.flags
+DENSE_STRIPS, DENSE_TILES, DENSE_TCGEN05 = 0, 1, 2
 
 EXPORTS = (
     "llattn_version", "llattn_last_error", "llattn_pick_bpc", "llattn_chunks_for", "llattn_tile_units", "llattn_kv_commit",
     "llattn_kv_commit_paged", "llattn_qk_norm_rope", "llattn_qkv_prepare_commit", "llattn_attn_partial", "llattn_attn_combine", "llattn_create", "llattn_destroy",
     "llattn_plan_create", "llattn_plan_destroy", "llattn_plan_get_stats", "llattn_plan_precise_warps", "llattn_plan_preview", "llattn_attention",
     "llattn_plan_update", "llattn_attention_host", "llattn_host_flush", "llattn_device_status",
-    "llattn_dense_w4a8", "llattn_dense_status", "llattn_dense_error_word", "llattn_kvpool_create", "llattn_kvpool_destroy", "llattn_kvpool_open", "llattn_kvpool_append", "llattn_kvpool_pages", "llattn_kvpool_mark_committed",
+    "llattn_dense_w4a8", "llattn_dense_preview", "llattn_dense_status", "llattn_dense_error_word", "llattn_kvpool_create", "llattn_kvpool_destroy", "llattn_kvpool_open", "llattn_kvpool_append", "llattn_kvpool_pages", "llattn_kvpool_mark_committed",
     "llattn_kvpool_close", "llattn_kvpool_stats", "llattn_attention_static", "llattn_wait_selftest",
 )
 
@@ -98,6 +99,7 @@ def lib() -> ctypes.CDLL:
         L.llattn_attention_host.argtypes = [c_void_p, c_void_p, POINTER(_IO), c_void_p]
         L.llattn_host_flush.argtypes = [c_void_p, c_void_p]
         L.llattn_dense_w4a8.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]
+        L.llattn_dense_preview.argtypes = [c_int, c_int, c_int, c_int, POINTER(c_int), POINTER(c_int)]
         L.llattn_dense_status.argtypes = [c_void_p, POINTER(c_int)]
         L.llattn_dense_error_word.argtypes = [POINTER(c_void_p)]
         L.llattn_kvpool_create.argtypes = [c_int, POINTER(c_void_p)]
@@ -228,6 +230,13 @@ def dense_w4a8(W, q, s, qsum, Y, err_word=None, stream=None) -> None:
     rows = Y.shape[1]
     _check(lib().llattn_dense_w4a8(_ptr(W), _ptr(q), _ptr(s), _ptr(qsum), _ptr(Y), ntokens, rows, K,
                                    _ptr(err_word) if err_word is not None else None, _stream(stream)))
+
+
+def dense_preview(rows: int, K: int, ntokens: int, num_sms: int):
+    """(kernel, tokens per CTA) that dense_w4a8 takes for these sizes on a device of num_sms SMs: DENSE_STRIPS, _TILES or _TCGEN05."""
+    kernel, tokens = c_int(), c_int()
+    _check(lib().llattn_dense_preview(rows, K, ntokens, num_sms, byref(kernel), byref(tokens)))
+    return kernel.value, tokens.value
 
 
 def dense_status(stream=None) -> int:

@@ -268,14 +268,46 @@ int dense_wide_tokens(int rows, int K, int ntokens, int sms) {
     consider(128, 6.9, 0.67);
     return wide;
 }
+
+// Which kernel takes a call and the tokens of a CTA, by the sizes and the SM count alone.
+struct DenseForm {
+    int kernel, tokens;
+};
+DenseForm dense_form(int rows, int K, int ntokens, int sms) {
+    if (ntokens <= DENSE_STRIP_MAX_TOKENS && dense_strips_win(rows, K, ntokens, sms)) return {LLATTN_DENSE_STRIPS, llattn::DS_TOK};
+    if (const int wide = dense_wide_tokens(rows, K, ntokens, sms)) return {LLATTN_DENSE_TCGEN05, wide};
+    // The largest tile is the cheapest per token, as long as the tiles fill the chip: with smaller ones while they do not.
+    // 2048 x 2048, in a graph: 65 .. 144 tokens 16.2 .. 16.6 us with 64 tokens a tile, 8.1 .. 8.7 with 16; 160 .. 288 tokens 16.7 and
+    // 11.3 .. 11.8 (32); at 512 tokens 16.8 (64) and 17.3 (32), at 1024 26.4 and 30.7.
+    // Never a tile larger than the tokens: 32,768 rows of K = 8192 and one token 43 us with 16, 85 with 64.
+    const long long row_tiles = rows / llattn::DN_ROWS;
+    if (ntokens <= 16 || row_tiles * ((ntokens + 15) / 16) <= sms) return {LLATTN_DENSE_TILES, 16};
+    if (ntokens <= 32 || row_tiles * ((ntokens + 31) / 32) <= sms) return {LLATTN_DENSE_TILES, 32};
+    return {LLATTN_DENSE_TILES, 64};
+}
+
+int check_dense_sizes(int rows, int K, int ntokens) {
+    if (ntokens < 0 || ntokens > 1 << 22) return fail(LLATTN_EINVAL, "dense_w4a8: ntokens = %d", ntokens);
+    if (rows <= 0 || rows % llattn::DN_ROWS || K <= 0 || K % llattn::DN_GROUP || K > 1 << 20 || rows > 1 << 20)
+        return fail(LLATTN_EINVAL, "dense_w4a8: rows = %d, K = %d (both multiples of 128)", rows, K);
+    return LLATTN_OK;
+}
 }  // namespace
+
+int llattn_dense_preview(int rows, int K, int ntokens, int num_sms, int* kernel, int* tokens_per_cta) {
+    if (!kernel || !tokens_per_cta) return fail(LLATTN_EINVAL, "dense_preview: null pointer");
+    if (int rc = check_dense_sizes(rows, K, ntokens)) return rc;
+    if (ntokens < 1 || num_sms < 1) return fail(LLATTN_EINVAL, "dense_preview: ntokens and num_sms must be positive");
+    const DenseForm f = dense_form(rows, K, ntokens, num_sms);
+    *kernel = f.kernel;
+    *tokens_per_cta = f.tokens;
+    return LLATTN_OK;
+}
 
 int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int32_t* sum, float* Y, int ntokens, int rows, int K,
                       int* err_word, void* stream) {
     if (!W || !q || !s || !sum || !Y) return fail(LLATTN_EINVAL, "dense_w4a8: null pointer");
-    if (ntokens < 0 || ntokens > 1 << 22) return fail(LLATTN_EINVAL, "dense_w4a8: ntokens = %d", ntokens);
-    if (rows <= 0 || rows % llattn::DN_ROWS || K <= 0 || K % llattn::DN_GROUP || K > 1 << 20 || rows > 1 << 20)
-        return fail(LLATTN_EINVAL, "dense_w4a8: rows = %d, K = %d (both multiples of 128)", rows, K);
+    if (int rc = check_dense_sizes(rows, K, ntokens)) return rc;
     if (ntokens == 0) return LLATTN_OK;
     if (!aligned16(W) || !aligned16(q)) return fail(LLATTN_EINVAL, "dense_w4a8: W and q must be 16-byte aligned");
     const llattn::DenseParams p{static_cast<const uint8_t*>(W), q, s, sum, Y, ntokens, rows, K, err_word};
@@ -294,26 +326,20 @@ int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int3
         });
     int sms = 0;
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (ntokens <= DENSE_STRIP_MAX_TOKENS && dense_strips_win(rows, K, ntokens, sms)) {
-        const dim3 grid(rows / 16, (ntokens + llattn::DS_TOK - 1) / llattn::DS_TOK);
-        llattn::dense_strip_kernel<<<grid, llattn::DS_THREADS, llattn::DS_SMEM_BYTES, as_stream(stream)>>>(p);
-    } else if (const int wide = dense_wide_tokens(rows, K, ntokens, sms)) {
-        const dim3 grid(rows / llattn::DN_ROWS, (ntokens + wide - 1) / wide);
-        if (wide == 32) llattn::dense_wide_kernel<32><<<grid, llattn::DW_THREADS, llattn::DenseWide<32>::SMEM, as_stream(stream)>>>(p);
-        else if (wide == 64) llattn::dense_wide_kernel<64><<<grid, llattn::DW_THREADS, llattn::DenseWide<64>::SMEM, as_stream(stream)>>>(p);
-        else llattn::dense_wide_kernel<128><<<grid, llattn::DW_THREADS, llattn::DenseWide<128>::SMEM, as_stream(stream)>>>(p);
+    const DenseForm f = dense_form(rows, K, ntokens, sms);
+    const bool strips = f.kernel == LLATTN_DENSE_STRIPS;
+    auto launch = [&](auto* kernel, int threads, int smem) {
+        kernel<<<dim3(rows / (strips ? 16 : llattn::DN_ROWS), (ntokens + f.tokens - 1) / f.tokens), threads, smem, as_stream(stream)>>>(p);
+    };
+    if (strips) launch(llattn::dense_strip_kernel, llattn::DS_THREADS, llattn::DS_SMEM_BYTES);
+    else if (f.kernel == LLATTN_DENSE_TCGEN05) {
+        if (f.tokens == 32) launch(llattn::dense_wide_kernel<32>, llattn::DW_THREADS, llattn::DenseWide<32>::SMEM);
+        else if (f.tokens == 64) launch(llattn::dense_wide_kernel<64>, llattn::DW_THREADS, llattn::DenseWide<64>::SMEM);
+        else launch(llattn::dense_wide_kernel<128>, llattn::DW_THREADS, llattn::DenseWide<128>::SMEM);
     } else {
-        // The largest tile is the cheapest per token, as long as the tiles fill the chip: with smaller ones while they do not.
-        // 2048 x 2048, in a graph: 65 .. 144 tokens 16.2 .. 16.6 us with 64 tokens a tile, 8.1 .. 8.7 with 16; 160 .. 288 tokens 16.7 and
-        // 11.3 .. 11.8 (32); at 512 tokens 16.8 (64) and 17.3 (32), at 1024 26.4 and 30.7.
-        const long long row_tiles = rows / llattn::DN_ROWS;
-        auto launch = [&](auto* kernel, int tok, int smem) {
-            kernel<<<dim3(rows / llattn::DN_ROWS, (ntokens + tok - 1) / tok), llattn::DT_THREADS, smem, as_stream(stream)>>>(p);
-        };
-        // Never a tile larger than the tokens: 32,768 rows of K = 8192 and one token 43 us with 16, 85 with 64.
-        if (ntokens <= 16 || row_tiles * ((ntokens + 15) / 16) <= sms) launch(llattn::dense_tile_kernel<16>, 16, llattn::DenseTile<16>::SMEM);
-        else if (ntokens <= 32 || row_tiles * ((ntokens + 31) / 32) <= sms) launch(llattn::dense_tile_kernel<32>, 32, llattn::DenseTile<32>::SMEM);
-        else launch(llattn::dense_tile_kernel<64>, 64, llattn::DenseTile<64>::SMEM);
+        if (f.tokens == 16) launch(llattn::dense_tile_kernel<16>, llattn::DT_THREADS, llattn::DenseTile<16>::SMEM);
+        else if (f.tokens == 32) launch(llattn::dense_tile_kernel<32>, llattn::DT_THREADS, llattn::DenseTile<32>::SMEM);
+        else launch(llattn::dense_tile_kernel<64>, llattn::DT_THREADS, llattn::DenseTile<64>::SMEM);
     }
     CU(cudaGetLastError());
     return LLATTN_OK;

@@ -232,13 +232,33 @@ def test_dense_status_argument_errors(api):
     assert api.lib().llattn_dense_error_word(None) == api.EINVAL
 
 
-# Where the tcgen05 form takes over: 32, 64 and 128 tokens a CTA, with a ragged last tile, one and several waves, an odd number of
-# groups (a stage of one), and more groups than factors held at a time (16)
+# Where the tcgen05 form takes over: 32, 64 and 128 tokens a CTA, each with a ragged last tile of few tokens and of all but one,
+# one and several waves, the fewest groups it takes, an odd number of groups (a stage of one), and more groups than factors held at a time (16)
+TCGEN05_CASES = [
+    (149, 2048, 2048, 32), (160, 2048, 2176, 32), (289, 2048, 2048, 64), (321, 2048, 2176, 64), (577, 2048, 2048, 128), (641, 2048, 1152, 128),
+    (1153, 2048, 2048, 128), (1217, 2048, 4096, 64), (2049, 1024, 4224, 128), (65, 8192, 2048, 64), (200, 8192, 4224, 128), (127, 4096, 2048, 32), (255, 4096, 2176, 64),
+    (577, 2048, 768, 128), (511, 2048, 1280, 64), (1151, 2048, 768, 128)]
+
+
+@pytest.mark.parametrize("ntokens,rows,K,tok", TCGEN05_CASES)
+def test_dense_tcgen05_cases_take_that_form(api, ntokens, rows, K, tok):
+    assert api.dense_preview(rows, K, ntokens, 148) == (api.DENSE_TCGEN05, tok)
+
+
+def test_dense_preview(api):
+    assert api.dense_preview(2048, 2048, 32, 148)[0] == api.DENSE_STRIPS
+    assert api.dense_preview(2048, 128, 2560, 148) == (api.DENSE_TILES, 64)
+    assert {t for *_, t in TCGEN05_CASES} == {32, 64, 128}
+    for bad in ((100, 128, 1, 148), (128, 128, 0, 148), (128, 128, 1, 0)):
+        with pytest.raises(api.LlattnError):
+            api.dense_preview(*bad)
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("ntokens,rows,K", [
-    (149, 2048, 2048), (160, 2048, 2176), (289, 2048, 2048), (321, 2048, 2176), (577, 2048, 2048), (641, 2048, 1152), (1153, 2048, 2048),
-    (2049, 1024, 4224), (65, 8192, 2048), (200, 8192, 4224)])
-def test_dense_tcgen05_form(api, orc, pkg, ntokens, rows, K):
+@pytest.mark.parametrize("ntokens,rows,K,tok", TCGEN05_CASES)
+def test_dense_tcgen05_form(api, orc, pkg, ntokens, rows, K, tok):
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert api.dense_preview(rows, K, ntokens, 148) == (api.DENSE_TCGEN05, tok)
     wl = pkg.workload
     strips, _, _, _ = wl.dense_weights(rows, K, 41)
     strips = strips.copy()
@@ -250,7 +270,11 @@ def test_dense_tcgen05_form(api, orc, pkg, ntokens, rows, K):
     Y0 = np.random.default_rng(43).normal(size=(ntokens, rows)).astype(np.float32)
     want = Y0.copy()
     orc.dense_w4a8(strips, q, s, qsum, want)
-    Y, err = _dev(Y0), torch.zeros(1, dtype=torch.int32, device="cuda")
-    api.dense_w4a8(_dev(strips), _dev(q), _dev(s), _dev(qsum), Y, err_word=err)
+    pad = torch.full((ntokens + 2 * tok, rows), 7.0, device="cuda")                  # a CTA's tokens before and after Y must not change
+    pad[tok:-tok] = _dev(Y0)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    api.dense_w4a8(_dev(strips), _dev(q), _dev(s), _dev(qsum), pad[tok:-tok], err_word=err)
     assert int(err.item()) == 0
-    assert np.array_equal(Y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    got = pad.cpu().numpy()
+    assert (got[:tok] == 7).all() and (got[-tok:] == 7).all()
+    assert np.array_equal(got[tok:-tok].view(np.uint32), want.view(np.uint32))
