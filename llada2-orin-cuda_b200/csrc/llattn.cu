@@ -244,8 +244,12 @@ bool dense_strips_win(int rows, int K, int ntokens, int sms) {
 // Tokens per CTA of the tcgen05 form, or 0 where the mma.sync tiles are the faster ones. A CTA of the former fills an SM and has a
 // long start (tensor memory, four roles, sixteen groups' factors), so it wins with the groups and with the tokens; the line follows
 // both sides' measured costs in microseconds, in a graph over 1024 .. 8192 rows, K = 128 .. 8192 and 80 .. 2560 tokens. 2048 rows,
-// tiles / tcgen05 with 32, 64 and 128 tokens: K = 2048, 80 tokens 8.4 / 10.4, 12.2, 17.1, 160 11.0 / 10.5, 12.2, 17.8, 320 16.7 / 19.1,
-// 12.3, 17.6, 640 26.5 / 28.3, 23.0, 17.9, 2560 62 / 82, 56, 51; K = 512, 320 tokens 6.7 / 10.4, 7.1, 9.6, 2560 22.7 / 43, 30, 26.5.
+// tiles / tcgen05 with 32, 64 and 128 tokens a CTA:
+//   K = 2048    80 tokens  8.4 / 10.4, 12.2, 17.1    160  11.0 / 10.5, 12.2, 17.8    320  16.7 / 19.1, 12.3, 17.6
+//              640 tokens 26.5 / 28.3, 23.0, 17.9   2560  62 / 82, 56, 51
+//   K = 512    320 tokens  6.7 / 10.4, 7.1, 9.6     2560  22.7 / 43, 30, 26.5
+// Checked over 128 .. 32,768 rows, 33 .. 4096 tokens (1,400 sizes): a call that takes the tcgen05 form is at most 3.6 % slower than
+// its tiles, at six groups, and takes up to 41 % less time (both without the votes at its waits, 1 to 1.5 %).
 int dense_wide_tokens(int rows, int K, int ntokens, int sms) {
     if (ntokens <= 32) return 0;
     const double groups = K / llattn::DN_GROUP, row_tiles = rows / llattn::DN_ROWS;
@@ -254,9 +258,10 @@ int dense_wide_tokens(int rows, int K, int ntokens, int sms) {
     if (ctas(16) <= sms) best = 2.1 + 0.38 * groups;
     else if (ctas(32) <= sms) best = 2.3 + 0.54 * groups;
     else if (ctas(64) <= sms) best = 2.6 + 0.88 * groups;
-    else {                                     // two CTAs an SM; a partly filled last wave counts half
-        const double waves = ctas(64) / (2 * sms);
-        best = std::max(1.0, (waves + std::ceil(waves)) / 2) * (2.9 + 1.42 * groups);
+    else {                                     // two CTAs an SM. A partly filled last wave counts half; behind six others, which have
+                                               // drifted apart by then, a fifth (K = 768, 16,384 rows, 1184 tokens: 87.8 as tiles, 94.5 here)
+        const double waves = ctas(64) / (2 * sms), idle = std::ceil(waves) - waves;
+        best = std::max(1.0, waves + idle * (waves > 6 ? 0.2 : 0.5)) * (2.9 + 1.42 * groups);
     }
     int wide = 0;
     auto consider = [&](int tok, double start, double group) {
