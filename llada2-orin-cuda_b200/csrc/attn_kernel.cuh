@@ -65,9 +65,6 @@ constexpr int LLATTN_TRACE_EVENTS = 2048;
 #else
 #define LLATTN_TR(ev, tile) do {} while (0)
 #endif
-#ifndef LLATTN_SKIP
-#define LLATTN_SKIP 0      // tuning builds only: bit 0 = no dequantisation, bit 1 = no exponentials (results are garbage)
-#endif
 
 constexpr int TILE_UNITS = 4;
 constexpr int KBLOCK = 128 * 128;                  // 16384: 128 keys x 64 channels of fp16, one swizzled block
@@ -103,9 +100,6 @@ constexpr int ATTN_SMEM_BYTES = SM_QSUM + QR * 4;
 #endif
 #ifndef LLATTN_SINGLE_ISSUER
 #define LLATTN_SINGLE_ISSUER 0     // 1: one warp issues PV(t) and then S(t+2); the tensor pipe runs one thread's MMAs in order
-#endif
-#ifndef LLATTN_WARP_ARRIVE
-#define LLATTN_WARP_ARRIVE 0       // 1: one arrival per softmax warp on the P barrier instead of one per thread
 #endif
 __host__ __device__ constexpr int softmax_warps(bool rows16) { return rows16 ? 8 : 4; }
 constexpr int DEQUANT_WARPS = LLATTN_DEQUANT_WARPS, GROUP_WARPS = LLATTN_GROUP_WARPS, DEQUANT_GROUPS = DEQUANT_WARPS / GROUP_WARPS;
@@ -262,29 +256,6 @@ __device__ __forceinline__ float rowmax16(const uint32_t (&r)[16]) {
     }
     return max3(max3(a, b, __uint_as_float(r[7])), __uint_as_float(r[15]), __uint_as_float(r[15]));
 }
-#ifndef LLATTN_POLY_MOD
-#define LLATTN_POLY_MOD 0      // n > 0: every n-th score pair takes its 2^x from the multiply-add pipes instead of the MUFU
-#endif
-// 2^x for two values on the multiply-add pipes: x is held above -125, split into round(x) and a fraction in [-0.5, 0.5]
-// by the add-a-large-constant trick, 2^fraction comes from a degree-4 polynomial (relative error 2e-6, far below the
-// fp16 rounding that follows) and round(x) is added into the exponent field.
-__device__ __forceinline__ void exp2_pair_poly(float x0, float x1, float& e0, float& e1) {
-    x0 = fmaxf(x0, -125.f); x1 = fmaxf(x1, -125.f);
-    unsigned long long x, t, n, f, q;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(x0), "f"(x1));
-    asm("{\n\t.reg .b64 m;\n\tmov.b64 m, 0x4b4000004b400000;\n\tadd.rn.f32x2 %0, %1, m;\n\t}" : "=l"(t) : "l"(x));        // 1.5 * 2^23 + round(x)
-    asm("{\n\t.reg .b64 m;\n\tmov.b64 m, 0xcb400000cb400000;\n\tadd.rn.f32x2 %0, %1, m;\n\t}" : "=l"(n) : "l"(t));        // round(x)
-    asm("{\n\t.reg .b64 m;\n\tmov.b64 m, 0xbf800000bf800000;\n\tfma.rn.f32x2 %0, %1, m, %2;\n\t}" : "=l"(f) : "l"(n), "l"(x));   // x - round(x)
-    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, 0x3c1803f73c1803f7;\n\tmov.b64 b, 0x3d64d2b93d64d2b9;\n\tfma.rn.f32x2 %0, %1, a, b;\n\t}" : "=l"(q) : "l"(f));   // 0.009278289 f + 0.055865023
-    asm("{\n\t.reg .b64 c;\n\tmov.b64 c, 0x3e76138d3e76138d;\n\tfma.rn.f32x2 %0, %0, %1, c;\n\t}" : "+l"(q) : "l"(f));                              // 0.24030896
-    asm("{\n\t.reg .b64 c;\n\tmov.b64 c, 0x3f3170f03f3170f0;\n\tfma.rn.f32x2 %0, %0, %1, c;\n\t}" : "+l"(q) : "l"(f));                              // 0.69312954
-    asm("{\n\t.reg .b64 c;\n\tmov.b64 c, 0x3f7fffdc3f7fffdc;\n\tfma.rn.f32x2 %0, %0, %1, c;\n\t}" : "+l"(q) : "l"(f));                              // 0.99999785
-    uint32_t q0, q1, t0, t1;
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(q0), "=r"(q1) : "l"(q));
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(t0), "=r"(t1) : "l"(t));
-    e0 = __uint_as_float(q0 + (t0 << 23));
-    e1 = __uint_as_float(q1 + (t1 << 23));
-}
 
 // Score pairs J0 .. J1-1 of 16 scores -> packed fp16 p. PRECISE: also the fp16 remainder p - fp16(p) (exact in fp32, then
 // rounded once more: together the pair carries p to about 22 bits).
@@ -292,12 +263,9 @@ template <int J0, int J1, bool PRECISE>
 __device__ __forceinline__ void exp_pairs16(const uint32_t (&r)[16], uint32_t* pk, uint32_t* pkl, unsigned long long sl2x2, unsigned long long nm2) {
 #pragma unroll
     for (int j = J0; j < J1; ++j) {
-        if (LLATTN_SKIP & 2) { pk[j] = r[2 * j] & 0x03ff03ffu; continue; }
         float x0, x1;
         fma2(r[2 * j], r[2 * j + 1], sl2x2, nm2, x0, x1);
-        float e0, e1;
-        if (LLATTN_POLY_MOD > 0 && j % (LLATTN_POLY_MOD > 0 ? LLATTN_POLY_MOD : 1) == LLATTN_POLY_MOD - 1) exp2_pair_poly(x0, x1, e0, e1);
-        else { e0 = ex2(x0); e1 = ex2(x1); }
+        const float e0 = ex2(x0), e1 = ex2(x1);
         const half2 h = __floats2half2_rn(e0, e1);
         pk[j] = *reinterpret_cast<const uint32_t*>(&h);
         if (PRECISE) {
@@ -664,7 +632,6 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM_MISC + 4);
     constexpr int SOFTMAX_WARPS = softmax_warps(ROWS16), WARP_SERVICE = SOFTMAX_WARPS + DEQUANT_WARPS, WARP_MMA_PV = WARP_SERVICE;
     constexpr int WARP_MMA = WARP_MMA_PV + 1, WARP_PRODUCER = WARP_MMA + 1, ATTN_THREADS = attn_threads(ROWS16);
-    constexpr int P_ARRIVALS = LLATTN_WARP_ARRIVE ? SOFTMAX_WARPS : 32 * SOFTMAX_WARPS;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar0 = ptx::smem_u32(bars);
     auto BAR = [&](int i) -> uint32_t { return bar0 + 8u * uint32_t(i); };
@@ -683,7 +650,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
         for (int i = 0; i < 2; ++i) {
             ptx::mbar_init(BAR(B_K_FULL + i), 32 * DEQUANT_WARPS); ptx::mbar_init(BAR(B_V_FULL + i), 32 * DEQUANT_WARPS);
             ptx::mbar_init(BAR(B_K_FREE + i), 1); ptx::mbar_init(BAR(B_PV_DONE + i), 1);
-            ptx::mbar_init(BAR(B_S_FULL + i), 1); ptx::mbar_init(BAR(B_P_FULL + i), P_ARRIVALS);
+            ptx::mbar_init(BAR(B_S_FULL + i), 1); ptx::mbar_init(BAR(B_P_FULL + i), 32 * SOFTMAX_WARPS);
         }
         ptx::mbar_init(BAR(B_Q_FULL), 32 * SOFTMAX_WARPS); ptx::mbar_init(BAR(B_O_FREE), 32 * SOFTMAX_WARPS);
         ptx::mbar_init(BAR(B_QSUM), 128);
@@ -798,12 +765,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                 if (!alive) break;
                 ptx::tmem_wait_st();
                 ptx::tc_fence_before();
-#if LLATTN_WARP_ARRIVE
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(BAR(B_P_FULL + b));
-#else
                 ptx::mbar_arrive(BAR(B_P_FULL + b));
-#endif
                 LLATTN_TR(4, t);
             }
             if (!alive) break;
@@ -1010,12 +972,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                 if (!alive) break;
                 ptx::tmem_wait_st();
                 ptx::tc_fence_before();
-#if LLATTN_WARP_ARRIVE
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(BAR(B_P_FULL + b));
-#else
                 ptx::mbar_arrive(BAR(B_P_FULL + b));
-#endif
                 LLATTN_TR(4, t);
             }
             if (!alive) break;
@@ -1156,8 +1113,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                 for (int u = 0; u < TILE_UNITS / DEQUANT_GROUPS; ++u) {
                     const uint32_t rr = r + grp + u * DEQUANT_GROUPS, slot = rr % NRAW;
                     if (!ptx::mbar_wait(BAR(B_RAW_FULL + slot), (rr / NRAW) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_DEQUANT; break; }
-                    if (!(LLATTN_SKIP & 1))
-                        dequant_k(smem + SM_RAW + slot * RAW_STRIDE, smem + SM_K + b * TILE_BYTES + (grp + u * DEQUANT_GROUPS) * UNIT_BYTES, dq);
+                    dequant_k(smem + SM_RAW + slot * RAW_STRIDE, smem + SM_K + b * TILE_BYTES + (grp + u * DEQUANT_GROUPS) * UNIT_BYTES, dq);
                 }
                 if (!alive) break;
                 LLATTN_TR(16, t);
@@ -1169,8 +1125,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
 #pragma unroll
                 for (int u = 0; u < TILE_UNITS / DEQUANT_GROUPS; ++u) {
                     const uint32_t rr = r + grp + u * DEQUANT_GROUPS, slot = rr % NRAW;
-                    if (!(LLATTN_SKIP & 1))
-                        dequant_v(smem + SM_RAW + slot * RAW_STRIDE, smem + SM_V + b * VTILE_BYTES + (grp + u * DEQUANT_GROUPS) * UNIT_BYTES, dq);
+                    dequant_v(smem + SM_RAW + slot * RAW_STRIDE, smem + SM_V + b * VTILE_BYTES + (grp + u * DEQUANT_GROUPS) * UNIT_BYTES, dq);
                     ptx::mbar_arrive(BAR(B_RAW_EMPTY + slot));
                 }
                 ptx::fence_proxy_async_smem();
@@ -1196,7 +1151,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                         LLATTN_TR(15, t);
                         if (!ptx::mbar_wait(BAR(B_RAW_FULL + slot), (rr / NRAW) & 1, abort_flag)) { alive = false; errbits |= ERR_WAIT_DEQUANT; break; }
                         LLATTN_TR(16, t);
-                        if (!(LLATTN_SKIP & 1)) dequant_k(smem + SM_RAW + slot * RAW_STRIDE, Kt + u * UNIT_BYTES, dq);
+                        dequant_k(smem + SM_RAW + slot * RAW_STRIDE, Kt + u * UNIT_BYTES, dq);
                     } else {          // the query block's own K, exact fp16
                         copy_fresh(p.Kf + f0, Kt + u * UNIT_BYTES, dt);
                     }
@@ -1213,7 +1168,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                     const int unit = TILE_UNITS * i + u;
                     if (unit < w.rec_count) {
                         const uint32_t slot = (r + u) % NRAW;       // landed: the K pass waited for it
-                        if (!(LLATTN_SKIP & 1)) dequant_v(smem + SM_RAW + slot * RAW_STRIDE, Vt + u * UNIT_BYTES, dq);
+                        dequant_v(smem + SM_RAW + slot * RAW_STRIDE, Vt + u * UNIT_BYTES, dq);
                         ptx::mbar_arrive(BAR(B_RAW_EMPTY + slot));
                     } else {
                         copy_fresh(p.Vf + f0, Vt + u * UNIT_BYTES, dt);
