@@ -182,7 +182,7 @@ typedef struct llattn_io {
  * (engine/attn.cu:261-263); a query row that one key partly dominates then carries that key's fp16 rounding (2^-12
  * relative), which at long contexts exceeds 2e-3 of the output RMS on a few elements. LLATTN_IO_PRECISE_P carries every
  * probability as an fp16 value plus an fp16 remainder (two P.V chains per tile): max-abs error against the fp64 oracle
- * stays within 2e-3 of the output RMS at 32 K tokens, at about two thirds of the throughput. No counterpart in the
+ * stays within 2e-3 of the output RMS at 32 K tokens, at about four fifths of the throughput. No counterpart in the
  * reference. */
 #define LLATTN_IO_PRECISE_P 1u
 

@@ -12,8 +12,8 @@
 //                   O += P V   (A = P read from TMEM as packed fp16, B = V MN-major in shared memory, fp32 O in TMEM);
 //                   V carries one extra column of ones, so the same MMA also accumulates the softmax row sum from
 //                   exactly the fp16 P the numerator uses (numerator and denominator then share their rounding)
-//   softmax warps : four warps, one thread per query row (TMEM lane), all keys of the row: no exchange between warps (the
-//                   precise form: eight warps, four threads per row, see softmax_tile_rows16).
+//   softmax warps : four warps, one thread per query row (TMEM lane), all keys of the row: no exchange between warps
+//                   (precise calls with long runs: eight warps, four threads per row, see softmax_tile_rows16).
 //                   One pass per tile: p = 2^(s*scale*log2e - mref) for 16 scores at a time while the next 16 arrive
 //                   from tensor memory, the chunk maximum taken on the way; P goes back over S in TMEM as fp16 pairs
 //                   (the 32 keys of chunk g at columns 32 g .. 32 g + 15, the first half of the S columns they were
@@ -24,7 +24,7 @@
 // reference maximum (log2 units) and row sum go to a partial slot in the format of the reference's Opart/Mpart/Lpart
 // (engine/attn.cu:291-305) and it counts itself in at the tile's arrival counter. When a CTA has no runs left it returns
 // to its split tiles: it waits (bounded) until every run of the tile is counted, then folds its share of the tile's
-// rows (run k of n takes rows k, k + n, ...; all sixteen warps, one or several per row; merge_kernel.cuh) and writes their
+// rows (run k of n takes rows k, k + n, ...; all warps of the CTA, one or several per row; merge_kernel.cuh) and writes their
 // outputs, so a tile cut into n runs is folded by n SMs at once. A CTA only ever waits after all of its own runs are
 // out, so the waits cannot form a cycle; they need every CTA of the launch to be on an SM, which a grid of at most one
 // CTA per SM launched cooperatively guarantees. With the reference-shaped operator pair the caller's attn_combine
@@ -86,12 +86,13 @@ constexpr int SM_FIRST = SM_MISC + 16;             // the CTA's first run descri
 // A softmax warp's way between its row-per-thread tensor memory and row-major global memory: 32 rows x 128 bytes, the 16-byte
 // chunk c of row r at chunk position c ^ (r % 8). Without it a warp's 16-byte accesses touch 32 lines each.
 constexpr int SM_STAGE = (SM_FIRST + int(sizeof(RunDesc)) + 127) / 128 * 128, STAGE_BYTES = 32 * 128;
-constexpr int SM_ROWREF = SM_STAGE + 4 * STAGE_BYTES;    // precise form: the run's final reference exponents, one per query row,
+constexpr int SM_ROWREF = SM_STAGE + 4 * STAGE_BYTES;    // eight softmax warps: the run's final reference exponents, one per query row,
 constexpr int SM_QSUM = SM_ROWREF + QR * 4;              // and for the int8 output the code sums of dims 64 .. 127
 constexpr int ATTN_SMEM_BYTES = SM_QSUM + QR * 4;
 // warps 0-3 softmax (warp w: TMEM lanes 32 w .. 32 w + 31, one query row per thread), 4-11 dequant (four groups of two
 // warps, group g takes unit g of every tile: a thread's scale / minimum words then serve eight passes over the record),
-// then the service warps. Every scheduler carries one softmax warp, two dequantising warps and one service warp.
+// then the service warps. Every scheduler carries one softmax warp, two dequantising warps and one service warp. With eight
+// softmax warps (two per quarter of the lanes, sixteen rows each): 0-7, then 8-15 and 16-19, and two softmax warps a scheduler.
 #ifndef LLATTN_DEQUANT_WARPS
 #define LLATTN_DEQUANT_WARPS 8
 #endif
@@ -108,7 +109,7 @@ constexpr int GROUP_THREADS = 32 * GROUP_WARPS, DQ_PASSES = 16 / GROUP_WARPS;   
 // issue and two copy producers that take alternate records, so that no scheduler carries much more than the others.
 constexpr int PRODUCERS = 2;
 __host__ __device__ constexpr int attn_threads(bool rows16) { return 32 * (softmax_warps(rows16) + DEQUANT_WARPS + 2 + PRODUCERS); }
-constexpr int ATTN_THREADS = attn_threads(false);  // 512; 640 in the precise form
+constexpr int ATTN_THREADS = attn_threads(false);  // 512; 640 with eight softmax warps
 constexpr int TMEM_COLS = 512;
 constexpr int TM_S = 0, TM_O = 256, TM_L = TM_O + 128, TM_Q = 400;   // S at columns 0 and 128, O at 256..383, row sum at 384, Q at 400..463
 // The reference exponent of a row moves when a score exceeds it by more than this many powers of two, the reference's own
@@ -139,8 +140,8 @@ struct KParams {
     int* err;
     // list mode with folding in the kernel
     bool fused;
-    int* tile_counters;            // [tiles][4]: [0] softmax warps whose rows of a run are out (4 per run), [1] warps that
-                                   // have folded their share (16 per run); both back at 0 when the launch ends
+    int* tile_counters;            // [tiles][4]: [0] softmax warps whose part of a run is out (4 or 8 per run), [1] warps that
+                                   // have folded their share (16 or 20 per run); both back at 0 when the launch ends
     MergeOut out;
     size_t cache_offset;           // bytes added to every sequence's cache pointer: the layer this launch reads
     // reference-grid mode (items == nullptr): CTA i is (kvh = i % 4, chunk = (i / 4) % ref_nchunks, jb = i / (4 * ref_nchunks))
@@ -370,11 +371,13 @@ __device__ __forceinline__ bool softmax_tile(float& mref, float sl2, unsigned lo
     return true;
 }
 
-// ---- The precise form's softmax: eight warps, two per lane quarter, sixteen rows each. It has half as much again to do per score (the
-// remainders: two conversions, two subtractions and a pack per pair), and with one warp on a scheduler that chain was the bound: 64
-// ragged sequences of up to 8 K tokens 169.5 us with four warps, 141 with eight, 9 x 201 blocks 41.1 and 38.2. The default form gains 1 % at
-// large batches from the same split and loses 4 % at a step of one sequence, whose run ends it lengthens (96 registers a thread instead
-// of 128; 20 layers 466 and 486 us), and keeps four. Votes are taken on P, two chunks at a time: a vote per chunk cost 3 %.
+// ---- The precise softmax for long runs: eight warps, two per lane quarter, sixteen rows each. It has half as much again to do per score
+// (the remainders: two conversions, two subtractions and a pack per pair), and with one warp on a scheduler that chain was the bound:
+// 64 ragged sequences of up to 8 K tokens 169.5 us with four warps, 141 with eight, 9 x 201 blocks 41.1 and 38.2. The ends of a run take
+// longer (precise_rows16, at the launch, has the line and both sides): half lines out of the staging rows, and 96 registers a thread
+// instead of 128, at which the compiler spills (216 bytes of stores, 172 of loads). The default form
+// gains 1 % at large batches from the same split, loses 4 % at a step of one sequence (20 layers 466 and 486 us) and keeps four.
+// Votes are taken on P, two chunks at a time: a vote per chunk cost 3 %.
 // The 16 scores that a thread holds of a 32-key chunk (16x256b fragment: two rows, eight keys each) -> packed fp16 p in the 16x128b
 // fragment. nmA, nmB: minus the rows' reference exponents. Also the fp16 remainder p - fp16(p) (exact in fp32, then
 // rounded once more: together the pair carries p to about 22 bits).
@@ -623,7 +626,8 @@ __device__ __forceinline__ void write_ones_column(uint8_t* smem, int lane) {
 // The whole CTA's work. `cta` is the CTA's index in the plan (list mode) or in the flattened reference grid
 // (kv head fastest, then chunk, then query block).
 // PRECISE: P is carried as fp16 value + fp16 remainder (two PV chains per tile), for callers that need the result to
-// within 2e-3 of the output RMS at long contexts and accept about half the throughput.
+// within 2e-3 of the output RMS at long contexts and accept four fifths of the throughput (64 sequences of 32 K tokens).
+// ROWS16: eight softmax warps of sixteen rows instead of four with a row per thread.
 template <bool PRECISE, bool ROWS16 = false>
 __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -631,7 +635,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM_MISC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM_MISC + 4);
     constexpr int SOFTMAX_WARPS = softmax_warps(ROWS16), WARP_SERVICE = SOFTMAX_WARPS + DEQUANT_WARPS, WARP_MMA_PV = WARP_SERVICE;
-    constexpr int WARP_MMA = WARP_MMA_PV + 1, WARP_PRODUCER = WARP_MMA + 1, ATTN_THREADS = attn_threads(ROWS16);
+    constexpr int WARP_MMA = WARP_MMA_PV + 1, WARP_PRODUCER = WARP_MMA + 1, WARPS = attn_threads(ROWS16) / 32;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar0 = ptx::smem_u32(bars);
     auto BAR = [&](int i) -> uint32_t { return bar0 + 8u * uint32_t(i); };
@@ -1383,7 +1387,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
 
     // ---- split tiles. Every run of this CTA is stored and counted by now, so nothing this CTA waits for depends on
     // this CTA: for each of its runs that is part of a split tile, wait (bounded) until all of the tile's runs are
-    // counted in, then all sixteen warps finish this run's share of the rows. The last warp to leave a
+    // counted in, then all warps of the CTA finish this run's share of the rows. The last warp to leave a
     // tile puts both of its counters back to zero for the next launch. Every thread of the CTA walks this loop the same
     // way (same runs, same outcome), so the CTA barrier inside it is reached by all.
     if (p.fused) {
@@ -1408,8 +1412,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                 *abort_flag = 1;
                 break;
             }
-            constexpr int NW = ATTN_THREADS / 32;
-            const int r0 = (w.slot - md.slot_begin) + md.nslots * warp, step = md.nslots * NW;
+            const int r0 = (w.slot - md.slot_begin) + md.nslots * warp, step = md.nslots * WARPS;
             if (md.nslots > FOLD_PART && md.nslots <= FOLD_SHARED_SLOTS) {
                 fold_rows_shared(p.Opart, p.Mpart, p.Lpart, md, w.slot - md.slot_begin, warp, lane, smem + SM_K, p.out);      // the tiles are done with
             } else if (md.nslots == 2) {
@@ -1431,7 +1434,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                 for (int r = r0; r < QR; r += step) fold_row_warp(p.Opart, p.Mpart, p.Lpart, md, r, lane, p.out);
             }
             __syncwarp();
-            if (lane == 0 && atomicAdd(counters + 1, 1) == (ATTN_THREADS / 32) * md.nslots - 1) { counters[0] = 0; counters[1] = 0; }
+            if (lane == 0 && atomicAdd(counters + 1, 1) == WARPS * md.nslots - 1) { counters[0] = 0; counters[1] = 0; }
         }
     }
 

@@ -292,16 +292,18 @@ __global__ void __launch_bounds__(DT_THREADS, TOK == 64 ? 2 : 3) dense_tile_kern
 }
 
 // ------------------------------------------------------------------------------------------------------- very many tokens
-// CTA = 128 rows x N tokens, one per SM, the products on tcgen05 kind::i8 (u8 x s8, M = 128), four times as fast as mma.sync
-// here, so that the fold is what is left: sixteen warps, six instructions per two outputs and group. The other roles run ahead of them through rings whose slots hold TWO groups: a warp by itself issues an instruction
-// every five cycles or so, and with a slot per group the barriers' instructions alone took a role 1,500 cycles a group.
+// CTA = 128 rows x N tokens, one per SM, the products on tcgen05 kind::i8 (u8 x s8, M = 128; 74 cycles for 128 x 128 x 32 of them,
+// where mma.sync takes 8.8 for 16 x 8 x 32 on each of four schedulers, both measured: 3.8 times the rate), so that the fold is what is
+// left: sixteen warps, six instructions per two outputs and group. The other roles run ahead of them through rings whose slots hold
+// TWO groups: a warp by itself issues an instruction every five cycles or so, and with a slot per group the barriers' instructions
+// alone took a role 1,500 cycles a group.
 //   producer warp  bulk copies of the strips' codes into a ring, 2 KB a copy
 //   unpack warps   codes -> u8 rows in the 128-byte-swizzle operand layout
 //   load warps     activations, cp.async straight into the operand layout (completion by mbarrier, no waiting)
 //   MMA warp       four K-steps a group into one of four accumulators
 // The factors of the fold (token scales and sums, row scales and zero points) of sixteen groups lie in shared memory as floats.
-// Measured, 2048 x 2048, launches in a graph, mma.sync tiles / this: 320 tokens 16.7 / 12.3 us, 640 26.5 / 17.9, 1024 26.0 / 17.6, 2048
-// 49.2 / 34.3. 1024 tokens are one CTA on 128 SMs: 0.66 us a group, half of the issue slots (16 folding warps x 110 instructions and the
+// Measured, 2048 x 2048, launches in a graph, mma.sync tiles / this: 320 tokens 16.7 / 12.5 us, 640 26.5 / 18.2, 1024 26.0 / 18.2, 2048
+// 49.2 / 35.0. 1024 tokens are one CTA on 128 SMs: 0.66 us a group, half of the issue slots (16 folding warps x 110 instructions and the
 // unpacking), and 7 us before the first and behind the last.
 constexpr int DW_FOLD_WARPS = 16, DW_UNPACK_WARPS = 4, DW_LOAD_WARPS = 1;
 constexpr int DW_WARP_UNPACK = DW_FOLD_WARPS, DW_WARP_LOAD = DW_WARP_UNPACK + DW_UNPACK_WARPS, DW_WARP_PRODUCER = DW_WARP_LOAD + DW_LOAD_WARPS,

@@ -518,7 +518,7 @@ extern "C" int llattn_wait_selftest(unsigned long long limit_ns, int* err_word, 
 }
 
 #ifdef LLATTN_TRACE
-// Tuning builds only: points the kernel's timeline hooks at a device buffer of 18 * 2048 64-bit words.
+// Tuning builds only: points the kernel's timeline hooks at a device buffer of 20 * 2048 64-bit words (2048 events for each of up to 20 warps).
 extern "C" int llattn_debug_set_trace(void* dev_ptr) {
     CU(cudaMemcpyToSymbol(llattn::g_trace_buf, &dev_ptr, sizeof(dev_ptr)));
     return LLATTN_OK;

@@ -208,7 +208,7 @@ __device__ __forceinline__ void fold_row_warp(const float* Opart, const float* M
     emit_row_warp(M, den, acc, md, r, lane, o);
 }
 
-// This CTA's rows k, k + n, ... of a tile cut into n runs, FOLD_PART < n <= FOLD_SHARED_SLOTS, by 16 warps (20 in the precise form): W warps share a
+// This CTA's rows k, k + n, ... of a tile cut into n runs, FOLD_PART < n <= FOLD_SHARED_SLOTS, by 16 or 20 warps: W warps share a
 // row, each folds n / W of its slots, the row's first warp adds their results up in slot order. With a warp per row, most of
 // the warps had none and the others went through their slots in several round trips: 22 runs a tile, 7,000 cycles from the last
 // count-in to the outputs. Two warps a row up to 32 slots (at most 8 rows), four above (at most 4 rows); the planner
