@@ -292,22 +292,27 @@ __global__ void __launch_bounds__(DT_THREADS, TOK == 64 ? 2 : 3) dense_tile_kern
 }
 
 // ------------------------------------------------------------------------------------------------------- very many tokens
-// CTA = 128 rows x N tokens, one per SM, the products on tcgen05 kind::i8 (u8 x s8, M = 128; 74 cycles for 128 x 128 x 32 of them,
-// where mma.sync takes 8.8 for 16 x 8 x 32 on each of four schedulers, both measured: 3.8 times the rate), so that the fold is what is
-// left: sixteen warps, six instructions per two outputs and group. The other roles run ahead of them through rings whose slots hold
-// TWO groups: a warp by itself issues an instruction every five cycles or so, and with a slot per group the barriers' instructions
-// alone took a role 1,500 cycles a group.
+// Tiles of 128 rows x N tokens, one CTA per SM that walks its share of them, the products on tcgen05 kind::i8 (u8 x s8, M = 128; 74 cycles for
+// 128 x 128 x 32 of them, where mma.sync takes 8.8 for 16 x 8 x 32 on each of four schedulers, both measured: 3.8 times the rate), so that
+// the fold is what is left: sixteen warps, six instructions per two outputs and group. The other roles run ahead of them, into the next
+// tile too, through rings whose slots hold TWO groups: a warp by itself issues an instruction every five cycles or so, and with a slot per
+// group the barriers' instructions alone took a role 1,500 cycles a group.
 //   producer warp  bulk copies of the strips' codes into a ring, 2 KB a copy
 //   unpack warps   codes -> u8 rows in the 128-byte-swizzle operand layout
 //   load warps     activations, cp.async straight into the operand layout (completion by mbarrier, no waiting)
 //   MMA warp       four K-steps a group into one of four accumulators
 // The factors of the fold (token scales and sums, row scales and zero points) of sixteen groups lie in shared memory as floats.
-// Measured, 2048 x 2048, launches in a graph, mma.sync tiles / this: 320 tokens 16.7 / 12.5 us, 640 26.5 / 18.2, 1024 26.0 / 18.2, 2048
-// 49.2 / 35.0. 1024 tokens are one CTA on 128 SMs: 0.66 us a group, half of the issue slots (16 folding warps x 110 instructions and the
-// unpacking), and 7 us before the first and behind the last.
-constexpr int DW_FOLD_WARPS = 16, DW_UNPACK_WARPS = 4, DW_LOAD_WARPS = 1;
+// Measured, 2048 x 2048, launches in a graph, mma.sync tiles / a CTA per tile, two rounds of accumulators a group / this: 320 tokens 16.7 /
+// 11.8 / 11.7 us, 640 26.5 / 17.4 / 16.5, 1024 26.0 / 17.7 / 16.8, 2048 49.7 / 34.3 / 30.6, 4096 - / 67.7 / 58.5. A tile of 128 tokens takes 0.68 us a
+// group, 56 % of the issue slots and 42 % of the fp32 pipe over the kernel; its start and end are 6 us for a CTA's first and 3 for the others.
+constexpr int DW_FOLD_WARPS = 16, DW_UNPACK_WARPS = 4, DW_LOAD_WARPS = 2;
 constexpr int DW_WARP_UNPACK = DW_FOLD_WARPS, DW_WARP_LOAD = DW_WARP_UNPACK + DW_UNPACK_WARPS, DW_WARP_PRODUCER = DW_WARP_LOAD + DW_LOAD_WARPS,
               DW_WARP_MMA = DW_WARP_PRODUCER + 1, DW_THREADS = 32 * (DW_WARP_MMA + 1);
+// Registers a thread: at launch, and after the roles have parted. The second split has to come out of the first, or its waits for registers
+// would not end; that the compiler gave each kernel the first number is checked before the first launch.
+constexpr int DW_LAUNCH_REGS = 80, DW_FOLD_REGS = 96, DW_OTHER_REGS = 48;
+static_assert(DW_FOLD_WARPS * DW_FOLD_REGS + (DW_THREADS / 32 - DW_FOLD_WARPS) * DW_OTHER_REGS <= DW_THREADS / 32 * DW_LAUNCH_REGS && DW_THREADS % 128 == 0 &&
+              DW_FOLD_WARPS % 4 == 0, "register split");
 constexpr int DW_RAW = 2, DW_A = 2, DW_B = 2, DW_ACC = 4, DW_SC = 16;      // ring slots; groups of factors held
 template <int N> struct DenseWide {
     static constexpr int A_GROUP = DN_ROWS * DN_GROUP, B_GROUP = N * DN_GROUP, RAW_GROUP = 8 * DN_TILE_BYTES;
@@ -347,7 +352,7 @@ __device__ __forceinline__ void mma_i8_group_warp(uint32_t d, uint32_t a_lo, uin
 // An arrival on `bar` once this thread's cp.async so far have landed.
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory"); }
 
-template <int N>
+template <int N, bool ONE>
 __global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DenseParams p) {
     using T = DenseWide<N>;
     extern __shared__ __align__(1024) uint8_t dw_smem[];
@@ -355,8 +360,11 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DensePa
     __shared__ int abort_word;
     volatile int* const abort_flag = &abort_word;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int row0 = blockIdx.x * DN_ROWS, n0 = blockIdx.y * N, live = min(N, p.ntokens - n0);
     const int ktot = p.K / DN_GROUP, nst = (ktot + 1) / 2;       // stages: two groups each, the last one perhaps a single one
+    const int row_tiles = p.rows / DN_ROWS, tiles = row_tiles * ((p.ntokens + N - 1) / N);
+    // ONE: a grid of row tiles x token tiles, a CTA each, which needs no divisions on its way
+    auto row_tile = [&](int tile) -> int { return ONE ? int(blockIdx.x) : tile % row_tiles; };
+    auto token_tile = [&](int tile) -> int { return ONE ? int(blockIdx.y) : tile / row_tiles; };
     const uint32_t sm0 = ptx::smem_u32(dw_smem), bar0 = sm0 + T::BAR;
     auto BAR = [&](int i) -> uint32_t { return bar0 + 8u * uint32_t(i); };
     if (sm0 & 1023u) {                         // the swizzled tiles need a 1024-byte aligned base: report, do nothing
@@ -379,7 +387,6 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DensePa
     ptx::tc_fence_after();
     const uint32_t tmem = tmem_slot;
     const size_t strip_bytes = size_t(ktot) * (DN_TILE_BYTES + DN_META_BYTES);
-    const uint8_t* strips = p.W + size_t(row0 >> 4) * strip_bytes;
     int errbits = 0;
     // Wait for use `u` of a slot to be filled / for the previous use of a slot to be over (the first needs no wait). The roles that go on to
     // warp-wide instructions take the form with one answer per warp. Its votes cost 1 to 1.5 % (2048 x 2048, 2048 tokens 34.6 -> 35.0 us);
@@ -397,9 +404,13 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DensePa
     };
     auto emptied_warp = [&](int bar, int u, int err) -> bool { return u == 0 || filled_warp(bar, u - 1, err); };
 
+    // The folding warps' registers come from the others: 96 take in all accumulators of a group at once (with 80, and two rounds of 16 of the
+    // 32, a tile of 128 x 128 x 2048 took 17.7 us, now 16.8; one of 64 tokens 12.5 and 11.7).
+    if (warp < DW_FOLD_WARPS) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(DW_FOLD_REGS));
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(DW_OTHER_REGS));
     if (warp < DW_FOLD_WARPS) {
         // ---- fold: a warp has 32 rows and COLS tokens, as an mma fragment: lane l rows l / 4 + 8 k, tokens 8 i + 2 (l % 4) and + 1. Two token
-        // factors then serve eight outputs (with a row a lane: two), and 80 registers a thread do without spills.
+        // factors then serve eight outputs (with a row a lane: two).
         constexpr int C = T::COLS;
         const int row = 32 * (warp & 3) + (lane >> 2), col = C * (warp >> 2) + 2 * (lane & 3);
         const uint32_t tacc = tmem + (uint32_t(32 * (warp & 3)) << 16) + C * (warp >> 2);
@@ -407,88 +418,88 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DensePa
         float* const sq = reinterpret_cast<float*>(dw_smem + T::SQ);
         float2* const wz = reinterpret_cast<float2*>(dw_smem + T::WZ);
         f32x2 c[C / 8][4];                             // per eight tokens: rows row, + 8, + 16, + 24
-#pragma unroll
-        for (int j = 0; j < C / 2; ++j) (&c[0][0])[j] = 0ull;
         const f32x2 magic = 0xCB400000CB400000ull;     // -1.5 * 2^23 twice
         bool alive = true;
+        int u = 0, ga = 0;                             // blocks of factors and groups so far, over all tiles
 #pragma unroll 1
-        for (int g0 = 0, u = 0; g0 < ktot && alive; g0 += DW_SC, ++u) {
-            // the factors of the next sixteen groups: thread = (token or row, group)
-            if (!emptied_warp(WB_SC_EMPTY, u, ERR_WAIT_SOFTMAX)) { alive = false; break; }
-            const int g = tid & 15, gi = min(g0 + g, ktot - 1);
+        for (int tile = blockIdx.x; tile < tiles && alive; tile += ONE ? tiles : int(gridDim.x)) {
+            const int row0 = row_tile(tile) * DN_ROWS, n0 = token_tile(tile) * N, live = min(N, p.ntokens - n0);
+            const uint8_t* strips = p.W + size_t(row0 >> 4) * strip_bytes;
 #pragma unroll
-            for (int k = 0; k < (N + 31) / 32; ++k) {
-                const int n = (tid >> 4) + 32 * k;
-                const size_t at = size_t(n0 + min(n, live - 1)) * ktot + gi;
-                sx[g * T::LD_T + n] = __ldg(p.s + at);
-                sq[g * T::LD_T + n] = float(__ldg(p.sum + at));
-            }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int r = (tid >> 4) + 32 * k, rr = r & 15;
-                const uint8_t* mt = strips + size_t(r >> 4) * strip_bytes + size_t(ktot) * DN_TILE_BYTES + size_t(gi) * DN_META_BYTES;
-                wz[g * T::LD_R + r] = make_float2(__half2float(__ushort_as_half(__ldg(reinterpret_cast<const uint16_t*>(mt + 4 * (rr & 7) + 2 * (rr >> 3))))),
-                                                  -float(__ldg(mt + 32 + 2 * (rr & 7) + (rr >> 3))));
-            }
-            ptx::mbar_arrive(BAR(WB_SC_FULL));
-            if (!filled_warp(WB_SC_FULL, u, ERR_WAIT_SOFTMAX)) { alive = false; break; }
-            const int ng = min(DW_SC, ktot - g0);
+            for (int j = 0; j < C / 2; ++j) (&c[0][0])[j] = 0ull;
 #pragma unroll 1
-            for (int i = 0; i < ng; ++i) {
-                const int slot = i % DW_ACC;           // DW_SC is a multiple of DW_ACC
-                f32x2 sw[4], nz[4];
+            for (int g0 = 0; g0 < ktot && alive; g0 += DW_SC, ++u) {
+                // the factors of the next sixteen groups: thread = (token or row, group)
+                if (!emptied_warp(WB_SC_EMPTY, u, ERR_WAIT_SOFTMAX)) { alive = false; break; }
+                const int g = tid & 15, gi = min(g0 + g, ktot - 1);
+#pragma unroll
+                for (int k = 0; k < (N + 31) / 32; ++k) {
+                    const int n = (tid >> 4) + 32 * k;
+                    const size_t at = size_t(n0 + min(n, live - 1)) * ktot + gi;
+                    sx[g * T::LD_T + n] = __ldg(p.s + at);
+                    sq[g * T::LD_T + n] = float(__ldg(p.sum + at));
+                }
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const float2 f = wz[i * T::LD_R + row + 8 * k];
-                    sw[k] = pack2(__float_as_uint(f.x), __float_as_uint(f.x)); nz[k] = pack2(__float_as_uint(f.y), __float_as_uint(f.y));
+                    const int r = (tid >> 4) + 32 * k, rr = r & 15;
+                    const uint8_t* mt = strips + size_t(r >> 4) * strip_bytes + size_t(ktot) * DN_TILE_BYTES + size_t(gi) * DN_META_BYTES;
+                    wz[g * T::LD_R + r] = make_float2(__half2float(__ushort_as_half(__ldg(reinterpret_cast<const uint16_t*>(mt + 4 * (rr & 7) + 2 * (rr >> 3))))),
+                                                      -float(__ldg(mt + 32 + 2 * (rr & 7) + (rr >> 3))));
                 }
-                if (!filled_warp(WB_ACC_FULL + slot, (g0 + i) / DW_ACC, ERR_WAIT_SOFTMAX)) { alive = false; break; }
-                ptx::tc_fence_after();
-                constexpr int H = C < 16 ? C : 16;     // tokens a round
+                ptx::mbar_arrive(BAR(WB_SC_FULL));
+                if (!filled_warp(WB_SC_FULL, u, ERR_WAIT_SOFTMAX)) { alive = false; break; }
+                const int ng = min(DW_SC, ktot - g0);
+#pragma unroll 1
+                for (int i = 0; i < ng; ++i, ++ga) {
+                    const int slot = ga % DW_ACC;
+                    f32x2 sw[4], nz[4];
 #pragma unroll
-                for (int h = 0; h < C; h += H) {
-                    uint32_t d0[H / 2], d1[H / 2];     // rows + 0, + 8 and rows + 16, + 24
-                    ptx::tmem_ld16x256_cols(tacc + slot * N + h, d0);
-                    ptx::tmem_ld16x256_cols(tacc + slot * N + h + (16u << 16), d1);
+                    for (int k = 0; k < 4; ++k) {
+                        const float2 f = wz[i * T::LD_R + row + 8 * k];
+                        sw[k] = pack2(__float_as_uint(f.x), __float_as_uint(f.x)); nz[k] = pack2(__float_as_uint(f.y), __float_as_uint(f.y));
+                    }
+                    if (!filled_warp(WB_ACC_FULL + slot, ga / DW_ACC, ERR_WAIT_SOFTMAX)) { alive = false; break; }
+                    ptx::tc_fence_after();
+                    uint32_t d0[C / 2], d1[C / 2];     // rows + 0, + 8 and rows + 16, + 24
+                    ptx::tmem_ld16x256_cols(tacc + slot * N, d0);
+                    ptx::tmem_ld16x256_cols(tacc + slot * N + (16u << 16), d1);
                     ptx::tmem_wait_ld_tied(d0);
                     ptx::tmem_wait_ld_tied(d1);
-                    if (h + H == C) {
-                        ptx::tc_fence_before();
-                        ptx::mbar_arrive(BAR(WB_ACC_EMPTY + slot));
-                    }
+                    ptx::tc_fence_before();
+                    ptx::mbar_arrive(BAR(WB_ACC_EMPTY + slot));
 #pragma unroll
-                    for (int j = 0; j < H / 8; ++j) {
-                        const f32x2 x = *reinterpret_cast<const f32x2*>(sx + i * T::LD_T + col + h + 8 * j), q = *reinterpret_cast<const f32x2*>(sq + i * T::LD_T + col + h + 8 * j);
+                    for (int j = 0; j < C / 8; ++j) {
+                        const f32x2 x = *reinterpret_cast<const f32x2*>(sx + i * T::LD_T + col + 8 * j), q = *reinterpret_cast<const f32x2*>(sq + i * T::LD_T + col + 8 * j);
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
                             const uint32_t *d = (k < 2 ? d0 : d1) + 4 * j + 2 * (k & 1);
                             // float(P - z sq) = (1.5 * 2^23 + P) + (-z sq - 1.5 * 2^23): both terms are whole numbers below 2^24 in
                             // magnitude (|P|, |z sq| <= 255 * 128 * 128 = 4,177,920), so every step is exact
                             const f32x2 v = add2(pack2(d[0] + 0x4B400000u, d[1] + 0x4B400000u), fma2v(nz[k], q, magic));
-                            f32x2& o = c[h / 8 + j][k];
-                            o = fma2v(mul2(sw[k], x), v, o);
+                            c[j][k] = fma2v(mul2(sw[k], x), v, c[j][k]);
                         }
                     }
                 }
+                ptx::mbar_arrive(BAR(WB_SC_EMPTY));
             }
-            if (g0 + DW_SC < ktot) ptx::mbar_arrive(BAR(WB_SC_EMPTY));
-        }
-        if (alive) {
-            // Y += c: a warp's access is eight rows of four tokens, whole sectors; all loads of eight tokens before the first add
-            float* y0 = p.Y + size_t(n0 + col) * p.rows + row0 + row;
+            if (alive) {
+                // Y += c: a warp's access is eight rows of four tokens, whole sectors; all loads before the first add
+                float* y0 = p.Y + size_t(n0 + col) * p.rows + row0 + row;
+                float y[C / 8][4][2];
 #pragma unroll
-            for (int j = 0; j < C / 8; ++j) {
-                float y[4][2];
+                for (int j = 0; j < C / 8; ++j)
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
+                    for (int k = 0; k < 4; ++k)
 #pragma unroll
-                    for (int e = 0; e < 2; ++e) y[k][e] = col + 8 * j + e < live ? __ldcg(y0 + size_t(8 * j + e) * p.rows + 8 * k) : 0.f;
+                        for (int e = 0; e < 2; ++e) y[j][k][e] = col + 8 * j + e < live ? __ldcg(y0 + size_t(8 * j + e) * p.rows + 8 * k) : 0.f;
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
+                for (int j = 0; j < C / 8; ++j)
 #pragma unroll
-                    for (int e = 0; e < 2; ++e)
-                        if (col + 8 * j + e < live)
-                            __stcg(y0 + size_t(8 * j + e) * p.rows + 8 * k, y[k][e] + __uint_as_float(uint32_t(e ? c[j][k] >> 32 : c[j][k])));
+                    for (int k = 0; k < 4; ++k)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e)
+                            if (col + 8 * j + e < live)
+                                __stcg(y0 + size_t(8 * j + e) * p.rows + 8 * k, y[j][k][e] + __uint_as_float(uint32_t(e ? c[j][k] >> 32 : c[j][k])));
             }
         }
     } else if (warp < DW_WARP_LOAD) {
@@ -500,8 +511,9 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DensePa
         const uint8_t* const src = dw_smem + T::RAW + s0 * 2 * DN_TILE_BYTES + 16 * lane;
         uint8_t* const dst0 = dw_smem + T::A + (16 * s0 + g) * 128 + (((2 * t) ^ g) << 4);
         uint8_t* const dst1 = dw_smem + T::A + (16 * s0 + g) * 128 + (((2 * t + 1) ^ g) << 4);
+        const int total = ONE ? nst : nst * ((tiles - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x));      // stages of all tiles of this CTA
 #pragma unroll 1
-        for (int i = 0; i < nst; ++i) {
+        for (int i = 0; i < total; ++i) {
             const int b = i & 1, u = i >> 1;
             static_assert(DW_RAW == 2 && DW_A == 2 && DW_B == 2, "slot = stage % 2");
             if (!filled(WB_RAW_FULL + b, u, ERR_WAIT_DEQUANT) || !emptied(WB_A_EMPTY + b, u, ERR_WAIT_DEQUANT)) break;
@@ -531,43 +543,55 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DensePa
         // ---- activations: 16-byte chunk c of token n at chunk position c ^ (n % 8), zeros for tokens past the end
         const int lt = tid - 32 * DW_WARP_LOAD, n = lt >> 3, cc = lt & 7;
         constexpr int STEP = 32 * DW_LOAD_WARPS / 8;   // tokens a round
+        static_assert(STEP % 8 == 0, "chunk positions of a thread's tokens");
         const uint32_t dst = sm0 + T::B + n * 128 + ((cc ^ (n & 7)) << 4);
-        const int8_t* const src = p.q + size_t(n0) * p.K + 16 * cc;
         const size_t step = size_t(STEP) * p.K;
+        bool alive = true;
+        int ia = 0;                                    // stages so far, over all tiles
 #pragma unroll 1
-        for (int i = 0; i < nst; ++i) {
-            const int b = i & 1;
-            if (!emptied(WB_B_EMPTY + b, i >> 1, ERR_WAIT_PRODUCER)) break;
-            const bool two = 2 * i + 1 < ktot;
-            const int8_t* at = src + size_t(n) * p.K + size_t(2 * i) * DN_GROUP;
-#pragma unroll
-            for (int k = 0; k < N / STEP; ++k, at += step) {
-                const bool on = n + STEP * k < live;
-                const int8_t* from = on ? at : src;
-                const uint32_t to = (dst ^ (STEP == 4 ? 64 * (k & 1) : 0)) + b * 2 * T::B_GROUP + k * STEP * 128;      // token n + 4: the other half of the chunks
-                cp_async16(to, from, on);
-                if (two) cp_async16(to + T::B_GROUP, from + (on ? DN_GROUP : 0), on);
+        for (int tile = blockIdx.x; tile < tiles && alive; tile += ONE ? tiles : int(gridDim.x)) {
+            const int row0 = row_tile(tile) * DN_ROWS, n0 = token_tile(tile) * N, live = min(N, p.ntokens - n0);
+            const int8_t* const src = p.q + size_t(n0) * p.K + 16 * cc;
+#pragma unroll 1
+            for (int i = 0; i < nst; ++i, ++ia) {
+                const int b = ia & 1;
+                if (!emptied(WB_B_EMPTY + b, ia >> 1, ERR_WAIT_PRODUCER)) { alive = false; break; }
+                const bool two = 2 * i + 1 < ktot;
+                const int8_t* at = src + size_t(n) * p.K + size_t(2 * i) * DN_GROUP;
+#pragma unroll 4                               // more of them do not fit into 48 registers
+                for (int k = 0; k < N / STEP; ++k, at += step) {
+                    const bool on = n + STEP * k < live;
+                    const int8_t* from = on ? at : src;
+                    const uint32_t to = dst + b * 2 * T::B_GROUP + k * STEP * 128;
+                    cp_async16(to, from, on);
+                    if (two) cp_async16(to + T::B_GROUP, from + (on ? DN_GROUP : 0), on);
+                }
+                cp_async_arrive(BAR(WB_B_FULL + b));
+                // the tile's part of Y into L2, wanted when the last group is folded
+                if (i == 0)
+                    for (int k = lt; k < live * 4; k += 32 * DW_LOAD_WARPS) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.Y + size_t(n0 + (k >> 2)) * p.rows + row0 + 32 * (k & 3)));
             }
-            cp_async_arrive(BAR(WB_B_FULL + b));
-            // the tile's part of Y into L2, wanted when the last group is folded
-            if (i == 0)
-                for (int k = lt; k < live * 4; k += 32 * DW_LOAD_WARPS) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.Y + size_t(n0 + (k >> 2)) * p.rows + row0 + 32 * (k & 3)));
         }
         cp_async_commit();
         cp_async_wait<0>();
     } else if (warp == DW_WARP_PRODUCER) {
         // ---- codes by bulk copy, one strip a lane
         int issued = 0;
+        bool alive = true;
 #pragma unroll 1
-        for (int i = 0; i < nst; ++i) {
-            const int b = i & 1;
-            if (!emptied_warp(WB_RAW_EMPTY + b, i >> 1, ERR_WAIT_PRODUCER)) break;
-            const uint32_t bytes = 2 * i + 1 < ktot ? 2 * DN_TILE_BYTES : DN_TILE_BYTES;
-            if (lane == 0) ptx::mbar_arrive_expect_tx(BAR(WB_RAW_FULL + b), 8 * bytes);
-            __syncwarp();
-            if (lane < 8)
-                ptx::bulk_g2s(sm0 + T::RAW + b * 2 * T::RAW_GROUP + lane * 2 * DN_TILE_BYTES, strips + lane * strip_bytes + size_t(2 * i) * DN_TILE_BYTES, bytes, BAR(WB_RAW_FULL + b));
-            issued = i + 1;
+        for (int tile = blockIdx.x; tile < tiles && alive; tile += ONE ? tiles : int(gridDim.x)) {
+            const uint8_t* strips = p.W + size_t(row_tile(tile) * (DN_ROWS / 16)) * strip_bytes;
+#pragma unroll 1
+            for (int i = 0; i < nst; ++i) {
+                const int b = issued & 1;
+                if (!emptied_warp(WB_RAW_EMPTY + b, issued >> 1, ERR_WAIT_PRODUCER)) { alive = false; break; }
+                const uint32_t bytes = 2 * i + 1 < ktot ? 2 * DN_TILE_BYTES : DN_TILE_BYTES;
+                if (lane == 0) ptx::mbar_arrive_expect_tx(BAR(WB_RAW_FULL + b), 8 * bytes);
+                __syncwarp();
+                if (lane < 8)
+                    ptx::bulk_g2s(sm0 + T::RAW + b * 2 * T::RAW_GROUP + lane * 2 * DN_TILE_BYTES, strips + lane * strip_bytes + size_t(2 * i) * DN_TILE_BYTES, bytes, BAR(WB_RAW_FULL + b));
+                ++issued;
+            }
         }
         // copies still in flight must land before the shared memory is given back
         if (*abort_flag)
@@ -580,21 +604,24 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DensePa
         const uint32_t hi = ptx::desc_hi(1024) | (2u << 29), idesc = idesc_i8_u8s8(DN_ROWS, N);
         const uint32_t a_lo = ptx::desc_lo(sm0 + T::A, 16), b_lo = ptx::desc_lo(sm0 + T::B, 16);
         bool alive = true;
+        int ia = 0, ga = 0;                            // stages and groups so far, over all tiles
 #pragma unroll 1
-        for (int i = 0; i < nst && alive; ++i) {
-            const int b = i & 1, u = i >> 1;
-            if (!filled_warp(WB_B_FULL + b, u, ERR_WAIT_MMA) || !filled_warp(WB_A_FULL + b, u, ERR_WAIT_MMA)) break;
-            ptx::fence_proxy_async_smem();             // the activations, written by other threads' cp.async and seen through the barrier
+        for (int tile = blockIdx.x; tile < tiles && alive; tile += ONE ? tiles : int(gridDim.x)) {
 #pragma unroll 1
-            for (int e = 0; e < 2; ++e) {
-                const int gi = 2 * i + e, slot = gi % DW_ACC;
-                if (gi >= ktot) break;
-                if (!emptied_warp(WB_ACC_EMPTY + slot, gi / DW_ACC, ERR_WAIT_MMA)) { alive = false; break; }
-                ptx::tc_fence_after();
-                mma_i8_group_warp(tmem + slot * N, a_lo + (2 * b + e) * (T::A_GROUP / 16), b_lo + (2 * b + e) * (T::B_GROUP / 16), hi, idesc, BAR(WB_ACC_FULL + slot));
+            for (int i = 0; i < nst && alive; ++i, ++ia) {
+                const int b = ia & 1, u = ia >> 1;
+                if (!filled_warp(WB_B_FULL + b, u, ERR_WAIT_MMA) || !filled_warp(WB_A_FULL + b, u, ERR_WAIT_MMA)) { alive = false; break; }
+                ptx::fence_proxy_async_smem();             // the activations, written by other threads' cp.async and seen through the barrier
+#pragma unroll 1
+                for (int e = 0; e < 2 && 2 * i + e < ktot; ++e, ++ga) {
+                    const int slot = ga % DW_ACC;
+                    if (!emptied_warp(WB_ACC_EMPTY + slot, ga / DW_ACC, ERR_WAIT_MMA)) { alive = false; break; }
+                    ptx::tc_fence_after();
+                    mma_i8_group_warp(tmem + slot * N, a_lo + (2 * b + e) * (T::A_GROUP / 16), b_lo + (2 * b + e) * (T::B_GROUP / 16), hi, idesc, BAR(WB_ACC_FULL + slot));
+                }
+                ptx::mma_commit_warp(BAR(WB_A_EMPTY + b));
+                ptx::mma_commit_warp(BAR(WB_B_EMPTY + b));
             }
-            ptx::mma_commit_warp(BAR(WB_A_EMPTY + b));
-            ptx::mma_commit_warp(BAR(WB_B_EMPTY + b));
         }
         ptx::mma_commit_warp(BAR(WB_SPARE));           // every MMA issued must have retired before tensor memory is released
         volatile int never = 0;

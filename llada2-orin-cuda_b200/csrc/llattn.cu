@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
 #include <algorithm>
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -243,13 +244,12 @@ bool dense_strips_win(int rows, int K, int ntokens, int sms) {
 
 // Tokens per CTA of the tcgen05 form, or 0 where the mma.sync tiles are the faster ones. A CTA of the former fills an SM and has a
 // long start (tensor memory, four roles, sixteen groups' factors), so it wins with the groups and with the tokens; the line follows
-// both sides' measured costs in microseconds, in a graph over 1024 .. 8192 rows, K = 128 .. 8192 and 80 .. 2560 tokens. 2048 rows,
-// tiles / tcgen05 with 32, 64 and 128 tokens a CTA:
-//   K = 2048    80 tokens  8.4 / 10.4, 12.2, 17.1    160  11.0 / 10.5, 12.2, 17.8    320  16.7 / 19.1, 12.3, 17.6
-//              640 tokens 26.5 / 28.3, 23.0, 17.9   2560  62 / 82, 56, 51
-//   K = 512    320 tokens  6.7 / 10.4, 7.1, 9.6     2560  22.7 / 43, 30, 26.5
-// Checked over 128 .. 32,768 rows, 33 .. 4096 tokens (1,400 sizes): a call that takes the tcgen05 form is at most 3.6 % slower than
-// its tiles, at six groups, and takes up to 41 % less time (both without the votes at its waits, 1 to 1.5 %).
+// both sides' measured costs in microseconds, in a graph over 1024 .. 4096 rows, K = 256 .. 4096 and 96 .. 4096 tokens. A CTA walks its
+// tiles without ending, so that a further one costs less than the first. 2048 rows, tiles / tcgen05 with 32, 64 and 128 tokens a CTA:
+//   K = 2048   160 tokens 11.1 / 10.6, 12.3, 17.2    320  16.8 / 18.0, 12.4, 17.2    640 26.6 / 25.1, 21.2, 17.3   2048 53.5 / -, 38.7, 31.8
+//   K = 512    320 tokens  6.8 / 8.9, 7.1, 9.3      2048  18.0 / -, 18.3, 14.6
+// Over those 198 sizes the choice costs 0.4 % over the fastest form in the mean (10 % at most, where the tiles' cost is off) and a call
+// that takes the tcgen05 form is never slower than its tiles.
 int dense_wide_tokens(int rows, int K, int ntokens, int sms) {
     if (ntokens <= 32) return 0;
     const double groups = K / llattn::DN_GROUP, row_tiles = rows / llattn::DN_ROWS;
@@ -264,13 +264,14 @@ int dense_wide_tokens(int rows, int K, int ntokens, int sms) {
         best = std::max(1.0, waves + idle * (waves > 6 ? 0.2 : 0.5)) * (2.9 + 1.42 * groups);
     }
     int wide = 0;
-    auto consider = [&](int tok, double start, double group) {
-        const double cost = std::ceil(ctas(tok) / sms) * (start + group * groups);
+    if (groups <= 2 || (groups <= 6 && ctas(64) > 6 * 2 * sms)) return 0;      // few groups in many waves, and the fewest at all: the tiles
+    auto consider = [&](int tok, double start, double group, double more, double group_more) {
+        const double cost = start + group * groups + (std::ceil(ctas(tok) / sms) - 1) * (more + group_more * groups);
         if (cost < best) { best = cost; wide = tok; }
     };
-    consider(32, 4.7, 0.355);
-    consider(64, 5.4, 0.42);
-    consider(128, 6.9, 0.67);
+    consider(32, 4.7, 0.388, 1.4, 0.375);
+    consider(64, 5.3, 0.455, 2.2, 0.445);
+    consider(128, 6.6, 0.68, 2.6, 0.685);
     return wide;
 }
 
@@ -317,30 +318,41 @@ int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int3
     if (!aligned16(W) || !aligned16(q)) return fail(LLATTN_EINVAL, "dense_w4a8: W and q must be 16-byte aligned");
     const llattn::DenseParams p{static_cast<const uint8_t*>(W), q, s, sum, Y, ntokens, rows, K, err_word};
     static std::once_flag once[64];
+    static std::atomic<int> split_ok[64];      // 1: the tcgen05 kernels have the registers that their roles divide
     int dev = 0;
     CU(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64)
-        std::call_once(once[dev], [] {
+        std::call_once(once[dev], [dev] {
+            bool ok = true;
+            auto wide = [&](auto* kernel, int smem) {
+                cudaFuncAttributes a{};
+                ok = ok && cudaFuncGetAttributes(&a, kernel) == cudaSuccess && a.numRegs >= llattn::DW_LAUNCH_REGS;
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            };
+            wide(llattn::dense_wide_kernel<32, false>, llattn::DenseWide<32>::SMEM); wide(llattn::dense_wide_kernel<32, true>, llattn::DenseWide<32>::SMEM);
+            wide(llattn::dense_wide_kernel<64, false>, llattn::DenseWide<64>::SMEM);
+            wide(llattn::dense_wide_kernel<128, false>, llattn::DenseWide<128>::SMEM);
+            split_ok[dev] = ok;
             cudaFuncSetAttribute(llattn::dense_strip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DS_SMEM_BYTES);
             cudaFuncSetAttribute(llattn::dense_tile_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseTile<16>::SMEM);
             cudaFuncSetAttribute(llattn::dense_tile_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseTile<32>::SMEM);
             cudaFuncSetAttribute(llattn::dense_tile_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseTile<64>::SMEM);
-            cudaFuncSetAttribute(llattn::dense_wide_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseWide<32>::SMEM);
-            cudaFuncSetAttribute(llattn::dense_wide_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseWide<64>::SMEM);
-            cudaFuncSetAttribute(llattn::dense_wide_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, llattn::DenseWide<128>::SMEM);
         });
     int sms = 0;
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const DenseForm f = dense_form(rows, K, ntokens, sms);
     const bool strips = f.kernel == LLATTN_DENSE_STRIPS;
-    auto launch = [&](auto* kernel, int threads, int smem) {
-        kernel<<<dim3(rows / (strips ? 16 : llattn::DN_ROWS), (ntokens + f.tokens - 1) / f.tokens), threads, smem, as_stream(stream)>>>(p);
-    };
+    if (f.kernel == LLATTN_DENSE_TCGEN05 && !(dev >= 0 && dev < 64 && split_ok[dev])) return fail(LLATTN_ECUDA, "dense_w4a8: a kernel was built with fewer registers than its roles divide");
+    const dim3 tiles(rows / (strips ? 16 : llattn::DN_ROWS), (ntokens + f.tokens - 1) / f.tokens);
+    // With 32 tokens a CTA and no more tiles than SMs, a CTA per tile in a kernel without the loop over them: 160 tokens 10.0 us, 10.4 with it.
+    const bool one = f.tokens == 32 && (long long)tiles.x * tiles.y <= sms;
+    const dim3 grid = f.kernel == LLATTN_DENSE_TCGEN05 && !one ? dim3(unsigned(std::min<long long>(sms, (long long)tiles.x * tiles.y))) : tiles;
+    auto launch = [&](auto* kernel, int threads, int smem) { kernel<<<grid, threads, smem, as_stream(stream)>>>(p); };
     if (strips) launch(llattn::dense_strip_kernel, llattn::DS_THREADS, llattn::DS_SMEM_BYTES);
     else if (f.kernel == LLATTN_DENSE_TCGEN05) {
-        if (f.tokens == 32) launch(llattn::dense_wide_kernel<32>, llattn::DW_THREADS, llattn::DenseWide<32>::SMEM);
-        else if (f.tokens == 64) launch(llattn::dense_wide_kernel<64>, llattn::DW_THREADS, llattn::DenseWide<64>::SMEM);
-        else launch(llattn::dense_wide_kernel<128>, llattn::DW_THREADS, llattn::DenseWide<128>::SMEM);
+        if (f.tokens == 32) launch(one ? llattn::dense_wide_kernel<32, true> : llattn::dense_wide_kernel<32, false>, llattn::DW_THREADS, llattn::DenseWide<32>::SMEM);
+        else if (f.tokens == 64) launch(llattn::dense_wide_kernel<64, false>, llattn::DW_THREADS, llattn::DenseWide<64>::SMEM);
+        else launch(llattn::dense_wide_kernel<128, false>, llattn::DW_THREADS, llattn::DenseWide<128>::SMEM);
     } else {
         if (f.tokens == 16) launch(llattn::dense_tile_kernel<16>, llattn::DT_THREADS, llattn::DenseTile<16>::SMEM);
         else if (f.tokens == 32) launch(llattn::dense_tile_kernel<32>, llattn::DT_THREADS, llattn::DenseTile<32>::SMEM);

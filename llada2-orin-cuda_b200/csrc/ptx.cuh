@@ -164,7 +164,7 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
 }
 
 // 16 lanes (lane field of taddr: the warp's quarter, + 16 for its second half) as an mma C fragment: thread t has columns 8 i + 2 (t % 4)
-// and + 1 of lane t / 4 in r[4 i], r[4 i + 1] and of lane t / 4 + 8 in r[4 i + 2], r[4 i + 3]. 8 or 16 columns.
+// and + 1 of lane t / 4 in r[4 i], r[4 i + 1] and of lane t / 4 + 8 in r[4 i + 2], r[4 i + 3]. 8, 16 or 32 columns.
 __device__ __forceinline__ void tmem_ld16x256_cols(uint32_t taddr, uint32_t (&r)[4]) {
     asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
 }
@@ -181,6 +181,7 @@ __device__ __forceinline__ void tmem_ld16x256_x4(uint32_t taddr, uint32_t (&r)[1
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr) : "memory");
 }
+__device__ __forceinline__ void tmem_ld16x256_cols(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16x256_x4(taddr, r); }
 __device__ __forceinline__ void tmem_st16x256_x4(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], "

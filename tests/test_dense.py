@@ -280,3 +280,20 @@ def test_dense_tcgen05_form(api, orc, pkg, ntokens, rows, K, tok):
     got = pad.cpu().numpy()
     assert (got[:tok] == 7).all() and (got[-tok:] == 7).all()
     assert np.array_equal(got[tok:-tok].view(np.uint32), want.view(np.uint32))
+
+
+# A CTA of the tcgen05 form walks several tiles: two and three of them, an odd number of groups (the rings and accumulators are then out of
+# step with the tile), more groups than factors held at a time, and a ragged last tile of tokens.
+@pytest.mark.gpu
+@pytest.mark.parametrize("ntokens,rows,K,tok", [(1280, 4096, 1152, 128), (2050, 2048, 1152, 128), (300, 16384, 1152, 128), (1217, 2048, 4224, 64)])
+def test_dense_tcgen05_several_tiles_per_cta(api, orc, pkg, ntokens, rows, K, tok):
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert api.dense_preview(rows, K, ntokens, 148) == (api.DENSE_TCGEN05, tok) and rows // 128 * -(-ntokens // tok) > 148
+    wl = pkg.workload
+    strips, _, _, _ = wl.dense_weights(rows, K, 71)
+    q, s, qsum = wl.int8_activations(ntokens, K, 72)
+    want = np.random.default_rng(73).normal(size=(ntokens, rows)).astype(np.float32)
+    Y, err = _dev(want), torch.zeros(1, dtype=torch.int32, device="cuda")
+    orc.dense_w4a8(strips, q, s, qsum, want)
+    api.dense_w4a8(_dev(strips), _dev(q), _dev(s), _dev(qsum), Y, err_word=err)
+    assert int(err.item()) == 0 and np.array_equal(Y.cpu().numpy().view(np.uint32), want.view(np.uint32))
