@@ -668,6 +668,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
     if (p.items && warp == 1 && lane < int(sizeof(RunDesc) / 4))
         reinterpret_cast<uint32_t*>(smem + SM_FIRST)[lane] = __ldg(reinterpret_cast<const uint32_t*>(p.first_runs + cta) + lane);
     if (warp == WARP_MMA) { ptx::tmem_alloc(ptx::smem_u32(tmem_slot), TMEM_COLS); ptx::tmem_relinquish(); }
+    // reference-grid mode may be a dependent launch itself: nothing is read or written before the kernel ahead has completed
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
@@ -1447,9 +1448,9 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
 
 template <bool PRECISE, bool ROWS16 = false>
 __global__ void __launch_bounds__(attn_threads(ROWS16), 1) attn_tile_kernel(const __grid_constant__ KParams p) {
-    // reference-grid mode: the folding launch behind this one carries the attribute of a dependent launch, may take its place
-    // on the SMs this one leaves idle, and waits there (nothing behind a list-mode launch carries it)
-    if (!PRECISE && !p.items) ptx::launch_dependents();
+    // Reference-grid mode: the folding launch behind this one carries the attribute of a dependent launch, may take its place
+    // on the SMs this one leaves idle, and waits there (nothing may do so behind a list-mode launch). This launch carries it too.
+    if (!PRECISE && !p.items) { ptx::launch_dependents(); ptx::grid_dependency_wait(); }
     attn_tile_body<PRECISE, ROWS16>(p, blockIdx.x);
 }
 

@@ -70,6 +70,7 @@ constexpr int DS_SMEM_BYTES = DS_WARPS * DS_TOK * DS_LD * 8;
 
 __global__ void __launch_bounds__(DS_THREADS, 1) dense_strip_kernel(const DenseParams p) {
     extern __shared__ __align__(16) uint8_t ds_smem[];
+    ptx::grid_dependency_wait();               // nothing is read or written before the kernel ahead has completed
     float2* pairs = reinterpret_cast<float2*>(ds_smem);               // [warp][token][DS_LD]: (float of the integer, s_w * s_x)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int strip = blockIdx.x, n0 = blockIdx.y * DS_TOK, live = min(DS_TOK, p.ntokens - n0);
@@ -184,6 +185,7 @@ template <int TOK>
 __global__ void __launch_bounds__(DT_THREADS, TOK == 64 ? 2 : 3) dense_tile_kernel(const DenseParams p) {
     using T = DenseTile<TOK>;
     extern __shared__ __align__(128) uint8_t dt_smem[];
+    ptx::grid_dependency_wait();               // nothing is read or written before the kernel ahead has completed
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int row0 = blockIdx.x * DN_ROWS, n0 = blockIdx.y * TOK, live = min(TOK, p.ntokens - n0);
     const int ktot = p.K / DN_GROUP;
@@ -382,6 +384,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DensePa
         abort_word = 0;
     }
     if (warp == DW_WARP_MMA) { ptx::tmem_alloc(ptx::smem_u32(&tmem_slot), T::TMEM); ptx::tmem_relinquish(); }
+    ptx::grid_dependency_wait();               // nothing is read or written before the kernel ahead has completed
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();

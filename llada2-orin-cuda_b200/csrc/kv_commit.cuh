@@ -9,6 +9,7 @@
 #pragma once
 #include <cuda_fp16.h>
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace llattn {
 
@@ -169,6 +170,7 @@ template <int NT>
 __global__ void __launch_bounds__(NT)
 kv_commit_kernel(const half* __restrict__ Kf, const half* __restrict__ Vf, uint8_t* __restrict__ records,
                  const int32_t* __restrict__ pages, int max_blocks, int blk) {
+    ptx::grid_dependency_wait();               // nothing is read or written before the kernel ahead has completed
     kv_commit_body<NT>(Kf, Vf, records, pages, max_blocks, blk);
 }
 

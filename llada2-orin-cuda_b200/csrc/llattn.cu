@@ -90,18 +90,28 @@ struct DeviceGuard {
     ~DeviceGuard() { if (prev >= 0) cudaSetDevice(prev); }
 };
 
-// A launch that may start before the kernel ahead of it in the stream has run out; its kernel waits with griddepcontrol.wait.
-// Behind a kernel that does not allow it, it is an ordinary launch.
+// A launch that may start before the kernel ahead of it in the stream has run out; its kernel waits with griddepcontrol.wait before it reads
+// or writes anything. Behind a kernel that does not allow it earlier, it takes its place when the last CTA of that one has left, and the
+// launch's own latency is hidden: every kernel of this library but the cooperative attention goes this way. Calls one after the other
+// through the Python binding, before / now: commit of 64 blocks 7.1 / 6.6 us, operator pair at 2 K tokens 16.6 / 14.6, 32 tokens through the
+// projection 8.2 / 7.2, 2048 33.0 / 31.0, a first pass over four prompts of 13 blocks 29.3 / 27.4; a 20-layer step in a graph, 1 x 8 K tokens 466 /
+// 440, four sequences within 0.5 %.
 template <typename... KArgs>
-cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, int threads, cudaStream_t stream, KArgs... args) {
+cudaError_t launch_dependent_smem(void (*kernel)(KArgs...), dim3 grid, int threads, int smem, cudaStream_t stream, KArgs... args) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.stream = stream;
+    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.stream = stream; cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e != cudaSuccess) cudaGetLastError();  // reported here, not to whoever asks next
+    return e;
+}
+template <typename... KArgs>
+cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, int threads, cudaStream_t stream, KArgs... args) {
+    return launch_dependent_smem(kernel, grid, threads, 0, stream, args...);
 }
 
 int ensure_kernel_attrs() {
@@ -160,9 +170,8 @@ int launch_commit(const void* Kf, const void* Vf, void* records, const int32_t* 
     const dim3 grid(llattn::NKV, nb);
     const half *k = static_cast<const half*>(Kf), *v = static_cast<const half*>(Vf);
     uint8_t* r = static_cast<uint8_t*>(records);
-    if (nb <= 2 * sms) llattn::kv_commit_kernel<512><<<grid, 512, 0, as_stream(stream)>>>(k, v, r, pages, max_blocks, blk);
-    else llattn::kv_commit_kernel<256><<<grid, 256, 0, as_stream(stream)>>>(k, v, r, pages, max_blocks, blk);
-    CU(cudaGetLastError());
+    if (nb <= 2 * sms) CU(launch_dependent(llattn::kv_commit_kernel<512>, grid, 512, as_stream(stream), k, v, r, pages, max_blocks, blk));
+    else CU(launch_dependent(llattn::kv_commit_kernel<256>, grid, 256, as_stream(stream), k, v, r, pages, max_blocks, blk));
     return LLATTN_OK;
 }
 }  // namespace
@@ -193,9 +202,8 @@ int launch_prepare(const float* qkv, const int32_t* pos, const float* gq, const 
     llattn::PrepArgs a{qkv, pos, gq, gk, inv_freq, eps, static_cast<half*>(q), static_cast<half*>(k), static_cast<half*>(v), T,
                        static_cast<uint8_t*>(records), pages, max_blocks, blk};
     const int blocks = (T + llattn::BLK - 1) / llattn::BLK;
-    if (records) llattn::qkv_prepare_kernel<true><<<dim3(blocks, 20), llattn::PREP_THREADS, 0, as_stream(stream)>>>(a);
-    else llattn::qkv_prepare_kernel<false><<<dim3(blocks, 24), llattn::PREP_THREADS, 0, as_stream(stream)>>>(a);
-    CU(cudaGetLastError());
+    if (records) CU(launch_dependent(llattn::qkv_prepare_kernel<true>, dim3(blocks, 20), llattn::PREP_THREADS, as_stream(stream), a));
+    else CU(launch_dependent(llattn::qkv_prepare_kernel<false>, dim3(blocks, 24), llattn::PREP_THREADS, as_stream(stream), a));
     return LLATTN_OK;
 }
 }  // namespace
@@ -246,10 +254,10 @@ bool dense_strips_win(int rows, int K, int ntokens, int sms) {
 // long start (tensor memory, four roles, sixteen groups' factors), so it wins with the groups and with the tokens; the line follows
 // both sides' measured costs in microseconds, in a graph over 1024 .. 4096 rows, K = 256 .. 4096 and 96 .. 4096 tokens. A CTA walks its
 // tiles without ending, so that a further one costs less than the first. 2048 rows, tiles / tcgen05 with 32, 64 and 128 tokens a CTA:
-//   K = 2048   160 tokens 11.1 / 10.6, 12.3, 17.2    320  16.8 / 18.0, 12.4, 17.2    640 26.6 / 25.1, 21.2, 17.3   2048 53.5 / -, 38.7, 31.8
-//   K = 512    320 tokens  6.8 / 8.9, 7.1, 9.3      2048  18.0 / -, 18.3, 14.6
-// Over those 198 sizes the choice costs 0.4 % over the fastest form in the mean (10 % at most, where the tiles' cost is off) and a call
-// that takes the tcgen05 form is never slower than its tiles.
+//   K = 2048   160 tokens 11.2 / 11.0, 12.3, 16.9    320  16.7 / 18.1, 12.2, 16.9    640 26.6 / 25.2, 21.4, 17.0   2048 49.7 / -, 39.1, 31.7
+//   K = 512    320 tokens  6.6 / 9.2, 7.1, 9.3      2048  18.2 / -, 19.2, 15.5
+// Over those 198 sizes the choice costs 0.6 % over the fastest form in the mean (10 % at most, where the tiles' cost is off) and a call
+// that takes the tcgen05 form is at most 1 % slower than its tiles.
 int dense_wide_tokens(int rows, int K, int ntokens, int sms) {
     if (ntokens <= 32) return 0;
     const double groups = K / llattn::DN_GROUP, row_tiles = rows / llattn::DN_ROWS;
@@ -347,7 +355,8 @@ int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int3
     // With 32 tokens a CTA and no more tiles than SMs, a CTA per tile in a kernel without the loop over them: 160 tokens 10.0 us, 10.4 with it.
     const bool one = f.tokens == 32 && (long long)tiles.x * tiles.y <= sms;
     const dim3 grid = f.kernel == LLATTN_DENSE_TCGEN05 && !one ? dim3(unsigned(std::min<long long>(sms, (long long)tiles.x * tiles.y))) : tiles;
-    auto launch = [&](auto* kernel, int threads, int smem) { kernel<<<grid, threads, smem, as_stream(stream)>>>(p); };
+    cudaError_t e = cudaSuccess;
+    auto launch = [&](auto* kernel, int threads, int smem) { e = launch_dependent_smem(kernel, grid, threads, smem, as_stream(stream), p); };
     if (strips) launch(llattn::dense_strip_kernel, llattn::DS_THREADS, llattn::DS_SMEM_BYTES);
     else if (f.kernel == LLATTN_DENSE_TCGEN05) {
         if (f.tokens == 32) launch(one ? llattn::dense_wide_kernel<32, true> : llattn::dense_wide_kernel<32, false>, llattn::DW_THREADS, llattn::DenseWide<32>::SMEM);
@@ -358,7 +367,7 @@ int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int3
         else if (f.tokens == 32) launch(llattn::dense_tile_kernel<32>, llattn::DT_THREADS, llattn::DenseTile<32>::SMEM);
         else launch(llattn::dense_tile_kernel<64>, llattn::DT_THREADS, llattn::DenseTile<64>::SMEM);
     }
-    CU(cudaGetLastError());
+    CU(e);
     return LLATTN_OK;
 }
 
@@ -465,8 +474,7 @@ extern "C" int llattn_attention_static(const void* Q, const void* Kf, const void
     p.ref_seq = SeqDesc{static_cast<const uint8_t*>(cache), nullptr, max_blocks, nblocks, nb, 0};
     p.ref_bpc = bpc;
     p.ref_nchunks = nchunks;
-    attn_tile_kernel<false><<<NKV * nchunks * nb, ATTN_THREADS, ATTN_SMEM_BYTES, as_stream(stream)>>>(p);
-    CU(cudaGetLastError());
+    CU(launch_dependent_smem(attn_tile_kernel<false>, dim3(NKV * nchunks * nb), ATTN_THREADS, ATTN_SMEM_BYTES, as_stream(stream), p));
     MergeOut o{static_cast<half*>(O16), O32, LSE, q8, s8, sum8};
     CU(launch_dependent(
         nchunks > FOLD_PART ? combine_ref_kernel<true> : combine_ref_kernel<false>, dim3(NKV, QR / MERGE_ROWS, nb), MERGE_THREADS, as_stream(stream),

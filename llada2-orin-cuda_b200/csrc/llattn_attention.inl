@@ -404,8 +404,7 @@ int llattn_attn_partial(const llattn_args* a, int nb, int* err_word, void* strea
     p.ref_seq = SeqDesc{static_cast<const uint8_t*>(a->cache), nullptr, a->max_blocks, a->nblocks, nb, 0};
     p.ref_bpc = a->blocks_per_chunk;
     p.ref_nchunks = a->nchunks;
-    attn_tile_kernel<false><<<NKV * a->nchunks * nb, ATTN_THREADS, ATTN_SMEM_BYTES, as_stream(stream)>>>(p);
-    CU(cudaGetLastError());
+    CU(launch_dependent_smem(attn_tile_kernel<false>, dim3(NKV * a->nchunks * nb), ATTN_THREADS, ATTN_SMEM_BYTES, as_stream(stream), p));
     return LLATTN_OK;
 }
 

@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include "common.cuh"
+#include "ptx.cuh"
 #include "kv_commit.cuh"
 
 namespace llattn {
@@ -72,6 +73,7 @@ __device__ __forceinline__ void rope_angle(const PrepArgs& a, int t, float freq,
 
 template <bool COMMIT>
 __global__ void __launch_bounds__(PREP_THREADS) qkv_prepare_kernel(const PrepArgs a) {
+    ptx::grid_dependency_wait();               // nothing is read or written before the kernel ahead has completed
     const int jb = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = jb * BLK;
     const float freq = a.inv_freq[lane];
