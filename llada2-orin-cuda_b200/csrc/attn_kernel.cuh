@@ -1450,7 +1450,8 @@ template <bool PRECISE, bool ROWS16 = false>
 __global__ void __launch_bounds__(attn_threads(ROWS16), 1) attn_tile_kernel(const __grid_constant__ KParams p) {
     // Reference-grid mode: the folding launch behind this one carries the attribute of a dependent launch, may take its place
     // on the SMs this one leaves idle, and waits there (nothing may do so behind a list-mode launch). This launch carries it too.
-    if (!PRECISE && !p.items) { ptx::launch_dependents(); ptx::grid_dependency_wait(); }
+    if (!PRECISE && !p.items) ptx::launch_dependents();
+    ptx::grid_dependency_wait();               // nothing is read or written before the kernel ahead has completed
     attn_tile_body<PRECISE, ROWS16>(p, blockIdx.x);
 }
 

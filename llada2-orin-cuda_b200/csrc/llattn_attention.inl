@@ -668,12 +668,23 @@ int llattn_attention(llattn_ctx* c, const llattn_plan* pl, const llattn_io* io, 
     p.tile_counters = static_cast<int*>(c->workspace);
     p.out = MergeOut{static_cast<half*>(io->O16), io->O32, io->LSE, io->q8, io->s8, io->sum8};
     p.cache_offset = io->cache_offset;
+    const bool precise = io->flags & LLATTN_IO_PRECISE_P, rows16 = precise && precise_rows16(pl, io->O32 != nullptr);
+    auto* const fn = rows16 ? attn_tile_kernel<true, true> : precise ? attn_tile_kernel<true> : attn_tile_kernel<false>;
+    const dim3 grid(pl->launch_ctas);
+    const int threads = attn_threads(rows16);
+    // Without a tile cut into several runs no CTA waits for another and the launch is an ordinary, dependent one. Not under capture: the
+    // graph's launch has to do for whatever plan_update makes of the plan.
+    if (pl->stats.nitems == pl->ntiles) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+        if (cudaStreamIsCapturing(as_stream(stream), &capture) != cudaSuccess) { cudaGetLastError(); capture = cudaStreamCaptureStatusActive; }
+        if (capture == cudaStreamCaptureStatusNone) {
+            CU(launch_dependent_smem(fn, grid, threads, ATTN_SMEM_BYTES, as_stream(stream), p));
+            return LLATTN_OK;
+        }
+    }
     // cooperative: the driver starts the grid only when all of its CTAs can be resident together (see plan_create)
     void* args[] = {&p};
-    const bool precise = io->flags & LLATTN_IO_PRECISE_P, rows16 = precise && precise_rows16(pl, io->O32 != nullptr);
-    const void* fn = rows16 ? reinterpret_cast<const void*>(attn_tile_kernel<true, true>)
-                   : precise ? reinterpret_cast<const void*>(attn_tile_kernel<true>) : reinterpret_cast<const void*>(attn_tile_kernel<false>);
-    CU(cudaLaunchCooperativeKernel(fn, dim3(pl->launch_ctas), dim3(attn_threads(rows16)), args, ATTN_SMEM_BYTES, as_stream(stream)));
+    CU(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(fn), grid, dim3(threads), args, ATTN_SMEM_BYTES, as_stream(stream)));
     return LLATTN_OK;
 }
 
