@@ -202,8 +202,13 @@ int launch_prepare(const float* qkv, const int32_t* pos, const float* gq, const 
     llattn::PrepArgs a{qkv, pos, gq, gk, inv_freq, eps, static_cast<half*>(q), static_cast<half*>(k), static_cast<half*>(v), T,
                        static_cast<uint8_t*>(records), pages, max_blocks, blk};
     const int blocks = (T + llattn::BLK - 1) / llattn::BLK;
-    if (records) CU(launch_dependent(llattn::qkv_prepare_kernel<true>, dim3(blocks, 20), llattn::PREP_THREADS, as_stream(stream), a));
-    else CU(launch_dependent(llattn::qkv_prepare_kernel<false>, dim3(blocks, 24), llattn::PREP_THREADS, as_stream(stream), a));
+    using namespace llattn;
+    int dev = 0, sms = 0;
+    if (records) { CU(cudaGetDevice(&dev)); CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)); }
+    if (!records) CU(launch_dependent(qkv_prepare_kernel<false, PREP_THREADS>, dim3(blocks, 6 * prep_parts(PREP_THREADS)), PREP_THREADS, as_stream(stream), a));
+    else if (9 * (long long)blocks <= 4 * sms)
+        CU(launch_dependent(qkv_prepare_kernel<true, PREP_FEW_THREADS>, dim3(blocks, NKV + 4 * prep_parts(PREP_FEW_THREADS)), PREP_FEW_THREADS, as_stream(stream), a));
+    else CU(launch_dependent(qkv_prepare_kernel<true, PREP_THREADS>, dim3(blocks, NKV + 4 * prep_parts(PREP_THREADS)), PREP_THREADS, as_stream(stream), a));
     return LLATTN_OK;
 }
 }  // namespace

@@ -11,11 +11,13 @@
 //
 // A warp takes the four heads of one group for one token: sixteen loads in flight, one sine and cosine for all of them.
 // Groups 0-3 are q heads, 4 the k heads, 5 the v heads; grid (blocks of 32 tokens, 24): group y / 4, tokens 8 (y % 4) ..,
-// 8 warps a CTA. With the commit, K and V of a (block, kv head) stay with one CTA: grid (blocks, 20), y < 16 as above,
-// y >= 16 kv head y - 16, a warp per four tokens.
+// 8 warps a CTA. With the commit, K and V of a (block, kv head) stay with one CTA: grid (blocks, 4 + 16), y < 4 kv head y, a warp per four
+// tokens, then the q groups as above. These four have the longest way and come first in the grid (52 blocks 8.0 -> 7.0 us in a graph,
+// 16 blocks 6.1 -> 5.2). For few blocks CTAs have 512 threads (grid (blocks, 4 + 8), a warp per two tokens of K and V: one block 4.6 ->
+// 3.7 us, 16 5.2 -> 4.5, 52 6.9 -> 6.7, 64 7.8 -> 7.7, 74 8.4 -> 8.6): up to 65 on 148 SMs, with 1.75 of the longer CTAs an SM.
 // Bound by latency in a decode step: the former split, 8 CTAs per block whose warps walked 16 rows one after the
-// other, took 7.8 us for one block in a graph; now 1.8 (with the commit 9.5 -> 5.1). HBM-bound from a few thousand tokens
-// on: 8192 tokens 38.9 -> 24.7 us = 6.1 TB/s.
+// other, took 7.8 us for one block in a graph; now 1.6 (with the commit 9.5 -> 3.7). HBM-bound from a few thousand tokens
+// on: 8192 tokens 38.9 -> 24.6 us = 6.1 TB/s.
 // Lane l holds dims l, l+32, l+64, l+96 of a row: the rotate-half partners
 // then share a lane and every global access of a warp is one contiguous segment. The float operations and their order
 // are the reference kernel's (sum of squares folded lane-wise then by a xor butterfly, rsqrtf, x*r*g, sincosf, one
@@ -29,7 +31,8 @@
 
 namespace llattn {
 
-constexpr int PREP_THREADS = 256;
+constexpr int PREP_THREADS = 256, PREP_FEW_THREADS = 512;      // with the commit, few blocks: the latter
+__host__ __device__ constexpr int prep_parts(int threads) { return BLK / (threads / 32); }      // CTAs that share a group's tokens of a block
 
 struct PrepArgs {
     const float* qkv;        // [T][3072]
@@ -71,15 +74,15 @@ __device__ __forceinline__ void rope_angle(const PrepArgs& a, int t, float freq,
     sn = __bfloat162float(__float2bfloat16(sn));
 }
 
-template <bool COMMIT>
-__global__ void __launch_bounds__(PREP_THREADS) qkv_prepare_kernel(const PrepArgs a) {
+template <bool COMMIT, int NT>
+__global__ void __launch_bounds__(NT) qkv_prepare_kernel(const PrepArgs a) {
     ptx::grid_dependency_wait();               // nothing is read or written before the kernel ahead has completed
     const int jb = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = jb * BLK;
     const float freq = a.inv_freq[lane];
-    if (!COMMIT || blockIdx.y < 16) {
+    if (!COMMIT || blockIdx.y >= NKV) {
         // ---- four heads of one token
-        const int grp = blockIdx.y >> 2, t = t0 + 8 * (blockIdx.y & 3) + warp;
+        const int part = int(blockIdx.y) - (COMMIT ? NKV : 0), grp = part / prep_parts(NT), t = t0 + NT / 32 * (part % prep_parts(NT)) + warp;
         if (t >= a.T) return;
         const float* src = a.qkv + size_t(t) * 3072 + 4 * grp * D + lane;
         float x[4][4];
@@ -104,8 +107,8 @@ __global__ void __launch_bounds__(PREP_THREADS) qkv_prepare_kernel(const PrepArg
     if constexpr (COMMIT) {
         // ---- kv head h: the block's K (normalised, rotated) and V (converted) as fp16 tiles in shared memory. Whole blocks.
         __shared__ CommitSmem sm;
-        const int h = blockIdx.y - 16;
-        constexpr int TOKS = BLK / (PREP_THREADS / 32);
+        const int h = blockIdx.y;
+        constexpr int TOKS = BLK / (NT / 32);
         float xk[TOKS][4], xv[TOKS][4];
 #pragma unroll
         for (int k = 0; k < TOKS; ++k) {
@@ -127,14 +130,14 @@ __global__ void __launch_bounds__(PREP_THREADS) qkv_prepare_kernel(const PrepArg
         }
         __syncthreads();
         // ---- fp16 K and V of the block to global memory, 16 bytes per thread and store
-        for (int i = threadIdx.x; i < BLK * 16; i += PREP_THREADS) {
+        for (int i = threadIdx.x; i < BLK * 16; i += NT) {
             const int tok = i >> 4, ch = i & 15;
             const size_t at = (size_t(t0 + tok) * NKV + h) * D + ch * 8;
             *reinterpret_cast<uint4*>(a.k + at) = *reinterpret_cast<const uint4*>(&sm.Ks[tok][ch * 8]);
             *reinterpret_cast<uint4*>(a.v + at) = *reinterpret_cast<const uint4*>(&sm.Vs[tok][ch * 8]);
         }
         const size_t ridx = a.pages ? size_t(a.pages[jb * NKV + h]) : size_t(h) * a.max_blocks + a.blk + jb;
-        commit_tiles<PREP_THREADS>(sm, a.records + ridx * REC_BYTES, threadIdx.x);
+        commit_tiles<NT>(sm, a.records + ridx * REC_BYTES, threadIdx.x);
     }
 }
 

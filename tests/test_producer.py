@@ -138,3 +138,29 @@ def test_producer_fused_with_commit(orc, pkg, nb, paged):
             assert torch.equal(ref, got)
     with pytest.raises(ValueError):
         api.qkv_prepare_commit(args[0][:T - 1], *args[1:], q1, k1, v1, got, max_blocks=maxb, blk=blk)
+
+
+# Both launch shapes of the fused commit, at the line between them (65 blocks on 148 SMs) and at the ends: what the producer and the commit
+# give one after the other, byte for byte.
+@pytest.mark.gpu
+@pytest.mark.parametrize("nb,paged", [(1, False), (3, True), (64, False), (65, True), (66, False), (150, True)])
+def test_fused_commit_launch_shapes(pkg, nb, paged):
+    torch = pytest.importorskip("torch")
+    api = importlib.import_module(pkg.__name__ + ".api")
+    T = 32 * nb
+    qkv, pos, gq, gk, eps = inputs(T, 90 + nb)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    args = (dev(qkv), dev(pos), dev(gq), dev(gk), float(eps), dev(api.inv_freq()))
+    outs = [[torch.full((T, n, 128), 7.0, dtype=torch.half, device="cuda") for n in (16, 4, 4)] for _ in range(2)]
+    caches = [torch.full((4, nb + 2, 4736), 9, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    pages = torch.from_numpy(np.random.default_rng(nb).permutation(4 * (nb + 2))[:4 * nb].astype(np.int32).reshape(nb, 4)).cuda() if paged else None
+    api.qk_norm_rope(*args, *outs[0])
+    K, V = outs[0][1].view(nb, 32, 4, 128), outs[0][2].view(nb, 32, 4, 128)
+    if paged:
+        api.kv_commit_paged(K, V, caches[0], pages)
+        api.qkv_prepare_commit(*args, *outs[1], caches[1], pages=pages)
+    else:
+        api.kv_commit(K, V, caches[0], nb + 2, 1)
+        api.qkv_prepare_commit(*args, *outs[1], caches[1], max_blocks=nb + 2, blk=1)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(*outs)) and torch.equal(*caches)
