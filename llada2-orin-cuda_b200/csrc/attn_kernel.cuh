@@ -8,7 +8,7 @@
 //                   alternate records: one service warp per scheduler keeps the schedulers' loads alike)
 //   dequant warps : nibbles -> fp16 (magic-number unpack, one fp16 FMA per pair as the reference's __hfma2), written
 //                   straight into the 128-byte-swizzle UMMA operand layout; fresh fp16 K/V are copied into the same layout
-//   MMA warps     : S = Q K^T  (tcgen05.mma kind::f16, A = Q in TMEM, B = K K-major in shared memory, fp32 S in TMEM)
+//   MMA warp      : S = Q K^T  (tcgen05.mma kind::f16, A = Q in TMEM, B = K K-major in shared memory, fp32 S in TMEM)
 //                   O += P V   (A = P read from TMEM as packed fp16, B = V MN-major in shared memory, fp32 O in TMEM);
 //                   V carries one extra column of ones, so the same MMA also accumulates the softmax row sum from
 //                   exactly the fp16 P the numerator uses (numerator and denominator then share their rounding)
@@ -73,9 +73,9 @@ constexpr int VTILE_BYTES = 3 * KBLOCK;            // V tile: dims 0-63, 64-127,
 constexpr int UNIT_BYTES = 32 * 128;               // a unit's 32 keys inside a block
 constexpr int PV_N = 144;                          // dims 0..127, column 128 = row sum, 129..143 unused
 #ifndef LLATTN_NRAW
-#define LLATTN_NRAW 8
+#define LLATTN_NRAW 10
 #endif
-constexpr int NRAW = LLATTN_NRAW;                  // records in flight (8 = two tiles' worth)
+constexpr int NRAW = LLATTN_NRAW;                  // records in flight: two tiles' worth and two more
 constexpr int RAW_STRIDE = 4864;                   // 4736 rounded up to a multiple of 128
 constexpr int SM_K = 0;                            // two K tiles (every tile base is 1024-byte aligned)
 constexpr int SM_V = SM_K + 2 * TILE_BYTES;        // two V tiles
@@ -99,14 +99,11 @@ constexpr int ATTN_SMEM_BYTES = SM_QSUM + QR * 4;
 #ifndef LLATTN_GROUP_WARPS
 #define LLATTN_GROUP_WARPS 2
 #endif
-#ifndef LLATTN_SINGLE_ISSUER
-#define LLATTN_SINGLE_ISSUER 0     // 1: one warp issues PV(t) and then S(t+2); the tensor pipe runs one thread's MMAs in order
-#endif
 __host__ __device__ constexpr int softmax_warps(bool rows16) { return rows16 ? 8 : 4; }
 constexpr int DEQUANT_WARPS = LLATTN_DEQUANT_WARPS, GROUP_WARPS = LLATTN_GROUP_WARPS, DEQUANT_GROUPS = DEQUANT_WARPS / GROUP_WARPS;
 constexpr int GROUP_THREADS = 32 * GROUP_WARPS, DQ_PASSES = 16 / GROUP_WARPS;      // a group converts one record: 32 keys, two per warp and pass
-// Service warps, one per scheduler (a warp runs on scheduler warp % 4 and the softmax warps cannot move): PV issue, S
-// issue and two copy producers that take alternate records, so that no scheduler carries much more than the others.
+// Service warps, one per scheduler (a warp runs on scheduler warp % 4 and the softmax warps cannot move): MMA issue, two copy producers
+// that take alternate records, so that no scheduler carries much more than the others, and one that writes V's ones column and is done.
 constexpr int PRODUCERS = 2;
 __host__ __device__ constexpr int attn_threads(bool rows16) { return 32 * (softmax_warps(rows16) + DEQUANT_WARPS + 2 + PRODUCERS); }
 constexpr int ATTN_THREADS = attn_threads(false);  // 512; 640 with eight softmax warps
@@ -120,7 +117,7 @@ constexpr float RESCALE_SLACK = 8.f;
 // barrier indices
 enum { B_RAW_FULL = 0, B_RAW_EMPTY = B_RAW_FULL + NRAW, B_K_FULL = B_RAW_EMPTY + NRAW, B_V_FULL = B_K_FULL + 2,
        B_K_FREE = B_V_FULL + 2, B_PV_DONE = B_K_FREE + 2, B_S_FULL = B_PV_DONE + 2, B_P_FULL = B_S_FULL + 2,
-       B_Q_FULL = B_P_FULL + 2, B_O_FREE, B_QSUM, B_SPARE, B_COUNT = B_SPARE + 2 };
+       B_Q_FULL = B_P_FULL + 2, B_O_FREE, B_QSUM, B_ONES, B_SPARE, B_COUNT };
 static_assert(B_COUNT * 8 <= 512, "barrier area");
 static_assert(ATTN_SMEM_BYTES <= 232448, "shared memory budget");
 static_assert((GROUP_WARPS == 2 || GROUP_WARPS == 4) && DEQUANT_WARPS % GROUP_WARPS == 0 && DEQUANT_GROUPS >= 1 && TILE_UNITS % DEQUANT_GROUPS == 0,
@@ -608,10 +605,10 @@ __device__ __forceinline__ void copy_fresh(const half* src, uint8_t* tile_unit, 
     }
 }
 
-// Third block of both V tiles: column 128 of V is all ones (O column 128 accumulates sum(P)), 129..143 zero. Written by the warp
-// that issues the MMAs which read it; its first tile is still on its way then. Unrolled 8 times not for its own sake, it runs once:
-// where the code behind it comes to lie moves the kernel's pace by up to 8 %, and this was the best over both forms (192 sequences at
-// 2 K tokens 176 us rolled up by the compiler, 171 with 8, 162 with 16; the precise form 247, 240 and 250; 24 x 32 tokens 8.6, 8.6, 8.7).
+// Third block of both V tiles: column 128 of V is all ones (O column 128 accumulates sum(P)), 129..143 zero. Written by a warp of its own
+// while the first records are on their way: by the issuing warp in front of its first S it cost a short call 0.4 us (128 tokens 8.5 and
+// 8.1). Unrolled 8 times not for its own sake, it runs once: where the code behind it comes to lie moves the kernel's pace (rolled up, 4, 8, 16
+// and 32 times: the 20-layer step 440, 439, 440, 442 and 448 us, 192 sequences at 2 K tokens with the precise form 194, 190, 187, 186 and 197).
 __device__ __forceinline__ void write_ones_column(uint8_t* smem, int lane) {
 #pragma unroll 8
     for (int idx = lane; idx < 2 * 128 * 8; idx += 32) {
@@ -659,7 +656,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
         ptx::mbar_init(BAR(B_Q_FULL), 32 * SOFTMAX_WARPS); ptx::mbar_init(BAR(B_O_FREE), 32 * SOFTMAX_WARPS);
         ptx::mbar_init(BAR(B_QSUM), 128);
         ptx::mbar_init(BAR(B_SPARE), 1);
-        ptx::mbar_init(BAR(B_SPARE + 1), 1);
+        ptx::mbar_init(BAR(B_ONES), 1);
         ptx::fence_mbar_init();
         *abort_flag = 0;
     }
@@ -1232,10 +1229,11 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
         const uint32_t klo0 = ptx::desc_lo(k_s, 16), klo1 = ptx::desc_lo(k_s + TILE_BYTES, 16), khi = ptx::desc_hi(1024) | (2u << 29);
         const uint32_t tmem = uniform_u32(tmem_any);
         const int i0 = uniform_i32(i0_any), i1 = uniform_i32(i1_any);
-#if LLATTN_SINGLE_ISSUER
-        write_ones_column(smem, lane);
         // This warp issues everything, per tile t in the order PV(t), S(t+2). S(t+2) overwrites the buffer that holds P(t);
-        // the tensor pipe executes the MMAs of one thread in issue order, so no wait for PV(t) to complete is needed.
+        // the tensor pipe executes the MMAs of one thread in issue order, so no wait for PV(t) to complete is needed. With a warp for S and one
+        // for PV, which had to see PV(t) complete before S(t+2), and eight records in flight instead of ten: 64 sequences of 1 K tokens 34.9 us
+        // (now 33.2), of 32 K 628 (616), 100 ragged ones of up to 8 K 142 (137), eight of 9.6 K 38.7 (37.2), 24 of 32 tokens 7.8 (7.4), the precise form at 64 x 1 K
+        // 42.4 (41.0); ten records for that form and eight for this one make no difference and 1 %.
         const uint32_t v_s = ptx::smem_u32(smem + SM_V);
         const uint32_t idO = ptx::idesc_f16(128, PV_N, false, true);
         const uint32_t vlo0 = ptx::desc_lo(v_s, KBLOCK), vlo1 = ptx::desc_lo(v_s + VTILE_BYTES, KBLOCK), vhi = ptx::desc_hi(1024) | (2u << 29);
@@ -1263,6 +1261,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
                 if (!uniform_i32(ptx::mbar_wait(BAR(B_V_FULL + b), (t >> 1) & 1, abort_flag))) { alive = false; errbits |= ERR_WAIT_MMA; break; }
                 if (!uniform_i32(ptx::mbar_wait(BAR(B_P_FULL + b), (t >> 1) & 1, abort_flag))) { alive = false; errbits |= ERR_WAIT_MMA; break; }
                 LLATTN_TR(24, t);
+                if (t == 0 && !uniform_i32(ptx::mbar_wait(BAR(B_ONES), 0, abort_flag))) { alive = false; errbits |= ERR_WAIT_MMA; break; }
                 // the previous item's epilogue must have read O before the first PV of this item overwrites it
                 if (i == 0 && itc > 0 && !uniform_i32(ptx::mbar_wait(BAR(B_O_FREE), (itc - 1) & 1, abort_flag))) { alive = false; errbits |= ERR_WAIT_MMA; break; }
                 ptx::tc_fence_after();
@@ -1292,33 +1291,6 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
             }
             ++itc;
         }
-#else
-        // S = Q K^T issue; the PV warp below issues O += P V. Two issuing warps halve the per-tile instruction chain.
-#pragma unroll 1
-        for (int ii = i0; ii < i1 && alive; ++ii) {
-            WorkItem w; SeqDesc s;
-            if (!uniform_i32(fetch_item(p, ii, w, s, first_run, i0_any))) continue;
-            const int U = uniform_i32(w.rec_count + w.fresh), ntiles = (U + TILE_UNITS - 1) / TILE_UNITS;
-            if (!uniform_i32(ptx::mbar_wait(BAR(B_Q_FULL), itc & 1, abort_flag))) { alive = false; errbits |= ERR_WAIT_MMA; break; }
-#pragma unroll 1
-            for (int i = 0; i < ntiles; ++i, ++t) {
-                const uint32_t b = t & 1;
-                const int nu = min(TILE_UNITS, U - TILE_UNITS * i);
-                LLATTN_TR(20, t);
-                if (!uniform_i32(ptx::mbar_wait(BAR(B_K_FULL + b), (t >> 1) & 1, abort_flag))) { alive = false; errbits |= ERR_WAIT_MMA; break; }
-                // S buffer b also holds P of tile t-2: PV of that tile must have consumed it
-                if (t >= 2 && !uniform_i32(ptx::mbar_wait(BAR(B_PV_DONE + b), ((t >> 1) - 1) & 1, abort_flag))) { alive = false; errbits |= ERR_WAIT_MMA; break; }
-                LLATTN_TR(21, t);
-                ptx::tc_fence_after();
-                {
-                    const uint32_t idS = ptx::idesc_f16(128, 32 * nu, false, false), ds = tmem + TM_S + b * 128;
-                    ptx::mma_ts_s8_warp<KBLOCK / 16>(ds, tmem + TM_Q, b ? klo1 : klo0, khi, idS, BAR(B_S_FULL + b), BAR(B_K_FREE + b));
-                }
-                LLATTN_TR(25, t);
-            }
-            ++itc;
-        }
-#endif
         // every MMA issued must have retired before tensor memory is released
         ptx::mma_commit_warp(BAR(B_SPARE));
         {
@@ -1326,65 +1298,10 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
             if (!ptx::mbar_wait(BAR(B_SPARE), 0, &never)) errbits |= ERR_WAIT_TEARDOWN;
         }
     } else {
-#if !LLATTN_SINGLE_ISSUER
-        // ================================================================== O += P V issue
-        uint32_t t = 0, itc = 0;
-        bool alive = true;
+        // ================================================================== V's ones column, ready before the first PV (the MMA warp waits)
         write_ones_column(smem, lane);
-        const uint32_t v_s = ptx::smem_u32(smem + SM_V);
-        const uint32_t idO = ptx::idesc_f16(128, PV_N, false, true);
-        // one base descriptor per V buffer (MN-major, 128-byte swizzle: 8-key groups 1024 B apart, 64-dim blocks KBLOCK apart)
-        const uint32_t vlo0 = ptx::desc_lo(v_s, KBLOCK), vlo1 = ptx::desc_lo(v_s + VTILE_BYTES, KBLOCK), vhi = ptx::desc_hi(1024) | (2u << 29);
-        const uint32_t tmem = uniform_u32(tmem_any);
-        const int i0 = uniform_i32(i0_any), i1 = uniform_i32(i1_any);
-#pragma unroll 1
-        for (int ii = i0; ii < i1 && alive; ++ii) {
-            WorkItem w; SeqDesc s;
-            if (!uniform_i32(fetch_item(p, ii, w, s, first_run, i0_any))) continue;
-            const int U = uniform_i32(w.rec_count + w.fresh), ntiles = (U + TILE_UNITS - 1) / TILE_UNITS;
-#pragma unroll 1
-            for (int i = 0; i < ntiles; ++i, ++t) {
-                const uint32_t b = t & 1;
-                const int nu = min(TILE_UNITS, U - TILE_UNITS * i);
-                LLATTN_TR(22, t);
-                if (!uniform_i32(ptx::mbar_wait(BAR(B_V_FULL + b), (t >> 1) & 1, abort_flag))) { alive = false; errbits |= ERR_WAIT_MMA; break; }
-                LLATTN_TR(23, t);
-                if (!uniform_i32(ptx::mbar_wait(BAR(B_P_FULL + b), (t >> 1) & 1, abort_flag))) { alive = false; errbits |= ERR_WAIT_MMA; break; }
-                LLATTN_TR(24, t);
-                // the previous item's epilogue must have read O before the first PV of this item overwrites it
-                if (i == 0 && itc > 0 && !uniform_i32(ptx::mbar_wait(BAR(B_O_FREE), (itc - 1) & 1, abort_flag))) { alive = false; errbits |= ERR_WAIT_MMA; break; }
-                ptx::tc_fence_after();
-                {
-                    // unit u = keys 32u..32u+31 = K-steps 2u, 2u+1; its P sits at columns 32u .. 32u+15 of the S buffer
-                    const uint32_t pb = tmem + TM_S + b * 128, vlo = b ? vlo1 : vlo0;
-                    if (nu == TILE_UNITS) {
-                        if (PRECISE) {
-                            ptx::mma_ts_pv8_warp<false>(tmem + TM_O, pb, vlo, vhi, idO, i == 0 ? 0u : 1u, 0u);
-                            ptx::mma_ts_pv8_warp<true>(tmem + TM_O, pb + 16, vlo, vhi, idO, 1u, BAR(B_PV_DONE + b));     // the remainders of P
-                        } else {
-                            ptx::mma_ts_pv8_warp<true>(tmem + TM_O, pb, vlo, vhi, idO, i == 0 ? 0u : 1u, BAR(B_PV_DONE + b));
-                        }
-                    } else {
-#pragma unroll
-                        for (int u = 0; u < TILE_UNITS - 1; ++u)
-                            if (u < nu) {
-                                const uint64_t d0 = (uint64_t(vhi) << 32) | (vlo + 256u * u);
-                                ptx::mma_ts_x2_warp(tmem + TM_O, pb + 32 * u, d0, d0 + 128, idO, (i == 0 && u == 0) ? 0u : 1u);
-                                if (PRECISE) ptx::mma_ts_x2_warp(tmem + TM_O, pb + 32 * u + 16, d0, d0 + 128, idO, 1u);
-                            }
-                        ptx::mma_commit_warp(BAR(B_PV_DONE + b));
-                    }
-                }
-                LLATTN_TR(26, t);
-            }
-            ++itc;
-        }
-        ptx::mma_commit_warp(BAR(B_SPARE + 1));
-        {
-            volatile int never = 0;
-            if (!ptx::mbar_wait(BAR(B_SPARE + 1), 0, &never)) errbits |= ERR_WAIT_TEARDOWN;
-        }
-#endif
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(BAR(B_ONES));
     }
 
     // ---- split tiles. Every run of this CTA is stored and counted by now, so nothing this CTA waits for depends on
