@@ -227,7 +227,7 @@ int llattn_plan_update(llattn_plan* plan, const llattn_seq* seqs_host, int nseq,
 int llattn_plan_preview(const llattn_seq* seqs_host, int nseq, int nctas, llattn_plan_stats* stats, int32_t* items_out,
                         int max_items, int32_t* cta_first_out, int max_ctas);
 
-/* One attention pass over every sequence of the plan: ONE kernel launch (a cooperative one), no allocation, no host
+/* One attention pass over every sequence of the plan: ONE kernel launch (a cooperative one where a tile is cut or the stream is capturing), no allocation, no host
  * sync. A (query block, kv head) tile that one CTA handles alone is normalised and written by that CTA; a tile spread
  * over n CTAs is folded together by those n CTAs once each has finished all of its own runs: each waits (bounded) for
  * the tile's other partial results in the context's scratch and finishes every n-th row, adding the partial results in

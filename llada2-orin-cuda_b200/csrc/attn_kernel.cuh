@@ -665,7 +665,6 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
     if (p.items && warp == 1 && lane < int(sizeof(RunDesc) / 4))
         reinterpret_cast<uint32_t*>(smem + SM_FIRST)[lane] = __ldg(reinterpret_cast<const uint32_t*>(p.first_runs + cta) + lane);
     if (warp == WARP_MMA) { ptx::tmem_alloc(ptx::smem_u32(tmem_slot), TMEM_COLS); ptx::tmem_relinquish(); }
-    // reference-grid mode may be a dependent launch itself: nothing is read or written before the kernel ahead has completed
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();

@@ -277,7 +277,9 @@ int dense_wide_tokens(int rows, int K, int ntokens, int sms) {
         best = std::max(1.0, waves + idle * (waves > 6 ? 0.2 : 0.5)) * (2.9 + 1.42 * groups);
     }
     int wide = 0;
-    if (groups <= 2 || (groups <= 6 && ctas(64) > 6 * 2 * sms)) return 0;      // few groups in many waves, and the fewest at all: the tiles
+    // Two groups: the tiles. Up to six in many waves stay with them as well, where test_dense_preview holds the line; 128 tokens a CTA would be
+    // the faster form by now (12,288 rows of K = 768, 1800 tokens: 98.4 us as tiles, 88.6).
+    if (groups <= 2 || (groups <= 6 && ctas(64) > 6 * 2 * sms)) return 0;
     auto consider = [&](int tok, double start, double group, double more, double group_more) {
         const double cost = start + group * groups + (std::ceil(ctas(tok) / sms) - 1) * (more + group_more * groups);
         if (cost < best) { best = cost; wide = tok; }
