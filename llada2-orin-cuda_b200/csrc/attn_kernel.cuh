@@ -1228,17 +1228,20 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
         const uint32_t klo0 = ptx::desc_lo(k_s, 16), klo1 = ptx::desc_lo(k_s + TILE_BYTES, 16), khi = ptx::desc_hi(1024) | (2u << 29);
         const uint32_t tmem = uniform_u32(tmem_any);
         const int i0 = uniform_i32(i0_any), i1 = uniform_i32(i1_any);
-        // This warp issues everything, per tile t in the order PV(t), S(t+2). S(t+2) overwrites the buffer that holds P(t);
-        // the tensor pipe executes the MMAs of one thread in issue order, so no wait for PV(t) to complete is needed. With a warp for S and one
-        // for PV, which had to see PV(t) complete before S(t+2), and eight records in flight instead of ten: 64 sequences of 1 K tokens 34.9 us
-        // (now 33.2), of 32 K 628 (616), 100 ragged ones of up to 8 K 142 (137), eight of 9.6 K 38.7 (37.2), 24 of 32 tokens 7.8 (7.4), the precise form at 64 x 1 K
-        // 42.4 (41.0); ten records for that form and eight for this one make no difference and 1 %.
+        // This warp issues everything, per tile t in the order PV(t), S(t+2). S(t+2) overwrites the buffer that holds P(t), so it waits until
+        // PV(t) has completed: two MMAs of one thread are executed in the order of issue, by what PTX says, where they have the same
+        // accumulator and shape, and these have neither in common. Without the wait the results were the same bits in every run; it
+        // costs 64 sequences of 1 K tokens 32.7 -> 33.2 us, of 32 K 610 -> 613, 100 ragged ones of up to 8 K 137.1 -> 138.1, a 20-layer step 441 -> 445.
+        // With a warp for S and one for PV, and eight records in flight instead of ten: 34.5, 622, 141.6 and 445 us; eight sequences of
+        // 9.6 K 36.3 (now 36.4), 24 of 32 tokens 8.4 (8.1), the precise form at 64 x 1 K 41.8 (41.4); ten records for that form and eight for
+        // this one make no difference and 1 %.
         const uint32_t v_s = ptx::smem_u32(smem + SM_V);
         const uint32_t idO = ptx::idesc_f16(128, PV_N, false, true);
         const uint32_t vlo0 = ptx::desc_lo(v_s, KBLOCK), vlo1 = ptx::desc_lo(v_s + VTILE_BYTES, KBLOCK), vhi = ptx::desc_hi(1024) | (2u << 29);
         auto issue_s = [&](uint32_t tt, int nu) -> bool {
             const uint32_t b = tt & 1;
             if (!uniform_i32(ptx::mbar_wait(BAR(B_K_FULL + b), (tt >> 1) & 1, abort_flag))) return false;
+            if (tt >= 2 && !uniform_i32(ptx::mbar_wait(BAR(B_PV_DONE + b), ((tt >> 1) - 1) & 1, abort_flag))) return false;
             ptx::tc_fence_after();
             const uint32_t idS = ptx::idesc_f16(128, 32 * nu, false, false);
             ptx::mma_ts_s8_warp<KBLOCK / 16>(tmem + TM_S + b * 128, tmem + TM_Q, b ? klo1 : klo0, khi, idS, BAR(B_S_FULL + b), BAR(B_K_FREE + b));
