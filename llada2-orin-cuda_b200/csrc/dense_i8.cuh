@@ -370,6 +370,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dense_wide_kernel(const DensePa
     const uint32_t sm0 = ptx::smem_u32(dw_smem), bar0 = sm0 + T::BAR;
     auto BAR = [&](int i) -> uint32_t { return bar0 + 8u * uint32_t(i); };
     if (sm0 & 1023u) {                         // the swizzled tiles need a 1024-byte aligned base: report, do nothing
+        ptx::grid_dependency_wait();           // and let no kernel behind this one start before the one ahead has completed
         if (tid == 0) report_error(p, ERR_SMEM_ALIGN);
         return;
     }
