@@ -1,8 +1,9 @@
-"""The attention kernel's build option LLATTN_SINGLE_ISSUER (one warp issues both MMA chains) gives the default build's
-numbers: whatever a role sets up in shared memory, it sets up in either form. The option's library is compiled here."""
+"""The library built with other values of its compile-time options gives the default build's numbers: LLATTN_NRAW=8, a ring of eight
+records in flight instead of ten in the attention kernel (its slots and phases then fall differently on the tiles). Compiled here."""
 import importlib
 import importlib.util
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -11,21 +12,30 @@ import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
-pytestmark = pytest.mark.gpu
+OPTIONS = {"LLATTN_NRAW": 8}
+
+
+def test_the_options_exist(pkg):
+    """A define that no source reads would test the default build against itself."""
+    bld = importlib.import_module(pkg.__name__ + ".build")
+    text = "".join(open(f).read() for f in bld.sources())
+    for name, value in OPTIONS.items():
+        default = re.search(rf"#ifndef {name}\n#define {name} (\d+)\n", text)
+        assert default and int(default.group(1)) != value and len(re.findall(rf"\b{name}\b", text)) > 2, name
 
 
 @pytest.fixture(scope="module")
-def single(pkg, tmp_path_factory):
+def other(pkg, tmp_path_factory):
     nvcc = os.environ.get("NVCC") or shutil.which("nvcc")
     if nvcc is None:
-        pytest.skip("needs nvcc: the option is a compile-time one")
+        pytest.skip("needs nvcc: the options are compile-time ones")
     bld = importlib.import_module(pkg.__name__ + ".build")
-    lib = str(tmp_path_factory.mktemp("single") / "libllattn_single.so")
-    subprocess.check_call([nvcc] + bld.NVCC_FLAGS + ["-DLLATTN_SINGLE_ISSUER=1", os.path.join(bld.CSRC, "llattn.cu"), "-o", lib])
+    lib = str(tmp_path_factory.mktemp("other") / "libllattn_other.so")
+    subprocess.check_call([nvcc] + bld.NVCC_FLAGS + [f"-D{k}={v}" for k, v in OPTIONS.items()] + [os.path.join(bld.CSRC, "llattn.cu"), "-o", lib])
     old = os.environ.get("LLATTN_LIB")
     os.environ["LLATTN_LIB"] = lib                             # read when the module is loaded
     try:
-        spec = importlib.util.spec_from_file_location("llattn_api_single", os.path.join(bld.HERE, "api.py"))
+        spec = importlib.util.spec_from_file_location("llattn_api_other", os.path.join(bld.HERE, "api.py"))
         api = sys.modules[spec.name] = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(api)
     finally:
@@ -36,9 +46,10 @@ def single(pkg, tmp_path_factory):
     return api
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("nblocks,nctas", [(0, 0), (3, 4), (5, 8), (33, 3), (130, 0)])
 @pytest.mark.parametrize("precise", [False, True])
-def test_single_issuer_matches_the_oracle(single, pkg, orc, nblocks, nctas, precise):
+def test_other_build_matches_the_oracle(other, pkg, orc, nblocks, nctas, precise):
     wl = pkg.workload
     Q, Kf, Vf = wl.query_blocks(1, seq=nblocks)
     cache = np.zeros((4, nblocks + 1, orc.REC_BYTES), np.uint8)
@@ -47,9 +58,9 @@ def test_single_issuer_matches_the_oracle(single, pkg, orc, nblocks, nctas, prec
         orc.kv_commit(Kc, Vc, cache, nblocks + 1, 0)
     dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
     want, lse = orc.attention(Q, Kf, Vf, cache, nblocks + 1, nblocks, dq_mode=1)
-    ctx = single.Context(0)
+    ctx = other.Context(0)
     cached = dev(cache)
-    plan = ctx.plan([single.Seq(cache=cached, nblocks=nblocks)], nctas)
+    plan = ctx.plan([other.Seq(cache=cached, nblocks=nblocks)], nctas)
     O, L = torch.zeros((32, 16, 128), device="cuda"), torch.zeros((32, 16), device="cuda")
     ctx.attention(plan, dev(Q), dev(Kf), dev(Vf), O32=O, LSE=L, precise=precise)
     assert ctx.device_status() == 0
