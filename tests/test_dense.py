@@ -283,9 +283,11 @@ def test_dense_tcgen05_form(api, orc, pkg, ntokens, rows, K, tok):
 
 
 # A CTA of the tcgen05 form walks several tiles: two and three of them, an odd number of groups (the rings and accumulators are then out of
-# step with the tile), more groups than factors held at a time, and a ragged last tile of tokens.
+# step with the tile), more groups than factors held at a time, and a ragged last tile of tokens; with 32 tokens a CTA, few groups are what
+# makes more tiles than SMs the choice.
 @pytest.mark.gpu
-@pytest.mark.parametrize("ntokens,rows,K,tok", [(1280, 4096, 1152, 128), (2050, 2048, 1152, 128), (300, 16384, 1152, 128), (1217, 2048, 4224, 64)])
+@pytest.mark.parametrize("ntokens,rows,K,tok", [(1280, 4096, 1152, 128), (2050, 2048, 1152, 128), (300, 16384, 1152, 128), (1217, 2048, 4224, 64),
+                                                   (657, 1792, 768, 32), (913, 1280, 640, 32), (81, 12544, 640, 32)])
 def test_dense_tcgen05_several_tiles_per_cta(api, orc, pkg, ntokens, rows, K, tok):
     if torch.cuda.get_device_properties(0).multi_processor_count == 148:
         assert api.dense_preview(rows, K, ntokens, 148) == (api.DENSE_TCGEN05, tok) and rows // 128 * -(-ntokens // tok) > 148
