@@ -98,7 +98,8 @@ int llattn_qkv_prepare_commit(const float* qkv, const int32_t* pos, const float*
 int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int32_t* sum, float* Y, int ntokens, int rows, int K,
                       int* err_word, void* stream);
 
-/* The kernel that a call of these sizes gets on a device of num_sms SMs, and the tokens of a CTA. Host only. */
+/* The kernel that a call of these sizes gets on a device of num_sms SMs, and the tokens of a CTA. Host only. (A build whose tcgen05 kernels
+ * came out with too few registers for their roles takes LLATTN_DENSE_TILES in their place.) */
 #define LLATTN_DENSE_STRIPS 0  /* a 16-row strip per CTA, a warp per 128-group */
 #define LLATTN_DENSE_TILES 1   /* 128 rows per CTA, mma.sync */
 #define LLATTN_DENSE_TCGEN05 2 /* 128 rows per CTA, tcgen05 */

@@ -311,8 +311,11 @@ constexpr int DW_FOLD_WARPS = 16, DW_UNPACK_WARPS = 4, DW_LOAD_WARPS = 2;
 constexpr int DW_WARP_UNPACK = DW_FOLD_WARPS, DW_WARP_LOAD = DW_WARP_UNPACK + DW_UNPACK_WARPS, DW_WARP_PRODUCER = DW_WARP_LOAD + DW_LOAD_WARPS,
               DW_WARP_MMA = DW_WARP_PRODUCER + 1, DW_THREADS = 32 * (DW_WARP_MMA + 1);
 // Registers a thread: at launch, and after the roles have parted. The second split has to come out of the first, or its waits for registers
-// would not end; that the compiler gave each kernel the first number is checked before the first launch.
-constexpr int DW_LAUNCH_REGS = 80, DW_FOLD_REGS = 96, DW_OTHER_REGS = 48;
+// would not end; that the compiler gave each kernel the first number is checked before the first launch, and without it the tiles take the call.
+#ifndef LLATTN_DW_LAUNCH_REGS
+#define LLATTN_DW_LAUNCH_REGS 80
+#endif
+constexpr int DW_LAUNCH_REGS = LLATTN_DW_LAUNCH_REGS, DW_FOLD_REGS = 96, DW_OTHER_REGS = 48;
 static_assert(DW_FOLD_WARPS * DW_FOLD_REGS + (DW_THREADS / 32 - DW_FOLD_WARPS) * DW_OTHER_REGS <= DW_THREADS / 32 * DW_LAUNCH_REGS && DW_THREADS % 128 == 0 &&
               DW_FOLD_WARPS % 4 == 0, "register split");
 constexpr int DW_RAW = 2, DW_A = 2, DW_B = 2, DW_ACC = 4, DW_SC = 16;      // ring slots; groups of factors held

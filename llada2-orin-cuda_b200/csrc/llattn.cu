@@ -290,13 +290,14 @@ int dense_wide_tokens(int rows, int K, int ntokens, int sms) {
     return wide;
 }
 
-// Which kernel takes a call and the tokens of a CTA, by the sizes and the SM count alone.
+// Which kernel takes a call and the tokens of a CTA, by the sizes and the SM count alone. `tcgen05`: that kernel can be launched.
 struct DenseForm {
     int kernel, tokens;
 };
-DenseForm dense_form(int rows, int K, int ntokens, int sms) {
+DenseForm dense_form(int rows, int K, int ntokens, int sms, bool tcgen05 = true) {
     if (ntokens <= DENSE_STRIP_MAX_TOKENS && dense_strips_win(rows, K, ntokens, sms)) return {LLATTN_DENSE_STRIPS, llattn::DS_TOK};
-    if (const int wide = dense_wide_tokens(rows, K, ntokens, sms)) return {LLATTN_DENSE_TCGEN05, wide};
+    if (tcgen05)
+        if (const int wide = dense_wide_tokens(rows, K, ntokens, sms)) return {LLATTN_DENSE_TCGEN05, wide};
     // The largest tile is the cheapest per token, as long as the tiles fill the chip: with smaller ones while they do not.
     // 2048 x 2048, in a graph: 65 .. 144 tokens 16.2 .. 16.6 us with 64 tokens a tile, 8.1 .. 8.7 with 16; 160 .. 288 tokens 16.7 and
     // 11.3 .. 11.8 (32); at 512 tokens 16.8 (64) and 17.3 (32), at 1024 26.4 and 30.7.
@@ -355,9 +356,8 @@ int llattn_dense_w4a8(const void* W, const int8_t* q, const float* s, const int3
         });
     int sms = 0;
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const DenseForm f = dense_form(rows, K, ntokens, sms);
+    const DenseForm f = dense_form(rows, K, ntokens, sms, dev >= 0 && dev < 64 && split_ok[dev]);
     const bool strips = f.kernel == LLATTN_DENSE_STRIPS;
-    if (f.kernel == LLATTN_DENSE_TCGEN05 && !(dev >= 0 && dev < 64 && split_ok[dev])) return fail(LLATTN_ECUDA, "dense_w4a8: a kernel was built with fewer registers than its roles divide");
     const dim3 tiles(rows / (strips ? 16 : llattn::DN_ROWS), (ntokens + f.tokens - 1) / f.tokens);
     // With 32 tokens a CTA and no more tiles than SMs, a CTA per tile in a kernel without the loop over them: 160 tokens 10.0 us, 10.4 with it.
     const bool one = f.tokens == 32 && (long long)tiles.x * tiles.y <= sms;

@@ -1,5 +1,6 @@
-"""The library built with other values of its compile-time options gives the default build's numbers: LLATTN_NRAW=8, a ring of eight
-records in flight instead of ten in the attention kernel (its slots and phases then fall differently on the tiles). Compiled here."""
+"""The library built with other values of its compile-time options gives the default build's numbers. Compiled here:
+LLATTN_NRAW=8: a ring of eight records in flight instead of ten in the attention kernel (its slots and phases then fall differently on the tiles);
+LLATTN_DW_LAUNCH_REGS=96: the projection's tcgen05 kernels, built with 80 registers a thread, have fewer than their roles are to divide."""
 import importlib
 import importlib.util
 import os
@@ -12,7 +13,7 @@ import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
-OPTIONS = {"LLATTN_NRAW": 8}
+OPTIONS = {"LLATTN_NRAW": 8, "LLATTN_DW_LAUNCH_REGS": 96}
 
 
 def test_the_options_exist(pkg):
@@ -69,3 +70,18 @@ def test_other_build_matches_the_oracle(other, pkg, orc, nblocks, nctas, precise
     assert np.abs(O.cpu().numpy() - want).max() <= (2e-3 if precise or nblocks <= 8 else 5e-3) * rms
     assert np.abs(L.cpu().numpy() - lse).max() <= 1e-3
     plan.close(); ctx.close()
+
+
+# The sizes of the tcgen05 form; without the registers for it the mma.sync tiles take the call, same bits.
+@pytest.mark.gpu
+@pytest.mark.parametrize("ntokens", [160, 577])
+def test_too_few_registers_for_the_split(other, pkg, orc, ntokens):
+    wl = pkg.workload
+    strips, _, _, _ = wl.dense_weights(2048, 2048, 81)
+    q, s, qsum = wl.int8_activations(ntokens, 2048, 82)
+    assert other.dense_preview(2048, 2048, ntokens, 148)[0] == other.DENSE_TCGEN05
+    want = np.random.default_rng(83).normal(size=(ntokens, 2048)).astype(np.float32)
+    Y = torch.from_numpy(want.copy()).cuda()
+    orc.dense_w4a8(strips, q, s, qsum, want)
+    other.dense_w4a8(*(torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (strips, q, s, qsum)), Y)
+    assert other.dense_status() == 0 and np.array_equal(Y.cpu().numpy().view(np.uint32), want.view(np.uint32))
