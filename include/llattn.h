@@ -140,7 +140,7 @@ int llattn_attn_partial(const llattn_args* args, int nb, int* err_word, void* st
 /* Stands in for attn::attn_combine<<<dim3(4, 16, nb), 256, 0, st>>>(Opart, Mpart, Lpart, nchunks, nblocks, bpc,
  * O, q8, s8, sum8) (engine/attn.cu:319; call sites engine/engine.cu:432 and :598). With q8 non-null the int8
  * activation form (fragment order, per-head scale, integer sum) is written and O is not, as in the reference.
- * A programmatic dependent launch: behind llattn_attn_partial it may take its place on the chip early, and it waits for all
+ * A programmatic dependent launch, as every launch here but the cooperative attention: behind llattn_attn_partial it may take its place on the chip early, and it waits for all
  * that is ahead of it before it reads or writes. In a captured graph the edge in front of it has that type. */
 int llattn_attn_combine(const float* Opart, const float* Mpart, const float* Lpart, int nchunks, int nblocks,
                         int blocks_per_chunk, void* O, int8_t* q8, float* s8, int32_t* sum8, int nb, void* stream);
@@ -228,8 +228,8 @@ int llattn_plan_update(llattn_plan* plan, const llattn_seq* seqs_host, int nseq,
 int llattn_plan_preview(const llattn_seq* seqs_host, int nseq, int nctas, llattn_plan_stats* stats, int32_t* items_out,
                         int max_items, int32_t* cta_first_out, int max_ctas);
 
-/* One attention pass over every sequence of the plan: ONE kernel launch (a cooperative one where a tile is cut or the stream is capturing), no allocation, no host
- * sync. A (query block, kv head) tile that one CTA handles alone is normalised and written by that CTA; a tile spread
+/* One attention pass over every sequence of the plan: ONE kernel launch (a cooperative one where a tile is cut or the
+ * stream is capturing, else a dependent one), no allocation, no host sync. A (query block, kv head) tile that one CTA handles alone is normalised and written by that CTA; a tile spread
  * over n CTAs is folded together by those n CTAs once each has finished all of its own runs: each waits (bounded) for
  * the tile's other partial results in the context's scratch and finishes every n-th row, adding the partial results in
  * a fixed order, so results do not depend on timing. Calls that share a context must not overlap on the GPU. */

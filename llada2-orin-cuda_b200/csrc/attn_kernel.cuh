@@ -607,8 +607,8 @@ __device__ __forceinline__ void copy_fresh(const half* src, uint8_t* tile_unit, 
 
 // Third block of both V tiles: column 128 of V is all ones (O column 128 accumulates sum(P)), 129..143 zero. Written by a warp of its own
 // while the first records are on their way: by the issuing warp in front of its first S it cost a short call 0.4 us (128 tokens 8.5 and
-// 8.1). Unrolled 8 times not for its own sake, it runs once: where the code behind it comes to lie moves the kernel's pace (rolled up, 4, 8, 16
-// and 32 times: the 20-layer step 440, 439, 440, 442 and 448 us, 192 sequences at 2 K tokens with the precise form 194, 190, 187, 186 and 197).
+// 8.1). Unrolled 8 times not for its own sake, it runs once: where the code behind it comes to lie moves the kernel's pace (rolled up, 4, 8 and
+// 16 times: the 20-layer step 440.6, 442.5, 443.3 and 444.8 us, 192 sequences at 2 K tokens 165, 160, 159 and 156, with the precise form 186.5, 186, 187.5 and 196.5).
 __device__ __forceinline__ void write_ones_column(uint8_t* smem, int lane) {
 #pragma unroll 8
     for (int idx = lane; idx < 2 * 128 * 8; idx += 32) {
@@ -631,8 +631,8 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM_BAR);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM_MISC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM_MISC + 4);
-    constexpr int SOFTMAX_WARPS = softmax_warps(ROWS16), WARP_SERVICE = SOFTMAX_WARPS + DEQUANT_WARPS, WARP_MMA_PV = WARP_SERVICE;
-    constexpr int WARP_MMA = WARP_MMA_PV + 1, WARP_PRODUCER = WARP_MMA + 1, WARPS = attn_threads(ROWS16) / 32;
+    constexpr int SOFTMAX_WARPS = softmax_warps(ROWS16), WARP_ONES = SOFTMAX_WARPS + DEQUANT_WARPS;
+    constexpr int WARP_MMA = WARP_ONES + 1, WARP_PRODUCER = WARP_MMA + 1, WARPS = attn_threads(ROWS16) / 32;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar0 = ptx::smem_u32(bars);
     auto BAR = [&](int i) -> uint32_t { return bar0 + 8u * uint32_t(i); };
@@ -1088,7 +1088,7 @@ __device__ __forceinline__ void attn_tile_body(const KParams& p, const int cta) 
             }
         }
         }
-    } else if (warp < WARP_SERVICE) {
+    } else if (warp < WARP_ONES) {
         // ================================================================== dequant: records -> fp16 operand tiles
         const int da = tid - 32 * SOFTMAX_WARPS;      // over all groups
         const int grp = da / GROUP_THREADS, dt = da % GROUP_THREADS;       // group g owns units g, g + groups, ... of every tile

@@ -92,10 +92,11 @@ struct DeviceGuard {
 
 // A launch that may start before the kernel ahead of it in the stream has run out; its kernel waits with griddepcontrol.wait before it reads
 // or writes anything. Behind a kernel that does not allow it earlier, it takes its place when the last CTA of that one has left, and the
-// launch's own latency is hidden: every kernel of this library but the cooperative attention goes this way. Calls one after the other
-// through the Python binding, before / now: commit of 64 blocks 7.1 / 6.6 us, operator pair at 2 K tokens 16.6 / 14.6, 32 tokens through the
-// projection 8.2 / 7.2, 2048 33.0 / 31.0, a first pass over four prompts of 13 blocks 29.3 / 27.4; a 20-layer step in a graph, 1 x 8 K tokens 466 /
-// 440, four sequences within 0.5 %.
+// launch's own latency is hidden: every kernel of this library but the cooperative attention goes this way. In a graph, the same build without
+// and with the attribute: commit of 64 blocks 4.05 / 3.9 us, 32 tokens through the projection 3.7 / 3.5, operator pair at 2 K tokens 14.1 / 13.7,
+// a 20-layer step of one sequence at 8 K tokens 441.4 / 439.3. Calls one after the other through the Python binding, whose host time of 5 to
+// 7 us covers the two short ones: pair 16.1 / 14.5, 2048 tokens through the projection 33.0 / 31.0, a first pass over four prompts of 13 blocks 29.3 / 27.1.
+// Under capture the edge in front of the kernel becomes a programmatic one.
 template <typename... KArgs>
 cudaError_t launch_dependent_smem(void (*kernel)(KArgs...), dim3 grid, int threads, int smem, cudaStream_t stream, KArgs... args) {
     cudaLaunchConfig_t cfg{};
@@ -272,13 +273,14 @@ int dense_wide_tokens(int rows, int K, int ntokens, int sms) {
     else if (ctas(32) <= sms) best = 2.3 + 0.54 * groups;
     else if (ctas(64) <= sms) best = 2.6 + 0.88 * groups;
     else {                                     // two CTAs an SM. A partly filled last wave counts half; behind six others, which have
-                                               // drifted apart by then, a fifth (K = 768, 16,384 rows, 1184 tokens: 87.8 as tiles, 94.5 here)
+                                               // drifted apart by then, a fifth (K = 768, 16,384 rows, 1184 tokens: 87.3 measured, 98 by a half, 96 by a fifth)
         const double waves = ctas(64) / (2 * sms), idle = std::ceil(waves) - waves;
         best = std::max(1.0, waves + idle * (waves > 6 ? 0.2 : 0.5)) * (2.9 + 1.42 * groups);
     }
     int wide = 0;
-    // Two groups: the tiles. Up to six in many waves stay with them as well, where test_dense_preview holds the line; 128 tokens a CTA would be
-    // the faster form by now (12,288 rows of K = 768, 1800 tokens: 98.4 us as tiles, 88.6).
+    // Two groups: the tiles. Up to six in many waves stay with them as well, a line drawn for a CTA per tile: since CTAs walk their tiles, 128
+    // tokens a CTA are the faster form there too (as tiles / so: 12,288 rows of K = 768, 1800 tokens 97.7 / 86.5 us, 16,384 rows, 1184 tokens
+    // 87.3 / 74.6, 8192 rows, 4096 tokens 144 / 111, 16,384 rows of K = 512, 2048 tokens 108.5 / 94.4, of K = 384 94 / 84).
     if (groups <= 2 || (groups <= 6 && ctas(64) > 6 * 2 * sms)) return 0;
     auto consider = [&](int tok, double start, double group, double more, double group_more) {
         const double cost = start + group * groups + (std::ceil(ctas(tok) / sms) - 1) * (more + group_more * groups);

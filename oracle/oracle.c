@@ -1,7 +1,7 @@
 /*
  * CPU oracle for the block-diffusion attention path over the "4c/4" int4 KV cache.
  *
- * TEST INFRASTRUCTURE ONLY. This file is the checker the CUDA path is compared with; nothing that ships may
+ * TEST INFRASTRUCTURE ONLY. The CUDA path is compared with this file; nothing that ships may
  * call it. It restates, in plain C, the arithmetic of the reference engine:
  *   - record layout                         engine/attn.cu:3-7,22-25
  *   - block-commit quantiser (kv_commit)    engine/attn.cu:369-418

@@ -248,7 +248,7 @@ def test_dense_tcgen05_cases_take_that_form(api, ntokens, rows, K, tok):
 def test_dense_preview(api):
     assert api.dense_preview(2048, 2048, 32, 148)[0] == api.DENSE_STRIPS
     assert api.dense_preview(2048, 128, 2560, 148) == (api.DENSE_TILES, 64)
-    # many waves of six groups: the tiles, 87.8 and 98.6 us where the tcgen05 form takes 94.5 and 104.7
+    # many waves of six groups: the tiles (87.3 and 97.7 us; with a CTA per tile the tcgen05 form took 94.5 and 104.7, walking them it takes 74.6 and 86.5)
     assert api.dense_preview(16384, 768, 1184, 148) == api.dense_preview(12288, 768, 1800, 148) == (api.DENSE_TILES, 64)
     assert {t for *_, t in TCGEN05_CASES} == {32, 64, 128}
     for bad in ((100, 128, 1, 148), (128, 128, 0, 148), (128, 128, 1, 0)):
